@@ -228,10 +228,8 @@ typedef struct spconvb_conv_params {
                            * from the w-th K chunk of every CTA on, so the consumer's wait must
                            * run out; the launch then ends with SPCONVB_ST_TIMEOUT in the status
                            * block, its output undefined, the context and TMEM usable */
-  /* Optional hint for the tensor-core kernel's L2 prefetch of input rows: the device-side
-   * row count of `in` and the rows its buffer holds.  NULL / 0: input rows are not
-   * prefetched (results are the same either way).  The prefetch is off unless the environment
-   * variable SPCONVB_CONV_PREFETCH gives a depth in tiles: it measured slower than no prefetch. */
+  /* Optional hint: the device-side row count of `in` and the rows its buffer holds (NULL / 0:
+   * unknown).  No kernel uses it at present; results are the same either way. */
   const uint32_t* n_in_ptr;
   uint32_t cap_in;
 } spconvb_conv_params;

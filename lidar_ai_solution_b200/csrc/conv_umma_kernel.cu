@@ -8,15 +8,11 @@
 // feature rows of o's neighbours (zeros where a neighbour is absent).  A
 // tcgen05.mma takes the same time whether its accumulator has 64 or 128 rows, and
 // its time grows with its columns, so the voxel rows are put on the wide side: the
-// weights are the M operand (64 or 128 accumulator rows = output channels, copied
-// w_rep times when Cout is smaller), a tile of up to 256 voxel rows is the N
-// operand, and the accumulator in TMEM is the transposed output tile
-// D[channel][row].  Copies of the weights let more epilogue warps share a tile.
-// When all chunks of the layer (times the copies) fit beside the row stages they
-// are loaded once and stay in shared memory; otherwise a chunk is streamed with
-// every stage.  The host side (conv_umma.cu) picks copies, residency and the depth
-// of the stage ring from the shared-memory budget.  The kernel is persistent (one
-// CTA per SM) and warp-specialised:
+// weights are the M operand (128 accumulator rows = output channels, copied 128 / Cout
+// times when Cout is smaller), a tile of up to 256 voxel rows is the N operand, and the
+// accumulator in TMEM is the transposed output tile D[channel][row].  Copies of the
+// weights let more epilogue warps share a tile.  The kernel is persistent (one CTA per
+// SM) and warp-specialised:
 //
 //   warps 0-7   epilogue: warp w reads its lane quadrant (its channels) and its
 //               share of the tile's rows from the accumulator with tcgen05.ld,
@@ -24,26 +20,33 @@
 //               with per-lane scale and bias, transposes 4x4 blocks inside lane
 //               quads with two shuffles, and stores 4 (int8) or 8 (fp16)
 //               contiguous bytes of one output row per lane
-//   warp  8     allocates TMEM; one lane issues tcgen05.mma (kind::i8 with int32
-//               accumulators or kind::f16 with fp32 accumulators)
+//   warp  8     allocates TMEM; walks the chunks converged, one elected lane issues
+//               tcgen05.mma (kind::i8 with int32 accumulators or kind::f16 with fp32)
 //   warps 9-24  producers, two groups of 8 warps that take the chunks in turn (the
 //               work of a warp per chunk is a chain of dependent steps - wait for
 //               the stage, neighbour indices, addresses, copies, arrival - that
 //               takes longer than the tensor pipe needs for the chunk; two groups
 //               give each warp two chunk periods for it).  Within a group each warp
 //               owns 32 rows of the tile.  A thread loads the 8 neighbour indices
-//               it needs for its next chunk straight into registers (two 16-byte
-//               loads, a round ahead) and gathers with 16-byte cp.async (8 lanes
+//               it needs for a chunk straight into registers (two 16-byte loads, two
+//               of its chunks ahead) and gathers with 16-byte cp.async (8 lanes
 //               per row, so a row is one contiguous request; zero-fill for missing
 //               neighbours) straight into the 128-byte-swizzled K-major layout the
-//               MMA reads.
-//               A producer never waits for its copies: every thread lets them
-//               arrive on the stage's mbarrier when they land, so all free stages
-//               of the ring are in flight.  One thread also streams the
-//               pre-swizzled weight chunk with one bulk async copy.  Optionally
-//               (UmmaArgs.prefetch > 0; off by default, it measured slower) a few
-//               lanes ask L2 (bulk prefetch) for the map lines, input rows and
-//               residual rows of the tile the CTA will reach some rounds later.
+//               MMA reads.  A producer never waits for its copies: every thread lets
+//               them arrive on the stage's mbarrier when they land, so all free
+//               stages of the ring are in flight.
+//   warp  25    streams the pre-swizzled weight chunks with bulk async copies into a
+//               ring of their own
+//
+// What bounds it.  The round trip of a stage - freed, gathered (a cp.async takes about a
+// microsecond under load), multiplied, freed - over the number of stages in flight, not a
+// pipe: in isolation the MMAs of a 256-row chunk take 513 cycles, its gather 460 (cp.async.cg;
+// 640 with .ca, which keeps a copy in L1 that nothing reads again) and its weights 310, and
+// they overlap freely, but with four stages of rows and weights together a chunk took 1000.
+// Hence two rings that are sized to the tile's height in the kernel (256 rows: 5 stages of
+// rows and 4 of weights; 160 rows: 6 and 6), and no work beside the MMAs in the issuing warp.
+// Measured with both, int8, us: 208 071 rows 64 -> 64 49.2 to 41.3, 128 -> 128 86.9 to 69.3
+// (730 cycles a chunk), fp16 181.6 to 158.1; 30 000 rows 128 -> 128 18.9 to 16.4.
 //
 // K is walked in chunks of 128 bytes (one swizzle atom per row): a chunk is 8
 // taps of a 16-byte row, ..., 1 tap of a 128-byte row, or half a 256-byte row.
@@ -55,41 +58,22 @@
 // drain their copies and free TMEM.
 #include "umma_common.cuh"
 
-// Per-role cycle accounting, compiled in only with -DSPCONVB_CONV_PROFILE (a measurement
-// build, never the shipped one): one lane of a producer warp, the MMA thread and one
-// epilogue lane add up the clock cycles they spend in each part of their loops, per CTA;
-// spconvb_debug_conv_profile() copies the table out.  In that build a negative
-// spconvb_conv_params.wait_test -f switches work off: f & 1 no gather copies, f & 2 no MMAs.
-#ifdef SPCONVB_CONV_PROFILE
-#define PROF(...) __VA_ARGS__
-#else
-#define PROF(...)
-#endif
-// The work switches alone (-DSPCONVB_CONV_SWITCHES, implied by the profile build): the same
-// experiments timed from outside, without the clock reads in the loops.
-#if defined(SPCONVB_CONV_PROFILE) || defined(SPCONVB_CONV_SWITCHES)
-#define DBG(...) __VA_ARGS__
-#else
-#define DBG(...)
-#endif
-
 namespace spconvb {
 
 using namespace umma_detail;
 
-PROF(__device__ unsigned long long g_conv_profile[148][16];)
-
 namespace {
 
 constexpr int kTileRows = 256;  // most voxel rows per tile: the largest N of the MMA
-constexpr int kRowsBytes = kTileRows * kChunk;  // gathered rows of one stage
 constexpr int kEpiWarps = 8;
 constexpr int kMmaWarp = 8;
 constexpr int kProdWarp0 = 9;
 constexpr int kProdThreads = 512;   // two groups of 8 producer warps
-constexpr int kCtaThreads = 32 * kProdWarp0 + kProdThreads;
+constexpr int kWeightWarp = kProdWarp0 + kProdThreads / 32;
+constexpr int kCtaThreads = 32 * (kWeightWarp + 1);
 constexpr uint32_t kTmemCols = 2 * kTileRows;
-constexpr size_t kMaxSmem = 232448;  // 227 KB: the most dynamic shared memory of a CTA
+constexpr size_t kSmemBytes = 232448;  // 227 KB: the most dynamic shared memory of a CTA
+constexpr uint32_t kRingBytes = kSmemBytes - 1024 - 256;  // less alignment slack and barriers
 
 // 32-bit instruction descriptor: [4,6) D format (1 = f32, 2 = s32), [7,10) A
 // format, [10,13) B format (f16 kind: 0 = f16; i8 kind: 1 = signed), bits 15/16
@@ -153,32 +137,24 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
   const int kbytes = a.kvol * RB;
   const int nchunk = (kbytes + kChunk - 1) / kChunk;
   const int last_ksteps = ((kbytes - (nchunk - 1) * kChunk) + 31) / 32;
-  const uint32_t w_rep = (uint32_t)a.w_rep;
-  const uint32_t m_rows = w_rep * COUT;            // accumulator rows of the MMA: 64 or 128
-  const bool w_resident = a.w_resident != 0;
-  const uint32_t w_chunk_smem = m_rows * kChunk;   // bytes of one chunk with its copies
-  const uint32_t nst = (uint32_t)a.nstages;
+  constexpr uint32_t kRep = 128 / COUT;            // copies of the weights along the accumulator rows
+  constexpr uint32_t kWeightBytes = 128 * kChunk;  // one chunk of weights with its copies
 
-  // Shared memory: the weights (all chunks, or one per stage), the gathered-row stages,
-  // the barriers.
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw_addr = smem_u32(smem_raw);
   uint8_t* smem = smem_raw + ((1024u - (raw_addr & 1023u)) & 1023u);
-  uint8_t* sW = smem;
-  uint8_t* sR = sW + (w_resident ? (uint32_t)nchunk : nst) * w_chunk_smem;
-  uint64_t* bars = (uint64_t*)(sR + nst * kRowsBytes);
-  uint32_t* tmem_holder = (uint32_t*)(bars + 2 * kMaxStages + 5);
+  uint64_t* bars = (uint64_t*)(smem + kRingBytes);
+  uint32_t* tmem_holder = (uint32_t*)(bars + 2 * kMaxStages + 4);
   volatile uint32_t* abort_flag = tmem_holder + 1;
 
   const uint32_t bar_full = smem_u32(bars);
   const uint32_t bar_empty = bar_full + 8 * kMaxStages;
   const uint32_t bar_tfull = bar_empty + 8 * kMaxStages;
   const uint32_t bar_tempty = bar_tfull + 16;
-  const uint32_t bar_w = bar_tempty + 16;  // resident weights have landed
 
   const int warp = threadIdx.x >> 5;
   const uint32_t lane = threadIdx.x & 31;
-  PROF(const long long k_c0 = clock64(); const unsigned long long k_t0 = global_ns();)
+  const uint32_t n_out = min(__ldg(a.n_out_ptr), a.cap);
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kMaxStages; ++s) {
@@ -189,7 +165,6 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
       mbar_init(bar_tfull + 8 * b, 1);
       mbar_init(bar_tempty + 8 * b, kEpiWarps);
     }
-    mbar_init(bar_w, 1);
     *abort_flag = 0u;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     fence_proxy_async();
@@ -206,7 +181,6 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
   tc_fence_after();
   const uint32_t tmem_base = *tmem_holder;
 
-  const uint32_t n_out = min(*a.n_out_ptr, a.cap);
   // Tile height: the rows are dealt out in rounds over the CTAs, so a fixed 256-row tile
   // can leave most CTAs idle in the last round (227 tiles on 148 CTAs run as long as 296).
   // The height is instead the smallest multiple of 32 with which every CTA gets the same
@@ -216,8 +190,45 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
   const uint32_t tile_rows =
       min((uint32_t)kTileRows, max(32u, ((per_cta + rounds - 1) / rounds + 31u) & ~31u));
   const uint32_t ntiles = (n_out + tile_rows - 1) / tile_rows;
+  // Two rings share the buffer: row stages as high as this launch's tile, and weight stages.
+  // As many of both as fit (low tiles get deeper rings); what is left over goes to the rows.
+  const uint32_t row_stage = tile_rows * kChunk;
+  const uint32_t nwst = min((uint32_t)kMaxStages, kRingBytes / (kWeightBytes + row_stage));
+  const uint32_t nst = min((uint32_t)kMaxStages, (kRingBytes - nwst * kWeightBytes) / row_stage);
+  const uint32_t sW = smem_u32(smem), sR = sW + nwst * kWeightBytes;
 
-  if (warp >= kProdWarp0) {
+  if (warp == kWeightWarp) {
+    // -------------------------------------------------------------- weights
+    // One lane streams the chunks' pre-swizzled weight images, its ring may be shallower than
+    // the rows': a weight stage is free when the chunk that used it last has been consumed.
+    if (lane == 0) {
+      uint32_t s = 0, ws = 0;    // row stage (whose barrier the copy signs), weight stage
+      uint32_t os = 0, oph = 0;  // row stage and phase of the chunk `nwst` before
+      uint32_t it = 0;
+      bool alive = true;
+      for (uint32_t tile = blockIdx.x; tile < ntiles && alive; tile += gridDim.x)
+        for (int j = 0; j < nchunk; ++j, ++it) {
+          if (it >= nwst) {
+            if (!mbar_wait(bar_empty + 8 * os, oph, abort_flag, a.status, 6u)) {
+              alive = false;
+              break;
+            }
+            if (++os == nst) {
+              os = 0;
+              oph ^= 1u;
+            }
+          }
+          mbar_expect_tx(bar_full + 8 * s, kWeightBytes);
+#pragma unroll
+          for (uint32_t c = 0; c < kRep; ++c)
+            bulk_g2s(sW + ws * kWeightBytes + c * (COUT * kChunk),
+                     a.wpk + (size_t)j * (COUT * kChunk), COUT * kChunk, bar_full + 8 * s);
+          if (++s == nst) s = 0;
+          if (++ws == nwst) ws = 0;
+        }
+    }
+    __syncwarp();
+  } else if (warp >= kProdWarp0) {
     // ------------------------------------------------------------ producers
     // Two groups of 8 warps take the chunks in turn (group g the chunks g, g + 2, ...), so a
     // warp has two chunk periods for the round trip of one chunk: wait for the stage, look
@@ -229,7 +240,6 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
     // branch-free and their address arithmetic and copies overlap.
     const uint32_t pw_all = (uint32_t)warp - kProdWarp0;
     const uint32_t grp = pw_all >> 3, pw = pw_all & 7u;
-    const bool w_thread = pw == 0u && lane == 0u;  // also streams the weights of its chunks
     const uint32_t seg = lane & 7u;        // 16-byte segment of the chunk this thread copies
     const uint32_t slot = lane >> 3;       // its 8 rows of the warp's 32
     // row R of the tile lives at (R / 8) * 1024 + (R % 8) * 128, its segments XOR-ed
@@ -261,46 +271,6 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
         for (uint32_t i = 0; i < 8; ++i) v[i] = (live && row + i < n_out) ? __ldg(src + i) : -1;
       }
     };
-    // L2 prefetch of what tile `pt` will read: its map lines (lanes 0-3 of every warp take
-    // the taps w, w+8, ...), its share of the input rows and its residual rows.  Bulk
-    // prefetches: one instruction per contiguous piece, nothing returns to the SM.
-    const uint32_t n_in = a.n_in_ptr ? min(*a.n_in_ptr, a.cap_in) : 0u;
-    const bool map_pf = (a.cap & 3u) == 0u && ((uintptr_t)a.map & 15u) == 0u;
-    auto prefetch_tile = [&](uint32_t pt) {
-      if (pt >= ntiles || lane > 4u) return;
-      const uint32_t prow0 = pt * tile_rows;
-      const uint32_t prows = min(tile_rows, n_out - prow0);
-      if (lane < 4u) {
-        const uint32_t k = pw + 8u * lane;
-        if (map_pf && k < (uint32_t)a.kvol)
-          bulk_prefetch_l2(a.map + (size_t)k * a.cap + prow0, ((prows + 3u) & ~3u) * 4u);
-      } else if (pw == 0u) {
-        if (n_in) {
-          const uint32_t in0 = (uint32_t)((unsigned long long)prow0 * n_in / n_out);
-          uint32_t cnt = (uint32_t)((unsigned long long)prows * n_in / n_out) + 1u;
-          if (in0 < n_in) {
-            cnt = min(cnt, n_in - in0);
-            bulk_prefetch_l2(a.in + (size_t)in0 * RB, cnt * (uint32_t)RB);
-          }
-        }
-      } else if (pw == 1u) {
-        if (a.ep.has_res) {
-          const uint32_t rb = (uint32_t)COUT * (a.ep.res_kind == SPCONVB_I8 ? 1u : 2u);
-          bulk_prefetch_l2(a.res + (size_t)prow0 * rb, prows * rb);
-        }
-      }
-    };
-    if (grp == 0u)
-      for (int p = 0; p < a.prefetch; ++p) prefetch_tile(blockIdx.x + (uint32_t)p * gridDim.x);
-
-    if (grp == 0u && w_thread && w_resident && blockIdx.x < ntiles) {
-      mbar_expect_tx(bar_w, (uint32_t)nchunk * w_chunk_smem);
-      for (int j = 0; j < nchunk; ++j)
-        for (uint32_t c = 0; c < w_rep; ++c)
-          bulk_g2s(smem_u32(sW + j * w_chunk_smem + c * (COUT * kChunk)),
-                   a.wpk + (size_t)j * (COUT * kChunk), COUT * kChunk, bar_w);
-    }
-
     // This group's chunks: numbers it = grp, grp + 2, ... of the CTA's chunk sequence (tile
     // after tile, nchunk chunks each); chunk `it` uses stage it % nst.
     auto advance2 = [&](uint32_t& tile, int& j) {  // two chunks on
@@ -311,154 +281,124 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
       }
     };
     uint32_t tile = blockIdx.x;
-    int j = 0;
-    if (grp == 1u) {
-      j = 1;
-      while (j >= nchunk) {
-        j -= nchunk;
-        tile += gridDim.x;
-      }
+    int j = grp == 1u ? 1 : 0;
+    while (j >= nchunk) {
+      j -= nchunk;
+      tile += gridDim.x;
     }
+    uint32_t ntile = tile;  // the chunk whose indices are loaded next
+    int nj = j;
     uint32_t it = grp, s = grp % nst, ph = (grp / nst) & 1u;
-    int32_t cur[8], nxt[8];
-    load_idx(tile, j, cur);
-    PROF(long long p_idx = 0, p_wait = 0, p_issue = 0, p_t0 = clock64(), t_a, t_b; uint32_t p_n = 0;)
-    DBG(const bool no_copies = a.wait_test < 0 && ((-a.wait_test) & 1);)
-    while (tile < ntiles) {
-      PROF(t_a = clock64();)
-      uint32_t ntile = tile;
-      int nj = j;
-      advance2(ntile, nj);
-      load_idx(ntile, nj, nxt);  // used a round from now
-      if (j == 0 && a.prefetch > 0) prefetch_tile(tile + (uint32_t)a.prefetch * gridDim.x);
-      PROF(t_b = clock64(); p_idx += t_b - t_a;)
+    // One chunk: its rows go from the indices in `idx` into the stage, and `idx` is then
+    // refilled for the chunk after next.  Two register sets take turns and are never copied,
+    // so the load has a whole chunk of the group's time to arrive.
+    auto step = [&](int32_t (&idx)[8]) -> bool {
+      if (tile >= ntiles) return false;
       // every lane polls: one shared-memory word, no divergence, no broadcast afterwards
-      if (!mbar_wait(bar_empty + 8 * s, ph ^ 1u, abort_flag, a.status, 1u)) break;
-      PROF(t_a = clock64(); p_wait += t_a - t_b;)
-      if (w_thread) {
-        if (w_resident) {
-          mbar_arrive(bar_full + 8 * s);
-        } else {
-          mbar_expect_tx(bar_full + 8 * s, w_chunk_smem);
-          for (uint32_t c = 0; c < w_rep; ++c)
-            bulk_g2s(smem_u32(sW + s * w_chunk_smem + c * (COUT * kChunk)),
-                     a.wpk + (size_t)j * (COUT * kChunk), COUT * kChunk, bar_full + 8 * s);
-        }
-      }
+      if (!mbar_wait(bar_empty + 8 * s, ph ^ 1u, abort_flag, a.status, 1u)) return false;
       // segments of the last chunk that lie in K steps past the kernel's last tap are never
       // read by an MMA: nothing to copy, nothing to zero
       const bool dead_seg = j == nchunk - 1 && (int)(seg >> 1) >= last_ksteps;
-      if (has_rows && !dead_seg DBG(&& !no_copies)) {
-        const uint32_t byte = seg_byte + (RB > kChunk ? (uint32_t)(j % CPT) * kChunk : 0u);
-        const uint32_t stage_addr = smem_u32(sR + s * kRowsBytes) + dst_base;
+      if (has_rows && !dead_seg) {
+        const uint8_t* src = a.in + seg_byte + (RB > kChunk ? (uint32_t)(j % CPT) * kChunk : 0u);
+        const uint32_t stage_addr = sR + s * row_stage + dst_base;
 #pragma unroll
         for (uint32_t i = 0; i < 8; ++i) {
-          const int32_t sr = cur[i];
+          const int32_t sr = idx[i];
           cp_async16(stage_addr + i * 128u + ((seg ^ i) << 4),
-                     a.in + (size_t)(sr < 0 ? 0 : sr) * RB + byte, sr < 0 ? 0u : 16u);
+                     src + (size_t)(sr < 0 ? 0 : sr) * RB, sr < 0 ? 0u : 16u);
         }
       }
       if (!(a.wait_test > 0 && it + 1u >= (uint32_t)a.wait_test))
         cp_async_arrive_noinc(bar_full + 8 * s);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) cur[i] = nxt[i];
-      tile = ntile;
-      j = nj;
+      load_idx(ntile, nj, idx);
+      advance2(ntile, nj);
+      advance2(tile, j);
       it += 2;
       s += 2;
       if (s >= nst) {
         s -= nst;
         ph ^= 1u;
       }
-      PROF(p_issue += clock64() - t_a; ++p_n;)
+      return true;
+    };
+    int32_t idx_a[8], idx_b[8];
+    load_idx(ntile, nj, idx_a);
+    advance2(ntile, nj);
+    load_idx(ntile, nj, idx_b);
+    advance2(ntile, nj);
+    while (step(idx_a) && step(idx_b)) {
     }
-    PROF(if (pw_all == 7 && lane == 0 && blockIdx.x < 148) {
-      unsigned long long* o = g_conv_profile[blockIdx.x];
-      o[0] = clock64() - p_t0; o[1] = p_idx; o[2] = p_wait; o[3] = p_issue; o[4] = 2 * p_n;
-    })
     cp_async_wait_all();  // nothing of this thread may still be writing when the CTA exits
   } else if (warp == kMmaWarp) {
     // ------------------------------------------------------------ MMA issue
-    if (lane == 0) {
-      // The tensor pipe takes one MMA at a time, and issuing the next one blocks until
-      // it is free.  Everything that is not an MMA therefore sits between the
-      // second-to-last and the last MMA of a chunk, or is short: the next stage's
-      // barrier is probed while the pipe is busy, so that the first MMA of the next
-      // chunk can follow the last one of this chunk without a bubble.
-      const uint32_t idesc =
-          make_idesc<INT8>() | ((tile_rows >> 3) << 17) | ((m_rows >> 4) << 24);
-      const uint64_t wdesc0 = make_smem_desc(smem_u32(sW));  // M operand: weights
-      const uint64_t rdesc0 = make_smem_desc(smem_u32(sR));  // N operand: gathered rows
-      uint32_t ph = 0, tl = 0;
-      bool alive = true;
-      if (w_resident && blockIdx.x < ntiles)
-        alive = mbar_wait_spin(bar_w, 0u, abort_flag, a.status, 6u);
-      // The loop is entered with the current chunk's stage known to be full.
-      if (blockIdx.x < ntiles && alive)
-        alive = mbar_wait_spin(bar_full, 0u, abort_flag, a.status, 3u);
-      // The thread that issues the MMAs runs one lane of one warp: every instruction
-      // between two MMAs that the tensor pipe cannot hide (it queues about one MMA ahead)
-      // is a bubble.  So the loop carries its descriptors and barrier addresses along
-      // instead of recomputing them, asks about the next stage once, early (right after
-      // the first MMA, so the answer is there when the last one has been issued), and
-      // issues the K steps of a full chunk without a loop.
-      // 32-bit arithmetic only: the descriptors differ in their low word (the address)
-      const uint32_t w_step = w_chunk_smem >> 4, r_step = (uint32_t)(kRowsBytes >> 4);
-      const uint32_t desc_hi = (uint32_t)(wdesc0 >> 32);
-      const uint32_t w_lo0 = (uint32_t)wdesc0, r_lo0 = (uint32_t)rdesc0;
-      uint32_t s = 0;  // stage of the current chunk
-      PROF(long long m_full = 0, m_issue = 0, m_tempty = 0, m_t0 = clock64(), t_a, t_b;)
-      DBG(const bool no_mma = a.wait_test < 0 && ((-a.wait_test) & 2);)
-      for (uint32_t tile = blockIdx.x; tile < ntiles && alive; tile += gridDim.x, ++tl) {
-        const uint32_t buf = tl & 1u;
-        PROF(t_a = clock64();)
-        if (!mbar_wait_spin(bar_tempty + 8 * buf, ((tl >> 1) & 1u) ^ 1u, abort_flag, a.status, 2u))
-          break;
-        PROF(m_tempty += clock64() - t_a;)
-        tc_fence_after();  // the epilogue's reads of this accumulator come before these MMAs
-        const uint32_t d_tmem = tmem_base + buf * kTileRows;
-        const bool last_tile = tile + gridDim.x >= ntiles;
-        for (int j = 0; j < nchunk; ++j) {
-          // No fence here: the rows arrive by cp.async completions on the stage's mbarrier,
-          // which is what the MMA's shared-memory reads are ordered behind.
-          const uint32_t rd = r_lo0 + s * r_step;
-          const uint32_t wd = w_lo0 + (w_resident ? (uint32_t)j : s) * w_step;
-          // the next stage (of this tile's next chunk or of the next tile's first)
-          const uint32_t s1 = s + 1 == nst ? 0u : s + 1;
-          const uint32_t ph1 = s1 == 0u ? ph ^ 1u : ph;
-          const uint32_t full_n = bar_full + 8 * s1;
-          const bool more = j + 1 < nchunk || !last_tile;
-          bool ready;
-          PROF(t_a = clock64();)
-          DBG(if (no_mma) ready = !more || mbar_test_wait(full_n, ph1); else)
-          if (j + 1 < nchunk) {
-            umma_lohi<INT8>(d_tmem, wd, rd, desc_hi, idesc, (uint32_t)(j != 0));
-            ready = mbar_test_wait(full_n, ph1);
+    // The whole warp walks the chunks and one elected lane issues: the loop's values stay
+    // warp-uniform, so an MMA costs its own time (measured in isolation, M = 128, N = 256: 513
+    // cycles per chunk against 583 when a single lane runs the loop, whose descriptors are moved
+    // to uniform registers one MMA after the other).
+    //
+    // The tensor pipe takes one MMA at a time, and issuing the next one blocks until it is
+    // free.  Everything that is not an MMA is short: the next stage's barrier is probed once,
+    // early, while the pipe is busy, so that the first MMA of the next chunk can follow the
+    // last one of this chunk without a bubble.
+    const bool leader = elect_one();
+    const uint32_t idesc = make_idesc<INT8>() | ((tile_rows >> 3) << 17) | ((128u >> 4) << 24);
+    const uint64_t wdesc0 = make_smem_desc(sW);  // M operand: weights
+    const uint64_t rdesc0 = make_smem_desc(sR);  // N operand: gathered rows
+    // 32-bit arithmetic only: the descriptors differ in their low word (the address)
+    const uint32_t w_step = kWeightBytes >> 4, r_step = row_stage >> 4;
+    const uint32_t desc_hi = (uint32_t)(wdesc0 >> 32);
+    const uint32_t w_lo0 = (uint32_t)wdesc0, r_lo0 = (uint32_t)rdesc0;
+    uint32_t ph = 0, tl = 0;
+    uint32_t s = 0, ws = 0;  // row and weight stage of the current chunk
+    // The loop is entered with the current chunk's stage known to be full.
+    bool alive = blockIdx.x < ntiles && mbar_wait_spin(bar_full, 0u, abort_flag, a.status, 3u);
+    for (uint32_t tile = blockIdx.x; tile < ntiles && alive; tile += gridDim.x, ++tl) {
+      const uint32_t buf = tl & 1u;
+      if (!mbar_wait_spin(bar_tempty + 8 * buf, ((tl >> 1) & 1u) ^ 1u, abort_flag, a.status, 2u))
+        break;
+      tc_fence_after();  // the epilogue's reads of this accumulator come before these MMAs
+      const uint32_t d_tmem = tmem_base + buf * kTileRows;
+      const bool last_tile = tile + gridDim.x >= ntiles;
+      for (int j = 0; j < nchunk; ++j) {
+        // No fence here: the rows arrive by cp.async completions on the stage's mbarrier,
+        // which is what the MMA's shared-memory reads are ordered behind.
+        const uint32_t rd = r_lo0 + s * r_step;
+        const uint32_t wd = w_lo0 + ws * w_step;
+        // the next stage (of this tile's next chunk or of the next tile's first)
+        const uint32_t s1 = s + 1 == nst ? 0u : s + 1;
+        const uint32_t ph1 = s1 == 0u ? ph ^ 1u : ph;
+        const uint32_t full_n = bar_full + 8 * s1;
+        const bool more = j + 1 < nchunk || !last_tile;
+        bool ready = true;
+        if (j + 1 < nchunk) {
+          if (leader) umma_lohi<INT8>(d_tmem, wd, rd, desc_hi, idesc, (uint32_t)(j != 0));
+          ready = mbar_test_wait(full_n, ph1);
+          if (leader) {
             umma_lohi<INT8>(d_tmem, wd + 2u, rd + 2u, desc_hi, idesc, 1u);
             umma_lohi<INT8>(d_tmem, wd + 4u, rd + 4u, desc_hi, idesc, 1u);
             umma_lohi<INT8>(d_tmem, wd + 6u, rd + 6u, desc_hi, idesc, 1u);
-          } else {
-            ready = !more || mbar_test_wait(full_n, ph1);
+            tc_commit(bar_empty + 8 * s);
+          }
+        } else {
+          if (more) ready = mbar_test_wait(full_n, ph1);
+          if (leader) {
             for (int ks = 0; ks < last_ksteps; ++ks)
               umma_lohi<INT8>(d_tmem, wd + 2u * ks, rd + 2u * ks, desc_hi, idesc,
                               (uint32_t)((j | ks) != 0));
+            tc_commit(bar_empty + 8 * s);
+            tc_commit(bar_tfull + 8 * buf);
           }
-          tc_commit(bar_empty + 8 * s);
-          PROF(t_b = clock64(); m_issue += t_b - t_a;)
-          if (!ready && more && !mbar_wait_spin(full_n, ph1, abort_flag, a.status, 3u)) {
-            alive = false;
-            break;
-          }
-          PROF(m_full += clock64() - t_b;)
-          s = s1;
-          ph = ph1;
         }
-        if (alive) tc_commit(bar_tfull + 8 * buf);
+        __syncwarp();
+        if (!ready && !mbar_wait_spin(full_n, ph1, abort_flag, a.status, 3u)) {
+          alive = false;
+          break;
+        }
+        s = s1;
+        ph = ph1;
+        if (++ws == nwst) ws = 0;
       }
-      PROF(if (blockIdx.x < 148) {
-        unsigned long long* o = g_conv_profile[blockIdx.x];
-        o[5] = clock64() - m_t0; o[6] = m_full; o[7] = m_issue; o[8] = m_tempty;
-      })
     }
     __syncwarp();
   } else {
@@ -468,27 +408,20 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
     // as one saturating round-to-nearest-even convert, and the layer-wide switches
     // hoisted out of the element loops.
     const Epilogue ep = a.ep;
-    // Accumulator row m holds channel m % COUT of weight copy m / COUT.  With 128 rows
-    // TMEM lane = m; with 64 rows the accumulator sits in lanes 0-15 of every 32-lane
-    // quadrant (m = 16 * quadrant + lane) and lanes 16-31 carry nothing.  Copy c owns the
-    // tile's rows [c, c + 1) * 256 / w_rep, and the two warps of a lane quadrant split
-    // those rows again, so a warp works on 128 / w_rep rows of the tile.
+    // Accumulator row m (TMEM lane m) holds channel m % COUT of weight copy m / COUT.  Copy c
+    // owns cols_rep rows of the tile from c * cols_rep on, and the two warps of a lane
+    // quadrant split those rows again: every warp has the same share of this launch's tile.
     const uint32_t q = (uint32_t)warp & 3u;        // TMEM lane quadrant of this warp
     const uint32_t half = (uint32_t)warp >> 2;
-    const bool wide = m_rows == 128u;
-    const bool lane_valid = wide || lane < 16u;
-    const uint32_t acc_row = wide ? 32u * q + lane : 16u * q + (lane & 15u);
-    const uint32_t acc_row0 = wide ? 32u * q : 16u * q;   // of lane 0 of the warp
+    const uint32_t acc_row = 32u * q + lane, acc_row0 = 32u * q;
     const uint32_t ch = acc_row % COUT;            // this lane's channel
     const uint32_t chq = ch & ~3u;                 // first of the 4 channels this lane stores
     const uint32_t j4 = lane & 3u;                 // row within a group of 4 this lane stores
-    const uint32_t cols_rep = (uint32_t)kTileRows / w_rep, cols_warp = cols_rep / 2u;
-    const bool lane_active = lane_valid && acc_row / COUT < w_rep;
-    const bool warp_active = acc_row0 / COUT < w_rep;
+    const uint32_t cols_rep = (tile_rows + 32u * kRep - 1u) / (32u * kRep) * 32u;
+    const uint32_t cols_warp = cols_rep / 2u;
     // first row (of the tile) of this lane, and of lane 0 of the warp: they differ only for
-    // COUT = 16 with 128 accumulator rows, where the two halves of a warp belong to
-    // different copies
-    const bool split_warp = COUT == 16 && wide && w_rep > 1u;
+    // COUT = 16, where the two halves of a warp belong to different copies
+    constexpr bool split_warp = COUT == 16;
     const uint32_t col_lane = (acc_row / COUT) * cols_rep + half * cols_warp;
     const uint32_t col_warp = (acc_row0 / COUT) * cols_rep + half * cols_warp;
     const float sc = (INT8 && a.scale) ? __ldg(a.scale + ch) : 1.f;
@@ -513,31 +446,24 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
       }
     };
     uint32_t tl = 0;
-    PROF(long long e_wait = 0, e_body = 0, e_t0 = clock64(), t_a, t_b;)
     for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++tl) {
       const uint32_t buf = tl & 1u;
       const uint32_t trow0 = tile * tile_rows + col_lane;
-      PROF(t_a = clock64();)
       // the first residual rows are fetched before the accumulator is waited for;
       // after that the loads run one group of 16 rows ahead of the arithmetic.  A group
       // lies inside the tile or not as a whole (the tile height is a multiple of 32);
       // rows past it belong to the next tile.
       uint2 rq[4];
-      if (ep.has_res) load_res(trow0, lane_active && col_lane < tile_rows, rq);
+      if (ep.has_res) load_res(trow0, col_lane < tile_rows, rq);
       uint32_t ok = 1u;
       if (lane == 0) {
-        PROF(if (a.wait_test < 0 && ((-a.wait_test) & 16)) {
-          for (int i = 0; i < 4000 && !mbar_test_wait(bar_tfull + 8 * buf, (tl >> 1) & 1u); ++i)
-            __nanosleep(500);
-        })
         ok = mbar_wait(bar_tfull + 8 * buf, (tl >> 1) & 1u, abort_flag, a.status, 4u) ? 1u : 0u;
       }
       ok = __shfl_sync(0xffffffffu, ok, 0);
       if (!ok) break;
-      PROF(t_b = clock64(); e_wait += t_b - t_a;)
       tc_fence_after();
       // groups of this warp that lie inside the tile (by its lower-numbered rows)
-      const uint32_t ng = (!warp_active || col_warp >= tile_rows)
+      const uint32_t ng = col_warp >= tile_rows
                               ? 0u
                               : min(cols_warp / 16u, (tile_rows - col_warp + 15u) / 16u);
       const uint32_t taddr = tmem_base + ((32u * q) << 16) + buf * kTileRows + col_warp;
@@ -549,7 +475,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
 #pragma unroll 1
       for (uint32_t g = 0; g < ng; ++g) {
         const uint32_t row0 = trow0 + 16u * g;
-        const bool in_tile = lane_active && col_lane + 16u * g < tile_rows;
+        const bool in_tile = col_lane + 16u * g < tile_rows;
         uint32_t v[16];
         tmem_ld16(taddr + 16u * g, v);
         if (split_warp) {
@@ -574,7 +500,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
 #pragma unroll
           for (int t = 0; t < 4; ++t) rcur[t] = rq[t];
           if (g + 1u < ng)
-            load_res(row0 + 16, lane_active && col_lane + 16u * (g + 1u) < tile_rows, rq);
+            load_res(row0 + 16, col_lane + 16u * (g + 1u) < tile_rows, rq);
         }
         float y[16];
 #pragma unroll
@@ -647,21 +573,12 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
           }
         }
       }
-      PROF(e_body += clock64() - t_b;)
     }
-    PROF(if (threadIdx.x == 0 && blockIdx.x < 148) {
-      unsigned long long* o = g_conv_profile[blockIdx.x];
-      o[9] = clock64() - e_t0; o[10] = e_wait; o[11] = e_body; o[12] = tl;
-    })
   }
 
   // ---------------------------------------------------------------- teardown
   tc_fence_before();
   __syncthreads();
-  PROF(if (threadIdx.x == 0 && blockIdx.x < 148) {
-    g_conv_profile[blockIdx.x][13] = clock64() - k_c0;   // SM cycles of the CTA ...
-    g_conv_profile[blockIdx.x][14] = global_ns() - k_t0;  // ... and the nanoseconds they took
-  })
   if (*abort_flag) {
     // give copies already issued a bounded time to land before the CTA exits
     const unsigned long long t0 = global_ns();
@@ -678,45 +595,42 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
 }
 
 template <bool INT8, int RB, int COUT>
-int launch_one(const UmmaArgs& args, uint32_t launch_rows, size_t smem, cudaStream_t st) {
+int launch_one(const UmmaArgs& args, uint32_t launch_rows, cudaStream_t st) {
   static bool attr_done[64] = {};
   int dev = 0;
   SPCONVB_CUDA_TRY(cudaGetDevice(&dev));
-  if (smem > kMaxSmem) return SPCONVB_E_UNSUPPORTED;
   if (dev < 0 || dev >= 64 || !attr_done[dev]) {
     SPCONVB_CUDA_TRY(cudaFuncSetAttribute(conv_umma_kernel<INT8, RB, COUT>,
                                           cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)kMaxSmem));
+                                          (int)kSmemBytes));
     if (dev >= 0 && dev < 64) attr_done[dev] = true;
   }
   uint32_t tiles = (launch_rows + 31) / 32;  // the kernel picks the tile height per launch
   int grid = (int)(tiles < (uint32_t)kSmCount ? (tiles ? tiles : 1u) : (uint32_t)kSmCount);
-  conv_umma_kernel<INT8, RB, COUT><<<grid, kCtaThreads, smem, st>>>(args);
+  conv_umma_kernel<INT8, RB, COUT><<<grid, kCtaThreads, kSmemBytes, st>>>(args);
   SPCONVB_LAUNCH_CHECK();
   return SPCONVB_OK;
 }
 
 template <bool INT8, int RB>
-int launch_cout(int cout, const UmmaArgs& args, uint32_t launch_rows, size_t smem,
-                cudaStream_t st) {
+int launch_cout(int cout, const UmmaArgs& args, uint32_t launch_rows, cudaStream_t st) {
   switch (cout) {
-    case 16: return launch_one<INT8, RB, 16>(args, launch_rows, smem, st);
-    case 32: return launch_one<INT8, RB, 32>(args, launch_rows, smem, st);
-    case 64: return launch_one<INT8, RB, 64>(args, launch_rows, smem, st);
-    case 128: return launch_one<INT8, RB, 128>(args, launch_rows, smem, st);
+    case 16: return launch_one<INT8, RB, 16>(args, launch_rows, st);
+    case 32: return launch_one<INT8, RB, 32>(args, launch_rows, st);
+    case 64: return launch_one<INT8, RB, 64>(args, launch_rows, st);
+    case 128: return launch_one<INT8, RB, 128>(args, launch_rows, st);
   }
   return SPCONVB_E_UNSUPPORTED;
 }
 
 template <bool INT8>
-int launch_rb(int rb, int cout, const UmmaArgs& args, uint32_t launch_rows, size_t smem,
-              cudaStream_t st) {
+int launch_rb(int rb, int cout, const UmmaArgs& args, uint32_t launch_rows, cudaStream_t st) {
   switch (rb) {
-    case 16: return launch_cout<INT8, 16>(cout, args, launch_rows, smem, st);
-    case 32: return launch_cout<INT8, 32>(cout, args, launch_rows, smem, st);
-    case 64: return launch_cout<INT8, 64>(cout, args, launch_rows, smem, st);
-    case 128: return launch_cout<INT8, 128>(cout, args, launch_rows, smem, st);
-    case 256: return launch_cout<INT8, 256>(cout, args, launch_rows, smem, st);
+    case 16: return launch_cout<INT8, 16>(cout, args, launch_rows, st);
+    case 32: return launch_cout<INT8, 32>(cout, args, launch_rows, st);
+    case 64: return launch_cout<INT8, 64>(cout, args, launch_rows, st);
+    case 128: return launch_cout<INT8, 128>(cout, args, launch_rows, st);
+    case 256: return launch_cout<INT8, 256>(cout, args, launch_rows, st);
   }
   return SPCONVB_E_UNSUPPORTED;
 }
@@ -724,16 +638,9 @@ int launch_rb(int rb, int cout, const UmmaArgs& args, uint32_t launch_rows, size
 }  // namespace
 
 int conv_umma_kernel_launch(const UmmaArgs& a, bool int8, int rb, int cout, uint32_t launch_rows,
-                            size_t smem, cudaStream_t st) {
-  return int8 ? launch_rb<true>(rb, cout, a, launch_rows, smem, st)
-              : launch_rb<false>(rb, cout, a, launch_rows, smem, st);
+                            cudaStream_t st) {
+  return int8 ? launch_rb<true>(rb, cout, a, launch_rows, st)
+              : launch_rb<false>(rb, cout, a, launch_rows, st);
 }
 
 }  // namespace spconvb
-
-#ifdef SPCONVB_CONV_PROFILE
-extern "C" __attribute__((visibility("default"))) int spconvb_debug_conv_profile(
-    unsigned long long* host) {
-  return (int)cudaMemcpyFromSymbol(host, spconvb::g_conv_profile, sizeof(spconvb::g_conv_profile));
-}
-#endif

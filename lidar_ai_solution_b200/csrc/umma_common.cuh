@@ -10,7 +10,7 @@ namespace umma_detail {
 
 constexpr int kChunk = 128;   // bytes of K per pipeline stage: one 128-byte swizzle atom per row
 constexpr int kMaxTaps = 27;  // most taps of a layer the tensor-core kernel takes
-constexpr int kMaxStages = 6; // deepest ring of gathered-row stages
+constexpr int kMaxStages = 8; // deepest ring of gathered-row stages
 constexpr unsigned long long kWaitLimitNs = 250ull * 1000 * 1000;
 
 struct UmmaArgs {
@@ -24,24 +24,10 @@ struct UmmaArgs {
   const uint8_t* res;
   uint8_t* out;
   uint32_t* status;
-  const uint32_t* n_in_ptr;  // rows of `in` (for the L2 prefetch of input rows); may be null
-  uint32_t cap_in;           // rows the buffer of `in` holds
   int kvol;
-  int w_rep;       // copies of each weight chunk along the accumulator rows: w_rep * Cout = 64 or 128
-  int w_resident;  // 1: all chunks stay in shared memory for the whole launch; 0: streamed
-  int nstages;     // depth of the ring of gathered-row stages (2..kMaxStages)
-  int prefetch;    // tiles (per CTA) the L2 prefetch runs ahead of the gather; 0 = off
   int wait_test;   // > 0: producers withhold "stage full" from this chunk on (self-test)
   Epilogue ep;
 };
-
-// Shared-memory footprint of one launch configuration (the kernel carves it the same way).
-__host__ __device__ inline size_t umma_smem_bytes(int cout, int nchunk, int w_rep, int w_resident,
-                                                  int nstages) {
-  const size_t wchunk = (size_t)w_rep * cout * kChunk;
-  const size_t w = w_resident ? (size_t)nchunk * wchunk : (size_t)nstages * wchunk;
-  return 1024 + w + (size_t)nstages * 256 * kChunk + 256;
-}
 
 // ------------------------------------------------------------- PTX wrappers
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
@@ -140,32 +126,14 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity,
   return mbar_wait_slow(bar, parity, abort_flag, status, where);
 }
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, uint32_t src_bytes) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src),
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src),
                "r"(src_bytes)
                : "memory");
-}
-__device__ __forceinline__ void cp_async4(uint32_t dst, const void* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
-}
-__device__ __forceinline__ void st_shared_s32(uint32_t dst, int32_t v) {
-  asm volatile("st.shared.s32 [%0], %1;" ::"r"(dst), "r"(v) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() {
-  asm volatile("cp.async.commit_group;" ::: "memory");
-}
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 // The calling thread's earlier cp.async copies arrive on the barrier when they have landed
 // (the barrier's expected count includes this arrival: "noinc").
 __device__ __forceinline__ void cp_async_arrive_noinc(uint32_t bar) {
   asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
-}
-// Asks L2 to fetch a contiguous piece of global memory: address 16-byte aligned, size a
-// multiple of 16 bytes.  No data reaches the SM.
-__device__ __forceinline__ void bulk_prefetch_l2(const void* src, uint32_t bytes) {
-  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
 }
 __device__ __forceinline__ void cp_async_wait_all() {
   asm volatile("cp.async.wait_all;" ::: "memory");
@@ -181,6 +149,15 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t
       "l"(src), "r"(bytes), "r"(bar)
       : "memory");
 }
+// One lane of a converged warp (the same one every time), in a form the compiler knows to be
+// a single lane.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(p));
+  return p != 0u;
+}
 __device__ __forceinline__ void tc_fence_before() {
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
 }
@@ -192,24 +169,7 @@ __device__ __forceinline__ void tc_commit(uint32_t bar) {
                    "r"(bar)
                : "memory");
 }
-template <bool INT8>
-__device__ __forceinline__ void umma(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc,
-                                     uint32_t idesc, uint32_t accumulate) {
-  if (INT8) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-        : "memory");
-  } else {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-        : "memory");
-  }
-}
-// The same with the shared-memory descriptors given as halves: only the low word (the
+// One MMA; the shared-memory descriptors are given as halves: only the low word (the
 // address field) changes from chunk to chunk, so the issuing thread does 32-bit arithmetic.
 template <bool INT8>
 __device__ __forceinline__ void umma_lohi(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo,

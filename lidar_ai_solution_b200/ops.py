@@ -156,8 +156,7 @@ def conv_forward(x, m, n_out_ptr, wts: ConvWeights, act=ACT_NONE, out_kind=F16,
                  inv_out_scale=1.0, res=None, res_scale=1.0, mid_kind=F16, mid_inv_scale=1.0,
                  mid_scale=1.0, res_relu=False, force_simt=False, status=None, launch_rows=0,
                  out=None, wait_test=0, n_in_ptr=None):
-    """``n_in_ptr`` (device row count of ``x``) lets the tensor-core kernel prefetch the input
-    rows into L2; results do not depend on it."""
+    """``n_in_ptr`` (device row count of ``x``) is a hint; results do not depend on it."""
     cap = m.shape[1]
     p = cabi.ConvParams()
     p.compute, p.cin, p.cout, p.kvol = wts.compute, wts.cin, wts.cout, wts.kvol
