@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "grid3.hpp"
 #include "spconvb.h"
 
 namespace spconvb {
@@ -31,11 +32,6 @@ inline int blocks_for(uint32_t rows, int threads, int max_waves = 8) {
   if (b < 1) b = 1;
   return (int)b;
 }
-
-struct Grid3 {
-  int32_t g[3];
-  int32_t batch;
-};
 
 __host__ __device__ inline uint32_t voxel_key(int b, int c0, int c1, int c2, const Grid3& g) {
   return (((uint32_t)b * g.g[0] + c0) * g.g[1] + c1) * g.g[2] + c2;
@@ -85,16 +81,25 @@ __device__ __forceinline__ int hash_insert(uint64_t* table, uint32_t mask, uint3
   return 2;
 }
 
-__device__ __forceinline__ int32_t hash_lookup(const uint64_t* __restrict__ table, uint32_t mask,
-                                               uint32_t key) {
+// The probes after the first.
+__device__ __forceinline__ int32_t hash_lookup_next(const uint64_t* __restrict__ table,
+                                                    uint32_t mask, uint32_t key) {
   uint32_t s = hash_first_slot(key, mask);
-  for (uint32_t probe = 0; probe <= (mask >> 3); ++probe) {
-    uint64_t v = __ldg((const unsigned long long*)(table + s));
+  for (uint32_t probe = 0; probe < (mask >> 3); ++probe) {
+    s = (s + 8u) & mask;
+    const uint64_t v = __ldg((const unsigned long long*)(table + s));
     if (v == 0ull) return -1;
     if ((uint32_t)(v >> 32) == key + 1u) return (int32_t)(uint32_t)v;
-    s = (s + 8u) & mask;
   }
   return -1;
+}
+
+__device__ __forceinline__ int32_t hash_lookup(const uint64_t* __restrict__ table, uint32_t mask,
+                                               uint32_t key) {
+  const uint64_t v = __ldg((const unsigned long long*)(table + hash_first_slot(key, mask)));
+  if (v == 0ull) return -1;
+  if ((uint32_t)(v >> 32) == key + 1u) return (int32_t)(uint32_t)v;
+  return hash_lookup_next(table, mask, key);
 }
 
 // ---------------------------------------------------------------- epilogue

@@ -56,6 +56,7 @@
 // Every wait is bounded: a wait that runs out sets SPCONVB_ST_TIMEOUT in the
 // status block, raises a CTA-wide abort flag and all roles leave their loops,
 // drain their copies and free TMEM.
+#include "pdl.cuh"
 #include "umma_common.cuh"
 
 namespace spconvb {
@@ -72,8 +73,12 @@ constexpr int kProdThreads = 512;   // two groups of 8 producer warps
 constexpr int kWeightWarp = kProdWarp0 + kProdThreads / 32;
 constexpr int kCtaThreads = 32 * (kWeightWarp + 1);
 constexpr uint32_t kTmemCols = 2 * kTileRows;
-constexpr size_t kSmemBytes = 232448;  // 227 KB: the most dynamic shared memory of a CTA
-constexpr uint32_t kRingBytes = kSmemBytes - 1024 - 256;  // less alignment slack and barriers
+// 5 stages of 256 rows and 4 of weights: all a CTA can have.  No other block fits beside this one:
+// 26 warps of 72 registers fill two of the SM's four register files.  With 64 registers and 12 KB
+// less a rulebook block fits and the two do overlap, but the convolutions then take 3 % longer,
+// which is what the overlap saves (batch of 8 frames 4.25 ms against 4.34).
+constexpr uint32_t kRingBytes = 5 * kTileRows * kChunk + 4 * 128 * kChunk;
+constexpr size_t kSmemBytes = kRingBytes + 1024 + 256;  // alignment slack, barriers
 
 // 32-bit instruction descriptor: [4,6) D format (1 = f32, 2 = s32), [7,10) A
 // format, [10,13) B format (f16 kind: 0 = f16; i8 kind: 1 = signed), bits 15/16
@@ -154,7 +159,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
 
   const int warp = threadIdx.x >> 5;
   const uint32_t lane = threadIdx.x & 31;
-  const uint32_t n_out = min(__ldg(a.n_out_ptr), a.cap);
+  pdl_trigger();
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kMaxStages; ++s) {
@@ -176,6 +181,8 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
+  pdl_wait();  // nothing above reads or writes what an earlier kernel may still be working on
+  const uint32_t n_out = min(__ldg(a.n_out_ptr), a.cap);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -191,7 +198,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
       min((uint32_t)kTileRows, max(32u, ((per_cta + rounds - 1) / rounds + 31u) & ~31u));
   const uint32_t ntiles = (n_out + tile_rows - 1) / tile_rows;
   // Two rings share the buffer: row stages as high as this launch's tile, and weight stages.
-  // As many of both as fit (low tiles get deeper rings); what is left over goes to the rows.
+  // Low tiles get deeper rings: as many of both as fit, and what is left over goes to the rows.
   const uint32_t row_stage = tile_rows * kChunk;
   const uint32_t nwst = min((uint32_t)kMaxStages, kRingBytes / (kWeightBytes + row_stage));
   const uint32_t nst = min((uint32_t)kMaxStages, (kRingBytes - nwst * kWeightBytes) / row_stage);
@@ -607,8 +614,8 @@ int launch_one(const UmmaArgs& args, uint32_t launch_rows, cudaStream_t st) {
   }
   uint32_t tiles = (launch_rows + 31) / 32;  // the kernel picks the tile height per launch
   int grid = (int)(tiles < (uint32_t)kSmCount ? (tiles ? tiles : 1u) : (uint32_t)kSmCount);
-  conv_umma_kernel<INT8, RB, COUT><<<grid, kCtaThreads, kSmemBytes, st>>>(args);
-  SPCONVB_LAUNCH_CHECK();
+  SPCONVB_CUDA_TRY(launch_pdl(conv_umma_kernel<INT8, RB, COUT>, dim3(grid), dim3(kCtaThreads),
+                              kSmemBytes, st, args));
   return SPCONVB_OK;
 }
 

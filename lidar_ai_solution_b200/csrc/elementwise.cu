@@ -1,6 +1,7 @@
 // HBM-bound helpers around the convolutions: Add / Add&ReLU / ReLU, precision
 // and channel-padding conversion, and the sparse -> dense BEV scatter.
 #include "common.cuh"
+#include "pdl.cuh"
 
 namespace spconvb {
 
@@ -174,6 +175,7 @@ __global__ void scatter_dense_kernel(const void* __restrict__ feat, int in_kind,
                                      __half* __restrict__ out) {
   extern __shared__ __half tile[];  // [channels][33]
   __shared__ long long s_cell[32];
+  pdl_wait();
   const uint32_t n = min(*n_ptr, cap);
   const int gp[3] = {g.g[p0], g.g[p1], g.g[p2]};
   const size_t vol = (size_t)gp[0] * gp[1] * gp[2];
@@ -398,10 +400,10 @@ extern "C++" int spconvb::scatter_dense_launch(const void* feat, int32_t in_kind
   size_t want_blocks = ((size_t)launch_rows + 31) / 32;
   if (want_blocks > (size_t)kSmCount * 16) want_blocks = (size_t)kSmCount * 16;
   const int blocks = (int)want_blocks;
-  scatter_dense_kernel<<<blocks, 256, sizeof(__half) * 33 * channels, st>>>(
-      feat, in_kind, in_scale, (const int4*)coords, n_ptr, launch_rows, channels, g, p[0], p[1],
-      p[2], (__half*)out);
-  SPCONVB_LAUNCH_CHECK();
+  SPCONVB_CUDA_TRY(launch_pdl(scatter_dense_kernel, dim3(blocks), dim3(256),
+                              sizeof(__half) * 33 * channels, st, feat, in_kind, in_scale,
+                              (const int4*)coords, n_ptr, launch_rows, channels, g, p[0], p[1], p[2],
+                              (__half*)out));
   return SPCONVB_OK;
 }
 

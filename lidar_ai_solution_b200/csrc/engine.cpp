@@ -64,7 +64,7 @@ int Builder::push(GNode&& n, const std::string& out_name) {
 // ------------------------------------------------------------------- engine
 Engine::~Engine() {
   free_prepared();
-  for (cudaEvent_t e : rule_ev_)
+  for (cudaEvent_t e : level_ev_)
     if (e) cudaEventDestroy(e);
   if (fork_ev_) cudaEventDestroy(fork_ev_);
   if (aux_) cudaStreamDestroy(aux_);
@@ -816,24 +816,165 @@ int Engine::prepare(const int32_t grid[3], int batch) {
     t.data = slots[pick].ptr;
   }
   if (cudaDeviceSynchronize() != cudaSuccess) return SPCONVB_E_NOMEM;
-  if (!(flags & SPCONVB_BUILD_SINGLE_STREAM) && !aux_) {
-    bool ok = cudaStreamCreateWithFlags(&aux_, cudaStreamNonBlocking) == cudaSuccess &&
-              cudaEventCreateWithFlags(&fork_ev_, cudaEventDisableTiming) == cudaSuccess;
-    rule_ev_.assign(steps.size(), nullptr);
-    for (size_t i = 0; ok && i < steps.size(); ++i)
-      if (is_rulebook_step(steps[i]))
-        ok = cudaEventCreateWithFlags(&rule_ev_[i], cudaEventDisableTiming) == cudaSuccess;
+  plan_waves();
+  if (!(flags & SPCONVB_BUILD_SINGLE_STREAM)) {
+    bool ok = true;
+    if (!aux_)
+      ok = cudaStreamCreateWithFlags(&aux_, cudaStreamNonBlocking) == cudaSuccess &&
+           cudaEventCreateWithFlags(&fork_ev_, cudaEventDisableTiming) == cudaSuccess;
+    const int levels = waves_.empty() ? 0 : waves_.back().level + 1;
+    while (ok && (int)level_ev_.size() < levels) {
+      cudaEvent_t e = nullptr;
+      ok = cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess;
+      if (ok) level_ev_.push_back(e);
+    }
     if (!ok) return SPCONVB_E_NOMEM;
   }
   prepared_ = true;
   return SPCONVB_OK;
 }
 
+// The rulebook steps as tasks, each on the earliest level where everything it reads is there:
+//   level 0   row count, padded features, hash table, bitmap of the first strided rulebook
+//   level 1   SubM map of the caller's rows, output rows of that rulebook, bitmap of the next
+//   level 2   its strided map and its SubM map, output rows of the next, bitmap of the one after
+//   ...
+// Tasks of one level share launches.  A backbone with four strided and four SubM rulebooks has 6
+// levels; one kernel per task is 24 launches whose latencies follow one another.
+void Engine::plan_waves() {
+  struct Planned { int level; RuleTask t; bool caller_rows; };
+  std::vector<Planned> tasks;
+  const int in_cs = rt[input_rt_].cs;
+  uint32_t* in_n = counts_ + 64 * (size_t)in_cs;
+  std::vector<int> mark_level(rules.size(), 0), emit_level(rules.size(), 0);
+  rule_level_.assign(rules.size(), 0);
+  pad_step_ = -1;
+
+  auto rows = [&](int32_t kind, int cs) {
+    RuleTask t;
+    const CoordSet& c = coordsets[cs];
+    t.kind = kind;
+    t.coords = (const int4*)c.coords;
+    t.n_ptr = c.external ? in_n : c.n_ptr;
+    t.cap = c.cap;
+    t.gin = make_grid(c.grid, batch_);
+    t.blocks = task_blocks(c.cap);
+    t.status = status;
+    return t;
+  };
+  auto put = [&](int level, const RuleTask& t, bool caller) { tasks.push_back({level, t, caller}); };
+
+  {
+    RuleTask t = rows(TASK_COUNT, in_cs);
+    t.blocks = 1;
+    t.n_out = in_n;
+    put(0, t, true);
+  }
+  bool first_feature_step = true;  // its buffer is not shared with an earlier tensor
+  for (size_t si = 0; si < steps.size(); ++si) {
+    const Step& s = steps[si];
+    const bool first = first_feature_step;
+    if (!is_rulebook_step(s)) first_feature_step = false;
+    if (s.kind == Step::CONVERT && first && s.in0 == input_rt_ && s.cout == 8 &&
+        rt[s.out].kind == SPCONVB_F16) {
+      RuleTask t = rows(TASK_PAD8, in_cs);
+      t.channels = s.cin;
+      t.feat_out = (uint4*)rt[s.out].data;
+      pad_step_ = (int)si;
+      put(0, t, true);
+    } else if (s.kind == Step::HASH) {
+      RuleTask t = rows(TASK_HASH, s.cs);
+      t.table = coordsets[s.cs].table;
+      t.mask = coordsets[s.cs].slots - 1;
+      put(0, t, true);
+    } else if (s.kind == Step::SUBM_MAP) {
+      const Rule& R = rules[s.rule];
+      const CoordSet& c = coordsets[R.in_cs];
+      RuleTask t = rows(c.external ? TASK_SUBM_HASH : TASK_SUBM_RANK, R.in_cs);
+      t.kr = make_kernel3(R.ksize, nullptr, nullptr, R.dil);
+      t.map = R.map;
+      if (c.external) {
+        t.table = c.table;
+        t.mask = c.slots - 1;
+      } else {
+        t.ws = down_ws(c.grid, batch_, rules[c.made_by_rule].ws);
+      }
+      rule_level_[s.rule] = c.external ? 1 : emit_level[c.made_by_rule] + 1;
+      put(rule_level_[s.rule], t, c.external);
+    } else if (s.kind == Step::DOWN_MAP) {
+      const Rule& R = rules[s.rule];
+      const CoordSet &ci = coordsets[R.in_cs], &co = coordsets[R.out_cs];
+      const int from = ci.made_by_rule;
+      RuleTask mark = rows(TASK_MARK_ROWS, R.in_cs);
+      mark.gout = make_grid(co.grid, batch_);
+      mark.kr = make_kernel3(R.ksize, R.stride, R.pad, R.dil);
+      mark.ws = down_ws(co.grid, batch_, R.ws);
+      if (from >= 0) mark.in_ws = down_ws(ci.grid, batch_, rules[from].ws);
+      RuleTask emit = rows(TASK_EMIT, R.out_cs), fill = mark;
+      if (from >= 0 && mark_from_bitmap(mark.kr)) {
+        mark.kind = TASK_MARK_BITMAP;
+        mark.blocks = mark_bitmap_blocks(co.grid, batch_);
+        mark_level[s.rule] = mark_level[from] + 1;
+      } else {
+        mark_level[s.rule] = from >= 0 ? emit_level[from] + 1 : 0;
+      }
+      put(mark_level[s.rule], mark, ci.external);
+      emit_level[s.rule] = mark_level[s.rule] + 1;
+      emit.gout = mark.gout;
+      emit.kr = mark.kr;
+      emit.ws = mark.ws;
+      emit.blocks = mark.ws.blocks;
+      emit.out_coords = (int4*)co.coords;
+      emit.n_out = co.n_ptr;
+      emit.map = from >= 0 ? nullptr : R.map;
+      put(emit_level[s.rule], emit, false);
+      fill.map = R.map;
+      if (from >= 0) {
+        fill.kind = TASK_GATHER;
+        fill.coords = (const int4*)co.coords;
+        fill.n_ptr = co.n_ptr;
+        fill.cap = co.cap;
+        fill.other_cap = ci.cap;
+        fill.blocks = task_blocks(co.cap);
+      } else {
+        fill.kind = TASK_SCATTER;
+        fill.map_cap = co.cap;
+      }
+      rule_level_[s.rule] = emit_level[s.rule] + 1;
+      put(rule_level_[s.rule], fill, ci.external);
+    } else if (s.kind == Step::INV_MAP) {
+      const Rule& R = rules[s.rule];
+      const Rule& F = rules[R.inverse_of];
+      RuleTask t = rows(TASK_INVERSE, R.out_cs);
+      t.blocks = task_blocks((unsigned long long)t.cap * R.kvol);
+      t.gout = make_grid(coordsets[F.out_cs].grid, batch_);
+      t.kr = make_kernel3(F.ksize, F.stride, F.pad, F.dil);
+      t.ws = down_ws(coordsets[F.out_cs].grid, batch_, F.ws);
+      t.other_cap = coordsets[F.out_cs].cap;
+      t.map = R.map;
+      rule_level_[s.rule] = emit_level[R.inverse_of] + 1;
+      put(rule_level_[s.rule], t, coordsets[R.out_cs].external);
+    }
+  }
+  std::stable_sort(tasks.begin(), tasks.end(),
+                   [](const Planned& a, const Planned& b) { return a.level < b.level; });
+  waves_.clear();
+  for (const Planned& p : tasks) {
+    if (waves_.empty() || waves_.back().level != p.level || waves_.back().wave.full()) {
+      waves_.emplace_back();
+      waves_.back().level = p.level;
+    }
+    PlannedWave& w = waves_.back();
+    w.caller_rows[w.wave.count] = p.caller_rows;
+    w.wave.add(p.t);
+  }
+}
+
 int Engine::forward(const void* features, const int32_t* indices, uint32_t cap_rows,
                     uint32_t n_host, const uint32_t* n_dev, const int32_t grid[3], int batch,
                     cudaStream_t caller_stream, const Profile* prof) {
   if (input_rt_ < 0 || !features || !indices || !grid) return SPCONVB_E_ARG;
-  cudaStream_t st = caller_stream;  // the stream run_step launches on; switched for rulebook steps
+  cudaStream_t st = caller_stream;
   int rc = prepare(grid, batch);
   if (rc != SPCONVB_OK) return rc;
   CoordSet& in = coordsets[rt[input_rt_].cs];
@@ -849,10 +990,12 @@ int Engine::forward(const void* features, const int32_t* indices, uint32_t cap_r
   // the caller's device-side value clamped to the rows the caller's buffers (and the model's
   // bound) hold, so that no kernel can be led past them.
   uint32_t* in_n = counts_ + 64 * (size_t)rt[input_rt_].cs;
-  if (n_dev) rc = launch_clamp_count(in_n, n_dev, in_cap, status, st);
-  else rc = launch_set_count(in_n, n_host, st);
-  if (rc != SPCONVB_OK) return rc;
-  ++last_launches;
+  if (prof) {
+    if (n_dev) rc = launch_clamp_count(in_n, n_dev, in_cap, status, st);
+    else rc = launch_set_count(in_n, n_host, st);
+    if (rc != SPCONVB_OK) return rc;
+    ++last_launches;
+  }
   rt[input_rt_].data = const_cast<void*>(features);
   last_in_n_ = in_n;
   last_in_cap_ = in_cap;
@@ -901,13 +1044,13 @@ int Engine::forward(const void* features, const int32_t* indices, uint32_t cap_r
                                        R.stride, R.pad, R.dil, rules[ci.made_by_rule].ws, R.ws,
                                        co.coords, co.n_ptr, co.cap, R.map, co.table, co.slots,
                                        SPCONVB_FLAG_PREZEROED, status, st);
-          last_launches += 4 + (co.table ? 1 : 0);  // mark, scan, emit, gather (+ hash)
+          last_launches += 3;  // mark, emit, gather
         } else {
           rc = spconvb_down_map(cs_coords(R.in_cs), cs_n(R.in_cs), cs_cap(R.in_cs),
                                 cs_launch(R.in_cs), ci.grid, batch, R.ksize, R.stride, R.pad,
                                 R.dil, ci.table, ci.slots, R.ws, co.coords, co.n_ptr, co.cap,
                                 R.map, co.table, co.slots, SPCONVB_FLAG_PREZEROED, status, st);
-          last_launches += 5 + (co.table ? 1 : 0);  // mark, scan, emit, map fill, scatter (+ hash)
+          last_launches += 3;  // mark, emit, scatter
         }
         break;
       }
@@ -969,28 +1112,51 @@ int Engine::forward(const void* features, const int32_t* indices, uint32_t cap_r
     if (cudaEventCreate(&ev0) != cudaSuccess || cudaEventCreate(&ev1) != cudaSuccess)
       return SPCONVB_E_NOMEM;
   }
-  // Fork: the rulebook steps go to the auxiliary stream in their original order; a feature
-  // step waits for the last rulebook step that precedes it in the program, which covers its
-  // rulebook, its coordinate set and its row count.  Nothing a rulebook step reads is written
-  // by a feature step.  The caller's stream joins the auxiliary one before returning, so the
-  // whole call remains one unit of work on that stream (and one capturable region).
-  const bool fork = !prof && aux_ != nullptr;
-  int last_rule = -1, waited = -1;
-  if (fork) {
+  // Rulebook waves.  Levels 0 and 1 (what the first convolutions need) go to the caller's
+  // stream; the others follow on the auxiliary stream, and a convolution waits for the level that
+  // completes its map.  Nothing a wave reads is written by a feature step.  Every level is waited
+  // for in the end, so the whole call remains one unit of work on the caller's stream (and one
+  // capturable region).  With one stream a level is launched when it is first needed.
+  size_t next_wave = 0;
+  auto launch_waves = [&](int up_to, cudaStream_t on) -> int {
+    int r = SPCONVB_OK;
+    for (; r == SPCONVB_OK && next_wave < waves_.size() && waves_[next_wave].level <= up_to;
+         ++next_wave) {
+      RuleWave w = waves_[next_wave].wave;
+      for (int i = 0; i < w.count; ++i) {
+        if (!waves_[next_wave].caller_rows[i]) continue;
+        RuleTask& t = w.t[i];
+        t.coords = (const int4*)indices;
+        t.feat = features;
+        if (waves_[next_wave].level == 0) {  // in_n is not there yet
+          t.n_ptr = n_dev;
+          t.n_host = n_host;
+          t.cap = in_cap;
+        }
+        if (!n_dev && t.kind != TASK_COUNT && t.kind != TASK_INVERSE)
+          t.blocks = std::min(t.blocks, task_blocks(n_host));
+      }
+      r = launch_rule_wave(w, on);
+      ++last_launches;
+    }
+    return r;
+  };
+  const int last_level = waves_.empty() ? -1 : waves_.back().level;
+  const bool fork = !prof && aux_ != nullptr && last_level >= 2;
+  int waited = 1;
+  std::vector<char> precleared(steps.size(), 0);
+  if (!prof && rc == SPCONVB_OK) rc = launch_waves(fork ? 1 : 0, st);
+  if (fork && rc == SPCONVB_OK) {
     if (cudaEventRecord(fork_ev_, caller_stream) != cudaSuccess ||
         cudaStreamWaitEvent(aux_, fork_ev_, 0) != cudaSuccess)
       return SPCONVB_E_DEVICE;
-  }
-  // Dense outputs are zeroed on the auxiliary stream right away (bandwidth the convolutions
-  // leave unused) when a rulebook step precedes the dense step: its event, which the dense step
-  // waits for, then also covers the zero fill.
-  std::vector<char> precleared(steps.size(), 0);
-  if (fork) {
-    bool rule_seen = false;
+    // Dense outputs are zeroed on the auxiliary stream right away (bandwidth the convolutions
+    // leave unused) when a convolution before them waits for one of its levels.
+    bool level_seen = false;
     for (size_t si = 0; si < steps.size() && rc == SPCONVB_OK; ++si) {
       const Step& s = steps[si];
-      if (is_rulebook_step(s)) rule_seen = true;
-      if (s.kind != Step::DENSE || !rule_seen) continue;
+      if (s.kind == Step::CONV && rule_level_[s.rule] >= 2) level_seen = true;
+      if (s.kind != Step::DENSE || !level_seen) continue;
       const CoordSet& cs = coordsets[s.cs];
       const size_t bytes = spconvb_dense_bytes(s.cout, batch, cs.grid, s.has_perm ? s.perm : nullptr,
                                                s.layout, rt[s.out].kind);
@@ -998,28 +1164,27 @@ int Engine::forward(const void* features, const int32_t* indices, uint32_t cap_r
       if (cudaMemsetAsync(rt[s.out].data, 0, bytes, aux_) != cudaSuccess) rc = SPCONVB_E_DEVICE;
       else precleared[si] = 1;
     }
+    for (int level = 2; level <= last_level && rc == SPCONVB_OK; ++level) {
+      rc = launch_waves(level, aux_);
+      if (cudaEventRecord(level_ev_[level], aux_) != cudaSuccess) rc = SPCONVB_E_DEVICE;
+    }
   }
   for (size_t si = 0; si < steps.size() && rc == SPCONVB_OK; ++si) {
     const Step& s = steps[si];
     clear_dense = !precleared[si];
-    if (fork) {
-      if (is_rulebook_step(s)) {
-        st = aux_;
-        rc = run_step(s);
-        st = caller_stream;
-        if (rc == SPCONVB_OK && cudaEventRecord(rule_ev_[si], aux_) != cudaSuccess)
-          rc = SPCONVB_E_DEVICE;
-        last_rule = (int)si;
-      } else {
-        if (last_rule > waited) {
-          if (cudaStreamWaitEvent(caller_stream, rule_ev_[last_rule], 0) != cudaSuccess)
+    if (!prof) {
+      if (is_rulebook_step(s) || (int)si == pad_step_) continue;
+      const int level = s.kind == Step::CONV ? rule_level_[s.rule] : 0;
+      if (fork) {
+        if (level > waited) {
+          if (cudaStreamWaitEvent(caller_stream, level_ev_[level], 0) != cudaSuccess)
             rc = SPCONVB_E_DEVICE;
-          waited = last_rule;
+          waited = level;
         }
-        if (rc == SPCONVB_OK) rc = run_step(s);
+      } else {
+        rc = launch_waves(level, st);
       }
-    } else if (!prof) {
-      rc = run_step(s);
+      if (rc == SPCONVB_OK) rc = run_step(s);
     } else {
       // Per-step device time: rulebook steps change state and run once; the
       // others overwrite their output and are repeated, each time behind an L2
@@ -1048,7 +1213,9 @@ int Engine::forward(const void* features, const int32_t* indices, uint32_t cap_r
       break;
     }
   }
-  if (fork) {  // join, also after a failed step, so that the auxiliary stream never outlives the call
+  if (!prof && !fork && rc == SPCONVB_OK) rc = launch_waves(last_level, st);
+  if (fork && (waited < last_level || rc != SPCONVB_OK)) {
+    // join, also after a failed step, so that the auxiliary stream never outlives the call
     if (cudaEventRecord(fork_ev_, aux_) != cudaSuccess ||
         cudaStreamWaitEvent(caller_stream, fork_ev_, 0) != cudaSuccess)
       rc = rc == SPCONVB_OK ? SPCONVB_E_DEVICE : rc;

@@ -10,6 +10,7 @@
 #include <unordered_map>
 #include <vector>
 
+#include "rulebook.hpp"
 #include "spconvb.h"
 
 namespace spconvb {
@@ -121,6 +122,14 @@ struct RTensor {
   size_t bytes = 0;
 };
 
+// A launch of rulebook tasks that depend on the levels before it only.  `caller_rows[i]`: task i
+// walks the caller's rows, whose address (and, on level 0, count) each call fills in.
+struct PlannedWave {
+  int level = 0;
+  RuleWave wave;
+  bool caller_rows[kMaxWaveTasks] = {};
+};
+
 struct LayerWeights {
   void* plain = nullptr;
   void* packed = nullptr;
@@ -186,11 +195,15 @@ class Engine {
   int32_t grid_[3] = {0, 0, 0};
   int batch_ = 0;
   std::vector<void*> allocations_;
-  // Rulebook steps depend on coordinates only: they run ahead on this stream while the
-  // caller's stream does the convolutions, joined by one event per rulebook step.
+  // Rulebook work, by level (see plan_waves).  The levels from 2 on run ahead on the auxiliary
+  // stream while the caller's stream does the convolutions, joined by one event per level.
+  std::vector<PlannedWave> waves_;
+  std::vector<int> rule_level_;  // level that completes a rule's map
+  int pad_step_ = -1;            // the step that pads the caller's features, done on level 0
   cudaStream_t aux_ = nullptr;
   cudaEvent_t fork_ev_ = nullptr;
-  std::vector<cudaEvent_t> rule_ev_;
+  std::vector<cudaEvent_t> level_ev_;
+  void plan_waves();
   void* zero_arena_ = nullptr;
   size_t zero_bytes_ = 0;
   uint32_t* counts_ = nullptr;

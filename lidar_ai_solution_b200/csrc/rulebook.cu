@@ -1,48 +1,31 @@
 // Rulebook construction: coordinate hash table, submanifold neighbour map and
-// strided-convolution map.  All HBM/L2-bound integer work; every kernel reads
-// its row count from device memory and strides, so launches never depend on
-// host knowledge of the counts.
+// strided-convolution map.  Integer work bound by L2 latency (small frames) or by the bytes of
+// the maps (batches); every task reads its row count from device memory and strides, so
+// launches never depend on host knowledge of the counts.
 //
 // Strided outputs are made unique and ordered without sorting: each candidate
-// output cell sets one bit in a bitmap over the output grid, an exclusive scan
-// of the per-word popcounts ranks the set bits, and the rank is the output row.
+// output cell sets one bit in a bitmap over the output grid, the popcounts of the words before
+// it rank a set bit, and the rank is the output row.
+//
+// The steps of one rulebook are short (2-20 us) and several rulebooks are independent of one
+// another, so they run as tasks of shared launches (RuleWave): a backbone of four strided and
+// four SubM rulebooks takes 6 launches where one kernel per step took 24.
 #include <mutex>
 
 #include "common.cuh"
+#include "pdl.cuh"
+#include "rulebook.hpp"
 
 namespace spconvb {
+namespace {
 
-constexpr int kThreads = 256;
-constexpr int kScanThreads = 1024;
-constexpr int kScanWordsPerBlock = kScanThreads;  // one bitmap word per thread
+constexpr int kTaskThreads = 128;
+constexpr int kTaskWarps = kTaskThreads / 32;
+constexpr uint32_t kScanWords = kTaskThreads;  // bitmap words per scan block: one a thread
 
-// ------------------------------------------------------------------ hash build
-__global__ void hash_build_kernel(const int4* __restrict__ coords, const uint32_t* n_ptr,
-                                  uint32_t cap, Grid3 g, uint64_t* table, uint32_t mask,
-                                  uint32_t* status) {
-  const uint32_t n = min(*n_ptr, cap);
-  if (blockIdx.x == 0 && threadIdx.x == 0 && *n_ptr > cap)
-    set_status(status, SPCONVB_ST_OVERFLOW, *n_ptr);
-  for (uint32_t row = blockIdx.x * blockDim.x + threadIdx.x; row < n;
-       row += gridDim.x * blockDim.x) {
-    int4 c = __ldg(coords + row);
-    if ((unsigned)c.x >= (unsigned)g.batch || (unsigned)c.y >= (unsigned)g.g[0] ||
-        (unsigned)c.z >= (unsigned)g.g[1] || (unsigned)c.w >= (unsigned)g.g[2]) {
-      set_status(status, SPCONVB_ST_COORD_RANGE, row);
-      continue;
-    }
-    hash_insert(table, mask, voxel_key(c.x, c.y, c.z, c.w, g), row, status);
-  }
+__device__ __forceinline__ uint32_t task_rows(const RuleTask& t) {
+  return min(t.n_ptr ? __ldg(t.n_ptr) : t.n_host, t.cap);
 }
-
-// ------------------------------------------------------------------- SubM map
-struct Kernel3 {
-  int32_t k[3];
-  int32_t s[3];
-  int32_t p[3];
-  int32_t d[3];
-  int32_t sh[3];  // log2 of the stride when it is a power of two (1, 2, 4, ...), else -1
-};
 
 // v % s == 0 and v / s for v >= 0, without the integer division when the stride is a power
 // of two (every strided layer of the lidar backbones has stride 1 or 2).
@@ -52,19 +35,75 @@ __device__ __forceinline__ bool stride_divides(int v, int s, int sh) {
 __device__ __forceinline__ int stride_quotient(int v, int s, int sh) {
   return sh >= 0 ? v >> sh : v / s;
 }
+__host__ __device__ inline bool unit_dilation(const Kernel3& kr) {
+  return kr.d[0] == 1 && kr.d[1] == 1 && kr.d[2] == 1;
+}
+__host__ __device__ inline bool is_k333(const Kernel3& kr) {
+  return kr.k[0] == 3 && kr.k[1] == 3 && kr.k[2] == 3 && unit_dilation(kr);
+}
 
-// One thread per row: the row's coordinate is read once, its taps are walked in tap order
-// (so a warp's stores of one tap land in one or two lines of map[k][.]), and the lookups of
-// the 27 taps are independent loads the compiler overlaps when the kernel size is known at
-// compile time (K333: the 3x3x3, dilation-1 case of every backbone layer).
+// Row of a cell from the bitmap and its ranks, -1 if the cell is empty or lies beyond the
+// capacity.
+__device__ __forceinline__ int32_t rank_lookup(const uint32_t* __restrict__ bitmap,
+                                               const uint32_t* __restrict__ prefix,
+                                               uint32_t cell, uint32_t cap) {
+  const uint32_t bits = __ldg(bitmap + (cell >> 5));
+  const uint32_t b = cell & 31u;
+  if (!((bits >> b) & 1u)) return -1;
+  const uint32_t row = __ldg(prefix + (cell >> 5)) + __popc(bits & ((1u << b) - 1u));
+  return row < cap ? (int32_t)row : -1;
+}
+
+// ---------------------------------------------------------------- the caller's rows
+__device__ __forceinline__ void task_count(const RuleTask& t) {
+  if (threadIdx.x != 0) return;
+  const uint32_t n = t.n_ptr ? __ldg(t.n_ptr) : t.n_host;
+  if (n > t.cap) set_status(t.status, SPCONVB_ST_OVERFLOW, n);
+  *t.n_out = min(n, t.cap);
+}
+
+// fp16 rows padded to 8 channels (the first layer of a lidar backbone: 4 or 5 point features in
+// 16-byte rows): one thread per row, one 16-byte store.
+__device__ __forceinline__ void task_pad8(const RuleTask& t, uint32_t first, uint32_t step) {
+  const uint32_t n = task_rows(t);
+  for (uint32_t row = first; row < n; row += step) {
+    const __half* src = (const __half*)t.feat + (size_t)row * t.channels;
+    uint16_t h[8];
+#pragma unroll
+    for (int c = 0; c < 8; ++c)
+      h[c] = c < t.channels ? __half_as_ushort(__ldg(src + c)) : (uint16_t)0;
+    t.feat_out[row] = make_uint4(h[0] | (uint32_t)h[1] << 16, h[2] | (uint32_t)h[3] << 16,
+                                 h[4] | (uint32_t)h[5] << 16, h[6] | (uint32_t)h[7] << 16);
+  }
+}
+
+__device__ __forceinline__ void task_hash(const RuleTask& t, uint32_t first, uint32_t step) {
+  const uint32_t n = task_rows(t);
+  if (first == 0 && t.n_ptr && *t.n_ptr > t.cap)
+    set_status(t.status, SPCONVB_ST_OVERFLOW, *t.n_ptr);
+  for (uint32_t row = first; row < n; row += step) {
+    const int4 c = __ldg(t.coords + row);
+    if ((unsigned)c.x >= (unsigned)t.gin.batch || (unsigned)c.y >= (unsigned)t.gin.g[0] ||
+        (unsigned)c.z >= (unsigned)t.gin.g[1] || (unsigned)c.w >= (unsigned)t.gin.g[2]) {
+      set_status(t.status, SPCONVB_ST_COORD_RANGE, row);
+      continue;
+    }
+    hash_insert(t.table, t.mask, voxel_key(c.x, c.y, c.z, c.w, t.gin), row, t.status);
+  }
+}
+
+// ------------------------------------------------------------------- SubM maps
+// One thread per row: the row's coordinate is read once, its taps are walked in tap order, so
+// a warp's stores of one tap land in one or two lines of map[k][.].
 template <bool K333, typename Lookup>
-__device__ __forceinline__ void subm_row_taps(const int4 c, uint32_t row, const Grid3& g,
-                                              const Kernel3& kr, uint32_t cap,
-                                              int32_t* __restrict__ map, Lookup lookup) {
+__device__ __forceinline__ void subm_row_taps(const int4 c, uint32_t row, const RuleTask& t,
+                                              Lookup lookup) {
+  const Grid3& g = t.gin;
+  const Kernel3& kr = t.kr;
   const int K0 = K333 ? 3 : kr.k[0], K1 = K333 ? 3 : kr.k[1], K2 = K333 ? 3 : kr.k[2];
   const int D0 = K333 ? 1 : kr.d[0], D1 = K333 ? 1 : kr.d[1], D2 = K333 ? 1 : kr.d[2];
   const bool bok = (unsigned)c.x < (unsigned)g.batch;
-  int32_t* dst = map + row;
+  int32_t* dst = t.map + row;
 #pragma unroll
   for (int k0 = 0; k0 < K0; ++k0) {
     const int p0 = c.y + (k0 - K0 / 2) * D0;
@@ -80,59 +119,74 @@ __device__ __forceinline__ void subm_row_taps(const int4 c, uint32_t row, const 
         if (k0 == K0 / 2 && k1 == K1 / 2 && k2 == K2 / 2) r = (int32_t)row;
         else if (ok1 && (unsigned)p2 < (unsigned)g.g[2]) r = lookup(voxel_key(c.x, p0, p1, p2, g));
         *dst = r;
-        dst += cap;
+        dst += t.cap;
       }
     }
   }
 }
 
-template <bool K333>
-__global__ void subm_map_kernel(const int4* __restrict__ coords, const uint32_t* n_ptr,
-                                uint32_t cap, Grid3 g, Kernel3 kr,
-                                const uint64_t* __restrict__ table, uint32_t mask,
-                                int32_t* __restrict__ map) {
-  const uint32_t n = min(*n_ptr, cap);
-  for (uint32_t row = blockIdx.x * blockDim.x + threadIdx.x; row < n;
-       row += gridDim.x * blockDim.x)
-    subm_row_taps<K333>(__ldg(coords + row), row, g, kr, cap, map,
-                        [&](uint32_t key) { return hash_lookup(table, mask, key); });
+// 3x3x3 lookups in the hash table.  A probe is a random L2 access of ~700 cycles and most find
+// nothing, so what counts is how many are in flight: the first probes of the 9 taps of a plane
+// are issued together and only then looked at (a probe loop per tap took its 27 latencies one
+// after the other).  Taps whose first slot holds another cell go on probing one by one.
+__device__ __forceinline__ void subm_hash_k333(const int4 c, uint32_t row, const RuleTask& t) {
+  const Grid3& g = t.gin;
+  const uint64_t* __restrict__ table = t.table;
+  const bool bok = (unsigned)c.x < (unsigned)g.batch;
+  int32_t* dst = t.map + row;
+#pragma unroll 1
+  for (int k0 = 0; k0 < 3; ++k0) {
+    const int p0 = c.y + k0 - 1;
+    const bool ok0 = bok && (unsigned)p0 < (unsigned)g.g[0];
+    unsigned long long v[9];
+#pragma unroll
+    for (int q = 0; q < 9; ++q) {
+      const int p1 = c.z + q / 3 - 1, p2 = c.w + q % 3 - 1;
+      v[q] = 0ull;
+      if (ok0 && (unsigned)p1 < (unsigned)g.g[1] && (unsigned)p2 < (unsigned)g.g[2])
+        v[q] = __ldg((const unsigned long long*)table +
+                     hash_first_slot(voxel_key(c.x, p0, p1, p2, g), t.mask));
+    }
+#pragma unroll
+    for (int q = 0; q < 9; ++q) {
+      int32_t r = -1;
+      if (v[q] != 0ull) {
+        const uint32_t key = voxel_key(c.x, p0, c.z + q / 3 - 1, c.w + q % 3 - 1, g);
+        r = (uint32_t)(v[q] >> 32) == key + 1u ? (int32_t)(uint32_t)v[q]
+                                               : hash_lookup_next(table, t.mask, key);
+      }
+      *dst = r;
+      dst += t.cap;
+    }
+  }
 }
 
-// ---------------------------------------------------------------- strided map
-// workspace layout (32-bit words):
-//   [0, W)        bitmap over the output grid
-//   [W, 2W)       exclusive popcount prefix per word (global after emit)
-//   [2W, 2W+B)    per-scan-block popcount sums
-struct DownWs {
-  uint32_t* bitmap;
-  uint32_t* prefix;
-  uint32_t* block_sums;
-  uint32_t words;
-  uint32_t blocks;
-};
-
-__host__ __device__ inline uint32_t down_words(const int32_t og[3], int batch) {
-  unsigned long long cells = (unsigned long long)batch * og[0] * og[1] * og[2];
-  return (uint32_t)((cells + 31) / 32);
+__device__ __forceinline__ void task_subm_hash(const RuleTask& t, uint32_t first, uint32_t step) {
+  const uint32_t n = task_rows(t);
+  const bool k333 = is_k333(t.kr);
+  for (uint32_t row = first; row < n; row += step) {
+    const int4 c = __ldg(t.coords + row);
+    if (k333)
+      subm_hash_k333(c, row, t);
+    else
+      subm_row_taps<false>(c, row, t,
+                           [&](uint32_t key) { return hash_lookup(t.table, t.mask, key); });
+  }
 }
 
-// The output cell that input coordinate c reaches through tap k of a strided conv, if any.
-__device__ __forceinline__ bool tap_output_cell(const int4 c, int k, const Grid3& gout,
-                                                const Kernel3& kr, uint32_t* cell) {
-  const int k2 = k % kr.k[2], k1 = (k / kr.k[2]) % kr.k[1], k0 = k / (kr.k[2] * kr.k[1]);
-  const int v0 = c.y + kr.p[0] - k0 * kr.d[0];
-  const int v1 = c.z + kr.p[1] - k1 * kr.d[1];
-  const int v2 = c.w + kr.p[2] - k2 * kr.d[2];
-  if (v0 < 0 || v1 < 0 || v2 < 0 || !stride_divides(v0, kr.s[0], kr.sh[0]) ||
-      !stride_divides(v1, kr.s[1], kr.sh[1]) || !stride_divides(v2, kr.s[2], kr.sh[2]))
-    return false;
-  const int o0 = stride_quotient(v0, kr.s[0], kr.sh[0]), o1 = stride_quotient(v1, kr.s[1], kr.sh[1]),
-            o2 = stride_quotient(v2, kr.s[2], kr.sh[2]);
-  if (o0 >= gout.g[0] || o1 >= gout.g[1] || o2 >= gout.g[2]) return false;
-  *cell = voxel_key(c.x, o0, o1, o2, gout);
-  return true;
+// Rows in cell order: a warp's lookups of one tap fall into the same or adjacent bitmap words.
+__device__ __forceinline__ void task_subm_rank(const RuleTask& t, uint32_t first, uint32_t step) {
+  const uint32_t n = task_rows(t);
+  const bool k333 = is_k333(t.kr);
+  auto look = [&](uint32_t key) { return rank_lookup(t.ws.bitmap, t.ws.prefix, key, t.cap); };
+  for (uint32_t row = first; row < n; row += step) {
+    const int4 c = __ldg(t.coords + row);
+    if (k333) subm_row_taps<true>(c, row, t, look);
+    else subm_row_taps<false>(c, row, t, look);
+  }
 }
 
+// ------------------------------------------------------------- strided maps: mark
 // Visits the output cells one input row reaches: for every axis only the taps with
 // (c + pad - k*dil) divisible by the stride and inside the output grid survive, so
 // the nest below does ~14 divisions per row instead of 81, and `visit` runs once
@@ -174,44 +228,39 @@ __device__ __forceinline__ AxisRange output_range(int c, int a, const Grid3& gou
   r.lo = t <= 0 ? 0 : stride_quotient(t + kr.s[a] - 1, kr.s[a], kr.sh[a]);
   return r;
 }
-__host__ __device__ inline bool unit_dilation(const Kernel3& kr) {
-  return kr.d[0] == 1 && kr.d[1] == 1 && kr.d[2] == 1;
+
+// Up to kvol inputs reach the same cells: look before the atomic, most find them set.
+__device__ __forceinline__ void mark_word(const DownWs& ws, uint32_t word, uint32_t bits) {
+  uint32_t* p = ws.bitmap + word;
+  if ((*(volatile uint32_t*)p & bits) != bits) atomicOr(p, bits);
 }
 
-__global__ void down_mark_kernel(const int4* __restrict__ coords, const uint32_t* n_ptr,
-                                 uint32_t cap, Grid3 gin, Grid3 gout, Kernel3 kr,
-                                 uint32_t* bitmap) {
-  const uint32_t n = min(*n_ptr, cap);
+__device__ __forceinline__ void task_mark_rows(const RuleTask& t, uint32_t first, uint32_t step) {
+  const uint32_t n = task_rows(t);
+  const Kernel3& kr = t.kr;
   const bool unit = unit_dilation(kr) && kr.k[2] <= 32 * kr.s[2];
-  for (uint32_t row = blockIdx.x * blockDim.x + threadIdx.x; row < n;
-       row += gridDim.x * blockDim.x) {
-    const int4 c = __ldg(coords + row);
-    if ((unsigned)c.x >= (unsigned)gin.batch) continue;
+  for (uint32_t row = first; row < n; row += step) {
+    const int4 c = __ldg(t.coords + row);
+    if ((unsigned)c.x >= (unsigned)t.gin.batch) continue;
     if (unit) {
       // the reached cells are a box; its cells along the innermost axis are adjacent bits,
       // set with one atomic (two when the run crosses a word)
-      const AxisRange r0 = output_range(c.y, 0, gout, kr), r1 = output_range(c.z, 1, gout, kr),
-                      r2 = output_range(c.w, 2, gout, kr);
+      const AxisRange r0 = output_range(c.y, 0, t.gout, kr), r1 = output_range(c.z, 1, t.gout, kr),
+                      r2 = output_range(c.w, 2, t.gout, kr);
       if (r2.lo > r2.hi) continue;
       const uint32_t nbits = (uint32_t)(r2.hi - r2.lo + 1);
       for (int o0 = r0.lo; o0 <= r0.hi; ++o0)
         for (int o1 = r1.lo; o1 <= r1.hi; ++o1) {
-          const uint32_t cell = voxel_key(c.x, o0, o1, r2.lo, gout);
+          const uint32_t cell = voxel_key(c.x, o0, o1, r2.lo, t.gout);
           const unsigned long long run =
               (nbits >= 64u ? ~0ull : (1ull << nbits) - 1ull) << (cell & 31u);
-          uint32_t* word = bitmap + (cell >> 5);
-          const uint32_t m0 = (uint32_t)run, m1 = (uint32_t)(run >> 32);
-          // up to kvol inputs reach the same cells: look before the atomic, most find them set
-          if ((*(volatile uint32_t*)word & m0) != m0) atomicOr(word, m0);
-          if (m1 && (*(volatile uint32_t*)(word + 1) & m1) != m1) atomicOr(word + 1, m1);
+          mark_word(t.ws, cell >> 5, (uint32_t)run);
+          if (run >> 32) mark_word(t.ws, (cell >> 5) + 1, (uint32_t)(run >> 32));
         }
       continue;
     }
-    for_each_output(c, gout, kr, [&](int, uint32_t cell) {
-      const uint32_t bit = 1u << (cell & 31);
-      uint32_t* word = bitmap + (cell >> 5);
-      if (!(*(volatile uint32_t*)word & bit)) atomicOr(word, bit);
-    });
+    for_each_output(c, t.gout, kr,
+                    [&](int, uint32_t cell) { mark_word(t.ws, cell >> 5, 1u << (cell & 31)); });
   }
 }
 
@@ -240,30 +289,34 @@ __device__ __forceinline__ unsigned long long line_bits64(const uint32_t* __rest
 // beyond the capacity of the input rows (an overflow the rulebook that made them has already
 // reported) count as set.
 constexpr int kMarkCells = 16;
-__global__ void down_mark_ranked_kernel(const uint32_t* __restrict__ in_bitmap, uint32_t in_words,
-                                        Grid3 gin, Grid3 gout, Kernel3 kr,
-                                        uint32_t* __restrict__ out_bitmap) {
-  const int segs = (gout.g[2] + kMarkCells - 1) / kMarkCells;
-  const unsigned long long lines = (unsigned long long)gout.batch * gout.g[0] * gout.g[1];
+__device__ __forceinline__ void task_mark_bitmap(const RuleTask& t, uint32_t first, uint32_t step) {
+  const Grid3 &gin = t.gin, &gout = t.gout;
+  const Kernel3& kr = t.kr;
+  const uint32_t segs = (uint32_t)(gout.g[2] + kMarkCells - 1) / kMarkCells;
+  const unsigned long long items =
+      (unsigned long long)gout.batch * gout.g[0] * gout.g[1] * segs;
   const unsigned long long kmask = (1ull << kr.k[2]) - 1ull;
-  for (unsigned long long item = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
-       item < lines * segs; item += (unsigned long long)gridDim.x * blockDim.x) {
-    const unsigned long long line = item / segs;
-    const int ox0 = (int)(item - line * segs) * kMarkCells;
+  for (unsigned long long item = first; item < items; item += step) {
+    // fewer than 2^32 cells (checked by the callers), so 32-bit arithmetic holds
+    const uint32_t line = (uint32_t)item / segs;
+    const int ox0 = (int)((uint32_t)item - line * segs) * kMarkCells;
     const int ncell = min(kMarkCells, gout.g[2] - ox0);
-    const int o1 = (int)(line % gout.g[1]);
-    const int o0 = (int)((line / gout.g[1]) % gout.g[0]);
-    const int b = (int)(line / ((unsigned long long)gout.g[1] * gout.g[0]));
+    const uint32_t plane = line / (uint32_t)gout.g[1];
+    const int o1 = (int)(line - plane * (uint32_t)gout.g[1]);
+    const int b = (int)(plane / (uint32_t)gout.g[0]);
+    const int o0 = (int)(plane - (uint32_t)b * (uint32_t)gout.g[0]);
     const int x0 = ox0 * kr.s[2] - kr.p[2];
-    const int count = (ncell - 1) * kr.s[2] + kr.k[2];  // <= 64 (checked by the launcher)
+    const int count = (ncell - 1) * kr.s[2] + kr.k[2];  // <= 64 (mark_from_bitmap)
     unsigned long long win = 0ull;
     for (int k0 = 0; k0 < kr.k[0]; ++k0) {
       const int i0 = o0 * kr.s[0] - kr.p[0] + k0;
       if ((unsigned)i0 >= (unsigned)gin.g[0]) continue;
+#pragma unroll 3
       for (int k1 = 0; k1 < kr.k[1]; ++k1) {
         const int i1 = o1 * kr.s[1] - kr.p[1] + k1;
         if ((unsigned)i1 >= (unsigned)gin.g[1]) continue;
-        win |= line_bits64(in_bitmap, in_words, voxel_key(b, i0, i1, 0, gin), x0, count, gin.g[2]);
+        win |= line_bits64(t.in_ws.bitmap, t.in_ws.words, voxel_key(b, i0, i1, 0, gin), x0,
+                           count, gin.g[2]);
       }
     }
     if (!win) continue;
@@ -272,312 +325,370 @@ __global__ void down_mark_ranked_kernel(const uint32_t* __restrict__ in_bitmap, 
     for (int i = 0; i < kMarkCells; ++i)
       if (i < ncell && ((win >> (i * kr.s[2])) & kmask)) r |= 1u << i;
     if (!r) continue;
-    const uint32_t cell = (uint32_t)(line * gout.g[2]) + (uint32_t)ox0;
+    const uint32_t cell = line * (uint32_t)gout.g[2] + (uint32_t)ox0;
     const unsigned long long run = (unsigned long long)r << (cell & 31u);
-    atomicOr(out_bitmap + (cell >> 5), (uint32_t)run);
-    if (run >> 32) atomicOr(out_bitmap + (cell >> 5) + 1, (uint32_t)(run >> 32));
+    atomicOr(t.ws.bitmap + (cell >> 5), (uint32_t)run);
+    if (run >> 32) atomicOr(t.ws.bitmap + (cell >> 5) + 1, (uint32_t)(run >> 32));
   }
 }
 
-// Row of an output cell from the bitmap and its (global) popcount prefix, -1 if
-// the cell is not an output or lies beyond the capacity.
-__device__ __forceinline__ int32_t rank_lookup(const uint32_t* __restrict__ bitmap,
-                                               const uint32_t* __restrict__ prefix,
-                                               uint32_t cell, uint32_t cap) {
-  const uint32_t bits = __ldg(bitmap + (cell >> 5));
-  const uint32_t b = cell & 31u;
-  if (!((bits >> b) & 1u)) return -1;
-  const uint32_t row = __ldg(prefix + (cell >> 5)) + __popc(bits & ((1u << b) - 1u));
-  return row < cap ? (int32_t)row : -1;
+// ------------------------------------------------------------- strided maps: emit
+struct EmitShared {
+  uint32_t before[kScanWords];  // set bits of the block's words before each
+  uint32_t word[kScanWords];
+  int4 cell[kScanWords];        // first cell of each word
+  uint32_t blk;
+  uint32_t warp_total[kTaskWarps];
+  uint32_t back[kTaskWarps];
+};
+
+// Set bits of all blocks before `blk`.  Every block publishes its count (plus 1) and adds it, with
+// an arrival, to the total of its group of 32; a block needs the totals of the groups before its own
+// and the counts of at most 31 blocks.  All of them are loaded at once (a batch of 8 frames has 21 000
+// blocks and 665 groups: 6 loads a thread); the chain of a look-back from block to block took 10 us
+// on 2 700 blocks that start together.  What is waited for was drawn from the same counter
+// before, so it is running or has finished; the wait is bounded like every other.
+__device__ __forceinline__ uint32_t bits_before(const RuleTask& t, uint32_t blk, uint32_t total,
+                                                EmitShared& sh) {
+  unsigned long long* groups = t.ws.scan_groups();
+  uint32_t* own = t.ws.scan_counts();
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, group = blk / kScanGroup;
+  if (threadIdx.x == 0) {
+    *(volatile uint32_t*)(own + blk) = total + 1u;
+    atomicAdd(groups + group, (1ull << 40) | total);
+  }
+  uint32_t sum = 0, spin = 0;
+  auto give_up = [&]() {
+    if (++spin < 1u << 21) {
+      __nanosleep(32);
+      return false;
+    }
+    set_status(t.status, SPCONVB_ST_TIMEOUT, 7u);
+    return true;
+  };
+  for (uint32_t i = threadIdx.x; i < group; i += kTaskThreads) {
+    unsigned long long v;
+    while (((v = *(volatile unsigned long long*)(groups + i)) >> 40) != kScanGroup)
+      if (give_up()) break;
+    sum += (uint32_t)v;  // fewer than 2^32 cells
+  }
+  const uint32_t mate = group * kScanGroup + threadIdx.x;
+  if (mate < blk && threadIdx.x < kScanGroup) {
+    uint32_t v;
+    while ((v = *(volatile uint32_t*)(own + mate)) == 0u)
+      if (give_up()) {
+        v = 1u;
+        break;
+      }
+    sum += v - 1u;
+  }
+  sum = __reduce_add_sync(0xffffffffu, sum);
+  if (lane == 0) sh.back[warp] = sum;
+  __syncthreads();
+  sum = 0;
+#pragma unroll
+  for (int w = 0; w < kTaskWarps; ++w) sum += sh.back[w];
+  return sum;
 }
 
-// Per block of kScanWordsPerBlock words: exclusive scan of popcounts.
-__global__ void __launch_bounds__(kScanThreads) down_scan_kernel(DownWs ws) {
-  __shared__ uint32_t warp_sums[kScanThreads / 32];
-  const uint32_t w = blockIdx.x * kScanWordsPerBlock + threadIdx.x;
-  const uint32_t local = w < ws.words ? __popc(ws.bitmap[w]) : 0u;
-  uint32_t incl = local;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+// Ranks every set bit of one scan block: writes the rank of each word's first bit, the output
+// coordinates and, for a map that is scattered into afterwards, the -1 of its rows; the last
+// block publishes the count.  One pass over the bitmap; block numbers are drawn in the order blocks
+// start, so that a wait can only be for a block that is running.
+__device__ __forceinline__ void task_emit(const RuleTask& t, EmitShared& sh) {
+  const DownWs& ws = t.ws;
+  const Grid3& gout = t.gout;
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  if (threadIdx.x == 0) sh.blk = atomicAdd(ws.scan_ticket(), 1u);
+  __syncthreads();
+  const uint32_t blk = sh.blk;
+  const uint32_t w0 = blk * kScanWords + threadIdx.x;
+  const uint32_t bits = w0 < ws.words ? ws.bitmap[w0] : 0u;
+  uint32_t incl = (uint32_t)__popc(bits);
 #pragma unroll
   for (int d = 1; d < 32; d <<= 1) {
-    uint32_t v = __shfl_up_sync(0xffffffffu, incl, d);
-    if (lane >= d) incl += v;
+    const uint32_t v = __shfl_up_sync(0xffffffffu, incl, d);
+    if ((int)lane >= d) incl += v;
   }
-  if (lane == 31) warp_sums[warp] = incl;
+  if (lane == 31u) sh.warp_total[warp] = incl;
   __syncthreads();
-  if (warp == 0) {
-    uint32_t v = warp_sums[lane];
-    uint32_t s = v;
+  uint32_t total = 0, before = incl - (uint32_t)__popc(bits);
 #pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      uint32_t t = __shfl_up_sync(0xffffffffu, s, d);
-      if (lane >= d) s += t;
-    }
-    warp_sums[lane] = s - v;  // exclusive
-    if (lane == 31) ws.block_sums[blockIdx.x] = s;
+  for (int i = 0; i < kTaskWarps; ++i) {
+    if (i < (int)warp) before += sh.warp_total[i];
+    total += sh.warp_total[i];
   }
-  __syncthreads();
-  if (w < ws.words) ws.prefix[w] = warp_sums[warp] + incl - local;
-}
-
-// Ranks every set bit: writes the output coordinate, makes the prefix global, and the
-// last block publishes the count.  No atomics.
-__global__ void __launch_bounds__(kScanThreads)
-down_emit_kernel(DownWs ws, Grid3 gout, int4* __restrict__ out_coords, uint32_t* n_out_ptr,
-                 uint32_t cap_out, uint32_t* status) {
-  __shared__ uint32_t red[32];
-  __shared__ uint32_t s_base;
-  uint32_t part = 0;
-  for (uint32_t i = threadIdx.x; i < blockIdx.x; i += blockDim.x) part += ws.block_sums[i];
+  sh.before[threadIdx.x] = before;
+  sh.word[threadIdx.x] = bits;
+  if (bits) {
+    uint32_t c = w0 << 5;
+    uint32_t q = c / (uint32_t)gout.g[2];
+    const int x = (int)(c - q * (uint32_t)gout.g[2]);
+    c = q / (uint32_t)gout.g[1];
+    const int y = (int)(q - c * (uint32_t)gout.g[1]);
+    q = c / (uint32_t)gout.g[0];
+    sh.cell[threadIdx.x] = make_int4((int)q, (int)(c - q * (uint32_t)gout.g[0]), y, x);
+  }
+  const uint32_t base = bits_before(t, blk, total, sh);
+  if (threadIdx.x == 0 && blk == ws.blocks - 1) {
+    if (base + total > t.cap) set_status(t.status, SPCONVB_ST_OVERFLOW, base + total);
+    *t.n_out = min(base + total, t.cap);
+  }
+  if (w0 < ws.words) ws.prefix[w0] = base + before;
+  // One thread per row: the row's word is the last one with at most that many bits before it,
+  // its bit is found by halving.  The stores coalesce and a block takes as long as its rows,
+  // which a lidar scene packs into few words: walking the words, a warp or a lane at a time, took
+  // 30-90 us on the dense grids of the later stages, blocks of 512 words still 45.
+  const uint32_t rows = base < t.cap ? min(total, t.cap - base) : 0u;
+  const int kvol = t.map ? t.kr.k[0] * t.kr.k[1] * t.kr.k[2] : 0;
+#pragma unroll 1
+  for (uint32_t r = threadIdx.x; r < rows; r += kTaskThreads) {
+    uint32_t w = 0;
 #pragma unroll
-  for (int d = 16; d > 0; d >>= 1) part += __shfl_xor_sync(0xffffffffu, part, d);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = part;
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    uint32_t v = red[threadIdx.x];
+    for (uint32_t half = kScanWords / 2; half > 0; half >>= 1)
+      if (sh.before[w + half] <= r) w += half;
+    uint32_t left = sh.word[w], nth = r - sh.before[w];
+    int4 c = sh.cell[w];
 #pragma unroll
-    for (int d = 16; d > 0; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
-    if (threadIdx.x == 0) {
-      s_base = v;
-      if (blockIdx.x == gridDim.x - 1) {
-        uint32_t total = v + ws.block_sums[blockIdx.x];
-        if (total > cap_out) set_status(status, SPCONVB_ST_OVERFLOW, total);
-        *n_out_ptr = min(total, cap_out);
+    for (int half = 16; half > 0; half >>= 1) {
+      const uint32_t low = (uint32_t)__popc(left & ((1u << half) - 1u));
+      if (nth >= low) {
+        nth -= low;
+        left >>= half;
+        c.w += half;
       }
     }
-  }
-  __syncthreads();
-  // Every thread reads one word and makes its prefix global; then the warp goes through its
-  // non-empty words together, one lane per bit: the rows of a word are consecutive, so the
-  // coordinate stores of a word coalesce, and no lane loops over the bits of a dense word
-  // while the others wait.
-  const uint32_t w = blockIdx.x * kScanWordsPerBlock + threadIdx.x;
-  const uint32_t lane = threadIdx.x & 31u;
-  uint32_t bits = 0, row0 = 0;
-  int c2 = 0, c1 = 0, c0 = 0, bq = 0;
-  if (w < ws.words) {
-    bits = ws.bitmap[w];
-    row0 = s_base + ws.prefix[w];
-    ws.prefix[w] = row0;
-    if (bits) {  // the word's first cell
-      uint32_t t = w << 5;
-      c2 = t % gout.g[2]; t /= gout.g[2];
-      c1 = t % gout.g[1]; t /= gout.g[1];
-      c0 = t % gout.g[0]; t /= gout.g[0];
-      bq = (int)t;
-    }
-  }
-  uint32_t nonempty = __ballot_sync(0xffffffffu, bits != 0u);
-  while (nonempty) {
-    const int src = __ffs(nonempty) - 1;
-    nonempty &= nonempty - 1;
-    const uint32_t wb = __shfl_sync(0xffffffffu, bits, src);
-    const uint32_t r0 = __shfl_sync(0xffffffffu, row0, src);
-    int x = __shfl_sync(0xffffffffu, c2, src) + (int)lane;
-    int y = __shfl_sync(0xffffffffu, c1, src);
-    int z = __shfl_sync(0xffffffffu, c0, src);
-    int b = __shfl_sync(0xffffffffu, bq, src);
-    if ((wb >> lane) & 1u) {
-      const uint32_t row = r0 + __popc(wb & ((1u << lane) - 1u));
-      while (x >= gout.g[2]) {
-        x -= gout.g[2];
-        if (++y >= gout.g[1]) {
-          y = 0;
-          if (++z >= gout.g[0]) { z = 0; ++b; }
-        }
+    while (c.w >= gout.g[2]) {
+      c.w -= gout.g[2];
+      if (++c.z >= gout.g[1]) {
+        c.z = 0;
+        if (++c.y >= gout.g[0]) { c.y = 0; ++c.x; }
       }
-      if (row < cap_out) out_coords[row] = make_int4(b, z, y, x);
+    }
+    t.out_coords[base + r] = c;
+    int32_t* m = t.map + base + r;
+#pragma unroll 9
+    for (int k = 0; k < kvol; ++k) {
+      *m = -1;
+      m += t.cap;
     }
   }
 }
 
-// The map rows of the outputs start as "no input" (-1); the scatter kernel then
-// writes the pairs that exist.  16-byte stores where the row range allows.
-__global__ void map_fill_kernel(const uint32_t* n_out_ptr, uint32_t cap_out, int kvol,
-                                int32_t* __restrict__ map) {
-  const uint32_t n = min(*n_out_ptr, cap_out);
-  const uint32_t n4 = (n + 3) / 4;  // int4 groups per tap (cap_out rows are 16-byte aligned
-                                    // only when cap_out % 4 == 0; else fall back to scalars)
-  const bool vec = (cap_out & 3u) == 0 && (((uintptr_t)map) & 15u) == 0;
-  const unsigned long long work = (unsigned long long)kvol * (vec ? n4 : n);
-  for (unsigned long long idx = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
-       idx < work; idx += (unsigned long long)gridDim.x * blockDim.x) {
-    if (vec) {
-      const uint32_t k = (uint32_t)(idx / n4), g4 = (uint32_t)(idx - (unsigned long long)k * n4);
-      ((int4*)(map + (size_t)k * cap_out))[g4] = make_int4(-1, -1, -1, -1);
-    } else {
-      const uint32_t k = (uint32_t)(idx / n), r = (uint32_t)(idx - (unsigned long long)k * n);
-      map[(size_t)k * cap_out + r] = -1;
-    }
-  }
-}
-
-// Input-stationary fill of the output-stationary map: every (input row, tap) pair
-// finds its output row by rank and writes itself there.  One rank query (two
-// cached loads) per existing pair, instead of kvol hash probes per output row.
-__global__ void down_scatter_kernel(const int4* __restrict__ coords, const uint32_t* n_ptr,
-                                    uint32_t cap, Grid3 gin, Grid3 gout, Kernel3 kr, DownWs ws,
-                                    uint32_t cap_out, int32_t* __restrict__ map) {
-  const uint32_t n = min(*n_ptr, cap);
+// ------------------------------------------------------------- strided maps: fill
+// Input-stationary fill of the output-stationary map: every (input row, tap) pair finds its
+// output row by rank and writes itself there.  The cells an input reaches were marked by it, so
+// with dilation 1 nothing is tested: word and rank are loaded side by side.
+__device__ __forceinline__ void task_scatter(const RuleTask& t, uint32_t first, uint32_t step) {
+  const uint32_t n = task_rows(t);
+  const Kernel3& kr = t.kr;
+  const uint32_t cap_out = t.map_cap;
   const bool unit = unit_dilation(kr);
-  for (uint32_t row = blockIdx.x * blockDim.x + threadIdx.x; row < n;
-       row += gridDim.x * blockDim.x) {
-    const int4 c = __ldg(coords + row);
-    if ((unsigned)c.x >= (unsigned)gin.batch) continue;
+  for (uint32_t row = first; row < n; row += step) {
+    const int4 c = __ldg(t.coords + row);
+    if ((unsigned)c.x >= (unsigned)t.gin.batch) continue;
     if (unit) {
-      const AxisRange r0 = output_range(c.y, 0, gout, kr), r1 = output_range(c.z, 1, gout, kr),
-                      r2 = output_range(c.w, 2, gout, kr);
+      const AxisRange r0 = output_range(c.y, 0, t.gout, kr), r1 = output_range(c.z, 1, t.gout, kr),
+                      r2 = output_range(c.w, 2, t.gout, kr);
       for (int o0 = r0.lo; o0 <= r0.hi; ++o0) {
         const int k0 = c.y + kr.p[0] - o0 * kr.s[0];
         for (int o1 = r1.lo; o1 <= r1.hi; ++o1) {
           const int k01 = k0 * kr.k[1] + (c.z + kr.p[1] - o1 * kr.s[1]);
+#pragma unroll 2
           for (int o2 = r2.lo; o2 <= r2.hi; ++o2) {
             const int k = k01 * kr.k[2] + (c.w + kr.p[2] - o2 * kr.s[2]);
-            const int32_t o =
-                rank_lookup(ws.bitmap, ws.prefix, voxel_key(c.x, o0, o1, o2, gout), cap_out);
-            if (o >= 0) map[(size_t)k * cap_out + o] = (int32_t)row;
+            const uint32_t cell = voxel_key(c.x, o0, o1, o2, t.gout);
+            const uint32_t o = __ldg(t.ws.prefix + (cell >> 5)) +
+                               __popc(__ldg(t.ws.bitmap + (cell >> 5)) & ((1u << (cell & 31u)) - 1u));
+            if (o < cap_out) t.map[(size_t)k * cap_out + o] = (int32_t)row;
           }
         }
       }
       continue;
     }
-    for_each_output(c, gout, kr, [&](int k, uint32_t cell) {
-      const int32_t o = rank_lookup(ws.bitmap, ws.prefix, cell, cap_out);
-      if (o >= 0) map[(size_t)k * cap_out + o] = (int32_t)row;
+    for_each_output(c, t.gout, kr, [&](int k, uint32_t cell) {
+      const int32_t o = rank_lookup(t.ws.bitmap, t.ws.prefix, cell, cap_out);
+      if (o >= 0) t.map[(size_t)k * cap_out + o] = (int32_t)row;
     });
-  }
-}
-
-// Optional: the outputs' hash table, for callers that want one.
-__global__ void hash_rows_kernel(const int4* __restrict__ coords, const uint32_t* n_ptr,
-                                 uint32_t cap, Grid3 g, uint64_t* table, uint32_t mask,
-                                 uint32_t* status) {
-  const uint32_t n = min(*n_ptr, cap);
-  for (uint32_t row = blockIdx.x * blockDim.x + threadIdx.x; row < n;
-       row += gridDim.x * blockDim.x) {
-    const int4 c = __ldg(coords + row);
-    hash_insert(table, mask, voxel_key(c.x, c.y, c.z, c.w, g), row, status);
-  }
-}
-
-// Submanifold map of a coordinate set that came out of down_map: neighbours are
-// found by rank in that set's bitmap, no hash table involved.  One thread per row;
-// rows are in cell order, so a warp's lookups of one tap fall into the same or
-// adjacent bitmap words and its map stores coalesce.
-template <bool K333>
-__global__ void subm_ranked_kernel(const int4* __restrict__ coords, const uint32_t* n_ptr,
-                                   uint32_t cap, Grid3 g, Kernel3 kr, DownWs ws,
-                                   int32_t* __restrict__ map) {
-  const uint32_t n = min(*n_ptr, cap);
-  for (uint32_t row = blockIdx.x * blockDim.x + threadIdx.x; row < n;
-       row += gridDim.x * blockDim.x)
-    subm_row_taps<K333>(__ldg(coords + row), row, g, kr, cap, map, [&](uint32_t key) {
-      return rank_lookup(ws.bitmap, ws.prefix, key, cap);
-    });
-}
-
-// Blocks for one thread per row: small blocks, so that a few thousand rows still spread
-// over the SMs, capped at a few waves (the kernels stride).
-static int row_blocks(uint32_t rows, int threads) {
-  unsigned long long b = ((unsigned long long)rows + threads - 1) / threads;
-  const unsigned long long most = (unsigned long long)kSmCount * 16;
-  if (b > most) b = most;
-  if (b < 1) b = 1;
-  return (int)b;
-}
-
-static bool is_k333(const Kernel3& kr) {
-  return kr.k[0] == 3 && kr.k[1] == 3 && kr.k[2] == 3 && kr.d[0] == 1 && kr.d[1] == 1 &&
-         kr.d[2] == 1;
-}
-
-static void set_stride_shifts(Kernel3& kr) {
-  for (int a = 0; a < 3; ++a) {
-    kr.sh[a] = -1;
-    for (int b = 0; b < 16; ++b)
-      if (kr.s[a] == (1 << b)) kr.sh[a] = b;
   }
 }
 
 // Output-stationary form of the strided map, for inputs that were themselves made by a
-// strided rulebook (their bitmap and rank prefix exist): one thread per output row walks the
+// strided rulebook (their bitmap and ranks exist): one thread per output row walks the
 // taps in tap order, finds the input cell of each (out * stride - pad + tap * dilation) and
 // ranks it in the input's bitmap.  Every map entry is written exactly once, so there is no
 // fill pass, and a warp's stores of one tap land in one or two lines of map[k][.].
 template <bool K333>
-__global__ void down_gather_ranked_kernel(const int4* __restrict__ out_coords,
-                                          const uint32_t* n_out_ptr, uint32_t cap_out, Grid3 gin,
-                                          Kernel3 kr, DownWs in_ws, uint32_t cap_in,
-                                          int32_t* __restrict__ map) {
-  const uint32_t n = min(*n_out_ptr, cap_out);
-  for (uint32_t row = blockIdx.x * blockDim.x + threadIdx.x; row < n;
-       row += gridDim.x * blockDim.x) {
-    const int4 c = __ldg(out_coords + row);
-    int32_t* dst = map + row;
-    if (K333) {
-      // 3x3x3, dilation 1: the taps unrolled, 27 independent rank lookups
-      const bool bok = (unsigned)c.x < (unsigned)gin.batch;
+__device__ __forceinline__ void gather_row(const int4 c, uint32_t row, const RuleTask& t) {
+  const Grid3& gin = t.gin;
+  const Kernel3& kr = t.kr;
+  const int K0 = K333 ? 3 : kr.k[0], K1 = K333 ? 3 : kr.k[1], K2 = K333 ? 3 : kr.k[2];
+  int32_t* dst = t.map + row;
+  const bool bok = (unsigned)c.x < (unsigned)gin.batch;
 #pragma unroll
-      for (int k0 = 0; k0 < 3; ++k0) {
-        const int p0 = c.y * kr.s[0] - kr.p[0] + k0;
-        const bool ok0 = bok && (unsigned)p0 < (unsigned)gin.g[0];
+  for (int k0 = 0; k0 < K0; ++k0) {
+    const int p0 = c.y * kr.s[0] - kr.p[0] + k0 * (K333 ? 1 : kr.d[0]);
+    const bool ok0 = bok && (unsigned)p0 < (unsigned)gin.g[0];
 #pragma unroll
-        for (int k1 = 0; k1 < 3; ++k1) {
-          const int p1 = c.z * kr.s[1] - kr.p[1] + k1;
-          const bool ok1 = ok0 && (unsigned)p1 < (unsigned)gin.g[1];
+    for (int k1 = 0; k1 < K1; ++k1) {
+      const int p1 = c.z * kr.s[1] - kr.p[1] + k1 * (K333 ? 1 : kr.d[1]);
+      const bool ok1 = ok0 && (unsigned)p1 < (unsigned)gin.g[1];
 #pragma unroll
-          for (int k2 = 0; k2 < 3; ++k2) {
-            const int p2 = c.w * kr.s[2] - kr.p[2] + k2;
-            int32_t r = -1;
-            if (ok1 && (unsigned)p2 < (unsigned)gin.g[2])
-              r = rank_lookup(in_ws.bitmap, in_ws.prefix, voxel_key(c.x, p0, p1, p2, gin), cap_in);
-            *dst = r;
-            dst += cap_out;
-          }
-        }
-      }
-      continue;
-    }
-    for (int k0 = 0; k0 < kr.k[0]; ++k0) {
-      const int p0 = c.y * kr.s[0] - kr.p[0] + k0 * kr.d[0];
-      const bool ok0 = (unsigned)p0 < (unsigned)gin.g[0];
-      for (int k1 = 0; k1 < kr.k[1]; ++k1) {
-        const int p1 = c.z * kr.s[1] - kr.p[1] + k1 * kr.d[1];
-        const bool ok1 = ok0 && (unsigned)p1 < (unsigned)gin.g[1];
-#pragma unroll 3
-        for (int k2 = 0; k2 < kr.k[2]; ++k2) {
-          const int p2 = c.w * kr.s[2] - kr.p[2] + k2 * kr.d[2];
-          int32_t r = -1;
-          if (ok1 && (unsigned)p2 < (unsigned)gin.g[2])
-            r = rank_lookup(in_ws.bitmap, in_ws.prefix, voxel_key(c.x, p0, p1, p2, gin), cap_in);
-          *dst = r;
-          dst += cap_out;
-        }
+      for (int k2 = 0; k2 < K2; ++k2) {
+        const int p2 = c.w * kr.s[2] - kr.p[2] + k2 * (K333 ? 1 : kr.d[2]);
+        int32_t r = -1;
+        if (ok1 && (unsigned)p2 < (unsigned)gin.g[2])
+          r = rank_lookup(t.in_ws.bitmap, t.in_ws.prefix, voxel_key(c.x, p0, p1, p2, gin),
+                          t.other_cap);
+        *dst = r;
+        dst += t.cap;
       }
     }
   }
 }
 
-// Fixed-size grids: a multiple of the SM count, independent of the row count.
-static int flat_blocks(unsigned long long work_cap) {
-  unsigned long long b = (work_cap + kThreads - 1) / kThreads;
-  const unsigned long long most = (unsigned long long)kSmCount * 8;
-  if (b > most) b = most;
-  if (b < 1) b = 1;
-  return (int)b;
+__device__ __forceinline__ void task_gather(const RuleTask& t, uint32_t first, uint32_t step) {
+  const uint32_t n = task_rows(t);
+  const bool k333 = is_k333(t.kr);
+  for (uint32_t row = first; row < n; row += step) {
+    const int4 c = __ldg(t.coords + row);
+    if (k333) gather_row<true>(c, row, t);
+    else gather_row<false>(c, row, t);
+  }
 }
 
-static bool grid_fits(const int32_t g[3], int batch) {
+// Map of an inverse (transposed) convolution: it runs over the pairs of a strided rulebook with
+// input and output swapped, so its outputs are that rulebook's input rows and map[k][i] is the
+// strided output row that input row i reaches through tap k.  One thread per (row, tap), rows
+// fastest: coalesced stores of map[k][row].
+__device__ __forceinline__ void task_inverse(const RuleTask& t, uint32_t first, uint32_t step) {
+  const uint32_t n = task_rows(t);
+  const Kernel3& kr = t.kr;
+  const int kvol = kr.k[0] * kr.k[1] * kr.k[2];
+  const unsigned long long work = (unsigned long long)n * kvol;
+  for (unsigned long long idx = first; idx < work; idx += step) {
+    const int k = (int)(idx / n);
+    const uint32_t row = (uint32_t)(idx - (unsigned long long)k * n);
+    const int4 c = __ldg(t.coords + row);
+    const int k2 = k % kr.k[2], k1 = (k / kr.k[2]) % kr.k[1], k0 = k / (kr.k[2] * kr.k[1]);
+    const int v0 = c.y + kr.p[0] - k0 * kr.d[0], v1 = c.z + kr.p[1] - k1 * kr.d[1],
+              v2 = c.w + kr.p[2] - k2 * kr.d[2];
+    int32_t o = -1;
+    if ((unsigned)c.x < (unsigned)t.gin.batch && v0 >= 0 && v1 >= 0 && v2 >= 0 &&
+        stride_divides(v0, kr.s[0], kr.sh[0]) && stride_divides(v1, kr.s[1], kr.sh[1]) &&
+        stride_divides(v2, kr.s[2], kr.sh[2])) {
+      const int o0 = stride_quotient(v0, kr.s[0], kr.sh[0]),
+                o1 = stride_quotient(v1, kr.s[1], kr.sh[1]),
+                o2 = stride_quotient(v2, kr.s[2], kr.sh[2]);
+      if (o0 < t.gout.g[0] && o1 < t.gout.g[1] && o2 < t.gout.g[2])
+        o = rank_lookup(t.ws.bitmap, t.ws.prefix, voxel_key(c.x, o0, o1, o2, t.gout), t.other_cap);
+    }
+    t.map[(size_t)k * t.cap + row] = o;
+  }
+}
+
+// ------------------------------------------------------------------------- launch
+__global__ void __launch_bounds__(kTaskThreads, 12)
+rule_wave_kernel(const __grid_constant__ RuleWave w) {
+  __shared__ EmitShared sh;
+  // No early trigger: the blocks of the next launch would take the places of this one's later
+  // blocks and wait there (SubM map of 120 000 rows 22 us, with it 28).
+  pdl_wait();
+  uint32_t blk = blockIdx.x;
+  int i = 0;
+  while (blk >= w.t[i].blocks) {
+    blk -= w.t[i].blocks;
+    ++i;
+  }
+  // by value: its fields are read once, into registers.  Through a reference every use would be
+  // a load from the parameter space again, after each store to the map (twice the time).
+  const RuleTask t = w.t[i];
+  const uint32_t first = blk * kTaskThreads + threadIdx.x, step = t.blocks * kTaskThreads;
+  switch (t.kind) {
+    case TASK_COUNT: task_count(t); break;
+    case TASK_PAD8: task_pad8(t, first, step); break;
+    case TASK_HASH: task_hash(t, first, step); break;
+    case TASK_SUBM_HASH: task_subm_hash(t, first, step); break;
+    case TASK_SUBM_RANK: task_subm_rank(t, first, step); break;
+    case TASK_MARK_ROWS: task_mark_rows(t, first, step); break;
+    case TASK_MARK_BITMAP: task_mark_bitmap(t, first, step); break;
+    case TASK_EMIT: task_emit(t, sh); break;
+    case TASK_SCATTER: task_scatter(t, first, step); break;
+    case TASK_GATHER: task_gather(t, first, step); break;
+    case TASK_INVERSE: task_inverse(t, first, step); break;
+  }
+}
+
+bool grid_fits(const int32_t g[3], int batch) {
   if (batch < 1 || g[0] < 1 || g[1] < 1 || g[2] < 1) return false;
   unsigned long long cells = (unsigned long long)batch * g[0] * g[1] * g[2];
   return cells < 0xffffffffull;
 }
 
-static Grid3 make_grid(const int32_t g[3], int batch) {
+uint32_t down_words(const int32_t og[3], int batch) {
+  unsigned long long cells = (unsigned long long)batch * og[0] * og[1] * og[2];
+  return (uint32_t)((cells + 31) / 32);
+}
+uint32_t scan_blocks(uint32_t words) { return (words + kScanWords - 1) / kScanWords; }
+
+}  // namespace
+
+int launch_rule_wave(const RuleWave& w, cudaStream_t st) {
+  uint32_t blocks = 0;
+  for (int i = 0; i < w.count; ++i) blocks += w.t[i].blocks;
+  if (!blocks) return SPCONVB_OK;
+  SPCONVB_CUDA_TRY(launch_pdl(rule_wave_kernel, dim3(blocks), dim3(kTaskThreads), 0, st, w));
+  return SPCONVB_OK;
+}
+
+// Blocks of a task that strides: one item per thread up to 12 blocks an SM, what fits on an empty
+// GPU.  (6 an SM: SubM map of 120 000 rows 31.6 us instead of 27.1, of 234 910 ranked rows 18.2
+// instead of 13.1.)
+uint32_t task_blocks(unsigned long long items) {
+  const unsigned long long b = (items + kTaskThreads - 1) / kTaskThreads, most = kSmCount * 12;
+  return (uint32_t)(b < 1 ? 1 : b < most ? b : most);
+}
+
+uint32_t mark_bitmap_blocks(const int32_t og[3], int batch) {
+  return task_blocks((unsigned long long)batch * og[0] * og[1] *
+                     (unsigned long long)((og[2] + kMarkCells - 1) / kMarkCells));
+}
+
+Grid3 make_grid(const int32_t g[3], int batch) {
   Grid3 r;
   r.g[0] = g[0]; r.g[1] = g[1]; r.g[2] = g[2];
   r.batch = batch;
   return r;
+}
+
+Kernel3 make_kernel3(const int32_t k[3], const int32_t s[3], const int32_t p[3],
+                     const int32_t d[3]) {
+  Kernel3 kr;
+  for (int a = 0; a < 3; ++a) {
+    kr.k[a] = k[a];
+    kr.s[a] = s ? s[a] : 1;
+    kr.p[a] = p ? p[a] : 0;
+    kr.d[a] = d[a];
+    kr.sh[a] = -1;
+    for (int b = 0; b < 16; ++b)
+      if (kr.s[a] == (1 << b)) kr.sh[a] = b;
+  }
+  return kr;
+}
+
+DownWs down_ws(const int32_t og[3], int batch, const void* workspace) {
+  DownWs ws;
+  ws.words = down_words(og, batch);
+  ws.blocks = scan_blocks(ws.words);
+  ws.bitmap = (uint32_t*)workspace;
+  ws.prefix = ws.bitmap + ws.words;
+  ws.scan = ws.prefix + ws.words;
+  return ws;
+}
+
+// A thread's window of input cells has to fit 64 bits.
+bool mark_from_bitmap(const Kernel3& kr) {
+  return unit_dilation(kr) && kr.k[2] <= 32 && (kMarkCells - 1) * kr.s[2] + kr.k[2] <= 64;
 }
 
 // ------------------------------------------------- allocation-free variant
@@ -613,11 +724,33 @@ static int static_scratch_for_current_device(void** out) {
 
 using namespace spconvb;
 
+// One task as a launch of its own.
+static int launch_task(const RuleTask& t, void* stream) {
+  RuleWave w;
+  w.add(t);
+  return launch_rule_wave(w, (cudaStream_t)stream);
+}
+
+static RuleTask row_task(int32_t kind, const int32_t* coords, const uint32_t* n_ptr, uint32_t cap,
+                         uint32_t launch_rows) {
+  RuleTask t;
+  t.kind = kind;
+  t.coords = (const int4*)coords;
+  t.n_ptr = n_ptr;
+  t.cap = cap;
+  t.blocks = task_blocks(launch_rows == 0 || launch_rows > cap ? cap : launch_rows);
+  return t;
+}
+
 extern "C" {
 
+// Four slots a row up to 8 MB (a table the L2 holds many times over), two beyond: at half load
+// every second lookup of an absent cell goes on to a second dependent probe or more.  120 000
+// rows: SubM map 68 us with 2 slots a row.
 uint32_t spconvb_hash_slots(uint32_t cap_rows) {
   uint32_t s = 1024;
   while (s < 2u * cap_rows && s < 0x80000000u) s <<= 1;
+  while (s < 4u * cap_rows && s < (1u << 20)) s <<= 1;
   return s;
 }
 
@@ -634,14 +767,15 @@ int spconvb_hash_build(const int32_t* coords, const uint32_t* n_ptr, uint32_t ca
   if (!coords || !n_ptr || !table || !grid) return SPCONVB_E_ARG;
   if (slots < 8 || (slots & (slots - 1)) || slots < 2ull * cap) return SPCONVB_E_ARG;
   if (!grid_fits(grid, batch)) return SPCONVB_E_RANGE;
-  cudaStream_t st = (cudaStream_t)stream;
   if (!(flags & SPCONVB_FLAG_PREZEROED))
-    SPCONVB_CUDA_TRY(cudaMemsetAsync(table, 0, sizeof(uint64_t) * (size_t)slots, st));
-  if (launch_rows == 0 || launch_rows > cap) launch_rows = cap;
-  hash_build_kernel<<<flat_blocks(launch_rows), kThreads, 0, st>>>(
-      (const int4*)coords, n_ptr, cap, make_grid(grid, batch), table, slots - 1, status);
-  SPCONVB_LAUNCH_CHECK();
-  return SPCONVB_OK;
+    SPCONVB_CUDA_TRY(cudaMemsetAsync(table, 0, sizeof(uint64_t) * (size_t)slots,
+                                     (cudaStream_t)stream));
+  RuleTask t = row_task(TASK_HASH, coords, n_ptr, cap, launch_rows);
+  t.gin = make_grid(grid, batch);
+  t.table = table;
+  t.mask = slots - 1;
+  t.status = status;
+  return launch_task(t, stream);
 }
 
 int spconvb_subm_map(const int32_t* coords, const uint32_t* n_ptr, uint32_t cap,
@@ -652,24 +786,16 @@ int spconvb_subm_map(const int32_t* coords, const uint32_t* n_ptr, uint32_t cap,
   if (!coords || !n_ptr || !table || !map || !grid || !ksize || !dilation) return SPCONVB_E_ARG;
   if (slots < 8 || (slots & (slots - 1))) return SPCONVB_E_ARG;
   if (!grid_fits(grid, batch)) return SPCONVB_E_RANGE;
-  Kernel3 kr;
-  for (int a = 0; a < 3; ++a) {
+  for (int a = 0; a < 3; ++a)
     if (ksize[a] < 1 || !(ksize[a] & 1) || dilation[a] < 1) return SPCONVB_E_ARG;
-    kr.k[a] = ksize[a]; kr.d[a] = dilation[a]; kr.s[a] = 1; kr.p[a] = 0;
-  }
-  const int kvol = ksize[0] * ksize[1] * ksize[2];
-  if (kvol > 65535) return SPCONVB_E_ARG;
-  if (launch_rows == 0 || launch_rows > cap) launch_rows = cap;
-  constexpr int kRowThreads = 128;
-  const int blocks = row_blocks(launch_rows, kRowThreads);
-  if (is_k333(kr))
-    subm_map_kernel<true><<<blocks, kRowThreads, 0, (cudaStream_t)stream>>>(
-        (const int4*)coords, n_ptr, cap, make_grid(grid, batch), kr, table, slots - 1, map);
-  else
-    subm_map_kernel<false><<<blocks, kRowThreads, 0, (cudaStream_t)stream>>>(
-        (const int4*)coords, n_ptr, cap, make_grid(grid, batch), kr, table, slots - 1, map);
-  SPCONVB_LAUNCH_CHECK();
-  return SPCONVB_OK;
+  if (ksize[0] * ksize[1] * ksize[2] > 65535) return SPCONVB_E_ARG;
+  RuleTask t = row_task(TASK_SUBM_HASH, coords, n_ptr, cap, launch_rows);
+  t.gin = make_grid(grid, batch);
+  t.kr = make_kernel3(ksize, nullptr, nullptr, dilation);
+  t.table = (uint64_t*)table;
+  t.mask = slots - 1;
+  t.map = map;
+  return launch_task(t, stream);
 }
 
 int spconvb_subm_map_ranked(const int32_t* coords, const uint32_t* n_ptr, uint32_t cap,
@@ -681,53 +807,15 @@ int spconvb_subm_map_ranked(const int32_t* coords, const uint32_t* n_ptr, uint32
   if (!coords || !n_ptr || !down_workspace || !map || !grid || !ksize || !dilation)
     return SPCONVB_E_ARG;
   if (!grid_fits(grid, batch)) return SPCONVB_E_RANGE;
-  Kernel3 kr;
-  for (int a2 = 0; a2 < 3; ++a2) {
-    if (ksize[a2] < 1 || !(ksize[a2] & 1) || dilation[a2] < 1) return SPCONVB_E_ARG;
-    kr.k[a2] = ksize[a2]; kr.d[a2] = dilation[a2]; kr.s[a2] = 1; kr.p[a2] = 0;
-  }
-  const int kvol = ksize[0] * ksize[1] * ksize[2];
-  if (kvol > 65535) return SPCONVB_E_ARG;
-  DownWs ws;
-  ws.words = down_words(grid, batch);
-  ws.blocks = (ws.words + kScanWordsPerBlock - 1) / kScanWordsPerBlock;
-  ws.bitmap = (uint32_t*)down_workspace;
-  ws.prefix = ws.bitmap + ws.words;
-  ws.block_sums = ws.prefix + ws.words;
-  if (launch_rows == 0 || launch_rows > cap) launch_rows = cap;
-  constexpr int kRowThreads = 128;
-  const int blocks = row_blocks(launch_rows, kRowThreads);
-  if (is_k333(kr))
-    subm_ranked_kernel<true><<<blocks, kRowThreads, 0, (cudaStream_t)stream>>>(
-        (const int4*)coords, n_ptr, cap, make_grid(grid, batch), kr, ws, map);
-  else
-    subm_ranked_kernel<false><<<blocks, kRowThreads, 0, (cudaStream_t)stream>>>(
-        (const int4*)coords, n_ptr, cap, make_grid(grid, batch), kr, ws, map);
-  SPCONVB_LAUNCH_CHECK();
-  return SPCONVB_OK;
-}
-
-// Map of an inverse (transposed) convolution: it runs over the pairs of a strided
-// rulebook with input and output swapped, so its outputs are that rulebook's input rows
-// and map[k][i] is the strided output row that input row i reaches through tap k.  One
-// thread per (row, tap): the strided conv's cell arithmetic for that tap, then a rank
-// lookup in the bitmap the strided rulebook left behind.
-__global__ void inverse_map_kernel(const int4* __restrict__ coords, const uint32_t* n_ptr,
-                                   uint32_t cap, Grid3 gin, Grid3 gout, Kernel3 kr, int kvol,
-                                   DownWs ws, uint32_t cap_coarse, int32_t* __restrict__ map) {
-  const uint32_t n = min(*n_ptr, cap);
-  const unsigned long long work = (unsigned long long)n * kvol;
-  for (unsigned long long idx = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
-       idx < work; idx += (unsigned long long)gridDim.x * blockDim.x) {
-    const int k = (int)(idx / n);  // rows fastest: coalesced stores of map[k][row]
-    const uint32_t row = (uint32_t)(idx - (unsigned long long)k * n);
-    const int4 c = __ldg(coords + row);
-    int32_t o = -1;
-    uint32_t cell;
-    if ((unsigned)c.x < (unsigned)gin.batch && tap_output_cell(c, k, gout, kr, &cell))
-      o = rank_lookup(ws.bitmap, ws.prefix, cell, cap_coarse);
-    map[(size_t)k * cap + row] = o;
-  }
+  for (int a = 0; a < 3; ++a)
+    if (ksize[a] < 1 || !(ksize[a] & 1) || dilation[a] < 1) return SPCONVB_E_ARG;
+  if (ksize[0] * ksize[1] * ksize[2] > 65535) return SPCONVB_E_ARG;
+  RuleTask t = row_task(TASK_SUBM_RANK, coords, n_ptr, cap, launch_rows);
+  t.gin = make_grid(grid, batch);
+  t.kr = make_kernel3(ksize, nullptr, nullptr, dilation);
+  t.ws = down_ws(grid, batch, down_workspace);
+  t.map = map;
+  return launch_task(t, stream);
 }
 
 int spconvb_inverse_map(const int32_t* coords, const uint32_t* n_ptr, uint32_t cap,
@@ -740,38 +828,32 @@ int spconvb_inverse_map(const int32_t* coords, const uint32_t* n_ptr, uint32_t c
       !map)
     return SPCONVB_E_ARG;
   if (!grid_fits(grid, batch)) return SPCONVB_E_RANGE;
-  Kernel3 kr;
   int32_t og[3];
-  for (int a2 = 0; a2 < 3; ++a2) {
-    if (ksize[a2] < 1 || stride[a2] < 1 || pad[a2] < 0 || dilation[a2] < 1) return SPCONVB_E_ARG;
-    kr.k[a2] = ksize[a2]; kr.s[a2] = stride[a2]; kr.p[a2] = pad[a2]; kr.d[a2] = dilation[a2];
-    og[a2] = spconvb_out_extent(grid[a2], ksize[a2], stride[a2], pad[a2], dilation[a2]);
-    if (og[a2] < 1) return SPCONVB_E_ARG;
+  for (int a = 0; a < 3; ++a) {
+    if (ksize[a] < 1 || stride[a] < 1 || pad[a] < 0 || dilation[a] < 1) return SPCONVB_E_ARG;
+    og[a] = spconvb_out_extent(grid[a], ksize[a], stride[a], pad[a], dilation[a]);
+    if (og[a] < 1) return SPCONVB_E_ARG;
   }
-  set_stride_shifts(kr);
   const int kvol = ksize[0] * ksize[1] * ksize[2];
   if (kvol > 65535) return SPCONVB_E_ARG;
   if (!grid_fits(og, batch)) return SPCONVB_E_RANGE;
-  DownWs ws;
-  ws.words = down_words(og, batch);
-  ws.blocks = (ws.words + kScanWordsPerBlock - 1) / kScanWordsPerBlock;
-  ws.bitmap = (uint32_t*)down_workspace;
-  ws.prefix = ws.bitmap + ws.words;
-  ws.block_sums = ws.prefix + ws.words;
-  if (launch_rows == 0 || launch_rows > cap) launch_rows = cap;
-  inverse_map_kernel<<<flat_blocks((unsigned long long)launch_rows * kvol), kThreads, 0,
-                       (cudaStream_t)stream>>>((const int4*)coords, n_ptr, cap,
-                                               make_grid(grid, batch), make_grid(og, batch), kr,
-                                               kvol, ws, cap_coarse, map);
-  SPCONVB_LAUNCH_CHECK();
-  return SPCONVB_OK;
+  RuleTask t = row_task(TASK_INVERSE, coords, n_ptr, cap, launch_rows);
+  t.blocks = task_blocks((unsigned long long)(launch_rows == 0 || launch_rows > cap ? cap
+                                                                                    : launch_rows) *
+                         kvol);
+  t.gin = make_grid(grid, batch);
+  t.gout = make_grid(og, batch);
+  t.kr = make_kernel3(ksize, stride, pad, dilation);
+  t.ws = down_ws(og, batch, down_workspace);
+  t.other_cap = cap_coarse;
+  t.map = map;
+  return launch_task(t, stream);
 }
 
 size_t spconvb_down_workspace_bytes(const int32_t out_grid[3], int32_t batch) {
   if (!out_grid || !grid_fits(out_grid, batch)) return 0;
-  size_t words = down_words(out_grid, batch);
-  size_t blocks = (words + kScanWordsPerBlock - 1) / kScanWordsPerBlock;
-  return sizeof(uint32_t) * (2 * words + blocks + 16);
+  const size_t words = down_words(out_grid, batch);
+  return sizeof(uint32_t) * (2 * words + scan_state_words(scan_blocks((uint32_t)words)) + 16);
 }
 
 // Shared body of spconvb_down_map and spconvb_down_map_ranked.
@@ -788,81 +870,74 @@ static int down_map_impl(const int32_t* in_coords, const uint32_t* n_in_ptr, uin
   if (out_table && (out_slots < 8 || (out_slots & (out_slots - 1)) || out_slots < 2ull * cap_out))
     return SPCONVB_E_ARG;
   if (!grid_fits(in_grid, batch)) return SPCONVB_E_RANGE;
-  Kernel3 kr;
   int32_t og[3];
   for (int a = 0; a < 3; ++a) {
     if (ksize[a] < 1 || stride[a] < 1 || dilation[a] < 1 || pad[a] < 0) return SPCONVB_E_ARG;
-    kr.k[a] = ksize[a]; kr.s[a] = stride[a]; kr.p[a] = pad[a]; kr.d[a] = dilation[a];
     og[a] = spconvb_out_extent(in_grid[a], ksize[a], stride[a], pad[a], dilation[a]);
     if (og[a] < 1) return SPCONVB_E_ARG;
   }
-  set_stride_shifts(kr);
   if (!grid_fits(og, batch)) return SPCONVB_E_RANGE;
-  const int kvol = ksize[0] * ksize[1] * ksize[2];
-  if (kvol > 65535) return SPCONVB_E_ARG;
+  if (ksize[0] * ksize[1] * ksize[2] > 65535) return SPCONVB_E_ARG;
   cudaStream_t st = (cudaStream_t)stream;
 
-  DownWs ws;
-  ws.words = down_words(og, batch);
-  ws.blocks = (ws.words + kScanWordsPerBlock - 1) / kScanWordsPerBlock;
-  ws.bitmap = (uint32_t*)workspace;
-  ws.prefix = ws.bitmap + ws.words;
-  ws.block_sums = ws.prefix + ws.words;
+  const DownWs ws = down_ws(og, batch, workspace);
   if (!(flags & SPCONVB_FLAG_PREZEROED)) {
     SPCONVB_CUDA_TRY(cudaMemsetAsync(ws.bitmap, 0, sizeof(uint32_t) * (size_t)ws.words, st));
+    SPCONVB_CUDA_TRY(
+        cudaMemsetAsync(ws.scan, 0, sizeof(uint32_t) * scan_state_words(ws.blocks), st));
     if (out_table)
       SPCONVB_CUDA_TRY(cudaMemsetAsync(out_table, 0, sizeof(uint64_t) * (size_t)out_slots, st));
   }
-  Grid3 gin = make_grid(in_grid, batch), gout = make_grid(og, batch);
-  if (launch_rows == 0 || launch_rows > cap_in) launch_rows = cap_in;
-  // rows made by a rulebook: their bitmap gives the outputs' bitmap directly (when a
-  // thread's window of input cells fits 64 bits)
-  const bool from_bitmap = in_workspace && unit_dilation(kr) && kr.k[2] <= 32 &&
-                           (kMarkCells - 1) * kr.s[2] + kr.k[2] <= 64;
-  if (from_bitmap) {
-    const unsigned long long items = (unsigned long long)batch * og[0] * og[1] *
-                                     (unsigned long long)((og[2] + kMarkCells - 1) / kMarkCells);
-    down_mark_ranked_kernel<<<flat_blocks(items), kThreads, 0, st>>>(
-        (const uint32_t*)in_workspace, down_words(in_grid, batch), gin, gout, kr, ws.bitmap);
-  } else {
-    down_mark_kernel<<<flat_blocks(launch_rows), kThreads, 0, st>>>(
-        (const int4*)in_coords, n_in_ptr, cap_in, gin, gout, kr, ws.bitmap);
+  RuleTask mark = row_task(TASK_MARK_ROWS, in_coords, n_in_ptr, cap_in, launch_rows);
+  mark.gin = make_grid(in_grid, batch);
+  mark.gout = make_grid(og, batch);
+  mark.kr = make_kernel3(ksize, stride, pad, dilation);
+  mark.ws = ws;
+  RuleTask fill = mark;
+  if (in_workspace) mark.in_ws = fill.in_ws = down_ws(in_grid, batch, in_workspace);
+  // rows made by a rulebook: their bitmap gives the outputs' bitmap directly
+  if (in_workspace && mark_from_bitmap(mark.kr)) {
+    mark.kind = TASK_MARK_BITMAP;
+    mark.blocks = mark_bitmap_blocks(og, batch);
   }
-  SPCONVB_LAUNCH_CHECK();
-  down_scan_kernel<<<ws.blocks, kScanThreads, 0, st>>>(ws);
-  SPCONVB_LAUNCH_CHECK();
-  down_emit_kernel<<<ws.blocks, kScanThreads, 0, st>>>(ws, gout, (int4*)out_coords, n_out_ptr,
-                                                       cap_out, status);
-  SPCONVB_LAUNCH_CHECK();
+  RuleTask emit;
+  emit.kind = TASK_EMIT;
+  emit.blocks = ws.blocks;
+  emit.cap = cap_out;
+  emit.gout = mark.gout;
+  emit.kr = mark.kr;
+  emit.ws = ws;
+  emit.out_coords = (int4*)out_coords;
+  emit.n_out = n_out_ptr;
+  emit.map = in_workspace ? nullptr : map;
+  emit.status = status;
+  fill.map = map;
   if (in_workspace) {
     // the inputs can be ranked: every map entry is looked up from the output side
-    DownWs in_ws;
-    in_ws.words = down_words(in_grid, batch);
-    in_ws.blocks = 0;
-    in_ws.bitmap = (uint32_t*)in_workspace;
-    in_ws.prefix = in_ws.bitmap + in_ws.words;
-    in_ws.block_sums = nullptr;
-    constexpr int kRowThreads = 128;
-    if (is_k333(kr))
-      down_gather_ranked_kernel<true><<<row_blocks(cap_out, kRowThreads), kRowThreads, 0, st>>>(
-          (const int4*)out_coords, n_out_ptr, cap_out, gin, kr, in_ws, cap_in, map);
-    else
-      down_gather_ranked_kernel<false><<<row_blocks(cap_out, kRowThreads), kRowThreads, 0, st>>>(
-          (const int4*)out_coords, n_out_ptr, cap_out, gin, kr, in_ws, cap_in, map);
+    fill.kind = TASK_GATHER;
+    fill.coords = (const int4*)out_coords;
+    fill.n_ptr = n_out_ptr;
+    fill.cap = cap_out;
+    fill.other_cap = cap_in;
+    fill.blocks = task_blocks(cap_out);
   } else {
-    map_fill_kernel<<<flat_blocks((unsigned long long)cap_out * kvol / 4 + 1), kThreads, 0, st>>>(
-        n_out_ptr, cap_out, kvol, map);
-    SPCONVB_LAUNCH_CHECK();
-    down_scatter_kernel<<<flat_blocks(launch_rows), kThreads, 0, st>>>(
-        (const int4*)in_coords, n_in_ptr, cap_in, gin, gout, kr, ws, cap_out, map);
+    fill.kind = TASK_SCATTER;
+    fill.map_cap = cap_out;
   }
-  if (out_table) {
-    SPCONVB_LAUNCH_CHECK();
-    hash_rows_kernel<<<flat_blocks(cap_out), kThreads, 0, st>>>(
-        (const int4*)out_coords, n_out_ptr, cap_out, gout, out_table, out_slots - 1, status);
+  int rc = launch_task(mark, stream);
+  if (rc == SPCONVB_OK) rc = launch_task(emit, stream);
+  if (rc != SPCONVB_OK) return rc;
+  RuleWave last;
+  last.add(fill);
+  if (out_table) {  // the outputs' hash table, for callers that want one
+    RuleTask hash = row_task(TASK_HASH, out_coords, n_out_ptr, cap_out, cap_out);
+    hash.gin = mark.gout;
+    hash.table = out_table;
+    hash.mask = out_slots - 1;
+    hash.status = status;
+    last.add(hash);
   }
-  SPCONVB_LAUNCH_CHECK();
-  return SPCONVB_OK;
+  return launch_rule_wave(last, st);
 }
 
 int spconvb_down_map(const int32_t* in_coords, const uint32_t* n_in_ptr, uint32_t cap_in,
@@ -922,11 +997,10 @@ int spconvb_down_map_static(const int32_t* in_coords, const uint32_t* n_in_ptr, 
   void* scratch = nullptr;
   int rc = static_scratch_for_current_device(&scratch);
   if (rc != SPCONVB_OK) return rc;
-  // The array still holds the previous call's bitmap: it is cleared on every
-  // call, whatever the caller says about its own buffers.
+  // The array still holds the previous call's bitmap and block totals: it is cleared on
+  // every call, whatever the caller says about its own buffers.
   cudaStream_t st = (cudaStream_t)stream;
-  const size_t bitmap_bytes = sizeof(uint32_t) * (size_t)down_words(og, batch);
-  SPCONVB_CUDA_TRY(cudaMemsetAsync(scratch, 0, bitmap_bytes, st));
+  SPCONVB_CUDA_TRY(cudaMemsetAsync(scratch, 0, need, st));
   if (out_table && !(flags & SPCONVB_FLAG_PREZEROED))
     SPCONVB_CUDA_TRY(cudaMemsetAsync(out_table, 0, sizeof(uint64_t) * (size_t)out_slots, st));
   return spconvb_down_map(in_coords, n_in_ptr, cap_in, launch_rows, in_grid, batch, ksize, stride,

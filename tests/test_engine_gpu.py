@@ -336,6 +336,33 @@ def test_auxiliary_stream_changes_no_result():
         assert np.array_equal(fast.output(0).cpu().numpy().view(np.uint16), want.view(np.uint16))
 
 
+@pytest.mark.parametrize("single_stream", [False, True])
+def test_many_rulebooks_on_one_level(single_stream):
+    """More independent rulebooks than one launch of rulebook tasks holds: ten strided convolutions
+    of different geometry on the input rows, each with a SubM layer behind it."""
+    eng = _engine_mod()
+    rng = np.random.default_rng(0)
+    ids, nodes, counter, outs = models._Ids(), [], [0, 0], []
+    for i in range(10):
+        k, s, p = (3, 3, 3), (2, 1 + i % 2, 2 + i % 3), (1, i % 2, i // 5)
+        y = models._conv(ids, rng, nodes, "0", 5, 16, k, s, p, False, "down%d" % i, "ReLU", counter,
+                         40000)
+        y = models._conv(ids, rng, nodes, y, 16, 16, k, (1, 1, 1), (1, 1, 1), True, "sub%d" % i,
+                         "ReLU", counter, 40000)
+        outs.append((y, [1, 16]))
+    model = {"kind": "layer", "inputs": [("0", [1, 5])], "outputs": outs, "nodes": nodes,
+             "roles": {"conv_input": [0]}, "in_channels": 5}
+    feats, coords = _frame(2500, seed=3)
+    e = eng.Engine.from_model(model, eng.PRECISION_FP16,
+                              eng.BUILD_FORCE_SIMT | eng.BUILD_KEEP_TENSORS |
+                              (eng.BUILD_SINGLE_STREAM if single_stream else 0))
+    e.forward(_dev(feats), _dev(coords), GRID)
+    torch.cuda.synchronize()
+    assert e.status()[0] == 0
+    _, T = graph_oracle.run(model, feats, coords, GRID, "fp16")
+    _compare_all(e, T, exact=True)
+
+
 def test_single_layer_sparse_output_and_bounds():
     eng = _engine_mod()
     feats, coords = _frame(5000, seed=5)

@@ -197,6 +197,37 @@ def test_down_map_geometries_match_the_oracle(k, s, p, d):
     assert np.array_equal(dm3.cpu().numpy()[:, :rn3], rdm3[:, :rn3])
 
 
+@pytest.mark.parametrize("grid,n", [
+    ((1, 1, 5), 3),             # one bitmap word, partly outside the grid
+    ((4, 32, 32), 3900),        # one scan block, nearly every cell set
+    ((4, 32, 33), 4224),        # a scan block and 4 words, every cell set
+    ((32, 64, 64), 40000),      # exactly one group of 32 scan blocks
+    ((32, 64, 65), 130000),     # a group and a bit
+    ((33, 257, 311), 2000),     # many blocks, most of them empty
+])
+def test_strided_rows_at_the_edges_of_scan_blocks(grid, n):
+    """Output rows, order, count and map where the scan's blocks (128 words of 32 cells) and groups
+    of blocks (32) begin and end; a 1x1x1 kernel of stride 1, so the outputs are the inputs."""
+    ops = _ops()
+    cells = np.sort(np.random.default_rng(n).permutation(int(np.prod(grid)))[:n])
+    coords = np.zeros((n, 4), np.int32)
+    coords[:, 1:] = np.stack(np.unravel_index(cells, grid), 1)
+    order = np.random.default_rng(n + 1).permutation(n)
+    st = ops.new_status()
+    one = (1, 1, 1)
+    oc, n_out, m, _, og, ws = ops.down_map(_dev(coords[order]), ops.device_count(n), grid, None, one,
+                                           one, (0, 0, 0), status=st, want_table=False,
+                                           return_ws=True)
+    _status_ok(st)
+    assert int(n_out.item()) == n and list(og) == list(grid)
+    assert np.array_equal(oc.cpu().numpy()[:n], coords)
+    assert np.array_equal(m.cpu().numpy()[0, :n], np.argsort(order))
+    sub = ops.subm_map_ranked(oc, n_out, grid, ws, status=st)
+    ref, _ = orc.subm_map(coords, grid)
+    _status_ok(st)
+    assert np.array_equal(sub.cpu().numpy()[:, :n], ref)
+
+
 def test_down_map_overflow_sets_status():
     ops = _ops()
     from lidar_ai_solution_b200 import cabi
