@@ -17,9 +17,10 @@
 //   warps 0-7   epilogue: warp w reads its lane quadrant (its channels) and its
 //               share of the tile's rows from the accumulator with tcgen05.ld,
 //               applies dequant + bias + activation (+ residual add) + requant
-//               with per-lane scale and bias, transposes 4x4 blocks inside lane
-//               quads with two shuffles, and stores 4 (int8) or 8 (fp16)
-//               contiguous bytes of one output row per lane
+//               with per-lane scale and bias, and stores one element a lane: a
+//               warp covers 32 contiguous channels of a row.  (Transposing 4x4
+//               blocks for 4-byte stores took more instructions than it saved:
+//               64 -> 64 with a residual 51.8 us, this way 45.9.)
 //   warp  8     allocates TMEM; walks the chunks converged, one elected lane issues
 //               tcgen05.mma (kind::i8 with int32 accumulators or kind::f16 with fp32)
 //   warps 9-24  producers, two groups of 8 warps that take the chunks in turn (the
@@ -68,10 +69,10 @@ namespace {
 constexpr int kTileRows = 256;  // most voxel rows per tile: the largest N of the MMA
 constexpr int kEpiWarps = 8;
 constexpr int kMmaWarp = 8;
-constexpr int kProdWarp0 = 9;
 constexpr int kProdThreads = 512;   // two groups of 8 producer warps
-constexpr int kWeightWarp = kProdWarp0 + kProdThreads / 32;
-constexpr int kCtaThreads = 32 * (kWeightWarp + 1);
+constexpr int kProdWarp0 = 9;       // 9, 10, ... 24: four of them on every TMEM lane quadrant
+constexpr int kWeightWarp = 25;
+constexpr int kCtaThreads = 32 * 26;
 constexpr uint32_t kTmemCols = 2 * kTileRows;
 // 5 stages of 256 rows and 4 of weights: all a CTA can have.  No other block fits beside this one:
 // 26 warps of 72 registers fill two of the SM's four register files.  With 64 registers and 12 KB
@@ -79,6 +80,11 @@ constexpr uint32_t kTmemCols = 2 * kTileRows;
 // which is what the overlap saves (batch of 8 frames 4.25 ms against 4.34).
 constexpr uint32_t kRingBytes = 5 * kTileRows * kChunk + 4 * 128 * kChunk;
 constexpr size_t kSmemBytes = kRingBytes + 1024 + 256;  // alignment slack, barriers
+
+// ceil(2^32 / n): with it x / n = umulhi(x, .) for x < 2^29
+__constant__ const uint32_t kReciprocal[9] = {0u,          0u,          0x80000000u,
+                                              0x55555556u, 0x40000000u, 0x33333334u,
+                                              0x2aaaaaabu, 0x24924925u, 0x20000000u};
 
 // 32-bit instruction descriptor: [4,6) D format (1 = f32, 2 = s32), [7,10) A
 // format, [10,13) B format (f16 kind: 0 = f16; i8 kind: 1 = signed), bits 15/16
@@ -88,48 +94,24 @@ __device__ __forceinline__ constexpr uint32_t make_idesc() {
   return INT8 ? ((2u << 4) | (1u << 7) | (1u << 10)) : (1u << 4);
 }
 
-// Transposes inside a quad of lanes (lane = 4g + j): they turn "my channel for a
-// few rows" into "4 adjacent channels of one row", and back.
-// A 16 x 4 byte block spread over a quad: lane j holds 4 words, word t = bytes of 4
-// consecutive rows 4t..4t+3 of channel j.  quad_words_transpose gives lane j word j
-// of every lane (2 x 2 shuffles); bytes_transpose4 then turns "word c = 4 rows of
-// channel c" into "word r = 4 channels of row r" inside the lane.  Together: lane j
-// holds rows 4j..4j+3 of the 4 channels, one word per row.  The inverse applies the
-// two steps in the opposite order (each is its own inverse).
-__device__ __forceinline__ void quad_words_transpose(uint32_t (&w)[4], uint32_t lane) {
-  const bool odd = lane & 1u, hi = lane & 2u;
-  uint32_t s0 = odd ? w[0] : w[1], s1 = odd ? w[2] : w[3];
-  s0 = __shfl_xor_sync(0xffffffffu, s0, 1);
-  s1 = __shfl_xor_sync(0xffffffffu, s1, 1);
-  const uint32_t a0 = odd ? s0 : w[0], a1 = odd ? w[1] : s0;
-  const uint32_t a2 = odd ? s1 : w[2], a3 = odd ? w[3] : s1;
-  uint32_t u0 = hi ? a0 : a2, u1 = hi ? a1 : a3;
-  u0 = __shfl_xor_sync(0xffffffffu, u0, 2);
-  u1 = __shfl_xor_sync(0xffffffffu, u1, 2);
-  w[0] = hi ? u0 : a0;
-  w[1] = hi ? u1 : a1;
-  w[2] = hi ? a2 : u0;
-  w[3] = hi ? a3 : u1;
-}
-__device__ __forceinline__ void bytes_transpose4(uint32_t (&w)[4]) {
-  const uint32_t l01 = __byte_perm(w[0], w[1], 0x5140), h01 = __byte_perm(w[0], w[1], 0x7362);
-  const uint32_t l23 = __byte_perm(w[2], w[3], 0x5140), h23 = __byte_perm(w[2], w[3], 0x7362);
-  w[0] = __byte_perm(l01, l23, 0x5410);
-  w[1] = __byte_perm(l01, l23, 0x7632);
-  w[2] = __byte_perm(h01, h23, 0x5410);
-  w[3] = __byte_perm(h01, h23, 0x7632);
-}
-// 16-bit elements: lane j holds 4 halves e[0..3] in two words; afterwards it holds
-// element j of lanes 0..3 of its quad, in lane order (the call is its own inverse).
-__device__ __forceinline__ void quad_transpose_h16(uint32_t& w0, uint32_t& w1, uint32_t lane) {
-  const bool odd = lane & 1u;
-  const uint32_t send = __byte_perm(w0, w1, odd ? 0x5410 : 0x7632);
-  const uint32_t recv = __shfl_xor_sync(0xffffffffu, send, 1);
-  w0 = __byte_perm(w0, recv, odd ? 0x3254 : 0x5410);
-  w1 = __byte_perm(w1, recv, odd ? 0x3276 : 0x7610);
-  const bool hi = lane & 2u;
-  const uint32_t other = __shfl_xor_sync(0xffffffffu, hi ? w0 : w1, 2);
-  if (hi) w0 = other; else w1 = other;
+// Bytes or halves of 16 rows of one channel, `pitch` bytes apart; `n` rows exist.
+template <bool I8>
+__device__ __forceinline__ void load_rows16(const uint8_t* p, uint32_t pitch, uint32_t n,
+                                            int32_t (&v)[16]) {
+  if (n >= 16u) {
+#pragma unroll
+    for (uint32_t i = 0; i < 16; ++i)
+      v[i] = I8 ? (int32_t)__ldg((const int8_t*)(p + i * pitch))
+                : (int32_t)__ldg((const uint16_t*)(p + i * pitch));
+  } else {
+#pragma unroll
+    for (uint32_t i = 0; i < 16; ++i) {
+      v[i] = 0;
+      if (i < n)
+        v[i] = I8 ? (int32_t)__ldg((const int8_t*)(p + i * pitch))
+                  : (int32_t)__ldg((const uint16_t*)(p + i * pitch));
+    }
+  }
 }
 
 // ------------------------------------------------------------------- kernel
@@ -191,12 +173,16 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
   // Tile height: the rows are dealt out in rounds over the CTAs, so a fixed 256-row tile
   // can leave most CTAs idle in the last round (227 tiles on 148 CTAs run as long as 296).
   // The height is instead the smallest multiple of 32 with which every CTA gets the same
-  // number of tiles: per-CTA rows / rounds, rounded up.
-  const uint32_t per_cta = (n_out + gridDim.x - 1) / gridDim.x;
-  const uint32_t rounds = max(1u, (per_cta + kTileRows - 1) / kTileRows);
-  const uint32_t tile_rows =
-      min((uint32_t)kTileRows, max(32u, ((per_cta + rounds - 1) / rounds + 31u) & ~31u));
-  const uint32_t ntiles = (n_out + tile_rows - 1) / tile_rows;
+  // number of tiles: per-CTA rows / rounds, rounded up.  Without integer divisions, which
+  // would stand between the row count and the first index load of every launch; a quotient
+  // that is off by one only makes another height.
+  const uint32_t per_cta = max(1u, __umulhi(n_out + gridDim.x - 1, a.grid_inv));
+  const uint32_t rounds = (per_cta + kTileRows - 1) / kTileRows;
+  const uint32_t high =
+      (uint32_t)(__fdividef((float)(per_cta + rounds - 1), (float)rounds) + 0.01f);
+  const uint32_t tile_rows = min((uint32_t)kTileRows, (high + 31u) & ~31u);
+  const uint32_t n32 = (n_out + 31u) >> 5, t32 = tile_rows >> 5;
+  const uint32_t ntiles = t32 == 1u ? n32 : __umulhi(n32 + t32 - 1u, kReciprocal[t32]);
   // Two rings share the buffer: row stages as high as this launch's tile, and weight stages.
   // Low tiles get deeper rings: as many of both as fit, and what is left over goes to the rows.
   const uint32_t row_stage = tile_rows * kChunk;
@@ -204,6 +190,15 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
   const uint32_t nst = min((uint32_t)kMaxStages, (kRingBytes - nwst * kWeightBytes) / row_stage);
   const uint32_t sW = smem_u32(smem), sR = sW + nwst * kWeightBytes;
 
+  const bool is_producer = warp > kMmaWarp && warp != kWeightWarp;
+  // Who drains accumulators: the epilogue warps every tile of the CTA; the producers, which have
+  // nothing left to gather by then, help with the last one.  It is the tail of every launch, and
+  // on a small frame the only tile (128 channels, 224 rows: 6 200 cycles with 8 warps, with a
+  // residual 15 000, beside 17 000 of MMAs).  A producer that is done knows that the MMAs are in
+  // the last tile, or about to be, only if a tile has at least as many chunks as the ring.
+  const bool shared_tail = (uint32_t)nchunk >= nst;
+  uint32_t drain_tile = blockIdx.x, drain_tl = 0;
+  bool drains = warp < kEpiWarps;
   if (warp == kWeightWarp) {
     // -------------------------------------------------------------- weights
     // One lane streams the chunks' pre-swizzled weight images, its ring may be shallower than
@@ -235,7 +230,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
         }
     }
     __syncwarp();
-  } else if (warp >= kProdWarp0) {
+  } else if (is_producer) {
     // ------------------------------------------------------------ producers
     // Two groups of 8 warps take the chunks in turn (group g the chunks g, g + 2, ...), so a
     // warp has two chunk periods for the round trip of one chunk: wait for the stage, look
@@ -245,7 +240,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
     // lanes per row, so the lanes that read the same neighbour row ask for one contiguous
     // piece of it).  Missing neighbours are zero-filled copies, so the 8 items are
     // branch-free and their address arithmetic and copies overlap.
-    const uint32_t pw_all = (uint32_t)warp - kProdWarp0;
+    const uint32_t pw_all = (uint32_t)(warp - kProdWarp0);
     const uint32_t grp = pw_all >> 3, pw = pw_all & 7u;
     const uint32_t seg = lane & 7u;        // 16-byte segment of the chunk this thread copies
     const uint32_t slot = lane >> 3;       // its 8 rows of the warp's 32
@@ -293,6 +288,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
       j -= nchunk;
       tile += gridDim.x;
     }
+    uint32_t tiles_done = 0;  // (of use where no step passes a tile: nchunk > 1)
     uint32_t ntile = tile;  // the chunk whose indices are loaded next
     int nj = j;
     uint32_t it = grp, s = grp % nst, ph = (grp / nst) & 1u;
@@ -313,14 +309,16 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
         for (uint32_t i = 0; i < 8; ++i) {
           const int32_t sr = idx[i];
           cp_async16(stage_addr + i * 128u + ((seg ^ i) << 4),
-                     src + (size_t)(sr < 0 ? 0 : sr) * RB, sr < 0 ? 0u : 16u);
+                     src + (int64_t)sr * RB, sr < 0 ? 0u : 16u);
         }
       }
       if (!(a.wait_test > 0 && it + 1u >= (uint32_t)a.wait_test))
         cp_async_arrive_noinc(bar_full + 8 * s);
       load_idx(ntile, nj, idx);
       advance2(ntile, nj);
+      const uint32_t was = tile;
       advance2(tile, j);
+      if (tile != was) ++tiles_done;
       it += 2;
       s += 2;
       if (s >= nst) {
@@ -337,6 +335,12 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
     while (step(idx_a) && step(idx_b)) {
     }
     cp_async_wait_all();  // nothing of this thread may still be writing when the CTA exits
+    __syncwarp();
+    if (shared_tail && tile >= ntiles && tiles_done > 0u) {
+      drains = true;
+      drain_tile = tile - gridDim.x;
+      drain_tl = tiles_done - 1u;
+    }
   } else if (warp == kMmaWarp) {
     // ------------------------------------------------------------ MMA issue
     // The whole warp walks the chunks and one elected lane issues: the loop's values stay
@@ -344,71 +348,77 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
     // cycles per chunk against 583 when a single lane runs the loop, whose descriptors are moved
     // to uniform registers one MMA after the other).
     //
-    // The tensor pipe takes one MMA at a time, and issuing the next one blocks until it is
-    // free.  Everything that is not an MMA is short: the next stage's barrier is probed once,
-    // early, while the pipe is busy, so that the first MMA of the next chunk can follow the
-    // last one of this chunk without a bubble.
+    // MMAs are queued: what a chunk costs here is the issue of its instructions, and with 24 other
+    // warps around every one takes tens of cycles.  So the loop carries addresses and nothing
+    // else, and a chunk is four MMAs, a commit and one test of the next stage's barrier.
     const bool leader = elect_one();
     const uint32_t idesc = make_idesc<INT8>() | ((tile_rows >> 3) << 17) | ((128u >> 4) << 24);
     const uint64_t wdesc0 = make_smem_desc(sW);  // M operand: weights
     const uint64_t rdesc0 = make_smem_desc(sR);  // N operand: gathered rows
     // 32-bit arithmetic only: the descriptors differ in their low word (the address)
-    const uint32_t w_step = kWeightBytes >> 4, r_step = row_stage >> 4;
     const uint32_t desc_hi = (uint32_t)(wdesc0 >> 32);
+    const uint32_t w_step = kWeightBytes >> 4, r_step = row_stage >> 4;
     const uint32_t w_lo0 = (uint32_t)wdesc0, r_lo0 = (uint32_t)rdesc0;
-    uint32_t ph = 0, tl = 0;
-    uint32_t s = 0, ws = 0;  // row and weight stage of the current chunk
+    const uint32_t w_end = w_lo0 + nwst * w_step, bar_end = bar_full + 8 * nst;
+    constexpr uint32_t kToEmpty = 8 * kMaxStages;  // from a stage's full barrier to its empty one
+    uint32_t bar = bar_full, rd = r_lo0, wd = w_lo0, ph = 0, tl = 0;
+    auto next_stage = [&]() {
+      bar += 8;
+      rd += r_step;
+      if (bar == bar_end) {
+        bar = bar_full;
+        rd = r_lo0;
+        ph ^= 1u;
+      }
+      wd += w_step;
+      if (wd == w_end) wd = w_lo0;
+    };
+    auto stage_full = [&]() -> bool {
+      return mbar_test_wait(bar, ph) || mbar_wait_spin(bar, ph, abort_flag, a.status, 3u);
+    };
     // The loop is entered with the current chunk's stage known to be full.
-    bool alive = blockIdx.x < ntiles && mbar_wait_spin(bar_full, 0u, abort_flag, a.status, 3u);
+    bool alive = blockIdx.x < ntiles && stage_full();
     for (uint32_t tile = blockIdx.x; tile < ntiles && alive; tile += gridDim.x, ++tl) {
       const uint32_t buf = tl & 1u;
       if (!mbar_wait_spin(bar_tempty + 8 * buf, ((tl >> 1) & 1u) ^ 1u, abort_flag, a.status, 2u))
         break;
       tc_fence_after();  // the epilogue's reads of this accumulator come before these MMAs
       const uint32_t d_tmem = tmem_base + buf * kTileRows;
-      const bool last_tile = tile + gridDim.x >= ntiles;
-      for (int j = 0; j < nchunk; ++j) {
-        // No fence here: the rows arrive by cp.async completions on the stage's mbarrier,
-        // which is what the MMA's shared-memory reads are ordered behind.
-        const uint32_t rd = r_lo0 + s * r_step;
-        const uint32_t wd = w_lo0 + ws * w_step;
-        // the next stage (of this tile's next chunk or of the next tile's first)
-        const uint32_t s1 = s + 1 == nst ? 0u : s + 1;
-        const uint32_t ph1 = s1 == 0u ? ph ^ 1u : ph;
-        const uint32_t full_n = bar_full + 8 * s1;
-        const bool more = j + 1 < nchunk || !last_tile;
-        bool ready = true;
-        if (j + 1 < nchunk) {
-          if (leader) umma_lohi<INT8>(d_tmem, wd, rd, desc_hi, idesc, (uint32_t)(j != 0));
-          ready = mbar_test_wait(full_n, ph1);
-          if (leader) {
-            umma_lohi<INT8>(d_tmem, wd + 2u, rd + 2u, desc_hi, idesc, 1u);
-            umma_lohi<INT8>(d_tmem, wd + 4u, rd + 4u, desc_hi, idesc, 1u);
-            umma_lohi<INT8>(d_tmem, wd + 6u, rd + 6u, desc_hi, idesc, 1u);
-            tc_commit(bar_empty + 8 * s);
-          }
-        } else {
-          if (more) ready = mbar_test_wait(full_n, ph1);
-          if (leader) {
-            for (int ks = 0; ks < last_ksteps; ++ks)
-              umma_lohi<INT8>(d_tmem, wd + 2u * ks, rd + 2u * ks, desc_hi, idesc,
-                              (uint32_t)((j | ks) != 0));
-            tc_commit(bar_empty + 8 * s);
-            tc_commit(bar_tfull + 8 * buf);
-          }
+      // No fence before the MMAs of a stage: its rows arrive by cp.async completions on the stage's
+      // mbarrier, which is what the MMA's shared-memory reads are ordered behind.
+      uint32_t accumulate = 0u;
+#pragma unroll 1
+      for (int j = nchunk - 1; j > 0; --j) {
+        if (leader) {
+          umma_lohi<INT8>(d_tmem, wd, rd, desc_hi, idesc, accumulate);
+          umma_lohi<INT8>(d_tmem, wd + 2u, rd + 2u, desc_hi, idesc, 1u);
+          umma_lohi<INT8>(d_tmem, wd + 4u, rd + 4u, desc_hi, idesc, 1u);
+          umma_lohi<INT8>(d_tmem, wd + 6u, rd + 6u, desc_hi, idesc, 1u);
+          tc_commit(bar + kToEmpty);
         }
-        __syncwarp();
-        if (!ready && !mbar_wait_spin(full_n, ph1, abort_flag, a.status, 3u)) {
+        accumulate = 1u;
+        next_stage();
+        if (!stage_full()) {
           alive = false;
           break;
         }
-        s = s1;
-        ph = ph1;
-        if (++ws == nwst) ws = 0;
       }
+      if (!alive) break;
+      if (leader) {
+        for (int ks = 0; ks < last_ksteps; ++ks) {
+          umma_lohi<INT8>(d_tmem, wd + 2u * ks, rd + 2u * ks, desc_hi, idesc, accumulate);
+          accumulate = 1u;
+        }
+        tc_commit(bar + kToEmpty);
+        tc_commit(bar_tfull + 8 * buf);
+      }
+      __syncwarp();
+      next_stage();
+      if (tile + gridDim.x < ntiles) alive = stage_full();
     }
     __syncwarp();
-  } else {
+  }
+  if (drains) {
     // ------------------------------------------------------------- epilogue
     // Same arithmetic as common.cuh:epilogue_value, written so that the per-element
     // work is a handful of instructions: ReLU as a max with 0 or -inf, float -> int8
@@ -416,52 +426,47 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
     // hoisted out of the element loops.
     const Epilogue ep = a.ep;
     // Accumulator row m (TMEM lane m) holds channel m % COUT of weight copy m / COUT.  Copy c
-    // owns cols_rep rows of the tile from c * cols_rep on, and the two warps of a lane
-    // quadrant split those rows again: every warp has the same share of this launch's tile.
+    // owns cols_rep rows of the tile from c * cols_rep on, and the warps of a lane quadrant take
+    // its groups of 16 rows in turn: two warps, in the CTA's last tile six.
     const uint32_t q = (uint32_t)warp & 3u;        // TMEM lane quadrant of this warp
-    const uint32_t half = (uint32_t)warp >> 2;
+    const uint32_t part = is_producer ? 2u + (((uint32_t)warp - kProdWarp0) >> 2) : (uint32_t)warp >> 2;
     const uint32_t acc_row = 32u * q + lane, acc_row0 = 32u * q;
     const uint32_t ch = acc_row % COUT;            // this lane's channel
-    const uint32_t chq = ch & ~3u;                 // first of the 4 channels this lane stores
-    const uint32_t j4 = lane & 3u;                 // row within a group of 4 this lane stores
     const uint32_t cols_rep = (tile_rows + 32u * kRep - 1u) / (32u * kRep) * 32u;
-    const uint32_t cols_warp = cols_rep / 2u;
-    // first row (of the tile) of this lane, and of lane 0 of the warp: they differ only for
-    // COUT = 16, where the two halves of a warp belong to different copies
+    // first row (of the tile) of this lane's copy, and of lane 0's: they differ only for COUT = 16,
+    // where the two halves of a warp belong to different copies
     constexpr bool split_warp = COUT == 16;
-    const uint32_t col_lane = (acc_row / COUT) * cols_rep + half * cols_warp;
-    const uint32_t col_warp = (acc_row0 / COUT) * cols_rep + half * cols_warp;
+    const uint32_t copy_lane = (acc_row / COUT) * cols_rep, copy_warp = (acc_row0 / COUT) * cols_rep;
+    // columns of lane 0's copy that lie inside the tile
+    const uint32_t cols = copy_warp < tile_rows ? min(cols_rep, tile_rows - copy_warp) : 0u;
     const float sc = (INT8 && a.scale) ? __ldg(a.scale + ch) : 1.f;
     const float bi = a.bias ? __ldg(a.bias + ch) : 0.f;
     const float lo = ep.act == SPCONVB_ACT_RELU ? 0.f : -INFINITY;
     const float lo2 = ep.res_relu ? 0.f : -INFINITY;
     const bool res_i8 = ep.res_kind == SPCONVB_I8;
-    const uint32_t out_b = ep.out_kind == SPCONVB_I8 ? 1u : 2u;
-    const uint32_t res_b = res_i8 ? 1u : 2u;
-    // residual words of 16 rows: lane (g, j) loads channels 4g..4g+3 of rows 4j + t
-    // (int8, a word each) or of rows 4t + j (fp16, two words each), t = 0..3
-    auto load_res = [&](uint32_t row0, bool in_tile, uint2 (&rq)[4]) {
-#pragma unroll
-      for (int t = 0; t < 4; ++t) {
-        const uint32_t row = res_i8 ? row0 + 4u * j4 + t : row0 + 4u * t + j4;
-        rq[t] = make_uint2(0u, 0u);
-        if (in_tile && row < n_out) {
-          const uint8_t* p = a.res + ((size_t)row * COUT + chq) * res_b;
-          if (res_i8) rq[t].x = __ldg((const uint32_t*)p);
-          else rq[t] = __ldg((const uint2*)p);
-        }
-      }
+    // A lane owns a channel, so a group of 16 rows is 16 loads or stores of one element each, at
+    // constant distances; the 32 lanes of a warp cover a contiguous piece of every row.
+    constexpr uint32_t kRow8 = COUT, kRow16 = 2 * COUT;  // bytes of an int8 / fp16 row
+    auto load_res = [&](uint32_t row, uint32_t n, int32_t (&r)[16]) {
+      if (res_i8) load_rows16<true>(a.res + (size_t)row * kRow8 + ch, kRow8, n, r);
+      else load_rows16<false>(a.res + (size_t)row * kRow16 + 2u * ch, kRow16, n, r);
     };
-    uint32_t tl = 0;
-    for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++tl) {
+    // rows of this lane's group of 16 that exist: a group lies inside the tile or not as a whole
+    // (the tile height is a multiple of 32); rows past the tile belong to the next one
+    auto rows_of = [&](uint32_t row, uint32_t col) -> uint32_t {
+      return col < tile_rows && row < n_out ? min(16u, n_out - row) : 0u;
+    };
+    uint32_t tl = drain_tl;
+    for (uint32_t tile = drain_tile; tile < ntiles; tile += gridDim.x, ++tl) {
       const uint32_t buf = tl & 1u;
-      const uint32_t trow0 = tile * tile_rows + col_lane;
-      // the first residual rows are fetched before the accumulator is waited for;
-      // after that the loads run one group of 16 rows ahead of the arithmetic.  A group
-      // lies inside the tile or not as a whole (the tile height is a multiple of 32);
-      // rows past it belong to the next tile.
-      uint2 rq[4];
-      if (ep.has_res) load_res(trow0, col_lane < tile_rows, rq);
+      const uint32_t step = shared_tail && tile + gridDim.x >= ntiles ? 6u * 16u : 2u * 16u;
+      const uint32_t trow0 = tile * tile_rows;
+      uint32_t col = 16u * part;  // of the copy
+      // the first residual rows are fetched before the accumulator is waited for; after that
+      // the loads run one group of 16 rows ahead of the arithmetic
+      int32_t rnext[16];
+      if (ep.has_res && col < cols)
+        load_res(trow0 + copy_lane + col, rows_of(trow0 + copy_lane + col, copy_lane + col), rnext);
       uint32_t ok = 1u;
       if (lane == 0) {
         ok = mbar_wait(bar_tfull + 8 * buf, (tl >> 1) & 1u, abort_flag, a.status, 4u) ? 1u : 0u;
@@ -469,46 +474,31 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
       ok = __shfl_sync(0xffffffffu, ok, 0);
       if (!ok) break;
       tc_fence_after();
-      // groups of this warp that lie inside the tile (by its lower-numbered rows)
-      const uint32_t ng = col_warp >= tile_rows
-                              ? 0u
-                              : min(cols_warp / 16u, (tile_rows - col_warp + 15u) / 16u);
-      const uint32_t taddr = tmem_base + ((32u * q) << 16) + buf * kTileRows + col_warp;
-      if (ng == 0u) {
+      const uint32_t taddr = tmem_base + ((32u * q) << 16) + buf * kTileRows + copy_warp;
+      auto release = [&]() {  // no more reads of this accumulator by this warp
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(bar_tempty + 8 * buf);
-      }
+        if (lane == 0 && !is_producer) mbar_arrive(bar_tempty + 8 * buf);
+      };
+      if (col >= cols) release();
 #pragma unroll 1
-      for (uint32_t g = 0; g < ng; ++g) {
-        const uint32_t row0 = trow0 + 16u * g;
-        const bool in_tile = col_lane + 16u * g < tile_rows;
+      for (; col < cols; col += step) {
+        const uint32_t row0 = trow0 + copy_lane + col;
+        const uint32_t rows = rows_of(row0, copy_lane + col);
         uint32_t v[16];
-        tmem_ld16(taddr + 16u * g, v);
+        tmem_ld16(taddr + col, v);
         if (split_warp) {
           // the upper half of the warp belongs to the next copy: its rows are one copy's
           // worth of columns further on
           uint32_t vm[16];
-          tmem_ld16(taddr + cols_rep + 16u * g, vm);
+          tmem_ld16(taddr + cols_rep + col, vm);
           tmem_ld_wait();
 #pragma unroll
           for (int i = 0; i < 16; ++i) v[i] = lane >= 16u ? vm[i] : v[i];
         } else {
           tmem_ld_wait();
         }
-        if (g + 1u == ng) {
-          // every accumulator element of this warp is in registers: release the buffer
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(bar_tempty + 8 * buf);
-        }
-        uint2 rcur[4];
-        if (ep.has_res) {
-#pragma unroll
-          for (int t = 0; t < 4; ++t) rcur[t] = rq[t];
-          if (g + 1u < ng)
-            load_res(row0 + 16, col_lane + 16u * (g + 1u) < tile_rows, rq);
-        }
+        if (col + step >= cols) release();
         float y[16];
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
@@ -517,66 +507,46 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
         }
         if (ep.has_res) {
           // the conv result as it would have been stored (mid), plus the residual
-          float rr[16];
-          if (res_i8) {
-            uint32_t w[4] = {rcur[0].x, rcur[1].x, rcur[2].x, rcur[3].x};
-            bytes_transpose4(w);
-            quad_words_transpose(w, lane);
-#pragma unroll
-            for (int t = 0; t < 4; ++t)
-#pragma unroll
-              for (int i = 0; i < 4; ++i)
-                rr[4 * t + i] = __fmul_rn((float)(int8_t)(w[t] >> (8 * i)), ep.res_scale);
-          } else {
-#pragma unroll
-            for (int t = 0; t < 4; ++t) {
-              uint32_t w0 = rcur[t].x, w1 = rcur[t].y;
-              quad_transpose_h16(w0, w1, lane);
-              const __half2 h0 = *(const __half2*)&w0, h1 = *(const __half2*)&w1;
-              rr[4 * t + 0] = __low2float(h0);
-              rr[4 * t + 1] = __high2float(h0);
-              rr[4 * t + 2] = __low2float(h1);
-              rr[4 * t + 3] = __high2float(h1);
-            }
-          }
           if (ep.mid_kind == SPCONVB_I8) {
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
-              const float m = __fmul_rn((float)cvt_sat_s8(__fmul_rn(y[i], ep.mid_inv_scale)),
-                                        ep.mid_scale);
-              y[i] = fmaxf(__fadd_rn(m, rr[i]), lo2);
-            }
+            for (int i = 0; i < 16; ++i)
+              y[i] = __fmul_rn((float)cvt_sat_s8(__fmul_rn(y[i], ep.mid_inv_scale)), ep.mid_scale);
+          } else {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) y[i] = __half2float(__float2half_rn(y[i]));
+          }
+          if (res_i8) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i)
+              y[i] = fmaxf(__fadd_rn(y[i], __fmul_rn((float)rnext[i], ep.res_scale)), lo2);
           } else {
 #pragma unroll
             for (int i = 0; i < 16; ++i)
-              y[i] = fmaxf(__fadd_rn(__half2float(__float2half_rn(y[i])), rr[i]), lo2);
+              y[i] = fmaxf(__fadd_rn(y[i], __half2float(__ushort_as_half((uint16_t)rnext[i]))), lo2);
           }
+          if (col + step < cols)
+            load_res(row0 + step, rows_of(row0 + step, copy_lane + col + step), rnext);
         }
         if (ep.out_kind == SPCONVB_I8) {
-          uint32_t w[4];
+          int8_t* o = (int8_t*)a.out + (size_t)row0 * kRow8 + ch;
+          if (rows == 16u) {
 #pragma unroll
-          for (int t = 0; t < 4; ++t)
-            w[t] = pack_s8x4(cvt_sat_s8(__fmul_rn(y[4 * t + 0], ep.inv_out_scale)),
-                             cvt_sat_s8(__fmul_rn(y[4 * t + 1], ep.inv_out_scale)),
-                             cvt_sat_s8(__fmul_rn(y[4 * t + 2], ep.inv_out_scale)),
-                             cvt_sat_s8(__fmul_rn(y[4 * t + 3], ep.inv_out_scale)));
-          quad_words_transpose(w, lane);
-          bytes_transpose4(w);
+            for (int i = 0; i < 16; ++i)
+              o[i * kRow8] = (int8_t)cvt_sat_s8(__fmul_rn(y[i], ep.inv_out_scale));
+          } else {
 #pragma unroll
-          for (int t = 0; t < 4; ++t) {
-            const uint32_t row = row0 + 4u * j4 + t;
-            if (in_tile && row < n_out) *(uint32_t*)(a.out + (size_t)row * COUT + chq) = w[t];
+            for (int i = 0; i < 16; ++i)
+              if (i < (int)rows) o[i * kRow8] = (int8_t)cvt_sat_s8(__fmul_rn(y[i], ep.inv_out_scale));
           }
         } else {
+          __half* o = (__half*)a.out + (size_t)row0 * COUT + ch;
+          if (rows == 16u) {
 #pragma unroll
-          for (int t = 0; t < 4; ++t) {
-            __half2 h0 = __floats2half2_rn(y[4 * t + 0], y[4 * t + 1]);
-            __half2 h1 = __floats2half2_rn(y[4 * t + 2], y[4 * t + 3]);
-            uint32_t w0 = *(uint32_t*)&h0, w1 = *(uint32_t*)&h1;
-            quad_transpose_h16(w0, w1, lane);
-            const uint32_t row = row0 + 4u * t + j4;
-            if (in_tile && row < n_out)
-              *(uint2*)(a.out + ((size_t)row * COUT + chq) * out_b) = make_uint2(w0, w1);
+            for (int i = 0; i < 16; ++i) o[i * COUT] = __float2half_rn(y[i]);
+          } else {
+#pragma unroll
+            for (int i = 0; i < 16; ++i)
+              if (i < (int)rows) o[i * COUT] = __float2half_rn(y[i]);
           }
         }
       }
@@ -613,9 +583,11 @@ int launch_one(const UmmaArgs& args, uint32_t launch_rows, cudaStream_t st) {
     if (dev >= 0 && dev < 64) attr_done[dev] = true;
   }
   uint32_t tiles = (launch_rows + 31) / 32;  // the kernel picks the tile height per launch
-  int grid = (int)(tiles < (uint32_t)kSmCount ? (tiles ? tiles : 1u) : (uint32_t)kSmCount);
+  const int grid = (int)(tiles < (uint32_t)kSmCount ? (tiles ? tiles : 1u) : (uint32_t)kSmCount);
+  UmmaArgs with_grid = args;
+  with_grid.grid_inv = grid > 1 ? 0xffffffffu / (uint32_t)grid + 1u : 0xffffffffu;
   SPCONVB_CUDA_TRY(launch_pdl(conv_umma_kernel<INT8, RB, COUT>, dim3(grid), dim3(kCtaThreads),
-                              kSmemBytes, st, args));
+                              kSmemBytes, st, with_grid));
   return SPCONVB_OK;
 }
 

@@ -328,6 +328,32 @@ def _f16_problem(n, cin, cout, seed, grid=(41, 180, 180), kvol=27):
     return coords, x, w, bias
 
 
+@pytest.mark.parametrize("n", [1, 31, 148 * 32, 148 * 32 + 1, 148 * 224 - 5, 148 * 256, 148 * 256 + 1,
+                               148 * 512 + 33])
+@pytest.mark.parametrize("cin,cout,kvol", [(16, 16, 27), (64, 64, 27), (128, 128, 27), (32, 128, 1),
+                                           (128, 32, 3)])
+def test_conv_int8_tile_heights_and_shared_tail(n, cin, cout, kvol):
+    """Row counts around the edges of the tile height the kernel picks (rows dealt to 148 CTAs in
+    multiples of 32, at most 256), for layers with fewer and with more K chunks than the stage
+    ring (in the latter the producers help to drain the last tile), with a residual; against the
+    CUDA-core kernel, bit for bit."""
+    ops = _ops()
+    rng = np.random.default_rng(n + cin)
+    nin = max(n // 2, 1)
+    m = _dev(np.where(rng.random((kvol, n)) < 0.5, rng.integers(0, nin, (kvol, n)), -1).astype(np.int32))
+    x = _dev(rng.integers(-128, 128, (nin, cin)).astype(np.int8))
+    res = _dev(rng.integers(-128, 128, (n, cout)).astype(np.int8))
+    wts = ops.ConvWeights(rng.integers(-127, 128, (cout, kvol, cin)).astype(np.int8), ops.I8,
+                          np.full(cout, 2e-4, np.float32), rng.standard_normal(cout))
+    n_ptr, st = ops.device_count(n), ops.new_status()
+    out = [ops.conv_forward(x, m, n_ptr, wts, out_kind=ops.I8, inv_out_scale=9.0, res=res,
+                            res_scale=0.1, mid_kind=ops.I8, mid_inv_scale=8.0, mid_scale=0.125,
+                            res_relu=True, force_simt=simt, status=st) for simt in (False, True)]
+    torch.cuda.synchronize()
+    _status_ok(st)
+    assert torch.equal(out[0], out[1])
+
+
 @pytest.mark.parametrize("c", [16, 32, 64, 128])
 def test_conv_fp16_tensor_core(c):
     """fp16 operands, fp32 accumulation in a different order than the oracle:
