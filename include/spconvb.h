@@ -69,6 +69,7 @@ extern "C" {
 
 /* flags */
 #define SPCONVB_FLAG_PREZEROED 1u /* caller already zeroed table / workspace */
+#define SPCONVB_FLAG_CLEAR_TAIL 2u /* rows after the last result are set to zero */
 
 SPCONVB_API const char* spconvb_version(void);
 SPCONVB_API const char* spconvb_error_string(int code);
@@ -84,6 +85,8 @@ SPCONVB_API const char* spconvb_error_string(int code);
  * have a power-of-two number of slots >= 8; its contents are opaque (the 8 cells of an
  * aligned run along the innermost axis share one 64-byte block of slots). */
 SPCONVB_API uint32_t spconvb_hash_slots(uint32_t cap_rows);
+/* A number of slots that makes lookups faster where memory is not short: up to four times as many. */
+SPCONVB_API uint32_t spconvb_hash_slots_fast(uint32_t cap_rows);
 
 /* Insert rows 0..*n_ptr-1 of `coords` into `table` (slot = (key+1)<<32 | row,
  * 0 = empty).  Zeroes the table first unless SPCONVB_FLAG_PREZEROED. */
@@ -347,6 +350,12 @@ SPCONVB_API int spconvb_voxelize(const spconvb_voxel_params* p, const void* poin
                                  uint32_t num_points, void* workspace, void* features,
                                  int32_t* indices, uint32_t* n_voxels_ptr, uint32_t* status,
                                  void* stream);
+/* The same with flags: SPCONVB_FLAG_CLEAR_TAIL zeroes the rows of features and indices after the last
+ * voxel, so that the caller need not clear the buffers first. */
+SPCONVB_API int spconvb_voxelize_flags(const spconvb_voxel_params* p, const void* points,
+                                       uint32_t num_points, void* workspace, void* features,
+                                       int32_t* indices, uint32_t* n_voxels_ptr, uint32_t flags,
+                                       uint32_t* status, void* stream);
 
 /* ------------------------------------------------------------------ engine
  * A whole backbone behind the C ABI.  These are the entry points the C++

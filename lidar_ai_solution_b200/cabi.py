@@ -7,6 +7,7 @@ if the shared object is missing, loading raises.
 from __future__ import annotations
 
 import ctypes as C
+import functools
 import os
 
 _PKG = os.path.dirname(os.path.abspath(__file__))
@@ -18,6 +19,7 @@ F16, I8 = 0, 1
 ACT_NONE, ACT_RELU = 0, 1
 ST_HASH_FULL, ST_DUPLICATE, ST_OVERFLOW, ST_TIMEOUT, ST_COORD_RANGE = 1, 2, 4, 8, 16
 FLAG_PREZEROED = 1
+FLAG_CLEAR_TAIL = 2
 E_SCRATCH_LIMIT = -8
 STATIC_SCRATCH_BYTES = 4 << 20
 
@@ -48,6 +50,7 @@ SYMBOLS = {
     "spconvb_version": (C.c_char_p, []),
     "spconvb_error_string": (C.c_char_p, [C.c_int]),
     "spconvb_hash_slots": (C.c_uint32, [C.c_uint32]),
+    "spconvb_hash_slots_fast": (C.c_uint32, [C.c_uint32]),
     "spconvb_hash_build": (C.c_int, [_VP, _VP, C.c_uint32, C.c_uint32, _I3, C.c_int32, _VP,
                                      C.c_uint32, C.c_uint32, _VP, _VP]),
     "spconvb_subm_map": (C.c_int, [_VP, _VP, C.c_uint32, C.c_uint32, _I3, C.c_int32, _I3, _I3, _VP,
@@ -87,6 +90,8 @@ SYMBOLS = {
     "spconvb_voxelize_workspace_bytes": (C.c_size_t, [C.POINTER(VoxelParams), C.c_uint32]),
     "spconvb_voxelize": (C.c_int, [C.POINTER(VoxelParams), _VP, C.c_uint32, _VP, _VP, _VP, _VP,
                                    _VP, _VP]),
+    "spconvb_voxelize_flags": (C.c_int, [C.POINTER(VoxelParams), _VP, C.c_uint32, _VP, _VP, _VP,
+                                         _VP, C.c_uint32, _VP, _VP]),
 }
 
 class CpHead(C.Structure):
@@ -137,8 +142,14 @@ def lib() -> C.CDLL:
     return _LIB
 
 
-def i3(v):
+@functools.lru_cache(maxsize=1024)
+def _i3(v):
     return (C.c_int32 * 3)(*[int(x) for x in v])
+
+
+def i3(v):
+    """Three numbers as the int32[3] the library reads (shared between calls: not to be written)."""
+    return _i3(tuple(v))
 
 
 def check(code: int, what: str = "spconvb call"):

@@ -164,7 +164,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   pdl_wait();  // nothing above reads or writes what an earlier kernel may still be working on
-  const uint32_t n_out = min(__ldg(a.n_out_ptr), a.cap);
+  const uint32_t n_out = min(load_after_wait(a.n_out_ptr), a.cap);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();

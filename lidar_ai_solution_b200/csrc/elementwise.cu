@@ -176,7 +176,7 @@ __global__ void scatter_dense_kernel(const void* __restrict__ feat, int in_kind,
   extern __shared__ __half tile[];  // [channels][33]
   __shared__ long long s_cell[32];
   pdl_wait();
-  const uint32_t n = min(*n_ptr, cap);
+  const uint32_t n = min(load_after_wait(n_ptr), cap);
   const int gp[3] = {g.g[p0], g.g[p1], g.g[p2]};
   const size_t vol = (size_t)gp[0] * gp[1] * gp[2];
   for (uint32_t row0 = blockIdx.x * 32; row0 < n; row0 += gridDim.x * 32) {

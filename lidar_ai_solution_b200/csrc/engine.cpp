@@ -743,7 +743,7 @@ int Engine::prepare(const int32_t grid[3], int batch) {
   for (size_t c = 0; c < coordsets.size(); ++c) {
     CoordSet& cs = coordsets[c];
     if (!cs.need_table) continue;
-    cs.slots = spconvb_hash_slots(cs.cap);
+    cs.slots = spconvb_hash_slots_fast(cs.cap);
     table_off[c] = zoff;
     zoff += align256(sizeof(uint64_t) * (size_t)cs.slots);
   }

@@ -6,12 +6,21 @@
 // before.
 #pragma once
 #include <cuda_runtime.h>
+#include <stdint.h>
 
 namespace spconvb {
 
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// A word an earlier kernel wrote.  Volatile: stays behind pdl_wait(), whatever the compiler knows
+// about the pointer.  (Loads that depend on its value stay behind it with it.)
+__device__ __forceinline__ uint32_t load_after_wait(const uint32_t* p) {
+  uint32_t v;
+  asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
 }
 
 template <typename... Params, typename... Args>

@@ -24,7 +24,7 @@ constexpr int kTaskWarps = kTaskThreads / 32;
 constexpr uint32_t kScanWords = kTaskThreads;  // bitmap words per scan block: one a thread
 
 __device__ __forceinline__ uint32_t task_rows(const RuleTask& t) {
-  return min(t.n_ptr ? __ldg(t.n_ptr) : t.n_host, t.cap);
+  return min(t.n_ptr ? load_after_wait(t.n_ptr) : t.n_host, t.cap);
 }
 
 // v % s == 0 and v / s for v >= 0, without the integer division when the stride is a power
@@ -57,7 +57,7 @@ __device__ __forceinline__ int32_t rank_lookup(const uint32_t* __restrict__ bitm
 // ---------------------------------------------------------------- the caller's rows
 __device__ __forceinline__ void task_count(const RuleTask& t) {
   if (threadIdx.x != 0) return;
-  const uint32_t n = t.n_ptr ? __ldg(t.n_ptr) : t.n_host;
+  const uint32_t n = t.n_ptr ? load_after_wait(t.n_ptr) : t.n_host;
   if (n > t.cap) set_status(t.status, SPCONVB_ST_OVERFLOW, n);
   *t.n_out = min(n, t.cap);
 }
@@ -744,13 +744,18 @@ static RuleTask row_task(int32_t kind, const int32_t* coords, const uint32_t* n_
 
 extern "C" {
 
-// Four slots a row up to 8 MB (a table the L2 holds many times over), two beyond: at half load
-// every second lookup of an absent cell goes on to a second dependent probe or more.  120 000
-// rows: SubM map 68 us with 2 slots a row.
 uint32_t spconvb_hash_slots(uint32_t cap_rows) {
   uint32_t s = 1024;
   while (s < 2u * cap_rows && s < 0x80000000u) s <<= 1;
-  while (s < 4u * cap_rows && s < (1u << 20)) s <<= 1;
+  return s;
+}
+
+// Eight slots a row up to 8 MB (a table the L2 holds many times over): at half load every second
+// lookup of an absent cell goes on to a second dependent probe or more.  120 000 rows: SubM map
+// 68 us with 2^18 slots, 33 with 2^19, 22 with 2^20.
+uint32_t spconvb_hash_slots_fast(uint32_t cap_rows) {
+  uint32_t s = spconvb_hash_slots(cap_rows);
+  while (s < 8u * cap_rows && s < (1u << 20)) s <<= 1;
   return s;
 }
 

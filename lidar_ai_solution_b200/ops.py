@@ -6,6 +6,7 @@ in exactly one ``spconvb_*`` call on the current CUDA stream.
 from __future__ import annotations
 
 import ctypes as C
+import math
 
 import numpy as np
 import torch
@@ -15,11 +16,11 @@ from .cabi import ACT_NONE, ACT_RELU, F16, I8  # noqa: F401
 
 
 def _stream():
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def _ptr(t):
-    return C.c_void_p(t.data_ptr()) if t is not None else None
+    return t.data_ptr() if t is not None else None
 
 
 def kind_of(t: torch.Tensor) -> int:
@@ -37,7 +38,7 @@ def device_count(n: int, device="cuda") -> torch.Tensor:
 
 def hash_build(coords, n_ptr, grid, batch=1, status=None, launch_rows=0):
     cap = coords.shape[0]
-    slots = cabi.lib().spconvb_hash_slots(cap)
+    slots = cabi.lib().spconvb_hash_slots_fast(cap)
     table = torch.empty(slots, dtype=torch.int64, device=coords.device)
     cabi.check(cabi.lib().spconvb_hash_build(_ptr(coords), _ptr(n_ptr), cap, launch_rows,
                                              cabi.i3(grid), batch, _ptr(table), slots, 0,
@@ -48,7 +49,7 @@ def hash_build(coords, n_ptr, grid, batch=1, status=None, launch_rows=0):
 def subm_map(coords, n_ptr, grid, table, ksize=(3, 3, 3), dilation=(1, 1, 1), batch=1,
              status=None, launch_rows=0):
     cap = coords.shape[0]
-    kvol = int(np.prod(ksize))
+    kvol = math.prod(ksize)
     m = torch.empty((kvol, cap), dtype=torch.int32, device=coords.device)
     cabi.check(cabi.lib().spconvb_subm_map(_ptr(coords), _ptr(n_ptr), cap, launch_rows,
                                            cabi.i3(grid), batch, cabi.i3(ksize),
@@ -73,8 +74,8 @@ def down_map(coords, n_ptr, grid, table, ksize, stride, pad, dilation=(1, 1, 1),
     cap_in = coords.shape[0]
     og = out_grid(grid, ksize, stride, pad, dilation)
     if cap_out is None:
-        cap_out = max(1, min(cap_in * int(np.prod(ksize)), batch * int(np.prod(og))))
-    kvol = int(np.prod(ksize))
+        cap_out = max(1, min(cap_in * math.prod(ksize), batch * math.prod(og)))
+    kvol = math.prod(ksize)
     ws = torch.empty(cabi.lib().spconvb_down_workspace_bytes(cabi.i3(og), batch),
                      dtype=torch.uint8, device=dev)
     oc = torch.zeros((cap_out, 4), dtype=torch.int32, device=dev)
@@ -104,7 +105,7 @@ def subm_map_ranked(coords, n_ptr, grid, ws, ksize=(3, 3, 3), dilation=(1, 1, 1)
                     status=None, launch_rows=0):
     """SubM map of rows that came out of ``down_map`` (ranked in its workspace ``ws``)."""
     cap = coords.shape[0]
-    kvol = int(np.prod(ksize))
+    kvol = math.prod(ksize)
     m = torch.empty((kvol, cap), dtype=torch.int32, device=coords.device)
     cabi.check(cabi.lib().spconvb_subm_map_ranked(_ptr(coords), _ptr(n_ptr), cap, launch_rows,
                                                   cabi.i3(grid), batch, cabi.i3(ksize),
@@ -118,7 +119,7 @@ def inverse_map(coords, n_ptr, grid, ws, cap_coarse, ksize, stride, pad, dilatio
     """Map of the inverse conv of a strided rulebook: ``coords`` are the rows that went INTO
     ``down_map`` (with ``return_ws=True``), ``ws`` its workspace, ``cap_coarse`` its cap_out."""
     cap = coords.shape[0]
-    kvol = int(np.prod(ksize))
+    kvol = math.prod(ksize)
     m = torch.empty((kvol, cap), dtype=torch.int32, device=coords.device)
     cabi.check(cabi.lib().spconvb_inverse_map(_ptr(coords), _ptr(n_ptr), cap, launch_rows,
                                               cabi.i3(grid), batch, cabi.i3(ksize), cabi.i3(stride),
@@ -158,15 +159,10 @@ def conv_forward(x, m, n_out_ptr, wts: ConvWeights, act=ACT_NONE, out_kind=F16,
                  out=None, wait_test=0, n_in_ptr=None):
     """``n_in_ptr`` (device row count of ``x``) is a hint; results do not depend on it."""
     cap = m.shape[1]
-    p = cabi.ConvParams()
-    p.compute, p.cin, p.cout, p.kvol = wts.compute, wts.cin, wts.cout, wts.kvol
-    p.act, p.out_kind, p.inv_out_scale = act, out_kind, inv_out_scale
-    p.res = res.data_ptr() if res is not None else None
-    p.res_kind = kind_of(res) if res is not None else F16
-    p.res_scale, p.mid_kind = res_scale, mid_kind
-    p.mid_inv_scale, p.mid_scale, p.res_relu = mid_inv_scale, mid_scale, int(res_relu)
-    p.force_simt = int(force_simt)
-    p.wait_test = int(wait_test)
+    p = cabi.ConvParams(
+        wts.compute, wts.cin, wts.cout, wts.kvol, act, out_kind, inv_out_scale, _ptr(res),
+        kind_of(res) if res is not None else F16, res_scale, mid_kind, mid_inv_scale, mid_scale,
+        int(res_relu), int(force_simt), int(wait_test))
     if n_in_ptr is not None:
         p.n_in_ptr, p.cap_in = n_in_ptr.data_ptr(), x.shape[0]
     if out is None:
@@ -261,12 +257,14 @@ def voxelize(points, params, status=None):
     """points: cuda tensor [n, F] float32/float16.  Returns (features, indices, n_ptr)."""
     n = points.shape[0]
     lib = cabi.lib()
-    ws = torch.empty(max(256, lib.spconvb_voxelize_workspace_bytes(C.byref(params), max(n, 1))),
-                     dtype=torch.uint8, device=points.device)
-    feat = torch.zeros((params.max_voxels, params.num_features), dtype=torch.float16,
-                       device=points.device)
-    idx = torch.zeros((params.max_voxels, 4), dtype=torch.int32, device=points.device)
-    n_ptr = torch.zeros(1, dtype=torch.int32, device=points.device)
-    cabi.check(lib.spconvb_voxelize(C.byref(params), _ptr(points), n, _ptr(ws), _ptr(feat),
-                                    _ptr(idx), _ptr(n_ptr), _ptr(status), _stream()), "voxelize")
+    dev = points.device
+    p = C.byref(params)
+    ws = torch.empty(max(256, lib.spconvb_voxelize_workspace_bytes(p, max(n, 1))),
+                     dtype=torch.uint8, device=dev)
+    feat = torch.empty((params.max_voxels, params.num_features), dtype=torch.float16, device=dev)
+    idx = torch.empty((params.max_voxels, 4), dtype=torch.int32, device=dev)
+    n_ptr = torch.empty(1, dtype=torch.int32, device=dev)
+    cabi.check(lib.spconvb_voxelize_flags(p, _ptr(points), n, _ptr(ws), _ptr(feat), _ptr(idx),
+                                          _ptr(n_ptr), cabi.FLAG_CLEAR_TAIL, _ptr(status),
+                                          _stream()), "voxelize")
     return feat, idx, n_ptr

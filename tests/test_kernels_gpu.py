@@ -702,3 +702,23 @@ def test_conv_int8_shape_sweep_bit_exact(cin, cout, n, kind, i8_out, seed):
     torch.cuda.synchronize()
     _status_ok(st)
     assert np.array_equal(out.cpu().numpy()[:n_out].view(np.uint8), ref[:n_out].view(np.uint8))
+
+
+@pytest.mark.parametrize("n", [1, 31, 511, 512, 513, 5000])
+@pytest.mark.parametrize("max_pts", [1, 2, 10, 16])
+def test_voxelizer_crowded_voxels_and_cleared_tail(n, max_pts):
+    """Few voxels with many points (every kept-slot cascade full), point counts around the scan
+    blocks, and the rows after the last voxel zero in buffers that were not."""
+    ops = _ops()
+    pts = np.random.default_rng(n).uniform(0, 3, (n, 4)).astype(np.float32)
+    params = ops.voxel_params((0, 0, 0, 3, 3, 3), (1, 1, 1), (3, 3, 3), 4, 0, max_pts, 40, 0)
+    st = ops.new_status()
+    torch.full((40 * 4 * 4 * 8,), 77, dtype=torch.int32, device="cuda")  # dirt for the allocator
+    feat, idx, n_ptr = ops.voxelize(_dev(pts), params, status=st)
+    _status_ok(st)
+    ref_f, ref_i, _ = orc.voxelize(pts, (0, 0, 0, 3, 3, 3), (1, 1, 1), (3, 3, 3), 40, max_pts)
+    k = int(n_ptr.item())
+    assert k == len(ref_f)
+    assert np.array_equal(idx[:k].cpu().numpy(), ref_i)
+    assert np.array_equal(feat[:k].cpu().numpy().view(np.uint16), ref_f.view(np.uint16))
+    assert int(feat[k:].abs().sum().item()) == 0 and int(idx[k:].abs().sum().item()) == 0
