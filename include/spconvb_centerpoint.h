@@ -75,6 +75,13 @@ SPCONVB_API int spconvb_cp_postprocess(const spconvb_cp_head* heads, int32_t num
                                        const spconvb_cp_params* p, void* workspace,
                                        size_t workspace_bytes, float* out_boxes,
                                        uint32_t* out_count, void* stream);
+/* The same; the number of boxes is also stored to host memory the device can write (pinned), where
+ * the host may read it once the stream has run: no copy of its own.  out_count_host may be NULL. */
+SPCONVB_API int spconvb_cp_postprocess_host(const spconvb_cp_head* heads, int32_t num_tasks,
+                                            const spconvb_cp_params* p, void* workspace,
+                                            size_t workspace_bytes, float* out_boxes,
+                                            uint32_t* out_count, uint32_t* out_count_host,
+                                            void* stream);
 
 /* Per-task intermediate results left in the workspace by the last call, for tests:
  * n_det detections ranked by score as [n_det][11] = x y z dx dy dz vx vy rot label score

@@ -115,6 +115,8 @@ SYMBOLS.update({
     "spconvb_cp_workspace_bytes": (C.c_size_t, [C.POINTER(CpParams), C.c_int32]),
     "spconvb_cp_postprocess": (C.c_int, [C.POINTER(CpHead), C.c_int32, C.POINTER(CpParams), _VP,
                                          C.c_size_t, _VP, _VP, _VP]),
+    "spconvb_cp_postprocess_host": (C.c_int, [C.POINTER(CpHead), C.c_int32, C.POINTER(CpParams), _VP,
+                                              C.c_size_t, _VP, _VP, _VP, _VP]),
     "spconvb_cp_task_detections": (C.c_int, [C.POINTER(CpParams), C.c_int32, _VP, C.c_int32,
                                              C.POINTER(_VP), C.POINTER(_VP)]),
     "spconvb_cp_rotated_iou": (C.c_int, [_VP, _VP, C.c_int32, _VP, _VP]),

@@ -8,6 +8,7 @@ out, with no host synchronisation in between.
 from __future__ import annotations
 
 import ctypes as C
+import struct
 
 import torch
 
@@ -48,8 +49,16 @@ class PostProcess:
         self.boxes = torch.zeros((num_tasks * self.params.nms_post_max, 11), dtype=torch.float32,
                                  device=device)
         self.count = torch.zeros(1, dtype=torch.int32, device=device)
+        # the kernels also store the count here, where the host reads it without a copy
+        self._count_host = torch.zeros(1, dtype=torch.int32).pin_memory()
+        self._count_view = self._count_host.numpy()
         self._heads = (cabi.CpHead * num_tasks)()
+        self._pack = struct.Struct("6Q2i" * num_tasks)
+        p = self.params
+        self._shapes = [(k, torch.Size((ch, p.H, p.W)), torch.Size((1, ch, p.H, p.W)))
+                        for k, ch in HEAD_CHANNELS.items()]
         self._keep = None
+        self._stream = None
 
     def run(self, heads, label_offsets=TASK_LABEL_OFFSET, stream=None):
         """heads: one dict per task of contiguous cuda fp16 tensors ``reg height dim rot vel hm``
@@ -57,29 +66,36 @@ class PostProcess:
         the stream has run."""
         assert len(heads) == self.num_tasks
         p = self.params
+        half = torch.float16
+        words = []
         for t, h in enumerate(heads):
-            for k, ch in HEAD_CHANNELS.items():
+            for k, chw, nchw in self._shapes:
                 x = h[k]
-                assert x.is_cuda and x.dtype == torch.float16 and x.is_contiguous()
-                assert tuple(x.shape[-3:]) == (ch, p.H, p.W), (k, tuple(x.shape))
-                setattr(self._heads[t], k, x.data_ptr())
+                shape = x.shape
+                assert x.dtype is half and x.is_cuda and x.is_contiguous()
+                assert shape == chw or shape == nchw or shape[-3:] == chw, (k, tuple(shape))
+                words.append(x.data_ptr())
             hm = h["hm"]
-            assert hm.is_cuda and hm.dtype == torch.float16 and hm.is_contiguous()
-            assert tuple(hm.shape[-2:]) == (p.H, p.W)
-            self._heads[t].hm = hm.data_ptr()
-            self._heads[t].num_classes = hm.shape[-3]
-            self._heads[t].label_offset = label_offsets[t]
+            shape = hm.shape
+            assert hm.dtype is half and hm.is_cuda and hm.is_contiguous()
+            assert shape[-2] == p.H and shape[-1] == p.W
+            words += (hm.data_ptr(), shape[-3], label_offsets[t])
+        self._pack.pack_into(self._heads, 0, *words)
         self._keep = heads
         s = stream if stream is not None else torch.cuda.current_stream()
-        cabi.check(self.lib.spconvb_cp_postprocess(
+        self._stream = s
+        cabi.check(self.lib.spconvb_cp_postprocess_host(
             self._heads, self.num_tasks, C.byref(p), self.workspace.data_ptr(),
             self.workspace.numel(), self.boxes.data_ptr(), self.count.data_ptr(),
-            C.c_void_p(s.cuda_stream)), "cp_postprocess")
+            self._count_host.data_ptr(), s.cuda_stream), "cp_postprocess")
 
     def result(self):
         """Synchronises and returns the kept boxes [n, 11] (a copy)."""
-        n = int(self.count.item())
-        return self.boxes[:n].clone()
+        s = torch.cuda.current_stream()
+        if self._stream is not None and self._stream != s:
+            self._stream.synchronize()
+        s.synchronize()
+        return self.boxes[:int(self._count_view[0])].clone()
 
     def task_detections(self, task):
         """Ranked detections of one task before NMS, [n, 11] = x y z dx dy dz vx vy rot label

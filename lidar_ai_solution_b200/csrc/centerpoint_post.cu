@@ -5,19 +5,19 @@
 // candidate list to the host, sorts it there, copies it back, copies the suppression mask to
 // the host and scans it there: three stream synchronisations per task, six tasks per frame.
 //
-// Here one call enqueues four kernels for all tasks together (blockIdx selects the task):
+// Here one call enqueues a clear and three kernels for all tasks together (blockIdx selects the
+// task); a few hundred boxes leave the GPU idle, so what counts is the number of dependent steps:
 //   candidates  one thread per heat-map cell: class arg-max of the sigmoid, score and centre
-//               range filters; survivors append a 64-bit key (score bits | cell | label)
-//   rank        one CTA per task: if more than 1024 candidates, an 8-pass radix select finds
-//               the max_det largest keys; a bitonic sort in shared memory orders them; the
-//               box parameters (exp, atan2) are evaluated for the ranked cells only
-//   mask        pairwise rotated IoU >= threshold above the diagonal, in tiles of 16 x 64
-//               pairs: a reach test queues the pairs that can overlap, then the queue is
-//               spread over full warps; corners and the trigonometry of every box are
-//               prepared once by the rank kernel
-//   scan        one warp per task walks the ranking with the mask in shared memory and keeps
-//               the first nms_post_max survivors; the last CTA to finish packs all tasks'
-//               boxes into the caller's list
+//               range filters; survivors append a 64-bit key (score bits | cell | label) and are
+//               counted in a histogram of their scores
+//   rank        16 CTAs per task: the histogram tells which scores the max_det best can have; the
+//               rank of a key is the number of greater keys among those, counted by a warp per
+//               key, so nothing is sorted; the box parameters (exp, atan2), corners and the
+//               trigonometry are evaluated for the ranked cells only
+//   mask        pairwise rotated IoU >= threshold below the diagonal, in tiles of 16 x 64
+//               pairs: cheap upper bounds queue the pairs whose IoU can reach the threshold, then
+//               the queue is spread over full warps; the last CTA of a task walks the ranking, 64
+//               boxes at a time, and the last task packs all boxes into the caller's list
 //
 // This file is compiled without multiply-add contraction so that every product and sum rounds
 // as in the reference's expression order on a CPU; only the library functions (expf, sinf,
@@ -28,6 +28,7 @@
 #include <stdint.h>
 
 #include "common.cuh"
+#include "pdl.cuh"
 #include "spconvb.h"
 #include "spconvb_centerpoint.h"
 
@@ -36,9 +37,15 @@ namespace {
 
 constexpr int kDet = 11;         // floats per detection
 constexpr int kBoxStride = 16;   // floats per prepared NMS box (struct BoxRec)
-constexpr int kRankThreads = 1024;
+constexpr int kMaxDet = 1024;
 constexpr int kMaskWords = 16;   // 64-bit words per mask row: 1024 / 64
-constexpr int kScanStagedRows = 320;  // mask rows the scan keeps in shared memory (40 KB)
+// Scores by their leading bits: bin 0 up to 2^-5, then 512 bins an octave (sigmoids end at 1).
+constexpr uint32_t kScoreBase = 0x3d000000u;  // bits of 2^-5
+constexpr int kScoreShift = 14;
+constexpr int kScoreBins = 2816;
+__device__ __forceinline__ uint32_t score_bin(uint32_t bits) {
+  return bits <= kScoreBase ? 0u : min((bits - kScoreBase) >> kScoreShift, (uint32_t)kScoreBins - 1u);
+}
 
 struct TaskBuffers {
   uint32_t* n_cand;
@@ -47,8 +54,10 @@ struct TaskBuffers {
   unsigned long long* cand;  // [H*W]
   float* det;                // [max_det][11]
   float* box;                // [max_det][16], BoxRec
-  unsigned long long* mask;  // [max_det][16]
-  float* kept;               // [post_max][11]
+  unsigned long long* mask;  // [max_det][16]: bit i of row j = the earlier box i suppresses box j
+  uint32_t* kept;            // [post_max] ranks of the boxes that stay
+  uint32_t* hist;            // [kScoreBins]
+  uint32_t* ticket;          // mask CTAs that are done
 };
 
 struct PostArgs {
@@ -59,6 +68,7 @@ struct PostArgs {
   uint32_t* ticket;
   float* out_boxes;
   uint32_t* out_count;
+  uint32_t* out_count_host;  // may be null
 };
 
 struct Layout {
@@ -72,13 +82,14 @@ __host__ inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a
 
 __host__ Layout layout_of(const spconvb_cp_params& p, int tasks) {
   Layout l{};
-  l.counters_bytes = align_up(sizeof(uint32_t) * (1 + 3 * (size_t)SPCONVB_CP_MAX_TASKS), 256);
+  l.counters_bytes = align_up(
+      sizeof(uint32_t) * (1 + 4 * (size_t)SPCONVB_CP_MAX_TASKS + kScoreBins * (size_t)tasks), 256);
   size_t off = 0;
   l.cand = off; off += align_up(sizeof(unsigned long long) * (size_t)p.H * p.W, 256);
   l.det = off;  off += align_up(sizeof(float) * kDet * (size_t)p.max_det, 256);
   l.box = off;  off += align_up(sizeof(float) * kBoxStride * (size_t)p.max_det, 256);
   l.mask = off; off += align_up(sizeof(unsigned long long) * kMaskWords * (size_t)p.max_det, 256);
-  l.kept = off; off += align_up(sizeof(float) * kDet * (size_t)p.nms_post_max, 256);
+  l.kept = off; off += align_up(sizeof(uint32_t) * (size_t)p.nms_post_max, 256);
   l.per_task = off;
   l.total = l.counters_bytes + l.per_task * (size_t)tasks;
   return l;
@@ -90,14 +101,16 @@ __host__ void bind_buffers(const Layout& l, void* workspace, int tasks, PostArgs
   a.ticket = counters;
   for (int t = 0; t < tasks; ++t) {
     char* tb = base + l.counters_bytes + l.per_task * (size_t)t;
-    a.buf[t].n_cand = counters + 1 + 3 * t;
-    a.buf[t].n_det = counters + 2 + 3 * t;
-    a.buf[t].n_kept = counters + 3 + 3 * t;
+    a.buf[t].n_cand = counters + 1 + 4 * t;
+    a.buf[t].n_det = counters + 2 + 4 * t;
+    a.buf[t].n_kept = counters + 3 + 4 * t;
+    a.buf[t].ticket = counters + 4 + 4 * t;
+    a.buf[t].hist = counters + 1 + 4 * SPCONVB_CP_MAX_TASKS + kScoreBins * t;
     a.buf[t].cand = (unsigned long long*)(tb + l.cand);
     a.buf[t].det = (float*)(tb + l.det);
     a.buf[t].box = (float*)(tb + l.box);
     a.buf[t].mask = (unsigned long long*)(tb + l.mask);
-    a.buf[t].kept = (float*)(tb + l.kept);
+    a.buf[t].kept = (uint32_t*)(tb + l.kept);
   }
 }
 
@@ -137,6 +150,7 @@ __global__ void cp_candidates_kernel(const PostArgs a) {
                                  (unsigned long long)label;
   const uint32_t slot = atomicAdd(a.buf[task].n_cand, 1u);
   a.buf[task].cand[slot] = key;  // at most one key per cell, so slot < H*W
+  atomicAdd(a.buf[task].hist + score_bin(__float_as_uint(score)), 1u);
 }
 
 // ------------------------------------------------------------------ rotated overlap
@@ -281,99 +295,65 @@ __device__ __forceinline__ void load_box(const float* p, BoxRec& r) {
 }
 
 // ------------------------------------------------------------------ rank
-__global__ void __launch_bounds__(kRankThreads) cp_rank_kernel(const PostArgs a) {
-  const int task = blockIdx.x;
-  const TaskBuffers& b = a.buf[task];
-  const spconvb_cp_head& hd = a.head[task];
-  const int HW = a.p.H * a.p.W;
+constexpr int kRankParts = 16;
+constexpr int kRankThreads = 256;
+constexpr int kRankList = 2048;  // keys a CTA compares with
+
+// The K-th largest key, most significant byte first (keys are distinct): for frames where so many
+// scores are equal to within a histogram bin that the list would not hold them.
+__device__ unsigned long long select_kth(const unsigned long long* cand, uint32_t n, uint32_t K,
+                                         uint32_t* hist, unsigned long long* s_prefix,
+                                         uint32_t* s_need) {
   const int tid = threadIdx.x;
-  __shared__ unsigned long long keys[kRankThreads];
-  __shared__ uint32_t hist[256];
-  __shared__ unsigned long long s_prefix;
-  __shared__ uint32_t s_need, s_fill;
-
-  const uint32_t n = min(*b.n_cand, (uint32_t)HW);
-  const uint32_t K = min(n, (uint32_t)a.p.max_det);
-  keys[tid] = 0ull;
-  if (n <= (uint32_t)kRankThreads) {
-    if ((uint32_t)tid < n) keys[tid] = b.cand[tid];
+  if (tid == 0) { *s_prefix = 0ull; *s_need = K; }
+  for (int shift = 56; shift >= 0; shift -= 8) {
+    hist[tid] = 0u;
     __syncthreads();
-  } else {
-    // the K-th largest key, most significant byte first (keys are distinct)
-    if (tid == 0) { s_prefix = 0ull; s_need = K; s_fill = 0u; }
-    for (int shift = 56; shift >= 0; shift -= 8) {
-      if (tid < 256) hist[tid] = 0u;
-      __syncthreads();
-      const unsigned long long prefix = s_prefix;
-      const unsigned long long hi = shift == 56 ? 0ull : (~0ull << (shift + 8));
-      for (uint32_t base = 0; base < n; base += kRankThreads) {
-        // keys of one score share their upper bytes: lanes with the same digit add once
-        const uint32_t i = base + tid;
-        const unsigned long long k = i < n ? b.cand[i] : 0ull;
-        const bool live = i < n && ((k ^ prefix) & hi) == 0ull;
-        const uint32_t digit = live ? ((uint32_t)(k >> shift) & 255u) : 256u;
-        const uint32_t peers = __match_any_sync(0xffffffffu, digit);
-        if (live && (tid & 31) == __ffs(peers) - 1) atomicAdd(&hist[digit], (uint32_t)__popc(peers));
-      }
-      __syncthreads();
-      if (tid < 32) {
-        // lane l owns bins 8l..8l+7; the digit is the highest bin whose count, together with
-        // everything above it, reaches what is still needed
-        uint32_t mine[8], sum = 0u;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) { mine[k] = hist[tid * 8 + k]; sum += mine[k]; }
-        uint32_t incl = sum;  // becomes the count in this lane's bins and in all higher lanes
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-          const uint32_t v = __shfl_down_sync(0xffffffffu, incl, d);
-          if (tid + d < 32) incl += v;
-        }
-        const uint32_t above = incl - sum;
-        const uint32_t need = s_need;
-        const bool here = above < need && incl >= need;  // exactly one lane
-        if (here) {
-          uint32_t acc = above;
-          int k = 7;
-          for (; k > 0; --k) {
-            if (acc + mine[k] >= need) break;
-            acc += mine[k];
-          }
-          s_need = need - acc;
-          s_prefix = prefix | ((unsigned long long)(tid * 8 + k) << shift);
-        }
-      }
-      __syncthreads();
+    const unsigned long long prefix = *s_prefix;
+    const unsigned long long hi = shift == 56 ? 0ull : (~0ull << (shift + 8));
+    for (uint32_t base = 0; base < n; base += kRankThreads) {
+      // keys of one score share their upper bytes: lanes with the same digit add once
+      const uint32_t i = base + tid;
+      const unsigned long long k = i < n ? cand[i] : 0ull;
+      const bool live = i < n && ((k ^ prefix) & hi) == 0ull;
+      const uint32_t digit = live ? ((uint32_t)(k >> shift) & 255u) : 256u;
+      const uint32_t peers = __match_any_sync(0xffffffffu, digit);
+      if (live && (tid & 31) == __ffs(peers) - 1) atomicAdd(&hist[digit], (uint32_t)__popc(peers));
     }
-    const unsigned long long kth = s_prefix;
-    for (uint32_t i = tid; i < n; i += kRankThreads) {
-      const unsigned long long k = b.cand[i];
-      if (k >= kth) {
-        const uint32_t pos = atomicAdd(&s_fill, 1u);
-        if (pos < (uint32_t)kRankThreads) keys[pos] = k;
+    __syncthreads();
+    if (tid < 32) {
+      // lane l owns bins 8l..8l+7; the digit is the highest bin whose count, together with
+      // everything above it, reaches what is still needed
+      uint32_t mine[8], sum = 0u;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) { mine[k] = hist[tid * 8 + k]; sum += mine[k]; }
+      uint32_t incl = sum;  // becomes the count in this lane's bins and in all higher lanes
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t v = __shfl_down_sync(0xffffffffu, incl, d);
+        if (tid + d < 32) incl += v;
+      }
+      const uint32_t above = incl - sum, need = *s_need;
+      if (above < need && incl >= need) {  // exactly one lane
+        uint32_t acc = above;
+        int k = 7;
+        for (; k > 0; --k) {
+          if (acc + mine[k] >= need) break;
+          acc += mine[k];
+        }
+        *s_need = need - acc;
+        *s_prefix = prefix | ((unsigned long long)(tid * 8 + k) << shift);
       }
     }
     __syncthreads();
   }
+  return *s_prefix;
+}
 
-  // bitonic sort, descending (padding keys are 0 and end up last)
-  const int filled = n <= (uint32_t)kRankThreads ? (int)n : (int)K;  // keys beyond are zero padding
-  int sort_n = 32;
-  while (sort_n < filled) sort_n <<= 1;
-  for (int size = 2; size <= sort_n; size <<= 1) {
-    for (int stride = size >> 1; stride > 0; stride >>= 1) {
-      const int partner = tid ^ stride;
-      if (partner > tid && partner < sort_n) {
-        const unsigned long long x = keys[tid], y = keys[partner];
-        const bool descending = (tid & size) == 0;
-        if ((x < y) == descending) { keys[tid] = y; keys[partner] = x; }
-      }
-      __syncthreads();
-    }
-  }
-
-  if (tid == 0) *b.n_det = K;
-  if ((uint32_t)tid >= K) return;
-  const unsigned long long key = keys[tid];
+// The detection and the prepared box of a ranked cell.
+__device__ __forceinline__ void rank_write(const PostArgs& a, const spconvb_cp_head& hd,
+                                           const TaskBuffers& b, unsigned long long key,
+                                           uint32_t rank, int HW) {
   const int cell = (int)(0xFFFFFFu - (uint32_t)((key >> 8) & 0xFFFFFFull));
   const int label = (int)(key & 0xFFull);
   const float score = __uint_as_float((uint32_t)(key >> 32));
@@ -388,12 +368,109 @@ __global__ void __launch_bounds__(kRankThreads) cp_rank_kernel(const PostArgs a)
   const float dz = expf(ldh(hd.dim, 2 * HW + cell));
   const float vx = ldh(hd.vel, cell), vy = ldh(hd.vel, HW + cell);
   const float rs = atan2f(ldh(hd.rot, cell), ldh(hd.rot, HW + cell));
-  float* d = b.det + (size_t)tid * kDet;
+  float* d = b.det + (size_t)rank * kDet;
   d[0] = xs; d[1] = ys; d[2] = zs; d[3] = dx; d[4] = dy; d[5] = dz;
   d[6] = vx; d[7] = vy; d[8] = rs; d[9] = (float)label; d[10] = score;
   // the box NMS sees: length and width swapped, yaw turned into the lidar frame
   const float nms_box[7] = {xs, ys, zs, dy, dx, dz, (float)(-(double)rs - 3.141592653 * 0.5)};
-  prepare_box(nms_box, *(BoxRec*)(b.box + (size_t)tid * kBoxStride));
+  prepare_box(nms_box, *(BoxRec*)(b.box + (size_t)rank * kBoxStride));
+}
+
+__global__ void __launch_bounds__(kRankThreads) cp_rank_kernel(const PostArgs a) {
+  const int task = blockIdx.y, part = blockIdx.x, tid = threadIdx.x;
+  const uint32_t lane = tid & 31u, warp = tid >> 5;
+  const TaskBuffers& b = a.buf[task];
+  const spconvb_cp_head& hd = a.head[task];
+  const int HW = a.p.H * a.p.W;
+  __shared__ unsigned long long list[kRankList], own[kRankList];
+  __shared__ uint16_t rank_of[kRankList];
+  __shared__ uint32_t hist[kRankThreads];
+  __shared__ unsigned long long s_prefix;
+  __shared__ uint32_t s_need, s_list, s_own;
+  pdl_wait();
+
+  const uint32_t n = min(load_after_wait(b.n_cand), (uint32_t)HW);
+  const uint32_t K = min(n, (uint32_t)a.p.max_det);
+  if (part == 0 && tid == 0) *b.n_det = K;
+  if (tid == 0) { s_list = 0u; s_own = 0u; s_need = 0u; }
+  __syncthreads();
+  unsigned long long least = 0ull;  // keys below cannot be among the K best
+  if (n > (uint32_t)kMaxDet) {
+    // the bin in which the K-th best score lies: every thread sums kBinsEach bins, the sums are
+    // scanned from the top
+    constexpr int kBinsEach = kScoreBins / kRankThreads;
+    static_assert(kBinsEach * kRankThreads == kScoreBins, "bins per thread");
+    uint32_t mine[kBinsEach], sum = 0u;
+#pragma unroll
+    for (int k = 0; k < kBinsEach; ++k) {
+      mine[k] = b.hist[tid * kBinsEach + k];
+      sum += mine[k];
+    }
+    uint32_t incl = sum;  // the bins of this lane and of all higher lanes of the warp
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const uint32_t v = __shfl_down_sync(0xffffffffu, incl, d);
+      if (lane + d < 32u) incl += v;
+    }
+    if (lane == 0) hist[warp] = incl;
+    __syncthreads();
+    uint32_t above = incl - sum;
+    for (uint32_t w = warp + 1; w < kRankThreads / 32; ++w) above += hist[w];
+    if (above < K && above + sum >= K) {  // exactly one thread
+      uint32_t acc = above;
+      int k = kBinsEach - 1;
+      for (; k > 0; --k) {
+        if (acc + mine[k] >= K) break;
+        acc += mine[k];
+      }
+      const uint32_t bin = (uint32_t)(tid * kBinsEach + k);
+      s_prefix = bin == 0u ? 0ull
+                           : (unsigned long long)(kScoreBase + (bin << kScoreShift)) << 32;
+      s_need = acc + mine[k];  // keys from that bin on
+    }
+    __syncthreads();
+    least = s_prefix;
+    if (s_need > (uint32_t)kRankList) {
+      __syncthreads();
+      least = select_kth(b.cand, n, K, hist, &s_prefix, &s_need);
+    }
+  }
+  // the keys that count, in any order; this part ranks those at positions 32 part, 32 (part +
+  // 16), ... of the candidates
+#pragma unroll 4
+  for (uint32_t base = 0; base < n; base += kRankThreads) {
+    const uint32_t i = base + tid;
+    const unsigned long long k = i < n ? b.cand[i] : 0ull;
+    const bool in = i < n && k >= least;
+    const uint32_t vote = __ballot_sync(0xffffffffu, in);
+    if (!vote) continue;
+    const bool mine = ((i >> 5) % kRankParts) == (uint32_t)part;
+    uint32_t at = 0, own_at = 0;
+    if (lane == 0) {
+      at = atomicAdd(&s_list, (uint32_t)__popc(vote));
+      if (mine) own_at = atomicAdd(&s_own, (uint32_t)__popc(vote));
+    }
+    const uint32_t off = __popc(vote & ((1u << lane) - 1u));
+    at = __shfl_sync(0xffffffffu, at, 0) + off;
+    own_at = __shfl_sync(0xffffffffu, own_at, 0) + off;
+    if (in && at < (uint32_t)kRankList) list[at] = k;
+    if (in && mine && own_at < (uint32_t)kRankList) own[own_at] = k;
+  }
+  __syncthreads();
+  const uint32_t count = min(s_list, (uint32_t)kRankList), owned = min(s_own, (uint32_t)kRankList);
+  for (uint32_t o = warp; o < owned; o += kRankThreads / 32) {
+    const unsigned long long k = own[o];
+    uint32_t greater = 0;
+    for (uint32_t i = lane; i < count; i += 32) greater += list[i] > k ? 1u : 0u;
+    greater = __reduce_add_sync(0xffffffffu, greater);
+    if (lane == 0) rank_of[o] = (uint16_t)greater;
+  }
+  __syncthreads();
+  for (uint32_t o = tid; o < owned; o += kRankThreads) {
+    const uint32_t r = rank_of[o];
+    if (r >= K) continue;
+    rank_write(a, hd, b, own[o], r, HW);
+  }
 }
 
 // ------------------------------------------------------------------ mask
@@ -401,151 +478,208 @@ constexpr int kMaskRows = 16;          // ranked boxes per tile; divides 64, so 
 constexpr int kMaskCtasPerTask = 148;
 constexpr int kMaskThreads = 128;
 
-// One tile = 16 rows x 64 partners.  Pass 1: every thread tests 8 pairs for reach (three floats
-// per box, staged in shared memory) and queues the few that can overlap.  Pass 2: the queued
-// pairs are spread over the threads one by one, so the long overlap computation runs with full
-// warps instead of one lane in 32.
+// The greedy walk over one task's ranking, by one CTA.  64 boxes at a time: two threads a box
+// look whether an earlier kept box suppresses it (its mask words are fetched while the 64 before
+// are decided), then the first warp decides among the 64: a box stays when every box of them that
+// suppresses it is out, and is out when one of them stays, so the rounds are as many as the
+// longest chain of suppressions and not as the boxes.  Boxes after the first nms_post_max
+// survivors cannot reach the output.
+__device__ void walk_ranking(const PostArgs& a, const TaskBuffers& b, int m) {
+  constexpr int kEach = kMaskWords / 2;
+  __shared__ unsigned long long s_keep[kMaskWords], s_inner[64];
+  __shared__ uint32_t s_gone[2], s_kept;
+  const int tid = threadIdx.x, box = tid >> 1, half = tid & 1;
+  const uint32_t lane = tid & 31u;
+  const int words = (m + 63) / 64;
+  unsigned long long next[kEach];
+  auto fetch = [&](int w) {
+#pragma unroll
+    for (int v = 0; v < kEach; ++v) {
+      const int word = 2 * v + half, j = w * 64 + box;
+      next[v] = w < words && word <= w && j < m ? __ldcg(b.mask + (size_t)j * kMaskWords + word) : 0ull;
+    }
+  };
+  if (tid == 0) s_kept = 0u;
+  fetch(0);
+  for (int w = 0; w < words; ++w) {
+    if (tid < 2) s_gone[tid] = 0u;
+    __syncthreads();
+    const uint32_t kept = s_kept;
+    if (kept >= (uint32_t)a.p.nms_post_max) break;
+    bool gone = w * 64 + box >= m;
+#pragma unroll
+    for (int v = 0; v < kEach; ++v) {
+      const int word = 2 * v + half;
+      if (word < w) gone = gone || (next[v] & s_keep[word]) != 0ull;
+      else if (word == w) s_inner[box] = next[v];
+    }
+    if (gone) atomicOr(&s_gone[box >> 5], 1u << (box & 31));
+    fetch(w + 1);
+    __syncthreads();
+    if (tid < 32) {
+      // lane l decides boxes l and 32 + l
+      const unsigned long long in0 = s_inner[lane], in1 = s_inner[lane + 32];
+      unsigned long long open = ~((unsigned long long)s_gone[0] | (unsigned long long)s_gone[1] << 32);
+      unsigned long long keep = 0ull;
+      while (open) {
+        const bool o0 = (open >> lane) & 1ull, o1 = (open >> (lane + 32)) & 1ull;
+        const bool k0 = o0 && (in0 & (open | keep)) == 0ull, k1 = o1 && (in1 & (open | keep)) == 0ull;
+        const bool d0 = o0 && (in0 & keep) != 0ull, d1 = o1 && (in1 & keep) != 0ull;
+        const unsigned long long nk = (unsigned long long)__ballot_sync(0xffffffffu, k0) |
+                                      (unsigned long long)__ballot_sync(0xffffffffu, k1) << 32;
+        const unsigned long long nd = (unsigned long long)__ballot_sync(0xffffffffu, d0) |
+                                      (unsigned long long)__ballot_sync(0xffffffffu, d1) << 32;
+        keep |= nk;
+        open &= ~(nk | nd);
+      }
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const uint32_t bit = lane + 32u * h;
+        const uint32_t at = kept + (uint32_t)__popcll(keep & ((1ull << bit) - 1ull));
+        if (((keep >> bit) & 1ull) && at < (uint32_t)a.p.nms_post_max)
+          b.kept[at] = (uint32_t)w * 64u + bit;
+      }
+      if (lane == 0) {
+        s_keep[w] = keep;
+        s_kept = kept + (uint32_t)__popcll(keep);
+      }
+    }
+    __syncthreads();
+  }
+  __syncthreads();
+  if (tid == 0) *b.n_kept = min(s_kept, (uint32_t)a.p.nms_post_max);
+}
+
+// The last task to get here packs every task's boxes into the caller's list, in task order.
+__device__ void pack_boxes(const PostArgs& a) {
+  __shared__ bool s_last_task;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) s_last_task = atomicAdd(a.ticket, 1u) == (uint32_t)(a.num_tasks - 1);
+  __syncthreads();
+  if (!s_last_task) return;
+  __threadfence();
+  uint32_t first[SPCONVB_CP_MAX_TASKS + 1];
+  first[0] = 0;
+#pragma unroll
+  for (int t = 0; t < SPCONVB_CP_MAX_TASKS; ++t)
+    first[t + 1] = first[t] + (t < a.num_tasks ? __ldcg(a.buf[t].n_kept) : 0u);
+  const uint32_t total = first[SPCONVB_CP_MAX_TASKS];
+  if (threadIdx.x == 0) {
+    *a.out_count = total;
+    if (a.out_count_host) {
+      *(volatile uint32_t*)a.out_count_host = total;
+      __threadfence_system();
+    }
+  }
+#pragma unroll 2
+  for (uint32_t e = threadIdx.x; e < total * kDet; e += blockDim.x) {
+    const uint32_t k = e / kDet, f = e % kDet;
+    int t = 0;
+    uint32_t from = 0;
+#pragma unroll
+    for (int q = 1; q < SPCONVB_CP_MAX_TASKS; ++q)
+      if (k >= first[q]) {
+        t = q;
+        from = first[q];
+      }
+    const uint32_t rank = __ldcg(a.buf[t].kept + (k - from));
+    float v = __ldcg(a.buf[t].det + (size_t)rank * kDet + f);
+    if (f == 9) v = (float)(a.head[t].label_offset + (int)v);
+    a.out_boxes[e] = v;
+  }
+}
+
+// Whether the IoU of two boxes is certain to stay below the threshold: the common part lies inside
+// the bounding box, along A's axes (and along B's), of what both cover there.  Half the pairs in
+// reach of one another are decided by this.  The margin covers the 1e-2 by which corners outside a
+// box still count as inside, the factors far more than any rounding; a NaN decides nothing.
+struct BoxBounds { float x, y, dx, dy, c, s; };
+__device__ __forceinline__ float cover_along(const BoxBounds& A, const BoxBounds& B) {
+  const float ddx = B.x - A.x, ddy = B.y - A.y;
+  const float rx = ddx * A.c - ddy * A.s, ry = ddx * A.s + ddy * A.c;
+  const float co = fabsf(A.c * B.c + A.s * B.s), si = fabsf(A.s * B.c - A.c * B.s);
+  const float ex = 0.5f * (co * B.dx + si * B.dy), ey = 0.5f * (si * B.dx + co * B.dy);
+  const float hx = 0.5f * A.dx, hy = 0.5f * A.dy;
+  const float wx = fminf(hx, rx + ex) - fmaxf(-hx, rx - ex) + 0.1f;
+  const float wy = fminf(hy, ry + ey) - fmaxf(-hy, ry - ey) + 0.1f;
+  return fmaxf(wx, 0.f) * fmaxf(wy, 0.f);
+}
+__device__ __forceinline__ bool surely_below(const BoxBounds& A, const BoxBounds& B, float threshold) {
+  const float cover = fminf(cover_along(A, B), cover_along(B, A)) * 1.02f + 1e-3f;
+  return cover < threshold * 0.999f * (A.dx * A.dy + B.dx * B.dy - cover);
+}
+
+// One tile = 16 boxes x 64 earlier ones.  Pass 1: every thread tests 8 pairs for reach (three
+// floats per box, staged in shared memory), bounds the IoU of the others and queues what is left.
+// Pass 2: the queued pairs are spread over the threads one by one, so the long overlap
+// computation runs with full warps instead of one lane in 32.  The CTA that finishes a task's
+// last tile walks that task's ranking.
 __global__ void __launch_bounds__(kMaskThreads) cp_mask_kernel(const PostArgs a) {
   const int task = blockIdx.y;
   const TaskBuffers& b = a.buf[task];
-  const int m = (int)*b.n_det;
   const int tid = threadIdx.x;
-  __shared__ float col_x[64], col_y[64], col_r[64], row_x[kMaskRows], row_y[kMaskRows], row_r[kMaskRows];
+  __shared__ BoxBounds s_col[64], s_row[kMaskRows];
+  __shared__ float s_reach[64 + kMaskRows];
   __shared__ unsigned long long words[kMaskRows];
   __shared__ uint16_t queue[kMaskRows * 64];
   __shared__ uint32_t queued;
-  const int col_blocks = (m + 63) / 64, row_groups = (m + kMaskRows - 1) / kMaskRows;
+  __shared__ bool s_last;
+  pdl_wait();
+  const int m = (int)load_after_wait(b.n_det);
+  const float threshold = a.p.nms_iou_threshold;
+  const int row_groups = (m + kMaskRows - 1) / kMaskRows, col_blocks = (m + 63) / 64;
   for (int tile = blockIdx.x; tile < col_blocks * row_groups; tile += gridDim.x) {
     const int row0 = (tile / col_blocks) * kMaskRows, col0 = (tile % col_blocks) * 64;
-    if (col0 / 64 < row0 / 64) continue;  // left of the diagonal: never read
+    if (col0 / 64 > row0 / 64) continue;  // right of the diagonal: never read
     __syncthreads();                      // the previous tile's shared state is no longer needed
-    if (tid < 64) {
-      const BoxRec* r = (const BoxRec*)(b.box + (size_t)min(col0 + tid, m - 1) * kBoxStride);
-      col_x[tid] = r->x; col_y[tid] = r->y; col_r[tid] = r->reach;
-    } else if (tid < 64 + kMaskRows) {
-      const int k = tid - 64;
-      const BoxRec* r = (const BoxRec*)(b.box + (size_t)min(row0 + k, m - 1) * kBoxStride);
-      row_x[k] = r->x; row_y[k] = r->y; row_r[k] = r->reach;
-      words[k] = 0ull;
-    } else if (tid == 64 + kMaskRows) {
-      queued = 0u;
+    if (tid < 64 + kMaskRows) {
+      const int box = tid < 64 ? col0 + tid : row0 + tid - 64;
+      const BoxRec* r = (const BoxRec*)(b.box + (size_t)min(box, m - 1) * kBoxStride);
+      const BoxBounds v = {r->x, r->y, r->dx, r->dy, r->cos_neg, r->sin_neg};
+      if (tid < 64) s_col[tid] = v;
+      else s_row[tid - 64] = v;
+      s_reach[tid] = r->reach;
     }
+    if (tid < kMaskRows) words[tid] = 0ull;
+    if (tid == kMaskThreads - 1) queued = 0u;
     __syncthreads();
     for (int pair = tid; pair < kMaskRows * 64; pair += kMaskThreads) {
       const int r = pair >> 6, c = pair & 63;
-      const int i = row0 + r, j = col0 + c;
-      if (i >= m || j >= m || j <= i) continue;
-      const float ddx = row_x[r] - col_x[c], ddy = row_y[r] - col_y[c];
-      const float far = row_r[r] + col_r[c] + 0.1f;
+      const int i = col0 + c, j = row0 + r;
+      if (j >= m || i >= j) continue;
+      const float ddx = s_col[c].x - s_row[r].x, ddy = s_col[c].y - s_row[r].y;
+      const float far = s_reach[c] + s_reach[64 + r] + 0.1f;
       if (ddx * ddx + ddy * ddy > far * far) continue;  // the same test rotated_iou starts with
+      if (surely_below(s_col[c], s_row[r], threshold)) continue;
       queue[atomicAdd(&queued, 1u)] = (uint16_t)pair;
     }
     __syncthreads();
     const uint32_t n_pairs = queued;
     for (uint32_t q = tid; q < n_pairs; q += kMaskThreads) {
       const int pair = queue[q], r = pair >> 6, c = pair & 63;
-      BoxRec A, B;
-      load_box(b.box + (size_t)(row0 + r) * kBoxStride, A);
-      load_box(b.box + (size_t)(col0 + c) * kBoxStride, B);
-      if (rotated_iou(A, B) >= a.p.nms_iou_threshold) atomicOr(&words[r], 1ull << c);
+      BoxRec A, B;  // the earlier box first
+      load_box(b.box + (size_t)(col0 + c) * kBoxStride, A);
+      load_box(b.box + (size_t)(row0 + r) * kBoxStride, B);
+      if (rotated_iou(A, B) >= threshold) atomicOr(&words[r], 1ull << c);
     }
     __syncthreads();
     if (tid < kMaskRows && row0 + tid < m)
       b.mask[(size_t)(row0 + tid) * kMaskWords + col0 / 64] = words[tid];
   }
-}
-
-// ------------------------------------------------------------------ scan
-__global__ void __launch_bounds__(512) cp_scan_kernel(const PostArgs a) {
-  __shared__ __align__(16) unsigned long long s_mask[kScanStagedRows * kMaskWords];
-  __shared__ bool s_last;
-  __shared__ int s_kept[kRankThreads];
-  __shared__ uint32_t s_nkept;
-  const int task = blockIdx.x;
-  const TaskBuffers& b = a.buf[task];
-  const int m = (int)*b.n_det;
-  const int words = (m + 63) / 64;
-  // The walk usually ends (nms_post_max survivors) within the first few hundred boxes: those
-  // rows are staged in shared memory, later ones are read from global memory when needed.
-  const int staged = min(m, kScanStagedRows);
-  {
-    // 16-byte loads issued back to back; words left of the diagonal tile and right of the last
-    // box were never written and are zeroed here
-    const ulonglong2* src = (const ulonglong2*)b.mask;
-    ulonglong2* dst = (ulonglong2*)s_mask;
-    const int vecs = staged * (kMaskWords / 2);
-#pragma unroll 5
-    for (int v = threadIdx.x; v < vecs; v += blockDim.x) {
-      ulonglong2 x = src[v];
-      const int row = v / (kMaskWords / 2), wd = (v % (kMaskWords / 2)) * 2;
-      if (wd < row / 64 || wd >= words) x.x = 0ull;
-      if (wd + 1 < row / 64 || wd + 1 >= words) x.y = 0ull;
-      dst[v] = x;
-    }
-  }
+  __threadfence();  // every thread's words are visible device-wide before the ticket is taken
   __syncthreads();
-  if (threadIdx.x < 32) {
-    const int lane = threadIdx.x;
-    unsigned long long removed = 0ull;  // lane w holds word w of the removed set
-    uint32_t kept = 0;
-    // Word by word: the lowest ranked box of the word that nobody has removed survives, its
-    // mask row joins the removed set, and so on; removed boxes cost nothing.  Boxes after the
-    // first nms_post_max survivors cannot reach the output.
-    for (int w = 0; w < words && kept < (uint32_t)a.p.nms_post_max; ++w) {
-      const unsigned long long valid =
-          (w == words - 1 && (m & 63)) ? ((1ull << (m & 63)) - 1ull) : ~0ull;
-      while (kept < (uint32_t)a.p.nms_post_max) {
-        const unsigned long long alive = ~__shfl_sync(0xffffffffu, removed, w) & valid;
-        if (alive == 0ull) break;
-        const int bit = __ffsll((long long)alive) - 1;
-        const int i = w * 64 + bit;
-        if (lane == 0) s_kept[kept] = i;
-        ++kept;
-        if (lane == w) removed |= 1ull << bit;  // done with this box
-        if (lane < kMaskWords) {
-          if (i < staged) removed |= s_mask[i * kMaskWords + lane];
-          else if (lane >= w && lane < words) removed |= b.mask[(size_t)i * kMaskWords + lane];
-        }
-      }
-    }
-    if (lane == 0) {
-      s_nkept = kept;
-      *b.n_kept = kept;
-    }
-  }
-  __syncthreads();
-  for (uint32_t e = threadIdx.x; e < s_nkept * kDet; e += blockDim.x) {
-    const uint32_t k = e / kDet, f = e % kDet;
-    float v = b.det[(size_t)s_kept[k] * kDet + f];
-    if (f == 9) v = (float)(a.head[task].label_offset + (int)v);
-    b.kept[e] = v;
-  }
-  __threadfence();  // every thread's rows are visible device-wide before the ticket is taken
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();
-    s_last = atomicAdd(a.ticket, 1u) == (uint32_t)(a.num_tasks - 1);
-  }
+  if (tid == 0) s_last = atomicAdd(b.ticket, 1u) == gridDim.x - 1u;
   __syncthreads();
   if (!s_last) return;
   __threadfence();
-  // the last task to finish packs every task's boxes into the caller's list, in task order
-  uint32_t count[SPCONVB_CP_MAX_TASKS], base = 0;
-#pragma unroll
-  for (int t = 0; t < SPCONVB_CP_MAX_TASKS; ++t)
-    count[t] = t < a.num_tasks ? __ldcg(a.buf[t].n_kept) : 0u;
-#pragma unroll
-  for (int t = 0; t < SPCONVB_CP_MAX_TASKS; ++t) {
-    for (uint32_t i = threadIdx.x; i < count[t] * kDet; i += blockDim.x)
-      a.out_boxes[(size_t)base * kDet + i] = __ldcg(a.buf[t].kept + i);
-    base += count[t];
-  }
-  if (threadIdx.x == 0) *a.out_count = base;
+  walk_ranking(a, b, m);
+  pack_boxes(a);
 }
 
 bool params_ok(const spconvb_cp_params* p) {
   return p && p->H >= 1 && p->W >= 1 && (size_t)p->H * p->W <= 0xFFFFFFu && p->max_det >= 1 &&
-         p->max_det <= kRankThreads && p->nms_post_max >= 1 && p->nms_post_max <= p->max_det;
+         p->max_det <= kMaxDet && p->nms_post_max >= 1 && p->nms_post_max <= p->max_det;
 }
 
 }  // namespace
@@ -577,6 +711,14 @@ size_t spconvb_cp_workspace_bytes(const spconvb_cp_params* p, int32_t num_tasks)
 int spconvb_cp_postprocess(const spconvb_cp_head* heads, int32_t num_tasks,
                            const spconvb_cp_params* p, void* workspace, size_t workspace_bytes,
                            float* out_boxes, uint32_t* out_count, void* stream) {
+  return spconvb_cp_postprocess_host(heads, num_tasks, p, workspace, workspace_bytes, out_boxes,
+                                     out_count, nullptr, stream);
+}
+
+int spconvb_cp_postprocess_host(const spconvb_cp_head* heads, int32_t num_tasks,
+                                const spconvb_cp_params* p, void* workspace,
+                                size_t workspace_bytes, float* out_boxes, uint32_t* out_count,
+                                uint32_t* out_count_host, void* stream) {
   if (!heads || !params_ok(p) || !workspace || !out_boxes || !out_count || num_tasks < 1 ||
       num_tasks > SPCONVB_CP_MAX_TASKS || ((uintptr_t)workspace & 255u))
     return SPCONVB_E_ARG;
@@ -594,18 +736,17 @@ int spconvb_cp_postprocess(const spconvb_cp_head* heads, int32_t num_tasks,
   a.num_tasks = num_tasks;
   a.out_boxes = out_boxes;
   a.out_count = out_count;
+  a.out_count_host = out_count_host;
   bind_buffers(l, workspace, num_tasks, a);
   cudaStream_t st = (cudaStream_t)stream;
   SPCONVB_CUDA_TRY(cudaMemsetAsync(workspace, 0, l.counters_bytes, st));
   const int HW = p->H * p->W;
   cp_candidates_kernel<<<dim3((HW + 255) / 256, num_tasks), 256, 0, st>>>(a);
   SPCONVB_LAUNCH_CHECK();
-  cp_rank_kernel<<<num_tasks, kRankThreads, 0, st>>>(a);
-  SPCONVB_LAUNCH_CHECK();
-  cp_mask_kernel<<<dim3(kMaskCtasPerTask, num_tasks), kMaskThreads, 0, st>>>(a);
-  SPCONVB_LAUNCH_CHECK();
-  cp_scan_kernel<<<num_tasks, 512, 0, st>>>(a);
-  SPCONVB_LAUNCH_CHECK();
+  SPCONVB_CUDA_TRY(launch_pdl(cp_rank_kernel, dim3(kRankParts, num_tasks), dim3(kRankThreads), 0,
+                              st, a));
+  SPCONVB_CUDA_TRY(launch_pdl(cp_mask_kernel, dim3(kMaskCtasPerTask, num_tasks), dim3(kMaskThreads),
+                              0, st, a));
   return SPCONVB_OK;
 }
 
