@@ -437,24 +437,32 @@ __global__ void __launch_bounds__(kRankThreads) cp_rank_kernel(const PostArgs a)
   }
   // the keys that count, in any order; this part ranks those at positions 32 part, 32 (part +
   // 16), ... of the candidates
-#pragma unroll 4
-  for (uint32_t base = 0; base < n; base += kRankThreads) {
-    const uint32_t i = base + tid;
-    const unsigned long long k = i < n ? b.cand[i] : 0ull;
-    const bool in = i < n && k >= least;
-    const uint32_t vote = __ballot_sync(0xffffffffu, in);
-    if (!vote) continue;
-    const bool mine = ((i >> 5) % kRankParts) == (uint32_t)part;
-    uint32_t at = 0, own_at = 0;
-    if (lane == 0) {
-      at = atomicAdd(&s_list, (uint32_t)__popc(vote));
-      if (mine) own_at = atomicAdd(&s_own, (uint32_t)__popc(vote));
+  constexpr int kAtOnce = 8;
+  for (uint32_t base = 0; base < n; base += kAtOnce * kRankThreads) {
+    unsigned long long k[kAtOnce];
+#pragma unroll
+    for (int u = 0; u < kAtOnce; ++u) {
+      const uint32_t i = base + u * kRankThreads + tid;
+      k[u] = i < n ? b.cand[i] : 0ull;  // no key is 0
     }
-    const uint32_t off = __popc(vote & ((1u << lane) - 1u));
-    at = __shfl_sync(0xffffffffu, at, 0) + off;
-    own_at = __shfl_sync(0xffffffffu, own_at, 0) + off;
-    if (in && at < (uint32_t)kRankList) list[at] = k;
-    if (in && mine && own_at < (uint32_t)kRankList) own[own_at] = k;
+#pragma unroll
+    for (int u = 0; u < kAtOnce; ++u) {
+      const bool in = k[u] != 0ull && k[u] >= least;
+      const uint32_t vote = __ballot_sync(0xffffffffu, in);
+      if (!vote) continue;
+      const uint32_t i = base + u * kRankThreads + tid;
+      const bool mine = ((i >> 5) % kRankParts) == (uint32_t)part;
+      uint32_t at = 0, own_at = 0;
+      if (lane == 0) {
+        at = atomicAdd(&s_list, (uint32_t)__popc(vote));
+        if (mine) own_at = atomicAdd(&s_own, (uint32_t)__popc(vote));
+      }
+      const uint32_t off = __popc(vote & ((1u << lane) - 1u));
+      at = __shfl_sync(0xffffffffu, at, 0) + off;
+      own_at = __shfl_sync(0xffffffffu, own_at, 0) + off;
+      if (in && at < (uint32_t)kRankList) list[at] = k[u];
+      if (in && mine && own_at < (uint32_t)kRankList) own[own_at] = k[u];
+    }
   }
   __syncthreads();
   const uint32_t count = min(s_list, (uint32_t)kRankList), owned = min(s_own, (uint32_t)kRankList);
@@ -474,7 +482,7 @@ __global__ void __launch_bounds__(kRankThreads) cp_rank_kernel(const PostArgs a)
 }
 
 // ------------------------------------------------------------------ mask
-constexpr int kMaskRows = 16;          // ranked boxes per tile; divides 64, so a tile's rows share a word
+constexpr int kMaskRows = 16;  // ranked boxes per tile; divides 64, so a tile's rows share a word
 constexpr int kMaskCtasPerTask = 148;
 constexpr int kMaskThreads = 128;
 
@@ -572,21 +580,39 @@ __device__ void pack_boxes(const PostArgs& a) {
       __threadfence_system();
     }
   }
-#pragma unroll 2
-  for (uint32_t e = threadIdx.x; e < total * kDet; e += blockDim.x) {
-    const uint32_t k = e / kDet, f = e % kDet;
-    int t = 0;
-    uint32_t from = 0;
+  // a thread takes four boxes at a time: their ranks, then 44 values, in flight together
+  constexpr int kAtOnce = 4;
+  for (uint32_t k0 = threadIdx.x; k0 < total; k0 += kAtOnce * kMaskThreads) {
+    const float* from[kAtOnce];
+    int offset[kAtOnce];
 #pragma unroll
-    for (int q = 1; q < SPCONVB_CP_MAX_TASKS; ++q)
-      if (k >= first[q]) {
-        t = q;
-        from = first[q];
-      }
-    const uint32_t rank = __ldcg(a.buf[t].kept + (k - from));
-    float v = __ldcg(a.buf[t].det + (size_t)rank * kDet + f);
-    if (f == 9) v = (float)(a.head[t].label_offset + (int)v);
-    a.out_boxes[e] = v;
+    for (int u = 0; u < kAtOnce; ++u) {
+      const uint32_t k = min(k0 + u * kMaskThreads, total - 1u);
+      const uint32_t* kept = a.buf[0].kept + k;
+      const float* det = a.buf[0].det;
+      offset[u] = a.head[0].label_offset;
+#pragma unroll
+      for (int q = 1; q < SPCONVB_CP_MAX_TASKS; ++q)
+        if (q < a.num_tasks && k >= first[q]) {
+          kept = a.buf[q].kept + (k - first[q]);
+          det = a.buf[q].det;
+          offset[u] = a.head[q].label_offset;
+        }
+      from[u] = det + (size_t)__ldcg(kept) * kDet;
+    }
+    float v[kAtOnce][kDet];
+#pragma unroll
+    for (int u = 0; u < kAtOnce; ++u)
+#pragma unroll
+      for (int f = 0; f < kDet; ++f) v[u][f] = __ldcg(from[u] + f);
+#pragma unroll
+    for (int u = 0; u < kAtOnce; ++u) {
+      const uint32_t k = k0 + u * kMaskThreads;
+      if (k >= total) break;
+      v[u][9] = (float)(offset[u] + (int)v[u][9]);
+#pragma unroll
+      for (int f = 0; f < kDet; ++f) a.out_boxes[(size_t)k * kDet + f] = v[u][f];
+    }
   }
 }
 
