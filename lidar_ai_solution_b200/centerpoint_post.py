@@ -19,6 +19,7 @@ from . import cabi
 TASK_LABEL_OFFSET = (0, 1, 3, 5, 6, 8)
 TASK_NUM_CLASSES = (1, 2, 2, 1, 2, 2)
 HEAD_CHANNELS = {"reg": 2, "height": 1, "dim": 3, "rot": 2, "vel": 2}
+HEAD_KEYS = (*HEAD_CHANNELS, "hm")
 
 
 def default_params(H=180, W=180, **overrides) -> cabi.CpParams:
@@ -58,6 +59,8 @@ class PostProcess:
         self._shapes = [(k, torch.Size((ch, p.H, p.W)), torch.Size((1, ch, p.H, p.W)))
                         for k, ch in HEAD_CHANNELS.items()]
         self._keep = None
+        self._known = [(None, 0)] * (6 * num_tasks)
+        self._words = None
         self._stream = None
 
     def run(self, heads, label_offsets=TASK_LABEL_OFFSET, stream=None):
@@ -66,21 +69,23 @@ class PostProcess:
         the stream has run."""
         assert len(heads) == self.num_tasks
         p = self.params
-        half = torch.float16
-        words = []
-        for t, h in enumerate(heads):
-            for k, chw, nchw in self._shapes:
+        # Bound buffers stay the same from frame to frame: a tensor that was here in the last call,
+        # at the same address, has been checked.
+        known = iter(self._known)
+        for h in heads:
+            for k in HEAD_KEYS:
                 x = h[k]
-                shape = x.shape
-                assert x.dtype is half and x.is_cuda and x.is_contiguous()
-                assert shape == chw or shape == nchw or shape[-3:] == chw, (k, tuple(shape))
-                words.append(x.data_ptr())
-            hm = h["hm"]
-            shape = hm.shape
-            assert hm.dtype is half and hm.is_cuda and hm.is_contiguous()
-            assert shape[-2] == p.H and shape[-1] == p.W
-            words += (hm.data_ptr(), shape[-3], label_offsets[t])
-        self._pack.pack_into(self._heads, 0, *words)
+                y, at = next(known)
+                if x is not y or x.data_ptr() != at:
+                    self._check(heads)
+                    break
+            else:
+                continue
+            break
+        words = self._words
+        if words[7::8] != [*label_offsets[:self.num_tasks]]:
+            words[7::8] = label_offsets[:self.num_tasks]
+            self._pack.pack_into(self._heads, 0, *words)
         self._keep = heads
         s = stream if stream is not None else torch.cuda.current_stream()
         self._stream = s
@@ -88,6 +93,27 @@ class PostProcess:
             self._heads, self.num_tasks, C.byref(p), self.workspace.data_ptr(),
             self.workspace.numel(), self.boxes.data_ptr(), self.count.data_ptr(),
             self._count_host.data_ptr(), s.cuda_stream), "cp_postprocess")
+
+    def _check(self, heads):
+        """Checks the heads' tensors and notes their addresses for the library."""
+        p = self.params
+        half = torch.float16
+        words, known = [], []
+        for h in heads:
+            for k, chw, nchw in self._shapes:
+                x = h[k]
+                shape = x.shape
+                assert x.dtype is half and x.is_cuda and x.is_contiguous()
+                assert shape == chw or shape == nchw or shape[-3:] == chw, (k, tuple(shape))
+                known.append((x, x.data_ptr()))
+                words.append(x.data_ptr())
+            hm = h["hm"]
+            shape = hm.shape
+            assert hm.dtype is half and hm.is_cuda and hm.is_contiguous()
+            assert shape[-2] == p.H and shape[-1] == p.W
+            known.append((hm, hm.data_ptr()))
+            words += (hm.data_ptr(), shape[-3], None)
+        self._words, self._known = words, known
 
     def result(self):
         """Synchronises and returns the kept boxes [n, 11] (a copy)."""

@@ -287,13 +287,6 @@ __global__ void rotated_iou_pairs_kernel(const float* a, const float* b, int n, 
   iou[i] = rotated_iou(A, B);
 }
 
-__device__ __forceinline__ void load_box(const float* p, BoxRec& r) {
-  float4* d = (float4*)&r;
-  const float4* s4 = (const float4*)p;
-#pragma unroll
-  for (int k = 0; k < 4; ++k) d[k] = s4[k];
-}
-
 // ------------------------------------------------------------------ rank
 constexpr int kRankParts = 16;
 constexpr int kRankThreads = 256;
@@ -484,26 +477,27 @@ __global__ void __launch_bounds__(kRankThreads) cp_rank_kernel(const PostArgs a)
 // ------------------------------------------------------------------ mask
 constexpr int kMaskRows = 16;  // ranked boxes per tile; divides 64, so a tile's rows share a word
 constexpr int kMaskCtasPerTask = 148;
-constexpr int kMaskThreads = 128;
+constexpr int kMaskThreads = 256;
+constexpr int kMaskSlots = 4;  // tiles of a CTA: at most 544 tiles a task
 
-// The greedy walk over one task's ranking, by one CTA.  64 boxes at a time: two threads a box
+// The greedy walk over one task's ranking, by one CTA.  64 boxes at a time: four threads a box
 // look whether an earlier kept box suppresses it (its mask words are fetched while the 64 before
 // are decided), then the first warp decides among the 64: a box stays when every box of them that
 // suppresses it is out, and is out when one of them stays, so the rounds are as many as the
 // longest chain of suppressions and not as the boxes.  Boxes after the first nms_post_max
 // survivors cannot reach the output.
 __device__ void walk_ranking(const PostArgs& a, const TaskBuffers& b, int m) {
-  constexpr int kEach = kMaskWords / 2;
+  constexpr int kEach = kMaskWords / 4;
   __shared__ unsigned long long s_keep[kMaskWords], s_inner[64];
   __shared__ uint32_t s_gone[2], s_kept;
-  const int tid = threadIdx.x, box = tid >> 1, half = tid & 1;
+  const int tid = threadIdx.x, box = tid >> 2, quarter = tid & 3;
   const uint32_t lane = tid & 31u;
   const int words = (m + 63) / 64;
   unsigned long long next[kEach];
   auto fetch = [&](int w) {
 #pragma unroll
     for (int v = 0; v < kEach; ++v) {
-      const int word = 2 * v + half, j = w * 64 + box;
+      const int word = 4 * v + quarter, j = w * 64 + box;
       next[v] = w < words && word <= w && j < m ? __ldcg(b.mask + (size_t)j * kMaskWords + word) : 0ull;
     }
   };
@@ -517,7 +511,7 @@ __device__ void walk_ranking(const PostArgs& a, const TaskBuffers& b, int m) {
     bool gone = w * 64 + box >= m;
 #pragma unroll
     for (int v = 0; v < kEach; ++v) {
-      const int word = 2 * v + half;
+      const int word = 4 * v + quarter;
       if (word < w) gone = gone || (next[v] & s_keep[word]) != 0ull;
       else if (word == w) s_inner[box] = next[v];
     }
@@ -636,62 +630,131 @@ __device__ __forceinline__ bool surely_below(const BoxBounds& A, const BoxBounds
   return cover < threshold * 0.999f * (A.dx * A.dy + B.dx * B.dy - cover);
 }
 
-// One tile = 16 boxes x 64 earlier ones.  Pass 1: every thread tests 8 pairs for reach (three
-// floats per box, staged in shared memory), bounds the IoU of the others and queues what is left.
-// Pass 2: the queued pairs are spread over the threads one by one, so the long overlap
-// computation runs with full warps instead of one lane in 32.  The CTA that finishes a task's
-// last tile walks that task's ranking.
+// rotated_iou(A, B) >= threshold by a whole warp: lane e < 16 looks for the crossing of edge e / 4
+// of A and e % 4 of B, lanes 16..23 at the corners, in the order in which the serial code appends
+// its points; sums run in that order and in the order of the angles, so every bit is the same.
+// Boxes with a coordinate that is not a number overlap nothing, as there.
+__device__ __forceinline__ bool iou_reaches(const BoxRec& A, const BoxRec& B, float threshold,
+                                            Pt* scratch) {
+  const uint32_t lane = threadIdx.x & 31u;
+  Pt p = {0.f, 0.f};
+  bool have = false;
+  if (lane < 16u) {
+    const int i = lane >> 2, j = lane & 3;
+    have = segments_cross(A.corner[(i + 1) & 3], A.corner[i], B.corner[(j + 1) & 3], B.corner[j], p);
+  } else if (lane < 24u) {
+    const int k = (lane - 16u) >> 1;
+    p = (lane & 1u) ? A.corner[k] : B.corner[k];
+    have = (lane & 1u) ? inside_with_margin(B, p) : inside_with_margin(A, p);
+  }
+  const uint32_t set = __ballot_sync(0xffffffffu, have);
+  const int cnt = __popc(set);
+  float iou = 0.f;
+  if (cnt != 0) {
+    Pt centre = {0.f, 0.f};
+    for (uint32_t left = set; left; left &= left - 1u) {
+      const int from = __ffs((int)left) - 1;
+      centre.x = centre.x + __shfl_sync(0xffffffffu, p.x, from);
+      centre.y = centre.y + __shfl_sync(0xffffffffu, p.y, from);
+    }
+    centre.x /= (float)cnt;
+    centre.y /= (float)cnt;
+    const float ang = have ? atan2f(p.y - centre.y, p.x - centre.x) : 0.f;
+    if (__any_sync(0xffffffffu, ang != ang)) return false;
+    // place in the stable ascending order of the angles
+    int place = 0;
+    for (uint32_t left = set; left; left &= left - 1u) {
+      const int from = __ffs((int)left) - 1;
+      const float other = __shfl_sync(0xffffffffu, ang, from);
+      if (other < ang || (other == ang && from < (int)lane)) ++place;
+    }
+    __syncwarp();
+    if (have) scratch[place] = p;
+    __syncwarp();
+    float term = 0.f;
+    if ((int)lane + 1 < cnt) {
+      const Pt p0 = scratch[0], pk = scratch[lane], pn = scratch[lane + 1];
+      const float ax = pk.x - p0.x, ay = pk.y - p0.y, bx = pn.x - p0.x, by = pn.y - p0.y;
+      term = ax * by - ay * bx;
+    }
+    float area = 0.f;
+    for (int k = 0; k + 1 < cnt; ++k) area += __shfl_sync(0xffffffffu, term, k);
+    const float overlap = fabsf(area) / 2.0f;
+    const float sa = A.dx * A.dy, sb = B.dx * B.dy;
+    iou = overlap / fmaxf(sa + sb - overlap, 1e-8f);
+  }
+  return iou >= threshold;
+}
+
+// One tile = 16 boxes x 64 earlier ones; a CTA takes all its tiles (up to four) through each pass
+// together.  Pass 1: every thread tests pairs for reach, bounds the IoU of the others and queues
+// what is left: 3 to 10 of a tile's 1 024, at most 30 in the benchmark's heads, so that what
+// counts is how long one pair takes and not how many there are.  Pass 2: a warp per queued pair.
+// The CTA that finishes a task's last tile walks that task's ranking.
 __global__ void __launch_bounds__(kMaskThreads) cp_mask_kernel(const PostArgs a) {
   const int task = blockIdx.y;
   const TaskBuffers& b = a.buf[task];
   const int tid = threadIdx.x;
-  __shared__ BoxBounds s_col[64], s_row[kMaskRows];
-  __shared__ float s_reach[64 + kMaskRows];
-  __shared__ unsigned long long words[kMaskRows];
-  __shared__ uint16_t queue[kMaskRows * 64];
+  constexpr int kBoxes = 64 + kMaskRows;
+  __shared__ __align__(16) BoxRec s_box[kMaskSlots][kBoxes];
+  __shared__ int s_first[kMaskSlots][2];
+  __shared__ unsigned long long words[kMaskSlots][kMaskRows];
+  __shared__ uint16_t queue[kMaskSlots * kMaskRows * 64];
+  __shared__ Pt scratch[kMaskThreads / 32][24];
   __shared__ uint32_t queued;
   __shared__ bool s_last;
   pdl_wait();
   const int m = (int)load_after_wait(b.n_det);
   const float threshold = a.p.nms_iou_threshold;
-  const int row_groups = (m + kMaskRows - 1) / kMaskRows, col_blocks = (m + 63) / 64;
-  for (int tile = blockIdx.x; tile < col_blocks * row_groups; tile += gridDim.x) {
-    const int row0 = (tile / col_blocks) * kMaskRows, col0 = (tile % col_blocks) * 64;
-    if (col0 / 64 > row0 / 64) continue;  // right of the diagonal: never read
-    __syncthreads();                      // the previous tile's shared state is no longer needed
-    if (tid < 64 + kMaskRows) {
-      const int box = tid < 64 ? col0 + tid : row0 + tid - 64;
-      const BoxRec* r = (const BoxRec*)(b.box + (size_t)min(box, m - 1) * kBoxStride);
-      const BoxBounds v = {r->x, r->y, r->dx, r->dy, r->cos_neg, r->sin_neg};
-      if (tid < 64) s_col[tid] = v;
-      else s_row[tid - 64] = v;
-      s_reach[tid] = r->reach;
+  // tiles on or below the diagonal: 4 row groups of 16 in block row G, G + 1 tiles each
+  const int groups = (m + kMaskRows - 1) / kMaskRows, whole = groups / 4;
+  const int tiles = 2 * whole * (whole + 1) + (groups - 4 * whole) * (whole + 1);
+  int slots = 0;
+  for (int tile = blockIdx.x; tile < tiles && slots < kMaskSlots; tile += gridDim.x, ++slots) {
+    int G = 0;
+    while (2 * (G + 1) * (G + 2) <= tile) ++G;
+    const int in = tile - 2 * G * (G + 1), row0 = (4 * G + in / (G + 1)) * kMaskRows;
+    const int col0 = in % (G + 1) * 64;
+    if (tid == 0) {
+      s_first[slots][0] = row0;
+      s_first[slots][1] = col0;
     }
-    if (tid < kMaskRows) words[tid] = 0ull;
-    if (tid == kMaskThreads - 1) queued = 0u;
-    __syncthreads();
-    for (int pair = tid; pair < kMaskRows * 64; pair += kMaskThreads) {
-      const int r = pair >> 6, c = pair & 63;
-      const int i = col0 + c, j = row0 + r;
-      if (j >= m || i >= j) continue;
-      const float ddx = s_col[c].x - s_row[r].x, ddy = s_col[c].y - s_row[r].y;
-      const float far = s_reach[c] + s_reach[64 + r] + 0.1f;
-      if (ddx * ddx + ddy * ddy > far * far) continue;  // the same test rotated_iou starts with
-      if (surely_below(s_col[c], s_row[r], threshold)) continue;
-      queue[atomicAdd(&queued, 1u)] = (uint16_t)pair;
+    for (int k = tid; k < kBoxes * 4; k += kMaskThreads) {
+      const int box = min(k < 256 ? col0 + k / 4 : row0 + k / 4 - 64, m - 1);
+      ((float4*)&s_box[slots][k / 4])[k & 3] =
+          ((const float4*)(b.box + (size_t)box * kBoxStride))[k & 3];
     }
-    __syncthreads();
-    const uint32_t n_pairs = queued;
-    for (uint32_t q = tid; q < n_pairs; q += kMaskThreads) {
-      const int pair = queue[q], r = pair >> 6, c = pair & 63;
-      BoxRec A, B;  // the earlier box first
-      load_box(b.box + (size_t)(col0 + c) * kBoxStride, A);
-      load_box(b.box + (size_t)(row0 + r) * kBoxStride, B);
-      if (rotated_iou(A, B) >= threshold) atomicOr(&words[r], 1ull << c);
-    }
-    __syncthreads();
-    if (tid < kMaskRows && row0 + tid < m)
-      b.mask[(size_t)(row0 + tid) * kMaskWords + col0 / 64] = words[tid];
+    if (tid < kMaskRows) words[slots][tid] = 0ull;
+  }
+  if (tid == 0) queued = 0u;
+  __syncthreads();
+  for (int pair = tid; pair < slots * kMaskRows * 64; pair += kMaskThreads) {
+    const int slot = pair >> 10, r = (pair >> 6) & (kMaskRows - 1), c = pair & 63;
+    const int i = s_first[slot][1] + c, j = s_first[slot][0] + r;
+    if (j >= m || i >= j) continue;
+    const BoxRec &A = s_box[slot][c], &B = s_box[slot][64 + r];
+    const float ddx = A.x - B.x, ddy = A.y - B.y;
+    const float far = A.reach + B.reach + 0.1f;
+    if (ddx * ddx + ddy * ddy > far * far) continue;  // the same test rotated_iou starts with
+    if (surely_below({A.x, A.y, A.dx, A.dy, A.cos_neg, A.sin_neg},
+                     {B.x, B.y, B.dx, B.dy, B.cos_neg, B.sin_neg}, threshold))
+      continue;
+    queue[atomicAdd(&queued, 1u)] = (uint16_t)pair;
+  }
+  __syncthreads();
+  const uint32_t n_pairs = queued;
+  for (uint32_t q = tid >> 5; q < n_pairs; q += kMaskThreads / 32) {
+    const int pair = queue[q], slot = pair >> 10, r = (pair >> 6) & (kMaskRows - 1), c = pair & 63;
+    // the earlier box first
+    if (iou_reaches(s_box[slot][c], s_box[slot][64 + r], threshold, scratch[tid >> 5]) &&
+        (tid & 31) == 0)
+      atomicOr(&words[slot][r], 1ull << c);
+  }
+  __syncthreads();
+  for (int k = tid; k < slots * kMaskRows; k += kMaskThreads) {
+    const int slot = k / kMaskRows, row = s_first[slot][0] + k % kMaskRows;
+    if (row < m)
+      b.mask[(size_t)row * kMaskWords + s_first[slot][1] / 64] = words[slot][k % kMaskRows];
   }
   __threadfence();  // every thread's words are visible device-wide before the ticket is taken
   __syncthreads();
