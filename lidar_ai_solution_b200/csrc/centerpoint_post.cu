@@ -42,7 +42,7 @@ constexpr int kMaskWords = 16;   // 64-bit words per mask row: 1024 / 64
 // Scores by their leading bits: bin 0 up to 2^-5, then 512 bins an octave (sigmoids end at 1).
 constexpr uint32_t kScoreBase = 0x3d000000u;  // bits of 2^-5
 constexpr int kScoreShift = 14;
-constexpr int kScoreBins = 2816;
+constexpr int kScoreBins = 2560;
 __device__ __forceinline__ uint32_t score_bin(uint32_t bits) {
   return bits <= kScoreBase ? 0u : min((bits - kScoreBase) >> kScoreShift, (uint32_t)kScoreBins - 1u);
 }
@@ -289,7 +289,7 @@ __global__ void rotated_iou_pairs_kernel(const float* a, const float* b, int n, 
 
 // ------------------------------------------------------------------ rank
 constexpr int kRankParts = 16;
-constexpr int kRankThreads = 256;
+constexpr int kRankThreads = 512;
 constexpr int kRankList = 2048;  // keys a CTA compares with
 
 // The K-th largest key, most significant byte first (keys are distinct): for frames where so many
@@ -300,7 +300,7 @@ __device__ unsigned long long select_kth(const unsigned long long* cand, uint32_
   const int tid = threadIdx.x;
   if (tid == 0) { *s_prefix = 0ull; *s_need = K; }
   for (int shift = 56; shift >= 0; shift -= 8) {
-    hist[tid] = 0u;
+    if (tid < 256) hist[tid] = 0u;
     __syncthreads();
     const unsigned long long prefix = *s_prefix;
     const unsigned long long hi = shift == 56 ? 0ull : (~0ull << (shift + 8));
@@ -377,7 +377,7 @@ __global__ void __launch_bounds__(kRankThreads) cp_rank_kernel(const PostArgs a)
   const int HW = a.p.H * a.p.W;
   __shared__ unsigned long long list[kRankList], own[kRankList];
   __shared__ uint16_t rank_of[kRankList];
-  __shared__ uint32_t hist[kRankThreads];
+  __shared__ uint32_t hist[256];
   __shared__ unsigned long long s_prefix;
   __shared__ uint32_t s_need, s_list, s_own;
   pdl_wait();
@@ -431,6 +431,9 @@ __global__ void __launch_bounds__(kRankThreads) cp_rank_kernel(const PostArgs a)
   // the keys that count, in any order; this part ranks those at positions 32 part, 32 (part +
   // 16), ... of the candidates
   constexpr int kAtOnce = 8;
+  auto is_mine = [&](uint32_t base) {
+    return (((base >> 5) + warp) % kRankParts) == (uint32_t)part;
+  };
   for (uint32_t base = 0; base < n; base += kAtOnce * kRankThreads) {
     unsigned long long k[kAtOnce];
 #pragma unroll
@@ -438,33 +441,52 @@ __global__ void __launch_bounds__(kRankThreads) cp_rank_kernel(const PostArgs a)
       const uint32_t i = base + u * kRankThreads + tid;
       k[u] = i < n ? b.cand[i] : 0ull;  // no key is 0
     }
+    uint32_t vote[kAtOnce], all = 0, mine = 0;
 #pragma unroll
     for (int u = 0; u < kAtOnce; ++u) {
-      const bool in = k[u] != 0ull && k[u] >= least;
-      const uint32_t vote = __ballot_sync(0xffffffffu, in);
-      if (!vote) continue;
-      const uint32_t i = base + u * kRankThreads + tid;
-      const bool mine = ((i >> 5) % kRankParts) == (uint32_t)part;
-      uint32_t at = 0, own_at = 0;
-      if (lane == 0) {
-        at = atomicAdd(&s_list, (uint32_t)__popc(vote));
-        if (mine) own_at = atomicAdd(&s_own, (uint32_t)__popc(vote));
+      vote[u] = __ballot_sync(0xffffffffu, k[u] != 0ull && k[u] >= least);
+      all += (uint32_t)__popc(vote[u]);
+      if (is_mine(base + u * kRankThreads)) mine += (uint32_t)__popc(vote[u]);
+    }
+    if (all == 0u) continue;
+    uint32_t at = 0, own_at = 0;
+    if (lane == 0) {
+      at = atomicAdd(&s_list, all);
+      if (mine) own_at = atomicAdd(&s_own, mine);
+    }
+    at = __shfl_sync(0xffffffffu, at, 0);
+    own_at = __shfl_sync(0xffffffffu, own_at, 0);
+#pragma unroll
+    for (int u = 0; u < kAtOnce; ++u) {
+      const uint32_t off = __popc(vote[u] & ((1u << lane) - 1u));
+      const bool in = (vote[u] >> lane) & 1u;
+      if (in && at + off < (uint32_t)kRankList) list[at + off] = k[u];
+      at += (uint32_t)__popc(vote[u]);
+      if (is_mine(base + u * kRankThreads)) {
+        if (in && own_at + off < (uint32_t)kRankList) own[own_at + off] = k[u];
+        own_at += (uint32_t)__popc(vote[u]);
       }
-      const uint32_t off = __popc(vote & ((1u << lane) - 1u));
-      at = __shfl_sync(0xffffffffu, at, 0) + off;
-      own_at = __shfl_sync(0xffffffffu, own_at, 0) + off;
-      if (in && at < (uint32_t)kRankList) list[at] = k[u];
-      if (in && mine && own_at < (uint32_t)kRankList) own[own_at] = k[u];
     }
   }
   __syncthreads();
   const uint32_t count = min(s_list, (uint32_t)kRankList), owned = min(s_own, (uint32_t)kRankList);
-  for (uint32_t o = warp; o < owned; o += kRankThreads / 32) {
-    const unsigned long long k = own[o];
-    uint32_t greater = 0;
-    for (uint32_t i = lane; i < count; i += 32) greater += list[i] > k ? 1u : 0u;
-    greater = __reduce_add_sync(0xffffffffu, greater);
-    if (lane == 0) rank_of[o] = (uint16_t)greater;
+  // a warp takes four keys through the list together
+  for (uint32_t o = warp * 4u; o < owned; o += kRankThreads / 32 * 4u) {
+    unsigned long long k[4];
+    uint32_t greater[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+    for (uint32_t u = 0; u < 4; ++u) k[u] = own[min(o + u, owned - 1u)];
+#pragma unroll 4
+    for (uint32_t i = lane; i < count; i += 32) {
+      const unsigned long long other = list[i];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) greater[u] += other > k[u] ? 1u : 0u;
+    }
+#pragma unroll
+    for (uint32_t u = 0; u < 4; ++u) {
+      greater[u] = __reduce_add_sync(0xffffffffu, greater[u]);
+      if (lane == 0 && o + u < owned) rank_of[o + u] = (uint16_t)greater[u];
+    }
   }
   __syncthreads();
   for (uint32_t o = tid; o < owned; o += kRankThreads) {
@@ -476,9 +498,9 @@ __global__ void __launch_bounds__(kRankThreads) cp_rank_kernel(const PostArgs a)
 
 // ------------------------------------------------------------------ mask
 constexpr int kMaskRows = 16;  // ranked boxes per tile; divides 64, so a tile's rows share a word
-constexpr int kMaskCtasPerTask = 148;
+constexpr int kMaskCtasPerTask = 98;  // six tasks: one wave of four CTAs an SM
 constexpr int kMaskThreads = 256;
-constexpr int kMaskSlots = 4;  // tiles of a CTA: at most 544 tiles a task
+constexpr int kMaskSlots = 6;  // tiles of a CTA: at most 544 tiles a task
 
 // The greedy walk over one task's ranking, by one CTA.  64 boxes at a time: four threads a box
 // look whether an earlier kept box suppresses it (its mask words are fetched while the 64 before
@@ -569,10 +591,7 @@ __device__ void pack_boxes(const PostArgs& a) {
   const uint32_t total = first[SPCONVB_CP_MAX_TASKS];
   if (threadIdx.x == 0) {
     *a.out_count = total;
-    if (a.out_count_host) {
-      *(volatile uint32_t*)a.out_count_host = total;
-      __threadfence_system();
-    }
+    if (a.out_count_host) *a.out_count_host = total;  // seen by the host when the kernel has ended
   }
   // a thread takes four boxes at a time: their ranks, then 44 values, in flight together
   constexpr int kAtOnce = 4;
@@ -686,7 +705,7 @@ __device__ __forceinline__ bool iou_reaches(const BoxRec& A, const BoxRec& B, fl
   return iou >= threshold;
 }
 
-// One tile = 16 boxes x 64 earlier ones; a CTA takes all its tiles (up to four) through each pass
+// One tile = 16 boxes x 64 earlier ones; a CTA takes all its tiles (up to six) through each pass
 // together.  Pass 1: every thread tests pairs for reach, bounds the IoU of the others and queues
 // what is left: 3 to 10 of a tile's 1 024, at most 30 in the benchmark's heads, so that what
 // counts is how long one pair takes and not how many there are.  Pass 2: a warp per queued pair.
@@ -696,7 +715,9 @@ __global__ void __launch_bounds__(kMaskThreads) cp_mask_kernel(const PostArgs a)
   const TaskBuffers& b = a.buf[task];
   const int tid = threadIdx.x;
   constexpr int kBoxes = 64 + kMaskRows;
-  __shared__ __align__(16) BoxRec s_box[kMaskSlots][kBoxes];
+  // 17 words a box: the lanes of a warp read the same field of 32 boxes
+  struct PaddedBox { BoxRec rec; float pad; };
+  __shared__ PaddedBox s_box[kMaskSlots][kBoxes];
   __shared__ int s_first[kMaskSlots][2];
   __shared__ unsigned long long words[kMaskSlots][kMaskRows];
   __shared__ uint16_t queue[kMaskSlots * kMaskRows * 64];
@@ -709,6 +730,9 @@ __global__ void __launch_bounds__(kMaskThreads) cp_mask_kernel(const PostArgs a)
   // tiles on or below the diagonal: 4 row groups of 16 in block row G, G + 1 tiles each
   const int groups = (m + kMaskRows - 1) / kMaskRows, whole = groups / 4;
   const int tiles = 2 * whole * (whole + 1) + (groups - 4 * whole) * (whole + 1);
+  // CTAs without a tile leave at once and are not waited for (one stays to walk an empty ranking)
+  const int ctas = max(1, min((int)gridDim.x, tiles));
+  if ((int)blockIdx.x >= ctas) return;
   int slots = 0;
   for (int tile = blockIdx.x; tile < tiles && slots < kMaskSlots; tile += gridDim.x, ++slots) {
     int G = 0;
@@ -719,10 +743,10 @@ __global__ void __launch_bounds__(kMaskThreads) cp_mask_kernel(const PostArgs a)
       s_first[slots][0] = row0;
       s_first[slots][1] = col0;
     }
-    for (int k = tid; k < kBoxes * 4; k += kMaskThreads) {
-      const int box = min(k < 256 ? col0 + k / 4 : row0 + k / 4 - 64, m - 1);
-      ((float4*)&s_box[slots][k / 4])[k & 3] =
-          ((const float4*)(b.box + (size_t)box * kBoxStride))[k & 3];
+#pragma unroll
+    for (int k = tid; k < kBoxes * kBoxStride; k += kMaskThreads) {
+      const int at = k / kBoxStride, box = min(at < 64 ? col0 + at : row0 + at - 64, m - 1);
+      ((float*)&s_box[slots][at])[k % kBoxStride] = b.box[(size_t)box * kBoxStride + k % kBoxStride];
     }
     if (tid < kMaskRows) words[slots][tid] = 0ull;
   }
@@ -732,7 +756,7 @@ __global__ void __launch_bounds__(kMaskThreads) cp_mask_kernel(const PostArgs a)
     const int slot = pair >> 10, r = (pair >> 6) & (kMaskRows - 1), c = pair & 63;
     const int i = s_first[slot][1] + c, j = s_first[slot][0] + r;
     if (j >= m || i >= j) continue;
-    const BoxRec &A = s_box[slot][c], &B = s_box[slot][64 + r];
+    const BoxRec &A = s_box[slot][c].rec, &B = s_box[slot][64 + r].rec;
     const float ddx = A.x - B.x, ddy = A.y - B.y;
     const float far = A.reach + B.reach + 0.1f;
     if (ddx * ddx + ddy * ddy > far * far) continue;  // the same test rotated_iou starts with
@@ -746,7 +770,7 @@ __global__ void __launch_bounds__(kMaskThreads) cp_mask_kernel(const PostArgs a)
   for (uint32_t q = tid >> 5; q < n_pairs; q += kMaskThreads / 32) {
     const int pair = queue[q], slot = pair >> 10, r = (pair >> 6) & (kMaskRows - 1), c = pair & 63;
     // the earlier box first
-    if (iou_reaches(s_box[slot][c], s_box[slot][64 + r], threshold, scratch[tid >> 5]) &&
+    if (iou_reaches(s_box[slot][c].rec, s_box[slot][64 + r].rec, threshold, scratch[tid >> 5]) &&
         (tid & 31) == 0)
       atomicOr(&words[slot][r], 1ull << c);
   }
@@ -758,7 +782,7 @@ __global__ void __launch_bounds__(kMaskThreads) cp_mask_kernel(const PostArgs a)
   }
   __threadfence();  // every thread's words are visible device-wide before the ticket is taken
   __syncthreads();
-  if (tid == 0) s_last = atomicAdd(b.ticket, 1u) == gridDim.x - 1u;
+  if (tid == 0) s_last = atomicAdd(b.ticket, 1u) == (uint32_t)ctas - 1u;
   __syncthreads();
   if (!s_last) return;
   __threadfence();
