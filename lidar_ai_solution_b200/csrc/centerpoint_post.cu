@@ -498,47 +498,52 @@ __global__ void __launch_bounds__(kRankThreads) cp_rank_kernel(const PostArgs a)
 
 // ------------------------------------------------------------------ mask
 constexpr int kMaskRows = 16;  // ranked boxes per tile; divides 64, so a tile's rows share a word
-constexpr int kMaskCtasPerTask = 98;  // six tasks: one wave of four CTAs an SM
+constexpr int kMaskCtasPerTask = 109;
 constexpr int kMaskThreads = 256;
-constexpr int kMaskSlots = 6;  // tiles of a CTA: at most 544 tiles a task
+constexpr int kMaskSlots = 5;  // tiles of a CTA: a task has at most 2 * 16 * 17 = 544
+static_assert(kMaskSlots * kMaskCtasPerTask >= 544, "tiles of a task");
 
 // The greedy walk over one task's ranking, by one CTA.  64 boxes at a time: four threads a box
-// look whether an earlier kept box suppresses it (its mask words are fetched while the 64 before
-// are decided), then the first warp decides among the 64: a box stays when every box of them that
+// look whether an earlier kept box suppresses it, then the first warp decides among the 64: a box stays when every box of them that
 // suppresses it is out, and is out when one of them stays, so the rounds are as many as the
 // longest chain of suppressions and not as the boxes.  Boxes after the first nms_post_max
 // survivors cannot reach the output.
-__device__ void walk_ranking(const PostArgs& a, const TaskBuffers& b, int m) {
-  constexpr int kEach = kMaskWords / 4;
+constexpr int kNearWords = 6;
+struct WalkShared {
+  unsigned long long word[kNearWords * 64][kNearWords];
+};
+__device__ void walk_ranking(const PostArgs& a, const TaskBuffers& b, int m, WalkShared& sh) {
   __shared__ unsigned long long s_keep[kMaskWords], s_inner[64];
   __shared__ uint32_t s_gone[2], s_kept;
   const int tid = threadIdx.x, box = tid >> 2, quarter = tid & 3;
   const uint32_t lane = tid & 31u;
   const int words = (m + 63) / 64;
-  unsigned long long next[kEach];
-  auto fetch = [&](int w) {
-#pragma unroll
-    for (int v = 0; v < kEach; ++v) {
-      const int word = 4 * v + quarter, j = w * 64 + box;
-      next[v] = w < words && word <= w && j < m ? __ldcg(b.mask + (size_t)j * kMaskWords + word) : 0ull;
-    }
-  };
   if (tid == 0) s_kept = 0u;
-  fetch(0);
+  // the walk usually ends within the first few hundred boxes: their words are fetched together
+  const int near = min(words, kNearWords);
+#pragma unroll
+  for (int k = tid; k < kNearWords * 64 * kNearWords; k += kMaskThreads) {
+    const int j = k / kNearWords, word = k % kNearWords;
+    sh.word[j][word] = j < m && word <= j / 64 ? __ldcg(b.mask + (size_t)j * kMaskWords + word) : 0ull;
+  }
+  __syncthreads();
   for (int w = 0; w < words; ++w) {
     if (tid < 2) s_gone[tid] = 0u;
     __syncthreads();
     const uint32_t kept = s_kept;
     if (kept >= (uint32_t)a.p.nms_post_max) break;
-    bool gone = w * 64 + box >= m;
+    const int j = w * 64 + box;
+    bool gone = j >= m;
 #pragma unroll
-    for (int v = 0; v < kEach; ++v) {
+    for (int v = 0; v < kMaskWords / 4; ++v) {
       const int word = 4 * v + quarter;
-      if (word < w) gone = gone || (next[v] & s_keep[word]) != 0ull;
-      else if (word == w) s_inner[box] = next[v];
+      if (word > w || j >= m) continue;
+      const unsigned long long bits =
+          w < near ? sh.word[j][word] : __ldcg(b.mask + (size_t)j * kMaskWords + word);
+      if (word < w) gone = gone || (bits & s_keep[word]) != 0ull;
+      else s_inner[box] = bits;
     }
     if (gone) atomicOr(&s_gone[box >> 5], 1u << (box & 31));
-    fetch(w + 1);
     __syncthreads();
     if (tid < 32) {
       // lane l decides boxes l and 32 + l
@@ -575,7 +580,12 @@ __device__ void walk_ranking(const PostArgs& a, const TaskBuffers& b, int m) {
 }
 
 // The last task to get here packs every task's boxes into the caller's list, in task order.
-__device__ void pack_boxes(const PostArgs& a) {
+constexpr int kPackBoxes = 1024;
+struct PackShared {
+  const float* from[kPackBoxes];
+  int offset[kPackBoxes];
+};
+__device__ void pack_boxes(const PostArgs& a, PackShared& sh) {
   __shared__ bool s_last_task;
   __threadfence();
   __syncthreads();
@@ -593,38 +603,31 @@ __device__ void pack_boxes(const PostArgs& a) {
     *a.out_count = total;
     if (a.out_count_host) *a.out_count_host = total;  // seen by the host when the kernel has ended
   }
-  // a thread takes four boxes at a time: their ranks, then 44 values, in flight together
-  constexpr int kAtOnce = 4;
-  for (uint32_t k0 = threadIdx.x; k0 < total; k0 += kAtOnce * kMaskThreads) {
-    const float* from[kAtOnce];
-    int offset[kAtOnce];
-#pragma unroll
-    for (int u = 0; u < kAtOnce; ++u) {
-      const uint32_t k = min(k0 + u * kMaskThreads, total - 1u);
-      const uint32_t* kept = a.buf[0].kept + k;
+  // where the boxes stand, then their values in the order of the list (coalesced both ways)
+  for (uint32_t base = 0; base < total; base += kPackBoxes) {
+    const uint32_t boxes = min(total - base, (uint32_t)kPackBoxes);
+    __syncthreads();
+    for (uint32_t k = threadIdx.x; k < boxes; k += kMaskThreads) {
+      const uint32_t* kept = a.buf[0].kept + base + k;
       const float* det = a.buf[0].det;
-      offset[u] = a.head[0].label_offset;
+      int offset = a.head[0].label_offset;
 #pragma unroll
       for (int q = 1; q < SPCONVB_CP_MAX_TASKS; ++q)
-        if (q < a.num_tasks && k >= first[q]) {
-          kept = a.buf[q].kept + (k - first[q]);
+        if (q < a.num_tasks && base + k >= first[q]) {
+          kept = a.buf[q].kept + (base + k - first[q]);
           det = a.buf[q].det;
-          offset[u] = a.head[q].label_offset;
+          offset = a.head[q].label_offset;
         }
-      from[u] = det + (size_t)__ldcg(kept) * kDet;
+      sh.from[k] = det + (size_t)__ldcg(kept) * kDet;
+      sh.offset[k] = offset;
     }
-    float v[kAtOnce][kDet];
-#pragma unroll
-    for (int u = 0; u < kAtOnce; ++u)
-#pragma unroll
-      for (int f = 0; f < kDet; ++f) v[u][f] = __ldcg(from[u] + f);
-#pragma unroll
-    for (int u = 0; u < kAtOnce; ++u) {
-      const uint32_t k = k0 + u * kMaskThreads;
-      if (k >= total) break;
-      v[u][9] = (float)(offset[u] + (int)v[u][9]);
-#pragma unroll
-      for (int f = 0; f < kDet; ++f) a.out_boxes[(size_t)k * kDet + f] = v[u][f];
+    __syncthreads();
+#pragma unroll 8
+    for (uint32_t e = threadIdx.x; e < boxes * kDet; e += kMaskThreads) {
+      const uint32_t k = e / kDet, f = e - k * kDet;
+      float v = __ldcg(sh.from[k] + f);
+      if (f == 9u) v = (float)(sh.offset[k] + (int)v);
+      a.out_boxes[(size_t)base * kDet + e] = v;
     }
   }
 }
@@ -653,8 +656,12 @@ __device__ __forceinline__ bool surely_below(const BoxBounds& A, const BoxBounds
 // of A and e % 4 of B, lanes 16..23 at the corners, in the order in which the serial code appends
 // its points; sums run in that order and in the order of the angles, so every bit is the same.
 // Boxes with a coordinate that is not a number overlap nothing, as there.
+struct IouScratch {
+  Pt point[24], sorted[24];
+  float value[24];
+};
 __device__ __forceinline__ bool iou_reaches(const BoxRec& A, const BoxRec& B, float threshold,
-                                            Pt* scratch) {
+                                            IouScratch& sh) {
   const uint32_t lane = threadIdx.x & 31u;
   Pt p = {0.f, 0.f};
   bool have = false;
@@ -670,34 +677,41 @@ __device__ __forceinline__ bool iou_reaches(const BoxRec& A, const BoxRec& B, fl
   const int cnt = __popc(set);
   float iou = 0.f;
   if (cnt != 0) {
+    // lane k goes on with point k; what is summed in order goes through shared memory
+    __syncwarp();
+    if (have) sh.point[__popc(set & ((1u << lane) - 1u))] = p;
+    __syncwarp();
     Pt centre = {0.f, 0.f};
-    for (uint32_t left = set; left; left &= left - 1u) {
-      const int from = __ffs((int)left) - 1;
-      centre.x = centre.x + __shfl_sync(0xffffffffu, p.x, from);
-      centre.y = centre.y + __shfl_sync(0xffffffffu, p.y, from);
+#pragma unroll 4
+    for (int k = 0; k < cnt; ++k) {
+      centre.x = centre.x + sh.point[k].x;
+      centre.y = centre.y + sh.point[k].y;
     }
     centre.x /= (float)cnt;
     centre.y /= (float)cnt;
-    const float ang = have ? atan2f(p.y - centre.y, p.x - centre.x) : 0.f;
+    const bool mine = (int)lane < cnt;
+    if (mine) p = sh.point[lane];
+    const float ang = mine ? atan2f(p.y - centre.y, p.x - centre.x) : 0.f;
+    if (mine) sh.value[lane] = ang;
     if (__any_sync(0xffffffffu, ang != ang)) return false;
     // place in the stable ascending order of the angles
     int place = 0;
-    for (uint32_t left = set; left; left &= left - 1u) {
-      const int from = __ffs((int)left) - 1;
-      const float other = __shfl_sync(0xffffffffu, ang, from);
-      if (other < ang || (other == ang && from < (int)lane)) ++place;
+#pragma unroll 4
+    for (int k = 0; k < cnt; ++k) {
+      const float other = sh.value[k];
+      if (other < ang || (other == ang && k < (int)lane)) ++place;
     }
+    if (mine) sh.sorted[place] = p;
     __syncwarp();
-    if (have) scratch[place] = p;
-    __syncwarp();
-    float term = 0.f;
     if ((int)lane + 1 < cnt) {
-      const Pt p0 = scratch[0], pk = scratch[lane], pn = scratch[lane + 1];
+      const Pt p0 = sh.sorted[0], pk = sh.sorted[lane], pn = sh.sorted[lane + 1];
       const float ax = pk.x - p0.x, ay = pk.y - p0.y, bx = pn.x - p0.x, by = pn.y - p0.y;
-      term = ax * by - ay * bx;
+      sh.value[lane] = ax * by - ay * bx;
     }
+    __syncwarp();
     float area = 0.f;
-    for (int k = 0; k + 1 < cnt; ++k) area += __shfl_sync(0xffffffffu, term, k);
+#pragma unroll 4
+    for (int k = 0; k + 1 < cnt; ++k) area += sh.value[k];
     const float overlap = fabsf(area) / 2.0f;
     const float sa = A.dx * A.dy, sb = B.dx * B.dy;
     iou = overlap / fmaxf(sa + sb - overlap, 1e-8f);
@@ -705,7 +719,7 @@ __device__ __forceinline__ bool iou_reaches(const BoxRec& A, const BoxRec& B, fl
   return iou >= threshold;
 }
 
-// One tile = 16 boxes x 64 earlier ones; a CTA takes all its tiles (up to six) through each pass
+// One tile = 16 boxes x 64 earlier ones; a CTA takes all its tiles (up to five) through each pass
 // together.  Pass 1: every thread tests pairs for reach, bounds the IoU of the others and queues
 // what is left: 3 to 10 of a tile's 1 024, at most 30 in the benchmark's heads, so that what
 // counts is how long one pair takes and not how many there are.  Pass 2: a warp per queued pair.
@@ -717,11 +731,18 @@ __global__ void __launch_bounds__(kMaskThreads) cp_mask_kernel(const PostArgs a)
   constexpr int kBoxes = 64 + kMaskRows;
   // 17 words a box: the lanes of a warp read the same field of 32 boxes
   struct PaddedBox { BoxRec rec; float pad; };
-  __shared__ PaddedBox s_box[kMaskSlots][kBoxes];
+  __shared__ union {
+    struct {
+      PaddedBox box[kMaskSlots][kBoxes];
+      uint16_t near[kMaskSlots * kMaskRows * 64];  // pairs in reach; those left go to its front
+    } tiles;
+    WalkShared walk;
+    PackShared pack;
+  } sh;
   __shared__ int s_first[kMaskSlots][2];
   __shared__ unsigned long long words[kMaskSlots][kMaskRows];
-  __shared__ uint16_t queue[kMaskSlots * kMaskRows * 64];
-  __shared__ Pt scratch[kMaskThreads / 32][24];
+  __shared__ IouScratch scratch[kMaskThreads / 32];
+  __shared__ uint32_t in_reach;
   __shared__ uint32_t queued;
   __shared__ bool s_last;
   pdl_wait();
@@ -733,44 +754,75 @@ __global__ void __launch_bounds__(kMaskThreads) cp_mask_kernel(const PostArgs a)
   // CTAs without a tile leave at once and are not waited for (one stays to walk an empty ranking)
   const int ctas = max(1, min((int)gridDim.x, tiles));
   if ((int)blockIdx.x >= ctas) return;
-  int slots = 0;
-  for (int tile = blockIdx.x; tile < tiles && slots < kMaskSlots; tile += gridDim.x, ++slots) {
+  const int slots = max(0, (tiles - (int)blockIdx.x + ctas - 1) / ctas);
+  if (tid < slots) {
+    const int tile = blockIdx.x + tid * ctas;
     int G = 0;
     while (2 * (G + 1) * (G + 2) <= tile) ++G;
-    const int in = tile - 2 * G * (G + 1), row0 = (4 * G + in / (G + 1)) * kMaskRows;
-    const int col0 = in % (G + 1) * 64;
-    if (tid == 0) {
-      s_first[slots][0] = row0;
-      s_first[slots][1] = col0;
+    const int in = tile - 2 * G * (G + 1);
+    s_first[tid][0] = (4 * G + in / (G + 1)) * kMaskRows;
+    s_first[tid][1] = in % (G + 1) * 64;
+  }
+  if (tid < kMaskSlots * kMaskRows) words[tid / kMaskRows][tid % kMaskRows] = 0ull;
+  if (tid == 0) in_reach = queued = 0u;
+  __syncthreads();
+  {
+    float4 v[kMaskSlots * kBoxes * 4 / kMaskThreads + 1];  // all in flight together
+#pragma unroll
+    for (int u = 0; u < kMaskSlots * kBoxes * 4 / kMaskThreads + 1; ++u) {
+      const int k = tid + u * kMaskThreads, slot = k / (kBoxes * 4), at = k / 4 % kBoxes;
+      if (slot >= slots) break;
+      const int box = min(at < 64 ? s_first[slot][1] + at : s_first[slot][0] + at - 64, m - 1);
+      v[u] = __ldcg((const float4*)(b.box + (size_t)box * kBoxStride) + (k & 3));
     }
 #pragma unroll
-    for (int k = tid; k < kBoxes * kBoxStride; k += kMaskThreads) {
-      const int at = k / kBoxStride, box = min(at < 64 ? col0 + at : row0 + at - 64, m - 1);
-      ((float*)&s_box[slots][at])[k % kBoxStride] = b.box[(size_t)box * kBoxStride + k % kBoxStride];
+    for (int u = 0; u < kMaskSlots * kBoxes * 4 / kMaskThreads + 1; ++u) {
+      const int k = tid + u * kMaskThreads, slot = k / (kBoxes * 4), at = k / 4 % kBoxes;
+      if (slot >= slots) break;
+      float* to = (float*)&sh.tiles.box[slot][at] + (k & 3) * 4;
+      to[0] = v[u].x; to[1] = v[u].y; to[2] = v[u].z; to[3] = v[u].w;
     }
-    if (tid < kMaskRows) words[slots][tid] = 0ull;
   }
-  if (tid == 0) queued = 0u;
   __syncthreads();
-  for (int pair = tid; pair < slots * kMaskRows * 64; pair += kMaskThreads) {
-    const int slot = pair >> 10, r = (pair >> 6) & (kMaskRows - 1), c = pair & 63;
-    const int i = s_first[slot][1] + c, j = s_first[slot][0] + r;
-    if (j >= m || i >= j) continue;
-    const BoxRec &A = s_box[slot][c].rec, &B = s_box[slot][64 + r].rec;
-    const float ddx = A.x - B.x, ddy = A.y - B.y;
-    const float far = A.reach + B.reach + 0.1f;
-    if (ddx * ddx + ddy * ddy > far * far) continue;  // the same test rotated_iou starts with
-    if (surely_below({A.x, A.y, A.dx, A.dy, A.cos_neg, A.sin_neg},
-                     {B.x, B.y, B.dx, B.dy, B.cos_neg, B.sin_neg}, threshold))
-      continue;
-    queue[atomicAdd(&queued, 1u)] = (uint16_t)pair;
+  for (int slot = 0; slot < slots; ++slot) {
+    // a thread keeps its column and takes every fourth row
+    const int c = tid & 63, i = s_first[slot][1] + c;
+    const BoxRec& A = sh.tiles.box[slot][c].rec;
+    const float x = A.x, y = A.y, reach = A.reach;
+#pragma unroll
+    for (int u = 0; u < kMaskRows / 4; ++u) {
+      const int r = (tid >> 6) + 4 * u, j = s_first[slot][0] + r;
+      const BoxRec& B = sh.tiles.box[slot][64 + r].rec;
+      const float ddx = x - B.x, ddy = y - B.y, far = reach + B.reach + 0.1f;
+      // the same test rotated_iou starts with
+      if (j < m && i < j && !(ddx * ddx + ddy * ddy > far * far))
+        sh.tiles.near[atomicAdd(&in_reach, 1u)] = (uint16_t)(slot << 10 | r << 6 | c);
+    }
+  }
+  __syncthreads();
+  const uint32_t n_reach = in_reach;
+  for (uint32_t q0 = 0; q0 < n_reach; q0 += kMaskThreads) {
+    const uint32_t q = q0 + tid;
+    bool stays = false;
+    uint16_t pair = 0;
+    if (q < n_reach) {
+      pair = sh.tiles.near[q];
+      const BoxRec& A = sh.tiles.box[pair >> 10][pair & 63].rec;
+      const BoxRec& B = sh.tiles.box[pair >> 10][64 + ((pair >> 6) & (kMaskRows - 1))].rec;
+      stays = !surely_below({A.x, A.y, A.dx, A.dy, A.cos_neg, A.sin_neg},
+                            {B.x, B.y, B.dx, B.dy, B.cos_neg, B.sin_neg}, threshold);
+    }
+    __syncthreads();  // this round's pairs are read; fewer than that are kept
+    if (stays) sh.tiles.near[atomicAdd(&queued, 1u)] = pair;
   }
   __syncthreads();
   const uint32_t n_pairs = queued;
   for (uint32_t q = tid >> 5; q < n_pairs; q += kMaskThreads / 32) {
-    const int pair = queue[q], slot = pair >> 10, r = (pair >> 6) & (kMaskRows - 1), c = pair & 63;
+    const int pair = sh.tiles.near[q], slot = pair >> 10, r = (pair >> 6) & (kMaskRows - 1);
+    const int c = pair & 63;
     // the earlier box first
-    if (iou_reaches(s_box[slot][c].rec, s_box[slot][64 + r].rec, threshold, scratch[tid >> 5]) &&
+    if (iou_reaches(sh.tiles.box[slot][c].rec, sh.tiles.box[slot][64 + r].rec, threshold,
+                    scratch[tid >> 5]) &&
         (tid & 31) == 0)
       atomicOr(&words[slot][r], 1ull << c);
   }
@@ -786,8 +838,8 @@ __global__ void __launch_bounds__(kMaskThreads) cp_mask_kernel(const PostArgs a)
   __syncthreads();
   if (!s_last) return;
   __threadfence();
-  walk_ranking(a, b, m);
-  pack_boxes(a);
+  walk_ranking(a, b, m, sh.walk);
+  pack_boxes(a, sh.pack);
 }
 
 bool params_ok(const spconvb_cp_params* p) {
