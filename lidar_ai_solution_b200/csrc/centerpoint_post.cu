@@ -498,9 +498,9 @@ __global__ void __launch_bounds__(kRankThreads) cp_rank_kernel(const PostArgs a)
 
 // ------------------------------------------------------------------ mask
 constexpr int kMaskRows = 16;  // ranked boxes per tile; divides 64, so a tile's rows share a word
-constexpr int kMaskCtasPerTask = 109;
+constexpr int kMaskCtasPerTask = 98;  // six tasks: one wave of four CTAs an SM
 constexpr int kMaskThreads = 256;
-constexpr int kMaskSlots = 5;  // tiles of a CTA: a task has at most 2 * 16 * 17 = 544
+constexpr int kMaskSlots = 6;  // tiles of a CTA: a task has at most 2 * 16 * 17 = 544
 static_assert(kMaskSlots * kMaskCtasPerTask >= 544, "tiles of a task");
 
 // The greedy walk over one task's ranking, by one CTA.  64 boxes at a time: four threads a box
@@ -622,12 +622,22 @@ __device__ void pack_boxes(const PostArgs& a, PackShared& sh) {
       sh.offset[k] = offset;
     }
     __syncthreads();
-#pragma unroll 8
-    for (uint32_t e = threadIdx.x; e < boxes * kDet; e += kMaskThreads) {
-      const uint32_t k = e / kDet, f = e - k * kDet;
-      float v = __ldcg(sh.from[k] + f);
-      if (f == 9u) v = (float)(sh.offset[k] + (int)v);
-      a.out_boxes[(size_t)base * kDet + e] = v;
+    // eight values a thread in flight (the stores may not be moved past loads, so by hand)
+    constexpr uint32_t kAtOnce = 8;
+    for (uint32_t e0 = threadIdx.x; e0 < boxes * kDet; e0 += kAtOnce * kMaskThreads) {
+      float v[kAtOnce];
+#pragma unroll
+      for (uint32_t u = 0; u < kAtOnce; ++u) {
+        const uint32_t e = min(e0 + u * kMaskThreads, boxes * kDet - 1u), k = e / kDet;
+        v[u] = __ldcg(sh.from[k] + (e - k * kDet));
+      }
+#pragma unroll
+      for (uint32_t u = 0; u < kAtOnce; ++u) {
+        const uint32_t e = e0 + u * kMaskThreads, k = e / kDet;
+        if (e >= boxes * kDet) break;
+        a.out_boxes[(size_t)base * kDet + e] =
+            e - k * kDet == 9u ? (float)(sh.offset[k] + (int)v[u]) : v[u];
+      }
     }
   }
 }
@@ -657,7 +667,7 @@ __device__ __forceinline__ bool surely_below(const BoxBounds& A, const BoxBounds
 // its points; sums run in that order and in the order of the angles, so every bit is the same.
 // Boxes with a coordinate that is not a number overlap nothing, as there.
 struct IouScratch {
-  Pt point[24], sorted[24];
+  Pt point[24];  // in the order of the serial code, then of the angles
   float value[24];
 };
 __device__ __forceinline__ bool iou_reaches(const BoxRec& A, const BoxRec& B, float threshold,
@@ -701,10 +711,10 @@ __device__ __forceinline__ bool iou_reaches(const BoxRec& A, const BoxRec& B, fl
       const float other = sh.value[k];
       if (other < ang || (other == ang && k < (int)lane)) ++place;
     }
-    if (mine) sh.sorted[place] = p;
+    if (mine) sh.point[place] = p;
     __syncwarp();
     if ((int)lane + 1 < cnt) {
-      const Pt p0 = sh.sorted[0], pk = sh.sorted[lane], pn = sh.sorted[lane + 1];
+      const Pt p0 = sh.point[0], pk = sh.point[lane], pn = sh.point[lane + 1];
       const float ax = pk.x - p0.x, ay = pk.y - p0.y, bx = pn.x - p0.x, by = pn.y - p0.y;
       sh.value[lane] = ax * by - ay * bx;
     }
@@ -719,7 +729,7 @@ __device__ __forceinline__ bool iou_reaches(const BoxRec& A, const BoxRec& B, fl
   return iou >= threshold;
 }
 
-// One tile = 16 boxes x 64 earlier ones; a CTA takes all its tiles (up to five) through each pass
+// One tile = 16 boxes x 64 earlier ones; a CTA takes all its tiles (up to six) through each pass
 // together.  Pass 1: every thread tests pairs for reach, bounds the IoU of the others and queues
 // what is left: 3 to 10 of a tile's 1 024, at most 30 in the benchmark's heads, so that what
 // counts is how long one pair takes and not how many there are.  Pass 2: a warp per queued pair.
