@@ -2,6 +2,7 @@
 // and channel-padding conversion, and the sparse -> dense BEV scatter.
 #include "common.cuh"
 #include "pdl.cuh"
+#include "rulebook.hpp"
 
 namespace spconvb {
 
@@ -166,52 +167,98 @@ __global__ void pad8_f16_kernel(const __half* __restrict__ x, int cin, const uin
   }
 }
 
-// 32 rows per block: rows are read coalesced into shared memory, then written
-// channel by channel so that neighbouring rows (neighbouring cells when the
-// rows are in canonical order) share write sectors.
-__global__ void scatter_dense_kernel(const void* __restrict__ feat, int in_kind, float in_scale,
-                                     const int4* __restrict__ coords, const uint32_t* n_ptr,
-                                     uint32_t cap, int channels, Grid3 g, int p0, int p1, int p2,
-                                     __half* __restrict__ out) {
+// Rows into [N, C, g(p0), g(p1), g(p2)].  A block takes 32 rows at a time through shared memory and
+// writes them channel by channel, a lane a cell, so that neighbouring cells share write sectors;
+// what bounds it is the number of sectors written, one per channel and run of neighbours.
+// BY_CELL: the 32 are the rows of 32 consecutive cells of the *output*, found by rank in the bitmap
+// of the strided rulebook that made them.  Taken when the output's axes are permuted: rows in their
+// own order then lie a line apart, every 2-byte store is a sector of its own, and the BEVFusion
+// sample frame took 43 us, this way 7.  (Not otherwise: it looks up all cells, and in row order the
+// runs are the same.)
+// VEC: fp16 rows of whole 16-byte pieces; 16-byte loads, one channel loop without divisions
+// (CenterPoint frame of 10 800 voxels 15 us, this way 6).
+template <bool BY_CELL, bool VEC>
+__global__ void __launch_bounds__(256)
+    scatter_dense_kernel(const void* __restrict__ feat, int in_kind, float in_scale,
+                         const int4* __restrict__ coords, const uint32_t* n_ptr, uint32_t cap,
+                         int channels, Grid3 g, int p0, int p1, int p2,
+                         const uint32_t* __restrict__ bitmap, const uint32_t* __restrict__ prefix,
+                         __half* __restrict__ out) {
   extern __shared__ __half tile[];  // [channels][33]
+  __shared__ int32_t s_row[32];
   __shared__ long long s_cell[32];
   pdl_wait();
-  const uint32_t n = min(load_after_wait(n_ptr), cap);
   const int gp[3] = {g.g[p0], g.g[p1], g.g[p2]};
   const size_t vol = (size_t)gp[0] * gp[1] * gp[2];
-  for (uint32_t row0 = blockIdx.x * 32; row0 < n; row0 += gridDim.x * 32) {
-    __syncthreads();
+  const uint32_t n = BY_CELL ? (uint32_t)vol * g.batch : min(load_after_wait(n_ptr), cap);
+  const uint32_t lane = threadIdx.x & 31u;
+  for (uint32_t at0 = blockIdx.x * 32; at0 < n; at0 += gridDim.x * 32) {
+    int any = 0;
     if (threadIdx.x < 32) {
+      const uint32_t at = at0 + threadIdx.x;
+      int32_t row = -1;
       long long cell = -1;
-      uint32_t row = row0 + threadIdx.x;
-      if (row < n) {
-        int4 c = coords[row];
-        const int sp[3] = {c.y, c.z, c.w};
-        const int s0 = sp[p0], s1 = sp[p1], s2 = sp[p2];
-        if ((unsigned)c.x < (unsigned)g.batch && (unsigned)s0 < (unsigned)gp[0] &&
-            (unsigned)s1 < (unsigned)gp[1] && (unsigned)s2 < (unsigned)gp[2])
-          cell = (long long)c.x * channels * (long long)vol + ((long long)s0 * gp[1] + s1) * gp[2] + s2;
+      if (at < n) {
+        if (BY_CELL) {
+          const uint32_t line = at / gp[2], s2 = at - line * gp[2];
+          const uint32_t plane = line / gp[1], s1 = line - plane * gp[1];
+          const uint32_t b = plane / gp[0], s0 = plane - b * gp[0];
+          int c[3];
+          c[p0] = (int)s0; c[p1] = (int)s1; c[p2] = (int)s2;
+          row = rank_lookup(bitmap, prefix, voxel_key((int)b, c[0], c[1], c[2], g), cap);
+          if (row >= 0)
+            cell = (long long)(at - b * (uint32_t)vol) + (long long)b * channels * (long long)vol;
+        } else {
+          const int4 c = coords[at];
+          const int sp[3] = {c.y, c.z, c.w};
+          const int s0 = sp[p0], s1 = sp[p1], s2 = sp[p2];
+          if ((unsigned)c.x < (unsigned)g.batch && (unsigned)s0 < (unsigned)gp[0] &&
+              (unsigned)s1 < (unsigned)gp[1] && (unsigned)s2 < (unsigned)gp[2]) {
+            row = (int32_t)at;
+            cell = (long long)c.x * channels * (long long)vol +
+                   ((long long)s0 * gp[1] + s1) * gp[2] + s2;
+          }
+        }
       }
+      s_row[threadIdx.x] = row;
       s_cell[threadIdx.x] = cell;
+      any = row >= 0;
     }
-    for (int i = threadIdx.x; i < 32 * channels; i += blockDim.x) {
-      const int r = i / channels, ch = i % channels;
-      const uint32_t row = row0 + r;
-      __half v = __float2half(0.f);
-      if (row < n) {
+    if (!__syncthreads_or(any)) continue;  // (every thread is past the tile of the round before)
+    if (VEC) {
+      const int segs = channels >> 3;
+      for (int i = threadIdx.x; i < 32 * segs; i += 256) {
+        const int r = i / segs, seg = i - r * segs;
+        const int32_t row = s_row[r];
+        if (row < 0) continue;
+        const uint4 v = __ldg((const uint4*)feat + (size_t)row * segs + seg);
+        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+        __half* to = tile + seg * 8 * 33 + r;
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+          to[q * 33] = __ushort_as_half((unsigned short)(w[q >> 1] >> (16 * (q & 1))));
+      }
+    } else {
+      for (int i = threadIdx.x; i < 32 * channels; i += 256) {
+        const int r = i / channels, ch = i - r * channels;
+        const int32_t row = s_row[r];
+        if (row < 0) continue;
         const size_t j = (size_t)row * channels + ch;
-        v = in_kind == SPCONVB_I8
+        tile[ch * 33 + r] =
+            in_kind == SPCONVB_I8
                 ? __float2half_rn(__fmul_rn((float)((const int8_t*)feat)[j], in_scale))
                 : ((const __half*)feat)[j];
       }
-      tile[ch * 33 + r] = v;
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < 32 * channels; i += blockDim.x) {
-      const int ch = i >> 5, r = i & 31;
-      const long long cell = s_cell[r];
-      if (cell >= 0) out[cell + (long long)ch * (long long)vol] = tile[ch * 33 + r];
+    const long long cell = s_cell[lane];
+    if (cell >= 0) {
+      __half* o = out + cell;
+#pragma unroll 4
+      for (int ch = threadIdx.x >> 5; ch < channels; ch += 8)
+        o[(size_t)ch * vol] = tile[ch * 33 + lane];
     }
+    __syncthreads();
   }
 }
 
@@ -275,12 +322,12 @@ static inline uint32_t clamp_u32(size_t v) { return v > 0xffffffffull ? 0xffffff
 int scatter_dense_launch(const void* feat, int32_t in_kind, float in_scale, const int32_t* coords,
                          const uint32_t* n_ptr, uint32_t launch_rows, int32_t channels,
                          int32_t batch, const int32_t grid[3], const int32_t perm[3], void* out,
-                         bool clear, void* stream);
+                         bool clear, const DownWs* rank, void* stream);
 int scatter_dense_layout_launch(const void* feat, int32_t in_kind, float in_scale,
                                 const int32_t* coords, const uint32_t* n_ptr, uint32_t launch_rows,
                                 int32_t channels, int32_t batch, const int32_t grid[3],
                                 const int32_t perm[3], int32_t layout, int32_t out_kind,
-                                float inv_out_scale, void* out, bool clear, void* stream);
+                                float inv_out_scale, void* out, bool clear, const DownWs* rank, void* stream);
 
 }  // namespace spconvb
 
@@ -361,14 +408,14 @@ int spconvb_scatter_dense(const void* feat, int32_t in_kind, float in_scale,
                           int32_t channels, int32_t batch, const int32_t grid[3],
                           const int32_t perm[3], void* out, void* stream) {
   return spconvb::scatter_dense_launch(feat, in_kind, in_scale, coords, n_ptr, launch_rows,
-                                       channels, batch, grid, perm, out, true, stream);
+                                       channels, batch, grid, perm, out, true, nullptr, stream);
 }
 
 extern "C++" int spconvb::scatter_dense_launch(const void* feat, int32_t in_kind, float in_scale,
                                   const int32_t* coords, const uint32_t* n_ptr,
                                   uint32_t launch_rows, int32_t channels, int32_t batch,
                                   const int32_t grid[3], const int32_t perm[3], void* out,
-                                  bool clear, void* stream) {
+                                  bool clear, const DownWs* rank, void* stream) {
   if (!feat || !coords || !n_ptr || !grid || !out || channels < 1 || channels > 1024 ||
       batch < 1 || launch_rows < 1)
     return SPCONVB_E_ARG;
@@ -378,18 +425,23 @@ extern "C++" int spconvb::scatter_dense_launch(const void* feat, int32_t in_kind
     if ((1 << p[0] | 1 << p[1] | 1 << p[2]) != 7) return SPCONVB_E_ARG;
   }
   cudaStream_t st = (cudaStream_t)stream;
+  // fp16 rows of 16-byte pieces; a permuted output with a rank index (see the kernel)
+  const bool vec = in_kind == SPCONVB_F16 && channels % 8 == 0 && ((uintptr_t)feat & 15u) == 0u;
+  const bool by_cell = rank != nullptr && p[2] != 2;
+  auto* kernel = by_cell ? (vec ? scatter_dense_kernel<true, true> : scatter_dense_kernel<true, false>)
+                         : (vec ? scatter_dense_kernel<false, true> : scatter_dense_kernel<false, false>);
   const size_t tile_bytes = sizeof(__half) * 33 * (size_t)channels;
-  if (tile_bytes > 48 * 1024) {
+  if (tile_bytes > 48 * 1024 - 512) {
     // wider rows than the default shared-memory window: raise the kernel's limit (once per
     // device; channels <= 1024 needs 66 KB)
-    static bool raised[64] = {};
+    static bool raised[64][4] = {};
     int dev = 0;
     SPCONVB_CUDA_TRY(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= 64 || !raised[dev]) {
-      SPCONVB_CUDA_TRY(cudaFuncSetAttribute(scatter_dense_kernel,
-                                            cudaFuncAttributeMaxDynamicSharedMemorySize,
+    const int which = 2 * by_cell + vec;
+    if (dev < 0 || dev >= 64 || !raised[dev][which]) {
+      SPCONVB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                             (int)(sizeof(__half) * 33 * 1024)));
-      if (dev >= 0 && dev < 64) raised[dev] = true;
+      if (dev >= 0 && dev < 64) raised[dev][which] = true;
     }
   }
   Grid3 g;
@@ -397,13 +449,15 @@ extern "C++" int spconvb::scatter_dense_launch(const void* feat, int32_t in_kind
   g.batch = batch;
   const size_t bytes = sizeof(__half) * (size_t)batch * channels * grid[0] * grid[1] * grid[2];
   if (clear) SPCONVB_CUDA_TRY(cudaMemsetAsync(out, 0, bytes, st));
-  size_t want_blocks = ((size_t)launch_rows + 31) / 32;
+  const size_t items = by_cell ? (size_t)batch * grid[0] * grid[1] * grid[2] : launch_rows;
+  size_t want_blocks = (items + 31) / 32;
   if (want_blocks > (size_t)kSmCount * 16) want_blocks = (size_t)kSmCount * 16;
   const int blocks = (int)want_blocks;
-  SPCONVB_CUDA_TRY(launch_pdl(scatter_dense_kernel, dim3(blocks), dim3(256),
-                              sizeof(__half) * 33 * channels, st, feat, in_kind, in_scale,
-                              (const int4*)coords, n_ptr, launch_rows, channels, g, p[0], p[1], p[2],
-                              (__half*)out));
+  const uint32_t* bitmap = by_cell ? rank->bitmap : nullptr;
+  const uint32_t* prefix = by_cell ? rank->prefix : nullptr;
+  SPCONVB_CUDA_TRY(launch_pdl(kernel, dim3(blocks), dim3(256), tile_bytes, st, feat, in_kind,
+                              in_scale, (const int4*)coords, n_ptr, launch_rows, channels, g, p[0],
+                              p[1], p[2], bitmap, prefix, (__half*)out));
   return SPCONVB_OK;
 }
 
@@ -414,7 +468,7 @@ int spconvb_scatter_dense_layout(const void* feat, int32_t in_kind, float in_sca
                                  int32_t out_kind, float inv_out_scale, void* out, void* stream) {
   return spconvb::scatter_dense_layout_launch(feat, in_kind, in_scale, coords, n_ptr, launch_rows,
                                               channels, batch, grid, perm, layout, out_kind,
-                                              inv_out_scale, out, true, stream);
+                                              inv_out_scale, out, true, nullptr, stream);
 }
 
 extern "C++" int spconvb::scatter_dense_layout_launch(const void* feat, int32_t in_kind, float in_scale,
@@ -422,11 +476,11 @@ extern "C++" int spconvb::scatter_dense_layout_launch(const void* feat, int32_t 
                                          uint32_t launch_rows, int32_t channels, int32_t batch,
                                          const int32_t grid[3], const int32_t perm[3],
                                          int32_t layout, int32_t out_kind, float inv_out_scale,
-                                         void* out, bool clear, void* stream) {
+                                         void* out, bool clear, const DownWs* rank, void* stream) {
   if (layout == 0) layout = 1;
   if (layout == 1 && out_kind == SPCONVB_F16)
     return scatter_dense_launch(feat, in_kind, in_scale, coords, n_ptr, launch_rows, channels,
-                                batch, grid, perm, out, clear, stream);
+                                batch, grid, perm, out, clear, rank, stream);
   if (!feat || !coords || !n_ptr || !grid || !out || channels < 1 || channels > 1024 ||
       batch < 1 || launch_rows < 1 || layout < 1 || layout > 3 ||
       (out_kind != SPCONVB_F16 && out_kind != SPCONVB_I8) ||

@@ -1095,11 +1095,13 @@ int Engine::forward(const void* features, const int32_t* indices, uint32_t cap_r
         break;
       case Step::DENSE: {
         const CoordSet& cs = coordsets[s.cs];
+        DownWs ws{};
+        if (cs.made_by_rule >= 0) ws = down_ws(cs.grid, batch_, rules[cs.made_by_rule].ws);
         rc = scatter_dense_layout_launch(rt[s.in0].data, rt[s.in0].kind, s.a_scale,
                                          cs_coords(s.cs), cs_n(s.cs), cs_launch(s.cs), s.cout,
                                          batch, cs.grid, s.has_perm ? s.perm : nullptr, s.layout,
                                          rt[s.out].kind, s.inv_out, rt[s.out].data, clear_dense,
-                                         st);
+                                         cs.made_by_rule >= 0 ? &ws : nullptr, st);
         last_launches += 2;  // the zero fill and the scatter
         break;
       }

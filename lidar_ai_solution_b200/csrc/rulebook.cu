@@ -42,18 +42,6 @@ __host__ __device__ inline bool is_k333(const Kernel3& kr) {
   return kr.k[0] == 3 && kr.k[1] == 3 && kr.k[2] == 3 && unit_dilation(kr);
 }
 
-// Row of a cell from the bitmap and its ranks, -1 if the cell is empty or lies beyond the
-// capacity.
-__device__ __forceinline__ int32_t rank_lookup(const uint32_t* __restrict__ bitmap,
-                                               const uint32_t* __restrict__ prefix,
-                                               uint32_t cell, uint32_t cap) {
-  const uint32_t bits = __ldg(bitmap + (cell >> 5));
-  const uint32_t b = cell & 31u;
-  if (!((bits >> b) & 1u)) return -1;
-  const uint32_t row = __ldg(prefix + (cell >> 5)) + __popc(bits & ((1u << b) - 1u));
-  return row < cap ? (int32_t)row : -1;
-}
-
 // ---------------------------------------------------------------- the caller's rows
 __device__ __forceinline__ void task_count(const RuleTask& t) {
   if (threadIdx.x != 0) return;

@@ -88,6 +88,20 @@ struct RuleWave {
   bool full() const { return count == kMaxWaveTasks; }
 };
 
+#ifdef __CUDACC__
+// Row of a cell from the bitmap and its ranks, -1 if the cell is empty or lies beyond the
+// capacity.
+__device__ __forceinline__ int32_t rank_lookup(const uint32_t* __restrict__ bitmap,
+                                               const uint32_t* __restrict__ prefix,
+                                               uint32_t cell, uint32_t cap) {
+  const uint32_t bits = __ldg(bitmap + (cell >> 5));
+  const uint32_t b = cell & 31u;
+  if (!((bits >> b) & 1u)) return -1;
+  const uint32_t row = __ldg(prefix + (cell >> 5)) + __popc(bits & ((1u << b) - 1u));
+  return row < cap ? (int32_t)row : -1;
+}
+#endif
+
 // One launch for the wave's tasks; an empty wave launches nothing.
 int launch_rule_wave(const RuleWave& w, cudaStream_t st);
 

@@ -481,6 +481,31 @@ def test_per_layer_parity_at_benchmark_sizes(kind, precision, voxels, seed):
     e.close()
 
 
+@pytest.mark.parametrize("grid,batch,channels", [((41, 40, 56), 1, (16, 32, 64, 128)),
+                                                  ((41, 264, 136), 2, (16, 16, 16, 16)),
+                                                  ((41, 72, 520), 3, (16, 16, 32, 64))])
+def test_transposed_dense_output_is_the_dense_output_transposed(grid, batch, channels):
+    """A permuted output is written from its own cells, by rank; lines that are no multiple of 32
+    cells, empty groups of cells and several frames included."""
+    frames = [scenes.make_coords(1500 + 700 * b, grid, b) for b in range(batch)]
+    for b, c in enumerate(frames):
+        c[:, 0] = b
+    coords = np.concatenate(frames)
+    feats = _dev(scenes.make_point_features(coords, 1))
+    outs, eng = [], _engine_mod()
+    for kind in ("centerpoint", "bevfusion"):
+        model = models.scn_backbone(kind, seed=2, grid_zyx=grid, output_bound=30000,
+                                    channels=channels)
+        e = eng.Engine.from_model(model, eng.PRECISION_FP16)
+        e.prepare(grid, batch)
+        e.forward(feats, _dev(coords), grid, batch=batch)
+        outs.append(e.output(0).cpu().numpy().copy())
+        assert e.status()[0] == 0
+    want = outs[0].reshape(batch, -1, *outs[0].shape[-2:]).swapaxes(-1, -2)
+    got = outs[1].reshape(want.shape)
+    assert np.any(want != 0) and np.array_equal(got, want)
+
+
 def test_batched_forward_equals_frame_by_frame():
     """Several frames in one engine call (told apart by the batch column of the indices) give,
     frame for frame, the bits of single-frame calls: dense output slices and every stage's rows.
