@@ -142,6 +142,33 @@ def test_tied_scores_rank_by_cell_index(max_det):
     assert np.allclose(got, boxes, rtol=RTOL, atol=1e-6)
 
 
+@pytest.mark.parametrize("n", [1, 2, 16, 17, 63, 64, 65, 513, 999, 1000, 1001, 1600])
+def test_candidate_counts_at_the_edges_of_tiles(n):
+    """``n`` cells in a block, boxes that overlap their neighbours: one box, full and ragged mask
+    tiles, as many as fit and more; long chains in which a suppressed box suppresses nothing."""
+    post = _post()
+    rng = np.random.default_rng(n)
+    H = W = 64
+    heads = scenes.make_centerpoint_heads(0, H=H, W=W, num_classes=(1,), objects=0)
+    head = {k: np.zeros_like(v) for k, v in heads[0].items()}
+    head["hm"][:] = -12.0
+    i = np.arange(n)
+    head["hm"][0, 5 + i // 40, 7 + i % 40] = rng.permutation(np.linspace(-1.5, 3.0, n))
+    head["dim"][:] = 0.5
+    head["rot"][1] = 1.0
+    prm = dict(nms_post_max=1000, post_center_range=(-100, -100, -10, 100, 100, 10))
+    det, _ = orc.centerpoint_decode(head, prm)
+    boxes, kept, margin = orc.centerpoint_nms(det, 0, prm)
+    assert len(det) == min(n, 1000) and margin > 1e-4
+    pp = post.PostProcess(post.default_params(H, W, **prm), num_tasks=1)
+    pp.run(_dev_heads([head]), label_offsets=(0,))
+    d = pp.task_detections(0).cpu().numpy()
+    assert np.array_equal(d[:, :3], det[:, :3])
+    got = pp.result().cpu().numpy()
+    assert got.shape == boxes.shape and np.array_equal(got[:, :3], boxes[:, :3])
+    assert np.allclose(got, boxes, rtol=RTOL, atol=1e-6)
+
+
 def test_postprocess_is_capturable_and_repeatable():
     """No host synchronisation inside: the call records into a CUDA graph; replays on new head
     values give the restatement's answer each time."""
