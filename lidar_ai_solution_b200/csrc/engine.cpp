@@ -858,7 +858,7 @@ void Engine::plan_waves() {
     t.n_ptr = c.external ? in_n : c.n_ptr;
     t.cap = c.cap;
     t.gin = make_grid(c.grid, batch_);
-    t.blocks = task_blocks(c.cap);
+    t.blocks = row_task_blocks(kind, c.cap);
     t.status = status;
     return t;
   };
@@ -935,7 +935,7 @@ void Engine::plan_waves() {
         fill.n_ptr = co.n_ptr;
         fill.cap = co.cap;
         fill.other_cap = ci.cap;
-        fill.blocks = task_blocks(co.cap);
+        fill.blocks = row_task_blocks(TASK_GATHER, co.cap);
       } else {
         fill.kind = TASK_SCATTER;
         fill.map_cap = co.cap;
@@ -1136,7 +1136,7 @@ int Engine::forward(const void* features, const int32_t* indices, uint32_t cap_r
           t.cap = in_cap;
         }
         if (!n_dev && t.kind != TASK_COUNT && t.kind != TASK_INVERSE)
-          t.blocks = std::min(t.blocks, task_blocks(n_host));
+          t.blocks = std::min(t.blocks, row_task_blocks(t.kind, n_host));
       }
       r = launch_rule_wave(w, on);
       ++last_launches;

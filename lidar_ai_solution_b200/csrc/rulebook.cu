@@ -83,17 +83,47 @@ __device__ __forceinline__ void task_hash(const RuleTask& t, uint32_t first, uin
 // ------------------------------------------------------------------- SubM maps
 // One thread per row: the row's coordinate is read once, its taps are walked in tap order, so
 // a warp's stores of one tap land in one or two lines of map[k][.].
-template <bool K333, typename Lookup>
-__device__ __forceinline__ void subm_row_taps(const int4 c, uint32_t row, const RuleTask& t,
-                                              Lookup lookup) {
+//
+// Planes of a 3x3x3 kernel (9 taps of one k0): where the rows are few, a thread takes one plane of a
+// row.  The lookups of a row are a chain of memory latencies, three planes in three threads are a
+// third of it, and on a small frame there is room for them: 7.5 us for the map of 10 800 of the
+// caller's rows, with a thread per row 13.9.  By rank as long as all planes run in one round (three
+// rounds of 9 lookups cost what one of 27 does); by hash, whose probes are dearer, up to two rounds (a
+// layer of 120 000 rows with its map 58.8 us, this way 56).
+struct Planes {
+  uint32_t n;  // items: rows, or three times the rows
+  bool split;
+};
+__device__ __forceinline__ Planes planes_of(uint32_t rows, bool k333, uint32_t most) {
+  Planes p;
+  p.split = k333 && rows <= most;
+  p.n = p.split ? 3u * rows : rows;
+  return p;
+}
+// Row of an item, and the k0 it starts at and stops before.
+__device__ __forceinline__ uint32_t plane_row(const Planes& p, uint32_t item, int& k0, int& k0_end) {
+  k0 = 0;
+  k0_end = 3;
+  if (!p.split) return item;
+  const uint32_t rows = p.n / 3u;
+  k0 = item >= 2u * rows ? 2 : item >= rows ? 1 : 0;
+  k0_end = k0 + 1;
+  return item - (uint32_t)k0 * rows;
+}
+
+// ONE: plane `plane` only
+template <bool K333, bool ONE, typename Lookup>
+__device__ __forceinline__ void subm_row_taps(const int4 c, uint32_t row, int plane,
+                                              const RuleTask& t, Lookup lookup) {
   const Grid3& g = t.gin;
   const Kernel3& kr = t.kr;
   const int K0 = K333 ? 3 : kr.k[0], K1 = K333 ? 3 : kr.k[1], K2 = K333 ? 3 : kr.k[2];
   const int D0 = K333 ? 1 : kr.d[0], D1 = K333 ? 1 : kr.d[1], D2 = K333 ? 1 : kr.d[2];
   const bool bok = (unsigned)c.x < (unsigned)g.batch;
-  int32_t* dst = t.map + row;
+  int32_t* dst = t.map + row + (size_t)(ONE ? plane * 9 : 0) * t.cap;
 #pragma unroll
-  for (int k0 = 0; k0 < K0; ++k0) {
+  for (int q = 0; q < (ONE ? 1 : K0); ++q) {
+    const int k0 = ONE ? plane : q;
     const int p0 = c.y + (k0 - K0 / 2) * D0;
     const bool ok0 = bok && (unsigned)p0 < (unsigned)g.g[0];
 #pragma unroll
@@ -117,13 +147,14 @@ __device__ __forceinline__ void subm_row_taps(const int4 c, uint32_t row, const 
 // nothing, so what counts is how many are in flight: the first probes of the 9 taps of a plane
 // are issued together and only then looked at (a probe loop per tap took its 27 latencies one
 // after the other).  Taps whose first slot holds another cell go on probing one by one.
-__device__ __forceinline__ void subm_hash_k333(const int4 c, uint32_t row, const RuleTask& t) {
+__device__ __forceinline__ void subm_hash_k333(const int4 c, uint32_t row, int k0_first, int k0_end,
+                                               const RuleTask& t) {
   const Grid3& g = t.gin;
   const uint64_t* __restrict__ table = t.table;
   const bool bok = (unsigned)c.x < (unsigned)g.batch;
-  int32_t* dst = t.map + row;
+  int32_t* dst = t.map + row + (size_t)(k0_first * 9) * t.cap;
 #pragma unroll 1
-  for (int k0 = 0; k0 < 3; ++k0) {
+  for (int k0 = k0_first; k0 < k0_end; ++k0) {
     const int p0 = c.y + k0 - 1;
     const bool ok0 = bok && (unsigned)p0 < (unsigned)g.g[0];
     unsigned long long v[9];
@@ -152,13 +183,16 @@ __device__ __forceinline__ void subm_hash_k333(const int4 c, uint32_t row, const
 __device__ __forceinline__ void task_subm_hash(const RuleTask& t, uint32_t first, uint32_t step) {
   const uint32_t n = task_rows(t);
   const bool k333 = is_k333(t.kr);
-  for (uint32_t row = first; row < n; row += step) {
+  const Planes pl = planes_of(n, k333, step - step / 3u);
+  for (uint32_t item = first; item < pl.n; item += step) {
+    int k0, k0_end;
+    const uint32_t row = plane_row(pl, item, k0, k0_end);
     const int4 c = __ldg(t.coords + row);
     if (k333)
-      subm_hash_k333(c, row, t);
+      subm_hash_k333(c, row, k0, k0_end, t);
     else
-      subm_row_taps<false>(c, row, t,
-                           [&](uint32_t key) { return hash_lookup(t.table, t.mask, key); });
+      subm_row_taps<false, false>(
+          c, row, 0, t, [&](uint32_t key) { return hash_lookup(t.table, t.mask, key); });
   }
 }
 
@@ -167,10 +201,14 @@ __device__ __forceinline__ void task_subm_rank(const RuleTask& t, uint32_t first
   const uint32_t n = task_rows(t);
   const bool k333 = is_k333(t.kr);
   auto look = [&](uint32_t key) { return rank_lookup(t.ws.bitmap, t.ws.prefix, key, t.cap); };
-  for (uint32_t row = first; row < n; row += step) {
+  const Planes pl = planes_of(n, k333, step / 3u);
+  for (uint32_t item = first; item < pl.n; item += step) {
+    int k0, k0_end;
+    const uint32_t row = plane_row(pl, item, k0, k0_end);
     const int4 c = __ldg(t.coords + row);
-    if (k333) subm_row_taps<true>(c, row, t, look);
-    else subm_row_taps<false>(c, row, t, look);
+    if (pl.split) subm_row_taps<true, true>(c, row, k0, t, look);
+    else if (k333) subm_row_taps<true, false>(c, row, 0, t, look);
+    else subm_row_taps<false, false>(c, row, 0, t, look);
   }
 }
 
@@ -330,6 +368,11 @@ struct EmitShared {
   uint32_t back[kTaskWarps];
 };
 
+__device__ __forceinline__ void publish_bits(const RuleTask& t, uint32_t blk, uint32_t total) {
+  *(volatile uint32_t*)(t.ws.scan_counts() + blk) = total + 1u;
+  atomicAdd(t.ws.scan_groups() + blk / kScanGroup, (1ull << 40) | total);
+}
+
 // Set bits of all blocks before `blk`.  Every block publishes its count (plus 1) and adds it, with
 // an arrival, to the total of its group of 32; a block needs the totals of the groups before its own
 // and the counts of at most 31 blocks.  All of them are loaded at once (a batch of 8 frames has 21 000
@@ -341,10 +384,7 @@ __device__ __forceinline__ uint32_t bits_before(const RuleTask& t, uint32_t blk,
   unsigned long long* groups = t.ws.scan_groups();
   uint32_t* own = t.ws.scan_counts();
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, group = blk / kScanGroup;
-  if (threadIdx.x == 0) {
-    *(volatile uint32_t*)(own + blk) = total + 1u;
-    atomicAdd(groups + group, (1ull << 40) | total);
-  }
+  if (threadIdx.x == 0) publish_bits(t, blk, total);
   uint32_t sum = 0, spin = 0;
   auto give_up = [&]() {
     if (++spin < 1u << 21) {
@@ -405,6 +445,13 @@ __device__ __forceinline__ void task_emit(const RuleTask& t, EmitShared& sh) {
   for (int i = 0; i < kTaskWarps; ++i) {
     if (i < (int)warp) before += sh.warp_total[i];
     total += sh.warp_total[i];
+  }
+  if (total == 0u && blk != ws.blocks - 1) {
+    // Nobody asks for ranks of words without bits: an empty block says so and makes room (the
+    // 2 658 blocks of a first strided map are one and a half rounds of what runs at once; 10 800 voxels
+    // 7.8 us, when they all waited for the blocks before them 13.8).
+    if (threadIdx.x == 0) publish_bits(t, blk, 0u);
+    return;
   }
   sh.before[threadIdx.x] = before;
   sh.word[threadIdx.x] = bits;
@@ -506,15 +553,17 @@ __device__ __forceinline__ void task_scatter(const RuleTask& t, uint32_t first, 
 // taps in tap order, finds the input cell of each (out * stride - pad + tap * dilation) and
 // ranks it in the input's bitmap.  Every map entry is written exactly once, so there is no
 // fill pass, and a warp's stores of one tap land in one or two lines of map[k][.].
-template <bool K333>
-__device__ __forceinline__ void gather_row(const int4 c, uint32_t row, const RuleTask& t) {
+template <bool K333, bool ONE>
+__device__ __forceinline__ void gather_row(const int4 c, uint32_t row, int plane,
+                                           const RuleTask& t) {
   const Grid3& gin = t.gin;
   const Kernel3& kr = t.kr;
   const int K0 = K333 ? 3 : kr.k[0], K1 = K333 ? 3 : kr.k[1], K2 = K333 ? 3 : kr.k[2];
-  int32_t* dst = t.map + row;
+  int32_t* dst = t.map + row + (size_t)(ONE ? plane * 9 : 0) * t.cap;
   const bool bok = (unsigned)c.x < (unsigned)gin.batch;
 #pragma unroll
-  for (int k0 = 0; k0 < K0; ++k0) {
+  for (int q = 0; q < (ONE ? 1 : K0); ++q) {
+    const int k0 = ONE ? plane : q;
     const int p0 = c.y * kr.s[0] - kr.p[0] + k0 * (K333 ? 1 : kr.d[0]);
     const bool ok0 = bok && (unsigned)p0 < (unsigned)gin.g[0];
 #pragma unroll
@@ -538,10 +587,14 @@ __device__ __forceinline__ void gather_row(const int4 c, uint32_t row, const Rul
 __device__ __forceinline__ void task_gather(const RuleTask& t, uint32_t first, uint32_t step) {
   const uint32_t n = task_rows(t);
   const bool k333 = is_k333(t.kr);
-  for (uint32_t row = first; row < n; row += step) {
+  const Planes pl = planes_of(n, k333, step / 3u);
+  for (uint32_t item = first; item < pl.n; item += step) {
+    int k0, k0_end;
+    const uint32_t row = plane_row(pl, item, k0, k0_end);
     const int4 c = __ldg(t.coords + row);
-    if (k333) gather_row<true>(c, row, t);
-    else gather_row<false>(c, row, t);
+    if (pl.split) gather_row<true, true>(c, row, k0, t);
+    else if (k333) gather_row<true, false>(c, row, 0, t);
+    else gather_row<false, false>(c, row, 0, t);
   }
 }
 
@@ -637,6 +690,12 @@ uint32_t task_blocks(unsigned long long items) {
   return (uint32_t)(b < 1 ? 1 : b < most ? b : most);
 }
 
+// The maps of 3x3x3 kernels may take a thread per plane of a row.
+uint32_t row_task_blocks(int32_t kind, unsigned long long rows) {
+  const bool planes = kind == TASK_SUBM_HASH || kind == TASK_SUBM_RANK || kind == TASK_GATHER;
+  return task_blocks(planes ? 3 * rows : rows);
+}
+
 uint32_t mark_bitmap_blocks(const int32_t og[3], int batch) {
   return task_blocks((unsigned long long)batch * og[0] * og[1] *
                      (unsigned long long)((og[2] + kMarkCells - 1) / kMarkCells));
@@ -726,7 +785,7 @@ static RuleTask row_task(int32_t kind, const int32_t* coords, const uint32_t* n_
   t.coords = (const int4*)coords;
   t.n_ptr = n_ptr;
   t.cap = cap;
-  t.blocks = task_blocks(launch_rows == 0 || launch_rows > cap ? cap : launch_rows);
+  t.blocks = row_task_blocks(kind, launch_rows == 0 || launch_rows > cap ? cap : launch_rows);
   return t;
 }
 
@@ -912,7 +971,7 @@ static int down_map_impl(const int32_t* in_coords, const uint32_t* n_in_ptr, uin
     fill.n_ptr = n_out_ptr;
     fill.cap = cap_out;
     fill.other_cap = cap_in;
-    fill.blocks = task_blocks(cap_out);
+    fill.blocks = row_task_blocks(TASK_GATHER, cap_out);
   } else {
     fill.kind = TASK_SCATTER;
     fill.map_cap = cap_out;

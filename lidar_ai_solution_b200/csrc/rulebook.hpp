@@ -111,6 +111,7 @@ Grid3 make_grid(const int32_t g[3], int batch);
 Kernel3 make_kernel3(const int32_t k[3], const int32_t s[3], const int32_t p[3], const int32_t d[3]);
 bool mark_from_bitmap(const Kernel3& kr);  // the bitmap-to-bitmap mark covers this geometry
 uint32_t task_blocks(unsigned long long items);
+uint32_t row_task_blocks(int32_t kind, unsigned long long rows);
 uint32_t mark_bitmap_blocks(const int32_t out_grid[3], int batch);
 
 }  // namespace spconvb

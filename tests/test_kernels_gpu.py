@@ -228,6 +228,36 @@ def test_strided_rows_at_the_edges_of_scan_blocks(grid, n):
     assert np.array_equal(sub.cpu().numpy()[:, :n], ref)
 
 
+@pytest.mark.parametrize("n", [1, 43, 128, 75776, 75777, 151552, 151553])
+def test_maps_where_threads_go_from_planes_to_rows(n):
+    """3x3x3 maps by hash and by rank, from one row up and on both sides of the row counts up to
+    which a thread takes one plane of a row (227 328 threads: a third of them by rank, two by hash);
+    then the strided map of those rows, gathered by rank."""
+    ops = _ops()
+    grid = (33, 96, 128)
+    cells = np.sort(np.random.default_rng(n).permutation(int(np.prod(grid)))[:n])
+    coords = np.zeros((n, 4), np.int32)
+    coords[:, 1:] = np.stack(np.unravel_index(cells, grid), 1)
+    shuffled = coords[np.random.default_rng(n + 1).permutation(n)]
+    dc, n_ptr, st = _dev(shuffled), ops.device_count(n), ops.new_status()
+    by_hash = ops.subm_map(dc, n_ptr, grid, ops.hash_build(dc, n_ptr, grid, status=st), status=st)
+    _status_ok(st)
+    assert np.array_equal(by_hash.cpu().numpy()[:, :n], orc.subm_map(shuffled, grid)[0])
+    one = (1, 1, 1)
+    oc, n_out, _, _, _, ws = ops.down_map(dc, n_ptr, grid, None, one, one, (0, 0, 0), status=st,
+                                          want_table=False, return_ws=True)
+    by_rank = ops.subm_map_ranked(oc, n_out, grid, ws, status=st)
+    _status_ok(st)
+    assert np.array_equal(by_rank.cpu().numpy()[:, :n], orc.subm_map(coords, grid)[0])
+    args = ((3, 3, 3), (2, 2, 2), one)
+    roc, rdm, _, _, rn = orc.down_map(coords, grid, *args)
+    goc, gn, gdm = ops.down_map(oc, n_out, grid, None, *args, cap_out=max(rn, 1), status=st,
+                                want_table=False, in_ws=ws)[:3]
+    _status_ok(st)
+    assert int(gn.item()) == rn and np.array_equal(goc.cpu().numpy()[:rn], roc[:rn])
+    assert np.array_equal(gdm.cpu().numpy()[:, :rn], rdm[:, :rn])
+
+
 def test_down_map_overflow_sets_status():
     ops = _ops()
     from lidar_ai_solution_b200 import cabi
