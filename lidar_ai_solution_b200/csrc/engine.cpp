@@ -1179,9 +1179,13 @@ int Engine::forward(const void* features, const int32_t* indices, uint32_t cap_r
       const int level = s.kind == Step::CONV ? rule_level_[s.rule] : 0;
       if (fork) {
         if (level > waited) {
-          if (cudaStreamWaitEvent(caller_stream, level_ev_[level], 0) != cudaSuccess)
+          // The second wait is for all levels that are left.  A launch behind a wait cannot start
+          // its prologue under the kernel before it (2 us each), and by then the waves, which run
+          // ahead, are done: 10 800 voxels 241.5 -> 236 us, 120 000 646.7 -> 641.
+          const int upto = waited > 1 ? last_level : level;
+          if (cudaStreamWaitEvent(caller_stream, level_ev_[upto], 0) != cudaSuccess)
             rc = SPCONVB_E_DEVICE;
-          waited = level;
+          waited = upto;
         }
       } else {
         rc = launch_waves(level, st);
