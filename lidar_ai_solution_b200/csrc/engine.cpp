@@ -816,6 +816,7 @@ int Engine::prepare(const int32_t grid[3], int batch) {
     t.data = slots[pick].ptr;
   }
   if (cudaDeviceSynchronize() != cudaSuccess) return SPCONVB_E_NOMEM;
+  rules_rc_ = check_rules();
   plan_waves();
   if (!(flags & SPCONVB_BUILD_SINGLE_STREAM)) {
     bool ok = true;
@@ -832,6 +833,31 @@ int Engine::prepare(const int32_t grid[3], int batch) {
   }
   prepared_ = true;
   return SPCONVB_OK;
+}
+
+// The argument checks of the kernel-level entry points for this model's rulebooks on this grid: the
+// tasks of a wave check nothing, and a model file may ask for anything.
+int Engine::check_rules() const {
+  int rc = SPCONVB_OK;
+  for (const Step& s : steps) {
+    int32_t og[3];
+    if (s.kind == Step::HASH) {
+      const CoordSet& c = coordsets[s.cs];
+      rc = check_hash(c.grid, batch_, c.cap, c.slots);
+    } else if (s.kind == Step::SUBM_MAP) {
+      const Rule& R = rules[s.rule];
+      rc = check_subm(coordsets[R.in_cs].grid, batch_, R.ksize, R.dil);
+    } else if (s.kind == Step::DOWN_MAP || s.kind == Step::INV_MAP) {
+      const Rule& R = rules[s.rule];  // (an inverse rule carries the strided one's geometry)
+      rc = check_strided(coordsets[s.kind == Step::INV_MAP ? R.out_cs : R.in_cs].grid, batch_, R.ksize,
+                         R.stride, R.pad, R.dil, og);
+    }
+    if (rc != SPCONVB_OK) {
+      log_msg(LOG_ERROR, "step '%s': %s", s.name.c_str(), spconvb_error_string(rc));
+      break;
+    }
+  }
+  return rc;
 }
 
 // The rulebook steps as tasks, each on the earliest level where everything it reads is there:
@@ -982,6 +1008,9 @@ int Engine::forward(const void* features, const int32_t* indices, uint32_t cap_r
     log_msg(LOG_ERROR, "%u input rows exceed the model's bound of %u", n_host, in.cap);
     return SPCONVB_E_ARG;
   }
+  if (rules_rc_ != SPCONVB_OK) return rules_rc_;
+  // (the convert step that a wave does in its place takes no empty buffer either)
+  if (pad_step_ >= 0 && n_dev && cap_rows == 0) return SPCONVB_E_ARG;
   last_launches = 0;
   cudaError_t ce = cudaMemsetAsync(zero_arena_, 0, zero_bytes_, st);
   if (ce != cudaSuccess) return (int)ce;

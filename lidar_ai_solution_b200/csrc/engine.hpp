@@ -201,10 +201,12 @@ class Engine {
   std::vector<PlannedWave> waves_;
   std::vector<int> rule_level_;  // level that completes a rule's map
   int pad_step_ = -1;            // the step that pads the caller's features, done on level 0
+  int rules_rc_ = 0;             // why the rulebooks cannot be built on this grid, or SPCONVB_OK
   cudaStream_t aux_ = nullptr;
   cudaEvent_t fork_ev_ = nullptr;
   std::vector<cudaEvent_t> level_ev_;
   void plan_waves();
+  int check_rules() const;
   void* zero_arena_ = nullptr;
   size_t zero_bytes_ = 0;
   uint32_t* counts_ = nullptr;

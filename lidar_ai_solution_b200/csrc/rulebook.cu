@@ -660,19 +660,47 @@ rule_wave_kernel(const __grid_constant__ RuleWave w) {
   }
 }
 
-bool grid_fits(const int32_t g[3], int batch) {
-  if (batch < 1 || g[0] < 1 || g[1] < 1 || g[2] < 1) return false;
-  unsigned long long cells = (unsigned long long)batch * g[0] * g[1] * g[2];
-  return cells < 0xffffffffull;
-}
-
 uint32_t down_words(const int32_t og[3], int batch) {
   unsigned long long cells = (unsigned long long)batch * og[0] * og[1] * og[2];
   return (uint32_t)((cells + 31) / 32);
 }
 uint32_t scan_blocks(uint32_t words) { return (words + kScanWords - 1) / kScanWords; }
 
+bool slots_ok(uint32_t cap, uint32_t slots) {
+  return slots >= 8 && !(slots & (slots - 1)) && slots >= 2ull * cap;
+}
+
 }  // namespace
+
+// (in 128 bits: the product of three extents and a batch may pass 2^64)
+bool grid_fits(const int32_t g[3], int batch) {
+  if (batch < 1 || g[0] < 1 || g[1] < 1 || g[2] < 1) return false;
+  return (unsigned __int128)batch * g[0] * g[1] * g[2] < 0xffffffffull;
+}
+
+int check_hash(const int32_t grid[3], int batch, uint32_t cap, uint32_t slots) {
+  if (!slots_ok(cap, slots)) return SPCONVB_E_ARG;
+  return grid_fits(grid, batch) ? SPCONVB_OK : SPCONVB_E_RANGE;
+}
+
+int check_subm(const int32_t grid[3], int batch, const int32_t k[3], const int32_t d[3]) {
+  if (!grid_fits(grid, batch)) return SPCONVB_E_RANGE;
+  for (int a = 0; a < 3; ++a)
+    if (k[a] < 1 || !(k[a] & 1) || d[a] < 1) return SPCONVB_E_ARG;
+  return (long long)k[0] * k[1] * k[2] <= 65535 ? SPCONVB_OK : SPCONVB_E_ARG;
+}
+
+int check_strided(const int32_t grid[3], int batch, const int32_t k[3], const int32_t s[3],
+                  const int32_t p[3], const int32_t d[3], int32_t og[3]) {
+  if (!grid_fits(grid, batch)) return SPCONVB_E_RANGE;
+  for (int a = 0; a < 3; ++a) {
+    if (k[a] < 1 || s[a] < 1 || d[a] < 1 || p[a] < 0) return SPCONVB_E_ARG;
+    og[a] = spconvb_out_extent(grid[a], k[a], s[a], p[a], d[a]);
+    if (og[a] < 1) return SPCONVB_E_ARG;
+  }
+  if (!grid_fits(og, batch)) return SPCONVB_E_RANGE;
+  return (long long)k[0] * k[1] * k[2] <= 65535 ? SPCONVB_OK : SPCONVB_E_ARG;
+}
 
 int launch_rule_wave(const RuleWave& w, cudaStream_t st) {
   uint32_t blocks = 0;
@@ -817,8 +845,8 @@ int spconvb_hash_build(const int32_t* coords, const uint32_t* n_ptr, uint32_t ca
                        uint64_t* table, uint32_t slots, uint32_t flags, uint32_t* status,
                        void* stream) {
   if (!coords || !n_ptr || !table || !grid) return SPCONVB_E_ARG;
-  if (slots < 8 || (slots & (slots - 1)) || slots < 2ull * cap) return SPCONVB_E_ARG;
-  if (!grid_fits(grid, batch)) return SPCONVB_E_RANGE;
+  const int rc = check_hash(grid, batch, cap, slots);
+  if (rc != SPCONVB_OK) return rc;
   if (!(flags & SPCONVB_FLAG_PREZEROED))
     SPCONVB_CUDA_TRY(cudaMemsetAsync(table, 0, sizeof(uint64_t) * (size_t)slots,
                                      (cudaStream_t)stream));
@@ -837,10 +865,8 @@ int spconvb_subm_map(const int32_t* coords, const uint32_t* n_ptr, uint32_t cap,
   (void)status;
   if (!coords || !n_ptr || !table || !map || !grid || !ksize || !dilation) return SPCONVB_E_ARG;
   if (slots < 8 || (slots & (slots - 1))) return SPCONVB_E_ARG;
-  if (!grid_fits(grid, batch)) return SPCONVB_E_RANGE;
-  for (int a = 0; a < 3; ++a)
-    if (ksize[a] < 1 || !(ksize[a] & 1) || dilation[a] < 1) return SPCONVB_E_ARG;
-  if (ksize[0] * ksize[1] * ksize[2] > 65535) return SPCONVB_E_ARG;
+  const int rc = check_subm(grid, batch, ksize, dilation);
+  if (rc != SPCONVB_OK) return rc;
   RuleTask t = row_task(TASK_SUBM_HASH, coords, n_ptr, cap, launch_rows);
   t.gin = make_grid(grid, batch);
   t.kr = make_kernel3(ksize, nullptr, nullptr, dilation);
@@ -858,10 +884,8 @@ int spconvb_subm_map_ranked(const int32_t* coords, const uint32_t* n_ptr, uint32
   (void)status;
   if (!coords || !n_ptr || !down_workspace || !map || !grid || !ksize || !dilation)
     return SPCONVB_E_ARG;
-  if (!grid_fits(grid, batch)) return SPCONVB_E_RANGE;
-  for (int a = 0; a < 3; ++a)
-    if (ksize[a] < 1 || !(ksize[a] & 1) || dilation[a] < 1) return SPCONVB_E_ARG;
-  if (ksize[0] * ksize[1] * ksize[2] > 65535) return SPCONVB_E_ARG;
+  const int rc = check_subm(grid, batch, ksize, dilation);
+  if (rc != SPCONVB_OK) return rc;
   RuleTask t = row_task(TASK_SUBM_RANK, coords, n_ptr, cap, launch_rows);
   t.gin = make_grid(grid, batch);
   t.kr = make_kernel3(ksize, nullptr, nullptr, dilation);
@@ -879,16 +903,10 @@ int spconvb_inverse_map(const int32_t* coords, const uint32_t* n_ptr, uint32_t c
   if (!coords || !n_ptr || !grid || !ksize || !stride || !pad || !dilation || !down_workspace ||
       !map)
     return SPCONVB_E_ARG;
-  if (!grid_fits(grid, batch)) return SPCONVB_E_RANGE;
   int32_t og[3];
-  for (int a = 0; a < 3; ++a) {
-    if (ksize[a] < 1 || stride[a] < 1 || pad[a] < 0 || dilation[a] < 1) return SPCONVB_E_ARG;
-    og[a] = spconvb_out_extent(grid[a], ksize[a], stride[a], pad[a], dilation[a]);
-    if (og[a] < 1) return SPCONVB_E_ARG;
-  }
+  const int rc = check_strided(grid, batch, ksize, stride, pad, dilation, og);
+  if (rc != SPCONVB_OK) return rc;
   const int kvol = ksize[0] * ksize[1] * ksize[2];
-  if (kvol > 65535) return SPCONVB_E_ARG;
-  if (!grid_fits(og, batch)) return SPCONVB_E_RANGE;
   RuleTask t = row_task(TASK_INVERSE, coords, n_ptr, cap, launch_rows);
   t.blocks = task_blocks((unsigned long long)(launch_rows == 0 || launch_rows > cap ? cap
                                                                                     : launch_rows) *
@@ -919,17 +937,10 @@ static int down_map_impl(const int32_t* in_coords, const uint32_t* n_in_ptr, uin
   if (!in_coords || !n_in_ptr || !in_grid || !ksize || !stride || !pad || !dilation ||
       !workspace || !out_coords || !n_out_ptr || !map)
     return SPCONVB_E_ARG;
-  if (out_table && (out_slots < 8 || (out_slots & (out_slots - 1)) || out_slots < 2ull * cap_out))
-    return SPCONVB_E_ARG;
-  if (!grid_fits(in_grid, batch)) return SPCONVB_E_RANGE;
+  if (out_table && !slots_ok(cap_out, out_slots)) return SPCONVB_E_ARG;
   int32_t og[3];
-  for (int a = 0; a < 3; ++a) {
-    if (ksize[a] < 1 || stride[a] < 1 || dilation[a] < 1 || pad[a] < 0) return SPCONVB_E_ARG;
-    og[a] = spconvb_out_extent(in_grid[a], ksize[a], stride[a], pad[a], dilation[a]);
-    if (og[a] < 1) return SPCONVB_E_ARG;
-  }
-  if (!grid_fits(og, batch)) return SPCONVB_E_RANGE;
-  if (ksize[0] * ksize[1] * ksize[2] > 65535) return SPCONVB_E_ARG;
+  int rc = check_strided(in_grid, batch, ksize, stride, pad, dilation, og);
+  if (rc != SPCONVB_OK) return rc;
   cudaStream_t st = (cudaStream_t)stream;
 
   const DownWs ws = down_ws(og, batch, workspace);
@@ -976,7 +987,7 @@ static int down_map_impl(const int32_t* in_coords, const uint32_t* n_in_ptr, uin
     fill.kind = TASK_SCATTER;
     fill.map_cap = cap_out;
   }
-  int rc = launch_task(mark, stream);
+  rc = launch_task(mark, stream);
   if (rc == SPCONVB_OK) rc = launch_task(emit, stream);
   if (rc != SPCONVB_OK) return rc;
   RuleWave last;
@@ -1033,21 +1044,14 @@ int spconvb_down_map_static(const int32_t* in_coords, const uint32_t* n_in_ptr, 
   if (!in_coords || !n_in_ptr || !in_grid || !ksize || !stride || !pad || !dilation ||
       !out_coords || !n_out_ptr || !map)
     return SPCONVB_E_ARG;
-  if (out_table && (out_slots < 8 || (out_slots & (out_slots - 1)) || out_slots < 2ull * cap_out))
-    return SPCONVB_E_ARG;
-  if (!grid_fits(in_grid, batch)) return SPCONVB_E_RANGE;
+  if (out_table && !slots_ok(cap_out, out_slots)) return SPCONVB_E_ARG;
   int32_t og[3];
-  for (int a = 0; a < 3; ++a) {
-    if (ksize[a] < 1 || stride[a] < 1 || dilation[a] < 1 || pad[a] < 0) return SPCONVB_E_ARG;
-    og[a] = spconvb_out_extent(in_grid[a], ksize[a], stride[a], pad[a], dilation[a]);
-    if (og[a] < 1) return SPCONVB_E_ARG;
-  }
-  if (ksize[0] * ksize[1] * ksize[2] > 65535) return SPCONVB_E_ARG;
+  int rc = check_strided(in_grid, batch, ksize, stride, pad, dilation, og);
+  if (rc != SPCONVB_OK) return rc;
   const size_t need = spconvb_down_workspace_bytes(og, batch);
-  if (need == 0) return SPCONVB_E_RANGE;
   if (need > kStaticScratchBytes) return SPCONVB_E_SCRATCH_LIMIT;
   void* scratch = nullptr;
-  int rc = static_scratch_for_current_device(&scratch);
+  rc = static_scratch_for_current_device(&scratch);
   if (rc != SPCONVB_OK) return rc;
   // The array still holds the previous call's bitmap and block totals: it is cleared on
   // every call, whatever the caller says about its own buffers.

@@ -105,6 +105,16 @@ __device__ __forceinline__ int32_t rank_lookup(const uint32_t* __restrict__ bitm
 // One launch for the wave's tasks; an empty wave launches nothing.
 int launch_rule_wave(const RuleWave& w, cudaStream_t st);
 
+// What a rulebook is refused for, by the kernel-level entry points and by the engine alike (its
+// waves are made of tasks, which check nothing).  A cell's number has to fit 32 bits: in a larger
+// grid different cells would share one.
+bool grid_fits(const int32_t g[3], int batch);
+int check_hash(const int32_t grid[3], int batch, uint32_t cap, uint32_t slots);
+int check_subm(const int32_t grid[3], int batch, const int32_t k[3], const int32_t d[3]);
+// and the output grid
+int check_strided(const int32_t grid[3], int batch, const int32_t k[3], const int32_t s[3],
+                  const int32_t p[3], const int32_t d[3], int32_t out_grid[3]);
+
 // Task makers: arguments already checked.
 DownWs down_ws(const int32_t out_grid[3], int batch, const void* workspace);
 Grid3 make_grid(const int32_t g[3], int batch);

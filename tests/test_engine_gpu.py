@@ -363,6 +363,51 @@ def test_many_rulebooks_on_one_level(single_stream):
     _compare_all(e, T, exact=True)
 
 
+@pytest.mark.parametrize("what,code", [("grid", -2), ("batch", -2), ("even kernel", -1), ("padding", -1),
+                                       ("dilation", -1), ("inverse padding", -1), ("no rows", -1)])
+def test_rulebooks_that_cannot_be_built_are_refused(what, code):
+    """forward() refuses what the kernel-level entry points refuse, in the same words as the
+    profiling pass, which calls them: more cells than 32-bit keys tell apart (by the grid, by the
+    batch), SubM kernels without a centre, strided geometry out of range, an empty buffer to pad."""
+    eng = _engine_mod()
+    from lidar_ai_solution_b200 import cabi
+    grid, batch = (8, 64, 64), 1
+    model = models.single_layer(16, 16, subm=what not in ("padding", "dilation"), output_bound=100)
+    conv = model["nodes"][0]
+    if what == "grid":
+        grid = (1024, 2048, 2048)
+    elif what == "batch":
+        grid, batch = models.GRID_ZYX, 51
+    elif what == "even kernel":
+        conv["kernel_size"] = [3, 2, 3]
+        conv["weight"] = np.ascontiguousarray(conv["weight"][:, :, :2])
+    elif what == "padding":
+        conv["padding"] = [1, -1, 1]
+    elif what == "dilation":
+        conv["dilation"] = [1, 1, 0]
+    elif what == "inverse padding":
+        model = models.encoder_decoder(16, output_bound=100)
+        for n in model["nodes"]:
+            if n.get("rulebook") == "down0":
+                n["padding"] = [1, 1, -1]
+    else:
+        model = models.single_layer(5, 16, output_bound=100)
+    e = eng.Engine.from_model(model, eng.PRECISION_FP16)
+    feats = torch.zeros((16, model["in_channels"]), dtype=torch.float16, device="cuda")
+    coords = torch.zeros((16, 4), dtype=torch.int32, device="cuda")
+    if what == "no rows":
+        n_dev = torch.zeros(1, dtype=torch.int32, device="cuda")
+        assert cabi.lib().spconvb_engine_forward_dds(
+            e._h, feats.data_ptr(), coords.data_ptr(), 0, n_dev.data_ptr(), cabi.i3(grid), 1,
+            torch.cuda.current_stream().cuda_stream) == code
+        return
+    for _ in range(2):  # the buffers exist from the first call on
+        with pytest.raises(RuntimeError, match=r"\(%d\)" % code):
+            e.forward(feats, coords, grid, batch=batch)
+    with pytest.raises(RuntimeError, match=r"\(%d\)" % code):
+        e.profile(feats, coords, grid, batch=batch)
+
+
 def test_single_layer_sparse_output_and_bounds():
     eng = _engine_mod()
     feats, coords = _frame(5000, seed=5)
