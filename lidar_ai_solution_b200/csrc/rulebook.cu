@@ -162,14 +162,17 @@ __device__ __forceinline__ void subm_hash_k333(const int4 c, uint32_t row, int k
     for (int q = 0; q < 9; ++q) {
       const int p1 = c.z + q / 3 - 1, p2 = c.w + q % 3 - 1;
       v[q] = 0ull;
-      if (ok0 && (unsigned)p1 < (unsigned)g.g[1] && (unsigned)p2 < (unsigned)g.g[2])
+      const bool centre = q == 4 && k0 == 1;
+      if (ok0 && !centre && (unsigned)p1 < (unsigned)g.g[1] && (unsigned)p2 < (unsigned)g.g[2])
         v[q] = __ldg((const unsigned long long*)table +
                      hash_first_slot(voxel_key(c.x, p0, p1, p2, g), t.mask));
     }
 #pragma unroll
     for (int q = 0; q < 9; ++q) {
       int32_t r = -1;
-      if (v[q] != 0ull) {
+      if (q == 4 && k0 == 1) {
+        r = (int32_t)row;  // the row itself, also where the table holds another row of its cell or none
+      } else if (v[q] != 0ull) {
         const uint32_t key = voxel_key(c.x, p0, c.z + q / 3 - 1, c.w + q % 3 - 1, g);
         r = (uint32_t)(v[q] >> 32) == key + 1u ? (int32_t)(uint32_t)v[q]
                                                : hash_lookup_next(table, t.mask, key);

@@ -85,6 +85,21 @@ def test_hash_reports_duplicates_and_range():
     assert bits & cabi.ST_DUPLICATE and bits & cabi.ST_COORD_RANGE
 
 
+@pytest.mark.parametrize("n", [6, 160000])
+def test_subm_centre_tap_is_the_row_itself(n):
+    """Also for rows the table does not hold: repeated cells (it keeps one of them) and cells outside
+    the grid; with a thread per plane of a row and with a thread per row."""
+    ops = _ops()
+    grid = (8, 64, 640)
+    coords = scenes.make_coords(min(n, 100000), grid, 3)
+    coords = np.concatenate([coords, coords, coords[:1]])[:n]
+    coords[n // 2] = (0, 9, 0, 0)
+    coords[n // 3] = (0, 0, -1, 0)
+    dc, n_ptr = _dev(coords), ops.device_count(n)
+    m = ops.subm_map(dc, n_ptr, grid, ops.hash_build(dc, n_ptr, grid))
+    assert np.array_equal(m[13].cpu().numpy(), np.arange(n))
+
+
 def _chain(coords, grid):
     """Stage 0 looks neighbours up in the hash table of the caller's rows; later stages rank
     them in the bitmap the strided rulebook left behind (no hash table)."""
