@@ -208,6 +208,8 @@ vox_emit_kernel(const void* __restrict__ points, uint32_t n, spconvb_voxel_param
   const uint32_t id = base + pre;
   const int3 v = voxel_of(sum[0], sum[1], sum[2], p);
   int cnt = 1;
+#pragma unroll
+  for (int f = 0; f < 8; ++f) sum[f] = __fadd_rn(0.f, sum[f]);  // sums start at 0: a lone -0 gives +0
   if (next != kNoPoint) {
     const uint32_t* k = w.kept + (size_t)i * per;
     for (int s = 0; s < per; ++s) {

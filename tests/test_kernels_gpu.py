@@ -767,3 +767,17 @@ def test_voxelizer_crowded_voxels_and_cleared_tail(n, max_pts):
     assert np.array_equal(idx[:k].cpu().numpy(), ref_i)
     assert np.array_equal(feat[:k].cpu().numpy().view(np.uint16), ref_f.view(np.uint16))
     assert int(feat[k:].abs().sum().item()) == 0 and int(idx[k:].abs().sum().item()) == 0
+
+
+def test_voxelizer_sums_start_at_zero():
+    """The mean of a voxel is 0 + x0 + x1 + ... in fp32: a negative zero comes out positive, whether
+    it is its voxel's only point or not."""
+    ops = _ops()
+    pts = np.full((3, 5), -0.0, np.float32)
+    pts[:, :3] = [[0.5, 0.5, 0.5], [1.5, 0.5, 0.5], [1.5, 0.5, 0.5]]
+    box = ((0, 0, 0, 3, 3, 3), (1, 1, 1), (3, 3, 3))
+    feat, _, n_ptr = ops.voxelize(_dev(pts), ops.voxel_params(*box, 5, 0, 10, 40, 0))
+    ref, _, n = orc.voxelize(pts, *box, 40, 10)
+    assert int(n_ptr.item()) == n == 2
+    assert np.array_equal(feat[:n].cpu().numpy().view(np.uint16), ref.view(np.uint16))
+    assert not np.signbit(ref).any()
