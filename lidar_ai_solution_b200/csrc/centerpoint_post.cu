@@ -703,6 +703,9 @@ __device__ __forceinline__ bool iou_reaches(const BoxRec& A, const BoxRec& B, fl
     if (mine) p = sh.point[lane];
     const float ang = mine ? atan2f(p.y - centre.y, p.x - centre.x) : 0.f;
     if (mine) sh.value[lane] = ang;
+    // a vote orders no memory: this orders the angles before their readers below, and the reads of
+    // the points above before the points are put in their places
+    __syncwarp();
     if (__any_sync(0xffffffffu, ang != ang)) return false;
     // place in the stable ascending order of the angles
     int place = 0;
