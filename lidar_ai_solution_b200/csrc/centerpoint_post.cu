@@ -665,7 +665,8 @@ __device__ __forceinline__ bool surely_below(const BoxBounds& A, const BoxBounds
 // rotated_iou(A, B) >= threshold by a whole warp: lane e < 16 looks for the crossing of edge e / 4
 // of A and e % 4 of B, lanes 16..23 at the corners, in the order in which the serial code appends
 // its points; sums run in that order and in the order of the angles, so every bit is the same.
-// Boxes with a coordinate that is not a number overlap nothing, as there.
+// Angles that are not numbers have no order: there the serial insertion decides which points end up
+// where (boxes of 1e12 m and more, whose crossings overflow: some of their overlaps are infinite).
 struct IouScratch {
   Pt point[24];  // in the order of the serial code, then of the angles
   float value[24];
@@ -706,15 +707,28 @@ __device__ __forceinline__ bool iou_reaches(const BoxRec& A, const BoxRec& B, fl
     // a vote orders no memory: this orders the angles before their readers below, and the reads of
     // the points above before the points are put in their places
     __syncwarp();
-    if (__any_sync(0xffffffffu, ang != ang)) return false;
-    // place in the stable ascending order of the angles
-    int place = 0;
+    if (!__any_sync(0xffffffffu, ang != ang)) {
+      // place in the stable ascending order of the angles
+      int place = 0;
 #pragma unroll 4
-    for (int k = 0; k < cnt; ++k) {
-      const float other = sh.value[k];
-      if (other < ang || (other == ang && k < (int)lane)) ++place;
+      for (int k = 0; k < cnt; ++k) {
+        const float other = sh.value[k];
+        if (other < ang || (other == ang && k < (int)lane)) ++place;
+      }
+      if (mine) sh.point[place] = p;
+    } else if (lane == 0) {
+      for (int k = 1; k < cnt; ++k) {
+        const Pt pk = sh.point[k];
+        const float ak = sh.value[k];
+        int j = k - 1;
+        for (; j >= 0 && sh.value[j] > ak; --j) {
+          sh.point[j + 1] = sh.point[j];
+          sh.value[j + 1] = sh.value[j];
+        }
+        sh.point[j + 1] = pk;
+        sh.value[j + 1] = ak;
+      }
     }
-    if (mine) sh.point[place] = p;
     __syncwarp();
     if ((int)lane + 1 < cnt) {
       const Pt p0 = sh.point[0], pk = sh.point[lane], pn = sh.point[lane + 1];

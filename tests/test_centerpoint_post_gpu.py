@@ -169,6 +169,53 @@ def test_candidate_counts_at_the_edges_of_tiles(n):
     assert np.allclose(got, boxes, rtol=RTOL, atol=1e-6)
 
 
+def _serial_nms(post, pp, threshold):
+    """Ranks kept of task 0's detections by a greedy walk over the one-thread overlaps of all pairs
+    within reach of one another (farther pairs are not looked at)."""
+    det = pp.task_detections(0)
+    d = det.cpu().numpy()
+    box = np.zeros((len(d), 7), np.float32)
+    box[:, :3], box[:, 3], box[:, 4], box[:, 5] = d[:, :3], d[:, 4], d[:, 3], d[:, 5]
+    box[:, 6] = (-d[:, 8].astype(np.float64) - 3.141592653 * 0.5).astype(np.float32)
+    i, j = np.triu_indices(len(d), 1)
+    dev = torch.from_numpy(box).cuda()
+    iou = post.rotated_iou(dev[i].contiguous(), dev[j].contiguous()).cpu().numpy()
+    with np.errstate(over="ignore", invalid="ignore"):
+        reach = np.float32(0.5) * np.sqrt(box[:, 3] * box[:, 3] + box[:, 4] * box[:, 4])
+        dx, dy = box[i, 0] - box[j, 0], box[i, 1] - box[j, 1]
+        far = reach[i] + reach[j] + np.float32(0.1)
+        near = ~(dx * dx + dy * dy > far * far)
+        hit = np.zeros((len(d), len(d)), bool)
+        hit[i, j] = near & (iou >= np.float32(threshold))
+    gone = np.zeros(len(d), bool)
+    for k in range(len(d)):
+        if not gone[k]:
+            gone |= hit[k]
+    return d[~gone], iou
+
+
+@pytest.mark.parametrize("seed", range(4))
+def test_overlaps_of_boxes_whose_crossings_overflow(seed):
+    """Boxes of 1e13 m: crossings are infinite, angles not numbers, overlaps infinite or not
+    numbers.  Every decision is that of the one-thread overlap."""
+    post = _post()
+    rng = np.random.default_rng(seed)
+    H = W = 32
+    heads = scenes.make_centerpoint_heads(0, H=H, W=W, num_classes=(1,), objects=0)
+    head = {k: np.zeros_like(v) for k, v in heads[0].items()}
+    head["hm"][0] = rng.permutation(np.linspace(-1.5, 3, H * W)).reshape(H, W)
+    head["dim"][:] = rng.uniform(29.5, 31, head["dim"].shape)
+    head["rot"][:] = rng.normal(0, 1, head["rot"].shape)
+    prm = dict(max_det=600, nms_post_max=600, pc_range=(-10., -10.),
+               post_center_range=(-100, -100, -10, 100, 100, 10))
+    pp = post.PostProcess(post.default_params(H, W, **prm), num_tasks=1)
+    pp.run(_dev_heads([head]), label_offsets=(0,))
+    got = pp.result().cpu().numpy()
+    want, iou = _serial_nms(post, pp, 0.2)
+    assert np.isinf(iou).any() and np.isnan(iou).any()
+    assert got.shape == want.shape and np.array_equal(got, want)
+
+
 def test_postprocess_is_capturable_and_repeatable():
     """No host synchronisation inside: the call records into a CUDA graph; replays on new head
     values give the restatement's answer each time."""
