@@ -216,6 +216,30 @@ def test_overlaps_of_boxes_whose_crossings_overflow(seed):
     assert got.shape == want.shape and np.array_equal(got, want)
 
 
+@pytest.mark.parametrize("seed", range(2))
+@pytest.mark.parametrize("at,threshold", [(1e7, 0.2), (-4e6, 0.1), (9e3, 0.2), (-10.0, 0.2), (-10.0, -3.0)])
+def test_overlap_decisions_where_positions_are_rounded(at, threshold, seed):
+    """Heads placed far from the origin, where corners and crossings are rounded to decimetres and
+    metres (no bound may decide a pair the overlap itself decides otherwise), near it, and with a
+    threshold every pair in reach passes."""
+    post = _post()
+    rng = np.random.default_rng(seed)
+    H = W = 32
+    heads = scenes.make_centerpoint_heads(0, H=H, W=W, num_classes=(1,), objects=0)
+    head = {k: np.zeros_like(v) for k, v in heads[0].items()}
+    head["hm"][0] = rng.permutation(np.linspace(-1.5, 3, H * W)).reshape(H, W)
+    head["dim"][:] = rng.uniform(-4 if threshold < 0 else -1, 2, head["dim"].shape)
+    head["rot"][:] = rng.normal(0, 1, head["rot"].shape)
+    prm = dict(max_det=600, nms_post_max=600, nms_iou_threshold=threshold, pc_range=(at, at),
+               post_center_range=(-2e7, -2e7, -10, 2e7, 2e7, 10))
+    pp = post.PostProcess(post.default_params(H, W, **prm), num_tasks=1)
+    pp.run(_dev_heads([head]), label_offsets=(0,))
+    got = pp.result().cpu().numpy()
+    want, _ = _serial_nms(post, pp, threshold)
+    assert 0 < len(want) < 600
+    assert got.shape == want.shape and np.array_equal(got, want)
+
+
 def test_postprocess_is_capturable_and_repeatable():
     """No host synchronisation inside: the call records into a CUDA graph; replays on new head
     values give the restatement's answer each time."""
