@@ -8,6 +8,7 @@ out, with no host synchronisation in between.
 from __future__ import annotations
 
 import ctypes as C
+import operator
 import struct
 
 import torch
@@ -20,6 +21,8 @@ TASK_LABEL_OFFSET = (0, 1, 3, 5, 6, 8)
 TASK_NUM_CLASSES = (1, 2, 2, 1, 2, 2)
 HEAD_CHANNELS = {"reg": 2, "height": 1, "dim": 3, "rot": 2, "vel": 2}
 HEAD_KEYS = (*HEAD_CHANNELS, "hm")
+_HEAD_TENSORS = operator.itemgetter(*HEAD_KEYS)
+_SHAPE, _DTYPE, _IS_CUDA = map(operator.attrgetter, ("shape", "dtype", "is_cuda"))
 
 
 def default_params(H=180, W=180, **overrides) -> cabi.CpParams:
@@ -55,12 +58,9 @@ class PostProcess:
         self._count_view = self._count_host.numpy()
         self._heads = (cabi.CpHead * num_tasks)()
         self._pack = struct.Struct("6Q2i" * num_tasks)
-        p = self.params
-        self._shapes = [(k, torch.Size((ch, p.H, p.W)), torch.Size((1, ch, p.H, p.W)))
-                        for k, ch in HEAD_CHANNELS.items()]
         self._keep = None
-        self._known = [(None, 0)] * (6 * num_tasks)
-        self._words = None
+        self._checked = None
+        self._classes = []
         self._stream = None
 
     def run(self, heads, label_offsets=TASK_LABEL_OFFSET, stream=None):
@@ -69,23 +69,22 @@ class PostProcess:
         the stream has run."""
         assert len(heads) == self.num_tasks
         p = self.params
-        # Bound buffers stay the same from frame to frame: a tensor that was here in the last call,
-        # at the same address, has been checked.
-        known = iter(self._known)
+        # Everything that is checked is read anew on every call (a tensor's shape, layout and storage
+        # can change in place); what is spared is taking the same answers apart again.
+        tensors = []
         for h in heads:
-            for k in HEAD_KEYS:
-                x = h[k]
-                y, at = next(known)
-                if x is not y or x.data_ptr() != at:
-                    self._check(heads)
-                    break
-            else:
-                continue
-            break
-        words = self._words
-        if words[7::8] != [*label_offsets[:self.num_tasks]]:
-            words[7::8] = label_offsets[:self.num_tasks]
-            self._pack.pack_into(self._heads, 0, *words)
+            tensors += _HEAD_TENSORS(h)
+        seen = [*map(_SHAPE, tensors), *map(_DTYPE, tensors), *map(_IS_CUDA, tensors),
+                *map(torch.Tensor.is_contiguous, tensors), p.H, p.W]
+        if seen != self._checked:
+            self._classes = self._check(heads)
+            self._checked = seen
+        address = [*map(torch.Tensor.data_ptr, tensors)]
+        words = []
+        for t, classes in enumerate(self._classes):
+            words += address[6 * t:6 * t + 6]
+            words += (classes, label_offsets[t])
+        self._pack.pack_into(self._heads, 0, *words)
         self._keep = heads
         s = stream if stream is not None else torch.cuda.current_stream()
         self._stream = s
@@ -95,25 +94,17 @@ class PostProcess:
             self._count_host.data_ptr(), s.cuda_stream), "cp_postprocess")
 
     def _check(self, heads):
-        """Checks the heads' tensors and notes their addresses for the library."""
+        """Checks the heads' tensors; the number of classes of each head."""
         p = self.params
-        half = torch.float16
-        words, known = [], []
+        classes = []
         for h in heads:
-            for k, chw, nchw in self._shapes:
+            for k, ch in (*HEAD_CHANNELS.items(), ("hm", None)):
                 x = h[k]
-                shape = x.shape
-                assert x.dtype is half and x.is_cuda and x.is_contiguous()
-                assert shape == chw or shape == nchw or shape[-3:] == chw, (k, tuple(shape))
-                known.append((x, x.data_ptr()))
-                words.append(x.data_ptr())
-            hm = h["hm"]
-            shape = hm.shape
-            assert hm.dtype is half and hm.is_cuda and hm.is_contiguous()
-            assert shape[-2] == p.H and shape[-1] == p.W
-            known.append((hm, hm.data_ptr()))
-            words += (hm.data_ptr(), shape[-3], None)
-        self._words, self._known = words, known
+                assert x.is_cuda and x.dtype == torch.float16 and x.is_contiguous(), k
+                shape = tuple(x.shape)
+                assert shape[-2:] == (p.H, p.W) and (ch is None or shape[-3:-2] == (ch,)), (k, shape)
+            classes.append(h["hm"].shape[-3])
+        return classes
 
     def result(self):
         """Synchronises and returns the kept boxes [n, 11] (a copy)."""

@@ -267,6 +267,39 @@ def test_postprocess_is_capturable_and_repeatable():
         assert np.allclose(got, want, rtol=RTOL, atol=1e-6)
 
 
+@pytest.mark.parametrize("change", ["transpose_", "set_", "data", "resize_", "classes"])
+def test_heads_changed_in_place_are_checked_again(change):
+    """The same tensors, bound again after their shape, strides, type or number of classes changed in
+    place, at the same address: what the kernels cannot read is refused, what they can is read as it
+    is now."""
+    post = _post()
+    heads = _dev_heads(scenes.make_centerpoint_heads(5, mean_logit=-5.0))
+    pp = post.PostProcess()
+    pp.run(heads)
+    want = pp.result()
+    if change == "classes":  # task 1 loses its second class: one plane of the same storage is left
+        hm = heads[1]["hm"]
+        hm.set_(hm.untyped_storage(), 0, (1, *hm.shape[1:]))
+        fresh = post.PostProcess()
+        fresh.run([dict(h, hm=h["hm"].clone()) for h in heads])
+        pp.run(heads)
+        assert not torch.equal(pp.result(), want) and torch.equal(pp.result(), fresh.result())
+        return
+    x = heads[2]["dim"]
+    at = x.data_ptr()
+    if change == "transpose_":
+        x.transpose_(1, 2)
+    elif change == "set_":
+        x.set_(x.untyped_storage(), 0, (3, 90, 360))
+    elif change == "data":
+        x.data = x.data.view(torch.int16)
+    else:
+        x.resize_(3, 180, 179)
+    assert x.data_ptr() == at
+    with pytest.raises(AssertionError):
+        pp.run(heads)
+
+
 def test_bad_arguments_are_refused():
     post = _post()
     from lidar_ai_solution_b200 import cabi
