@@ -760,7 +760,7 @@ DownWs down_ws(const int32_t og[3], int batch, const void* workspace) {
   ws.blocks = scan_blocks(ws.words);
   ws.bitmap = (uint32_t*)workspace;
   ws.prefix = ws.bitmap + ws.words;
-  ws.scan = ws.prefix + ws.words;
+  ws.scan = (uint32_t*)(((uintptr_t)(ws.prefix + ws.words) + 7u) & ~(uintptr_t)7u);
   return ws;
 }
 

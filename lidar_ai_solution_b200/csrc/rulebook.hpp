@@ -21,8 +21,9 @@ struct Kernel3 {
 //   [0, W)        bitmap over the output grid                     (zero before the mark task)
 //   [W, 2W)       rank of the word's first set bit (after the emit task)
 //   [2W, ...)     state of the emit task's scan                    (zero before the emit task):
-//                 totals of groups of 32 scan blocks (64 bits each), a counter of the blocks
-//                 started, counts of the scan blocks of 128 words
+//                 totals of groups of 32 scan blocks (64 bits each, from the next 8-byte boundary
+//                 on: the workspace may start at any word), a counter of the blocks started,
+//                 counts of the scan blocks of 128 words
 constexpr uint32_t kScanGroup = 32;
 struct DownWs {
   uint32_t* bitmap;

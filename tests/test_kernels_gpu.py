@@ -273,6 +273,48 @@ def test_maps_where_threads_go_from_planes_to_rows(n):
     assert np.array_equal(gdm.cpu().numpy()[:, :rn], rdm[:, :rn])
 
 
+def _carved_down_map(coords, grid, args, shift, cap_out, flags=0, zero="all", runs=1):
+    """spconvb_down_map on a workspace `shift` bytes into a buffer; what lies behind it stays as it is.
+    With a `zero` other than "none" the bitmap, or all of the workspace, is cleared before each run."""
+    ops = _ops()
+    from lidar_ai_solution_b200 import cabi
+    lib, n = cabi.lib(), len(coords)
+    og = ops.out_grid(grid, *args)
+    need = lib.spconvb_down_workspace_bytes(cabi.i3(og), 1)
+    words = (int(np.prod(og)) + 31) // 32
+    kvol = int(np.prod(args[0]))
+    buf = torch.full((shift + need + 64,), 0xA5, dtype=torch.uint8, device="cuda")
+    dc, n_ptr, st = _dev(coords), ops.device_count(n), ops.new_status()
+    for _ in range(runs):
+        if zero != "none":
+            buf[shift:shift + (need if zero == "all" else 4 * words)].zero_()
+        oc = torch.zeros((cap_out, 4), dtype=torch.int32, device="cuda")
+        n_out = torch.zeros(1, dtype=torch.int32, device="cuda")
+        m = torch.full((kvol, cap_out), -1, dtype=torch.int32, device="cuda")
+        cabi.check(lib.spconvb_down_map(
+            dc.data_ptr(), n_ptr.data_ptr(), n, 0, cabi.i3(grid), 1, *[cabi.i3(a) for a in args],
+            cabi.i3((1, 1, 1)), None, 0, buf.data_ptr() + shift, oc.data_ptr(), n_out.data_ptr(),
+            cap_out, m.data_ptr(), None, 0, flags, st.data_ptr(),
+            torch.cuda.current_stream().cuda_stream))
+        torch.cuda.synchronize()
+    _status_ok(st)
+    assert int((buf[:shift] != 0xA5).sum()) == 0 and int((buf[shift + need:] != 0xA5).sum()) == 0
+    k = int(n_out.item())
+    return oc.cpu().numpy()[:k], m.cpu().numpy()[:, :k]
+
+
+@pytest.mark.parametrize("shift", [0, 4, 8, 12])
+@pytest.mark.parametrize("grid", [(9, 70, 83), (41, 180, 180)])
+def test_down_map_workspace_may_start_at_any_word(grid, shift):
+    """A workspace carved out of a larger buffer at any multiple of 4 bytes gives the oracle's rows and
+    map, and nothing beside it is written."""
+    coords = scenes.make_coords(6000, grid, 5)
+    args = ((3, 3, 3), (2, 2, 2), (1, 1, 1))
+    roc, rdm, _, _, rn = orc.down_map(coords, grid, *args)
+    oc, m = _carved_down_map(coords, grid, args, shift, rn)
+    assert np.array_equal(oc, roc) and np.array_equal(m, rdm[:, :rn])
+
+
 def test_down_map_overflow_sets_status():
     ops = _ops()
     from lidar_ai_solution_b200 import cabi
