@@ -48,7 +48,8 @@ __host__ inline VoxWs vox_layout(void* base, const spconvb_voxel_params& p, uint
   w.blocks = (max_points + kVoxScanThreads - 1) / kVoxScanThreads;
   if (w.blocks < 1) w.blocks = 1;
   uint8_t* b = (uint8_t*)base;
-  size_t off = 0;
+  // the table's 64-bit slots start at the next 8-byte boundary: the workspace may start at any word
+  size_t off = (8u - ((uintptr_t)base & 7u)) & 7u;
   w.table = (unsigned long long*)(b + off); off += align_up(sizeof(uint64_t) * (size_t)w.slots, 256);
   if (zero_bytes) *zero_bytes = off;
   w.block_sums = (uint32_t*)(b + off); off += align_up(sizeof(uint32_t) * (size_t)w.blocks, 256);
@@ -56,7 +57,7 @@ __host__ inline VoxWs vox_layout(void* base, const spconvb_voxel_params& p, uint
   w.pprefix = (uint32_t*)(b + off); off += align_up(sizeof(uint32_t) * (size_t)max_points, 256);
   w.kept = (uint32_t*)(b + off);
   off += align_up(sizeof(uint32_t) * (size_t)max_points * (p.max_points_per_voxel - 1), 256);
-  if (total_bytes) *total_bytes = off;
+  if (total_bytes) *total_bytes = off + 256;  // (room for that)
   return w;
 }
 

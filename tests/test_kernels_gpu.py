@@ -823,3 +823,29 @@ def test_voxelizer_sums_start_at_zero():
     assert int(n_ptr.item()) == n == 2
     assert np.array_equal(feat[:n].cpu().numpy().view(np.uint16), ref.view(np.uint16))
     assert not np.signbit(ref).any()
+
+
+@pytest.mark.parametrize("shift", [0, 4, 8, 12])
+def test_voxelizer_workspace_may_start_at_any_word(shift):
+    """A workspace carved out of a larger buffer at any multiple of 4 bytes gives the same voxels, and
+    nothing beside it is written."""
+    ops = _ops()
+    from lidar_ai_solution_b200 import cabi
+    lib, n = cabi.lib(), 3000
+    pts = np.random.default_rng(shift).uniform(0, 20, (n, 5)).astype(np.float32)
+    box = ((0, 0, 0, 20, 20, 20), (1, 1, 1), (20, 20, 20))
+    params = ops.voxel_params(*box, 5, 0, 4, 4000, 0)
+    need = lib.spconvb_voxelize_workspace_bytes(cabi.C.byref(params), n)
+    buf = torch.full((shift + need + 64,), 0xA5, dtype=torch.uint8, device="cuda")
+    feat = torch.empty((4000, 5), dtype=torch.float16, device="cuda")
+    idx = torch.empty((4000, 4), dtype=torch.int32, device="cuda")
+    n_ptr, st, d = ops.device_count(0), ops.new_status(), _dev(pts)
+    cabi.check(lib.spconvb_voxelize(cabi.C.byref(params), d.data_ptr(), n, buf.data_ptr() + shift,
+                                    feat.data_ptr(), idx.data_ptr(), n_ptr.data_ptr(), st.data_ptr(),
+                                    torch.cuda.current_stream().cuda_stream))
+    _status_ok(st)
+    ref_f, ref_i, k = orc.voxelize(pts, *box, 4000, 4)
+    assert int(n_ptr.item()) == k
+    assert np.array_equal(idx[:k].cpu().numpy(), ref_i)
+    assert np.array_equal(feat[:k].cpu().numpy().view(np.uint16), ref_f.view(np.uint16))
+    assert int((buf[:shift] != 0xA5).sum()) == 0 and int((buf[shift + need:] != 0xA5).sum()) == 0
