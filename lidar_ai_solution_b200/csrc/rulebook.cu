@@ -372,46 +372,36 @@ struct EmitShared {
 };
 
 __device__ __forceinline__ void publish_bits(const RuleTask& t, uint32_t blk, uint32_t total) {
-  *(volatile uint32_t*)(t.ws.scan_counts() + blk) = total + 1u;
   atomicAdd(t.ws.scan_groups() + blk / kScanGroup, (1ull << 40) | total);
 }
 
-// Set bits of all blocks before `blk`.  Every block publishes its count (plus 1) and adds it, with
-// an arrival, to the total of its group of 32; a block needs the totals of the groups before its own
-// and the counts of at most 31 blocks.  All of them are loaded at once (a batch of 8 frames has 21 000
-// blocks and 665 groups: 6 loads a thread); the chain of a look-back from block to block took 10 us
-// on 2 700 blocks that start together.  What is waited for was drawn from the same counter
-// before, so it is running or has finished; the wait is bounded like every other.
+// Set bits of all blocks before `blk`.  Every block adds its count, with an arrival, to the total of
+// its group of 16; a block needs the totals of the groups before its own, and counts the bits of the
+// blocks before it in its group itself (at most 15 words a thread, from L2: counts of their own
+// would make the workspace larger, and to wait for).  All totals are loaded at once (a
+// batch of 8 frames has 21 000 blocks and 1 330 groups: 11 loads a thread); the chain of a look-back from block
+// to block took 10 us on 2 700 blocks that start together.  What is waited for was drawn from the same
+// counter before, so it is running or has finished; the wait is bounded like every other.
 __device__ __forceinline__ uint32_t bits_before(const RuleTask& t, uint32_t blk, uint32_t total,
                                                 EmitShared& sh) {
   unsigned long long* groups = t.ws.scan_groups();
-  uint32_t* own = t.ws.scan_counts();
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, group = blk / kScanGroup;
   if (threadIdx.x == 0) publish_bits(t, blk, total);
   uint32_t sum = 0, spin = 0;
-  auto give_up = [&]() {
-    if (++spin < 1u << 21) {
-      __nanosleep(32);
-      return false;
-    }
-    set_status(t.status, SPCONVB_ST_TIMEOUT, 7u);
-    return true;
-  };
+#pragma unroll 5
+  for (uint32_t w = group * kScanGroup * kScanWords + threadIdx.x; w < blk * kScanWords; w += kTaskThreads)
+    sum += (uint32_t)__popc(t.ws.bitmap[w]);
   for (uint32_t i = threadIdx.x; i < group; i += kTaskThreads) {
     unsigned long long v;
-    while (((v = *(volatile unsigned long long*)(groups + i)) >> 40) != kScanGroup)
-      if (give_up()) break;
-    sum += (uint32_t)v;  // fewer than 2^32 cells
-  }
-  const uint32_t mate = group * kScanGroup + threadIdx.x;
-  if (mate < blk && threadIdx.x < kScanGroup) {
-    uint32_t v;
-    while ((v = *(volatile uint32_t*)(own + mate)) == 0u)
-      if (give_up()) {
-        v = 1u;
-        break;
+    while (((v = *(volatile unsigned long long*)(groups + i)) >> 40) != kScanGroup) {
+      if (++spin < 1u << 21) {
+        __nanosleep(32);
+        continue;
       }
-    sum += v - 1u;
+      set_status(t.status, SPCONVB_ST_TIMEOUT, 7u);
+      break;
+    }
+    sum += (uint32_t)v;  // fewer than 2^32 cells
   }
   sum = __reduce_add_sync(0xffffffffu, sum);
   if (lane == 0) sh.back[warp] = sum;
@@ -925,8 +915,11 @@ int spconvb_inverse_map(const int32_t* coords, const uint32_t* n_ptr, uint32_t c
 
 size_t spconvb_down_workspace_bytes(const int32_t out_grid[3], int32_t batch) {
   if (!out_grid || !grid_fits(out_grid, batch)) return 0;
+  // The scan's state takes two words for 2 048 of the bitmap, one and what its alignment takes: inside
+  // one word for 1 024 and 16.  (The size is part of the interface: it decides which grids
+  // spconvb_down_map_static takes.)
   const size_t words = down_words(out_grid, batch);
-  return sizeof(uint32_t) * (2 * words + scan_state_words(scan_blocks((uint32_t)words)) + 16);
+  return sizeof(uint32_t) * (2 * words + (words + 1023) / 1024 + 16);
 }
 
 // Shared body of spconvb_down_map and spconvb_down_map_ranked.

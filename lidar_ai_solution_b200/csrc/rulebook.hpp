@@ -21,10 +21,10 @@ struct Kernel3 {
 //   [0, W)        bitmap over the output grid                     (zero before the mark task)
 //   [W, 2W)       rank of the word's first set bit (after the emit task)
 //   [2W, ...)     state of the emit task's scan                    (zero before the emit task):
-//                 totals of groups of 32 scan blocks (64 bits each, from the next 8-byte boundary
-//                 on: the workspace may start at any word), a counter of the blocks started,
-//                 counts of the scan blocks of 128 words
-constexpr uint32_t kScanGroup = 32;
+//                 totals of groups of 16 scan blocks of 128 words (64 bits each, from the next
+//                 8-byte boundary on: the workspace may start at any word), a counter of the blocks
+//                 started
+constexpr uint32_t kScanGroup = 16;
 struct DownWs {
   uint32_t* bitmap;
   uint32_t* prefix;
@@ -36,11 +36,10 @@ struct DownWs {
   __device__ uint32_t* scan_ticket() const {
     return scan + 2 * ((blocks + kScanGroup - 1) / kScanGroup);
   }
-  __device__ uint32_t* scan_counts() const { return scan_ticket() + 1; }
 #endif
 };
 inline size_t scan_state_words(uint32_t blocks) {
-  return 2 * (size_t)((blocks + kScanGroup - 1) / kScanGroup) + 1 + blocks;
+  return 2 * (size_t)((blocks + kScanGroup - 1) / kScanGroup) + 1;
 }
 
 enum RuleTaskKind : int32_t {

@@ -79,6 +79,22 @@ def test_argument_checks_come_before_any_device_work():
     assert lib.spconvb_convert(fake, cabi.F16, 5, cabi.F16, 4, 1.0, fake, 100, fake, None) == -1
 
 
+def test_workspace_of_a_strided_rulebook_keeps_its_size():
+    """Two words for 32 cells, one for 1 024 of those, 16 to spare: what decides which grids the
+    allocation-free entry point takes, up to 16 768 768 cells in a row and no more."""
+    cabi, lib = _lib()
+    for cells in (1, 32, 33, 4096, 4097, 131072, 131073, 10 ** 6, 16768768, 2 ** 32 - 2):
+        words = -(-cells // 32)
+        grid = (1, 1, cells) if cells < 2 ** 31 else (2, 1, cells // 2)
+        assert lib.spconvb_down_workspace_bytes(cabi.i3(grid), 1) == \
+            4 * (2 * words + -(-words // 1024) + 16)
+        # the scan's groups of 16 blocks of 128 words, its ticket and its alignment fit behind the ranks
+        blocks = -(-words // 128)
+        assert 2 * -(-blocks // 16) + 1 + 1 <= -(-words // 1024) + 16
+    size = [lib.spconvb_down_workspace_bytes(cabi.i3((1, 1, c)), 1) for c in (16768768, 16768769)]
+    assert size[0] <= cabi.STATIC_SCRATCH_BYTES < size[1]
+
+
 def test_weight_packing_layout():
     """Chunk j, row n, 16-byte segment c is stored at segment c ^ (n % 8) of row n."""
     cabi, lib = _lib()

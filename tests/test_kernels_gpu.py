@@ -216,13 +216,15 @@ def test_down_map_geometries_match_the_oracle(k, s, p, d):
     ((1, 1, 5), 3),             # one bitmap word, partly outside the grid
     ((4, 32, 32), 3900),        # one scan block, nearly every cell set
     ((4, 32, 33), 4224),        # a scan block and 4 words, every cell set
-    ((32, 64, 64), 40000),      # exactly one group of 32 scan blocks
-    ((32, 64, 65), 130000),     # a group and a bit
+    ((16, 64, 64), 30000),      # exactly one group of 16 scan blocks
+    ((16, 64, 65), 66000),      # a group and a bit
+    ((32, 64, 64), 40000),      # exactly two groups
+    ((32, 64, 65), 130000),     # two groups and a bit
     ((33, 257, 311), 2000),     # many blocks, most of them empty
 ])
 def test_strided_rows_at_the_edges_of_scan_blocks(grid, n):
     """Output rows, order, count and map where the scan's blocks (128 words of 32 cells) and groups
-    of blocks (32) begin and end; a 1x1x1 kernel of stride 1, so the outputs are the inputs."""
+    of blocks (16) begin and end; a 1x1x1 kernel of stride 1, so the outputs are the inputs."""
     ops = _ops()
     cells = np.sort(np.random.default_rng(n).permutation(int(np.prod(grid)))[:n])
     coords = np.zeros((n, 4), np.int32)

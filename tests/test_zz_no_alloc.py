@@ -71,6 +71,27 @@ def test_static_scratch_variant_matches_workspace_variant_twice():
         assert torch.equal(sub_new[:, :k], sub_ref[:, :k])
 
 
+def test_static_scratch_variant_takes_the_largest_grid_that_fits():
+    """16 768 768 output cells fill the scratch area; one more is refused."""
+    from lidar_ai_solution_b200 import cabi, ops
+    grid, one = (8, 32, 65503), (1, 1, 1)
+    n = 40000
+    cells = np.sort(np.random.default_rng(0).choice(int(np.prod(grid)), n, replace=False))
+    cells[-1] = int(np.prod(grid)) - 1
+    coords = np.zeros((n, 4), np.int32)
+    coords[:, 1:] = np.stack(np.unravel_index(cells, grid), 1)
+    order = np.random.default_rng(1).permutation(n)
+    dc, n_ptr, st = _dev(coords[order]), ops.device_count(n), ops.new_status()
+    table = ops.hash_build(dc, n_ptr, grid, status=st)
+    rc, oc, n_out, m, _ = _static_down_map(ops, cabi, dc, n_ptr, grid, table, one, one, (0, 0, 0), n, st)
+    torch.cuda.synchronize()
+    assert rc == cabi.OK and int(st.cpu()[0]) == 0 and int(n_out.item()) == n
+    assert np.array_equal(oc.cpu().numpy(), coords)
+    assert np.array_equal(m.cpu().numpy()[0], np.argsort(order))
+    rc = _static_down_map(ops, cabi, dc, n_ptr, (1, 1, 16768769), table, one, one, (0, 0, 0), n, st)[0]
+    assert rc == cabi.E_SCRATCH_LIMIT
+
+
 def test_static_scratch_variant_rejects_grids_beyond_its_limit():
     from lidar_ai_solution_b200 import cabi, ops
     grid = (41, 1440, 1440)      # stride 1 keeps 85 M output cells: far beyond the scratch area
