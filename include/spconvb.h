@@ -139,6 +139,9 @@ SPCONVB_API size_t spconvb_down_workspace_bytes(const int32_t out_grid[3], int32
  * cap_out, SPCONVB_ST_OVERFLOW on clipping), the map [kvol][cap_out] and, when
  * out_table != NULL, the hash table of the outputs.  `workspace` keeps the
  * outputs' bitmap and rank prefix afterwards (see spconvb_subm_map_ranked).
+ * It may start at any multiple of 4 bytes.  With SPCONVB_FLAG_PREZEROED its first
+ * cells / 32 words, rounded up (the bitmap over the batch's output cells), must be zero
+ * for every call, and out_table; the rest may hold anything.
  * `in_table` / `in_slots` are not used (kept in the signature; may be NULL / 0). */
 SPCONVB_API int spconvb_down_map(const int32_t* in_coords, const uint32_t* n_in_ptr,
                                  uint32_t cap_in, uint32_t launch_rows, const int32_t in_grid[3],

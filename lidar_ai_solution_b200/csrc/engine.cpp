@@ -750,8 +750,8 @@ int Engine::prepare(const int32_t grid[3], int batch) {
   for (size_t r = 0; r < rules.size(); ++r) {
     if (rules[r].subm || rules[r].inverse_of >= 0) continue;
     ws_off[r] = zoff;
-    // only the bitmap (first third of the workspace) must be zero, but the
-    // rest is small next to it and one memset is cheaper than two
+    // the bitmap and, behind the ranks, the scan's state must be zero before every call; the ranks
+    // (half of the workspace) need not be, but one memset is cheaper than two
     zoff += align256(rules[r].ws_bytes);
   }
   zero_bytes_ = zoff;

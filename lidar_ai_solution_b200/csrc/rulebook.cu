@@ -940,10 +940,11 @@ static int down_map_impl(const int32_t* in_coords, const uint32_t* n_in_ptr, uin
   cudaStream_t st = (cudaStream_t)stream;
 
   const DownWs ws = down_ws(og, batch, workspace);
+  // PREZEROED speaks of the bitmap (and the table): the scan's state is this library's own and is
+  // cleared on every call.  A stale ticket would number blocks past the end.
+  SPCONVB_CUDA_TRY(cudaMemsetAsync(ws.scan, 0, sizeof(uint32_t) * scan_state_words(ws.blocks), st));
   if (!(flags & SPCONVB_FLAG_PREZEROED)) {
     SPCONVB_CUDA_TRY(cudaMemsetAsync(ws.bitmap, 0, sizeof(uint32_t) * (size_t)ws.words, st));
-    SPCONVB_CUDA_TRY(
-        cudaMemsetAsync(ws.scan, 0, sizeof(uint32_t) * scan_state_words(ws.blocks), st));
     if (out_table)
       SPCONVB_CUDA_TRY(cudaMemsetAsync(out_table, 0, sizeof(uint64_t) * (size_t)out_slots, st));
   }
@@ -1049,10 +1050,11 @@ int spconvb_down_map_static(const int32_t* in_coords, const uint32_t* n_in_ptr, 
   void* scratch = nullptr;
   rc = static_scratch_for_current_device(&scratch);
   if (rc != SPCONVB_OK) return rc;
-  // The array still holds the previous call's bitmap and block totals: it is cleared on
-  // every call, whatever the caller says about its own buffers.
+  // The array still holds the previous call's bitmap: it is cleared on every call, whatever the
+  // caller says about its own buffers.
   cudaStream_t st = (cudaStream_t)stream;
-  SPCONVB_CUDA_TRY(cudaMemsetAsync(scratch, 0, need, st));
+  SPCONVB_CUDA_TRY(
+      cudaMemsetAsync(scratch, 0, sizeof(uint32_t) * (size_t)down_words(og, batch), st));
   if (out_table && !(flags & SPCONVB_FLAG_PREZEROED))
     SPCONVB_CUDA_TRY(cudaMemsetAsync(out_table, 0, sizeof(uint64_t) * (size_t)out_slots, st));
   return spconvb_down_map(in_coords, n_in_ptr, cap_in, launch_rows, in_grid, batch, ksize, stride,

@@ -317,6 +317,18 @@ def test_down_map_workspace_may_start_at_any_word(grid, shift):
     assert np.array_equal(oc, roc) and np.array_equal(m, rdm[:, :rn])
 
 
+@pytest.mark.parametrize("zero,flags", [("all", 1), ("bitmap", 1), ("none", 0)])
+def test_down_map_on_a_used_workspace(zero, flags):
+    """What a call must find zero: with PREZEROED the bitmap, without it nothing; the rest of the
+    workspace, the scan's state among it, may be as another use or the call before has left it."""
+    grid = (41, 180, 180)
+    coords = scenes.make_coords(6000, grid, 6)
+    args = ((3, 3, 3), (2, 2, 2), (1, 1, 1))
+    roc, rdm, _, _, rn = orc.down_map(coords, grid, *args)
+    oc, m = _carved_down_map(coords, grid, args, 0, rn, flags, zero, runs=2)
+    assert np.array_equal(oc, roc) and np.array_equal(m, rdm[:, :rn])
+
+
 def test_down_map_overflow_sets_status():
     ops = _ops()
     from lidar_ai_solution_b200 import cabi
