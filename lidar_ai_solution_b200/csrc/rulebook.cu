@@ -10,6 +10,8 @@
 // The steps of one rulebook are short (2-20 us) and several rulebooks are independent of one
 // another, so they run as tasks of shared launches (RuleWave): a backbone of four strided and
 // four SubM rulebooks takes 6 launches where one kernel per step took 24.
+#include <limits.h>
+
 #include <mutex>
 
 #include "common.cuh"
@@ -247,14 +249,17 @@ __device__ __forceinline__ void for_each_output(const int4 c, const Grid3& gout,
 // With dilation 1 the outputs an input coordinate c reaches along one axis are a range:
 // tap k = c + pad - o * stride lies in [0, K) exactly for
 // ceil((c + pad - K + 1) / stride) <= o <= floor((c + pad) / stride), clipped to the grid.
-// No divisibility tests, no tap loop.
+// No divisibility tests, no tap loop.  Nothing has checked the coordinate: none below -pad reaches a
+// cell (the quotient would be rounded towards zero, to a cell and a tap that do not exist), and the
+// sums stay inside an int for every value.
 struct AxisRange { int lo, hi; };
 __device__ __forceinline__ AxisRange output_range(int c, int a, const Grid3& gout,
                                                   const Kernel3& kr) {
+  AxisRange r = {0, -1};
+  if (c < -kr.p[a] || c > INT_MAX - kr.p[a]) return r;
   const int top = c + kr.p[a], t = top - kr.k[a] + 1;
-  AxisRange r;
   r.hi = min(stride_quotient(top, kr.s[a], kr.sh[a]), gout.g[a] - 1);
-  r.lo = t <= 0 ? 0 : stride_quotient(t + kr.s[a] - 1, kr.s[a], kr.sh[a]);
+  if (t > 0) r.lo = stride_quotient(t - 1, kr.s[a], kr.sh[a]) + 1;
   return r;
 }
 

@@ -275,6 +275,42 @@ def test_maps_where_threads_go_from_planes_to_rows(n):
     assert np.array_equal(gdm.cpu().numpy()[:, :rn], rdm[:, :rn])
 
 
+@pytest.mark.parametrize("s", [(3, 3, 3), (2, 2, 2), (5, 1, 3), (1, 1, 1)])
+@pytest.mark.parametrize("k,p", [((3, 3, 3), (1, 0, 1)), ((2, 1, 4), (0, 0, 2)), ((1, 1, 1), (0, 0, 0))])
+def test_strided_rows_outside_the_grid(k, s, p):
+    """Nothing checks a coordinate before the strided rulebook: rows outside the grid, up to the ends of
+    an int, reach the cells that tap = c + pad - cell * stride in [0, K) gives, and no others."""
+    ops = _ops()
+    grid = (7, 12, 15)
+    rng = np.random.default_rng(3)
+    coords = np.zeros((3000, 4), np.int32)
+    coords[:, 1:] = rng.integers(-6, 20, (3000, 3))
+    ends = np.iinfo(np.int32)
+    coords[:12, 1:][np.arange(12), np.arange(12) % 3] = [ends.min, ends.max, ends.min + 1, ends.max - 1] * 3
+    coords = coords[np.sort(np.unique(coords, axis=0, return_index=True)[1])]  # each cell once
+    og = ops.out_grid(grid, k, s, p)
+    reached = {}
+    for row, c in enumerate(coords[:, 1:].astype(np.int64)):
+        axes = [[(o, c[a] + p[a] - o * s[a]) for o in range(og[a]) if 0 <= c[a] + p[a] - o * s[a] < k[a]]
+                for a in range(3)]
+        for o0, k0 in axes[0]:
+            for o1, k1 in axes[1]:
+                for o2, k2 in axes[2]:
+                    reached.setdefault((o0, o1, o2), {})[(k0 * k[1] + k1) * k[2] + k2] = row
+    cells = sorted(reached)
+    want = np.full((int(np.prod(k)), len(cells)), -1, np.int32)
+    for o, cell in enumerate(cells):
+        for tap, row in reached[cell].items():
+            want[tap, o] = row
+    st = ops.new_status()
+    oc, n_out, m, _, _ = ops.down_map(_dev(coords), ops.device_count(len(coords)), grid, None, k, s, p,
+                                      cap_out=len(cells) + 50, status=st, want_table=False)
+    _status_ok(st)
+    assert int(n_out.item()) == len(cells) > 0
+    assert np.array_equal(oc.cpu().numpy()[:len(cells), 1:], np.array(cells))
+    assert np.array_equal(m.cpu().numpy()[:, :len(cells)], want)
+
+
 def _carved_down_map(coords, grid, args, shift, cap_out, flags=0, zero="all", runs=1):
     """spconvb_down_map on a workspace `shift` bytes into a buffer; what lies behind it stays as it is.
     With a `zero` other than "none" the bitmap, or all of the workspace, is cleared before each run."""
