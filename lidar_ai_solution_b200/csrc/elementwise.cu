@@ -192,13 +192,14 @@ __global__ void __launch_bounds__(256)
   const size_t vol = (size_t)gp[0] * gp[1] * gp[2];
   const uint32_t n = BY_CELL ? (uint32_t)vol * g.batch : min(load_after_wait(n_ptr), cap);
   const uint32_t lane = threadIdx.x & 31u;
-  for (uint32_t at0 = blockIdx.x * 32; at0 < n; at0 += gridDim.x * 32) {
+  // (64 bits: there may be almost 2^32 cells)
+  for (unsigned long long first = blockIdx.x * 32ull; first < n; first += gridDim.x * 32ull) {
     int any = 0;
     if (threadIdx.x < 32) {
-      const uint32_t at = at0 + threadIdx.x;
+      const uint32_t at = (uint32_t)first + threadIdx.x;
       int32_t row = -1;
       long long cell = -1;
-      if (at < n) {
+      if (first + threadIdx.x < n) {
         if (BY_CELL) {
           const uint32_t line = at / gp[2], s2 = at - line * gp[2];
           const uint32_t plane = line / gp[1], s1 = line - plane * gp[1];
