@@ -1,5 +1,7 @@
 // HBM-bound helpers around the convolutions: Add / Add&ReLU / ReLU, precision
 // and channel-padding conversion, and the sparse -> dense BEV scatter.
+#include <type_traits>
+
 #include "common.cuh"
 #include "pdl.cuh"
 #include "rulebook.hpp"
@@ -170,14 +172,17 @@ __global__ void pad8_f16_kernel(const __half* __restrict__ x, int cin, const uin
 // Rows into [N, C, g(p0), g(p1), g(p2)].  A block takes 32 rows at a time through shared memory and
 // writes them channel by channel, a lane a cell, so that neighbouring cells share write sectors;
 // what bounds it is the number of sectors written, one per channel and run of neighbours.
-// BY_CELL: the 32 are the rows of 32 consecutive cells of the *output*, found by rank in the bitmap
-// of the strided rulebook that made them.  Taken when the output's axes are permuted: rows in their
-// own order then lie a line apart, every 2-byte store is a sector of its own, and the BEVFusion
-// sample frame took 43 us, this way 7.  (Not otherwise: it looks up all cells, and in row order the
-// runs are the same.)
+// RANKED (the output's axes are permuted and the rows were made by a strided rulebook): the 32 may
+// also be the rows of 32 consecutive cells of the *output*, found by rank in that rulebook's bitmap.
+// In their own order rows then lie a line apart and every 2-byte store is a sector of its own; the
+// BEVFusion sample frame took 43 us, by cells 7.  (Not otherwise: in row order the runs are the same.)
+// But all cells are looked up, so it depends on how many there are for a row and on the row's width:
+// by cells while they are at most rows x channels / 4.  By cells / by rows, us, at cells per row:
+// 128 channels 48 / 85 at 4, 44 / 42 at 13, 89 / 95 at 32, 60 / 46 at 130; 32 channels 52 / 73 at 3, 50 / 34
+// at 11; 16 channels 13 / 20 at 1, 81 / 47 at 7, 217 / 58 at 10 900.
 // VEC: fp16 rows of whole 16-byte pieces; 16-byte loads, one channel loop without divisions
 // (CenterPoint frame of 10 800 voxels 15 us, this way 6).
-template <bool BY_CELL, bool VEC>
+template <bool RANKED, bool VEC>
 __global__ void __launch_bounds__(256)
     scatter_dense_kernel(const void* __restrict__ feat, int in_kind, float in_scale,
                          const int4* __restrict__ coords, const uint32_t* n_ptr, uint32_t cap,
@@ -190,17 +195,21 @@ __global__ void __launch_bounds__(256)
   pdl_wait();
   const int gp[3] = {g.g[p0], g.g[p1], g.g[p2]};
   const size_t vol = (size_t)gp[0] * gp[1] * gp[2];
-  const uint32_t n = BY_CELL ? (uint32_t)vol * g.batch : min(load_after_wait(n_ptr), cap);
+  const uint32_t rows = min(load_after_wait(n_ptr), cap);
+  const uint32_t cells = RANKED ? (uint32_t)vol * g.batch : 0u;
+  const bool by_cell = RANKED && cells <= (unsigned long long)rows * channels / 4;
+  const uint32_t n = by_cell ? cells : rows;
   const uint32_t lane = threadIdx.x & 31u;
-  // (64 bits: there may be almost 2^32 cells)
-  for (unsigned long long first = blockIdx.x * 32ull; first < n; first += gridDim.x * 32ull) {
+  // there may be almost 2^32 cells
+  using Index = std::conditional_t<RANKED, unsigned long long, uint32_t>;
+  for (Index first = blockIdx.x * 32u; first < n; first += gridDim.x * 32u) {
     int any = 0;
     if (threadIdx.x < 32) {
       const uint32_t at = (uint32_t)first + threadIdx.x;
       int32_t row = -1;
       long long cell = -1;
       if (first + threadIdx.x < n) {
-        if (BY_CELL) {
+        if (by_cell) {
           const uint32_t line = at / gp[2], s2 = at - line * gp[2];
           const uint32_t plane = line / gp[1], s1 = line - plane * gp[1];
           const uint32_t b = plane / gp[0], s0 = plane - b * gp[0];
@@ -426,10 +435,11 @@ extern "C++" int spconvb::scatter_dense_launch(const void* feat, int32_t in_kind
     if ((1 << p[0] | 1 << p[1] | 1 << p[2]) != 7) return SPCONVB_E_ARG;
   }
   cudaStream_t st = (cudaStream_t)stream;
-  // fp16 rows of 16-byte pieces; a permuted output with a rank index (see the kernel)
+  // fp16 rows of 16-byte pieces; a permuted output with a rank index (see the kernel, which also
+  // decides whether to go by its cells: the number of rows is known there)
   const bool vec = in_kind == SPCONVB_F16 && channels % 8 == 0 && ((uintptr_t)feat & 15u) == 0u;
-  const bool by_cell = rank != nullptr && p[2] != 2;
-  auto* kernel = by_cell ? (vec ? scatter_dense_kernel<true, true> : scatter_dense_kernel<true, false>)
+  const bool ranked = rank != nullptr && p[2] != 2;
+  auto* kernel = ranked ? (vec ? scatter_dense_kernel<true, true> : scatter_dense_kernel<true, false>)
                          : (vec ? scatter_dense_kernel<false, true> : scatter_dense_kernel<false, false>);
   const size_t tile_bytes = sizeof(__half) * 33 * (size_t)channels;
   if (tile_bytes > 48 * 1024 - 512) {
@@ -438,7 +448,7 @@ extern "C++" int spconvb::scatter_dense_launch(const void* feat, int32_t in_kind
     static bool raised[64][4] = {};
     int dev = 0;
     SPCONVB_CUDA_TRY(cudaGetDevice(&dev));
-    const int which = 2 * by_cell + vec;
+    const int which = 2 * ranked + vec;
     if (dev < 0 || dev >= 64 || !raised[dev][which]) {
       SPCONVB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                             (int)(sizeof(__half) * 33 * 1024)));
@@ -450,12 +460,12 @@ extern "C++" int spconvb::scatter_dense_launch(const void* feat, int32_t in_kind
   g.batch = batch;
   const size_t bytes = sizeof(__half) * (size_t)batch * channels * grid[0] * grid[1] * grid[2];
   if (clear) SPCONVB_CUDA_TRY(cudaMemsetAsync(out, 0, bytes, st));
-  const size_t items = by_cell ? (size_t)batch * grid[0] * grid[1] * grid[2] : launch_rows;
+  const size_t items = ranked ? (size_t)batch * grid[0] * grid[1] * grid[2] : launch_rows;
   size_t want_blocks = (items + 31) / 32;
   if (want_blocks > (size_t)kSmCount * 16) want_blocks = (size_t)kSmCount * 16;
   const int blocks = (int)want_blocks;
-  const uint32_t* bitmap = by_cell ? rank->bitmap : nullptr;
-  const uint32_t* prefix = by_cell ? rank->prefix : nullptr;
+  const uint32_t* bitmap = ranked ? rank->bitmap : nullptr;
+  const uint32_t* prefix = ranked ? rank->prefix : nullptr;
   SPCONVB_CUDA_TRY(launch_pdl(kernel, dim3(blocks), dim3(256), tile_bytes, st, feat, in_kind,
                               in_scale, (const int4*)coords, n_ptr, launch_rows, channels, g, p[0],
                               p[1], p[2], bitmap, prefix, (__half*)out));

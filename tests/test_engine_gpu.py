@@ -551,6 +551,39 @@ def test_transposed_dense_output_is_the_dense_output_transposed(grid, batch, cha
     assert np.any(want != 0) and np.array_equal(got, want)
 
 
+@pytest.mark.parametrize("grid,channels,rows", [((2, 40, 50), 32, 500), ((2, 40, 50), 32, 499),
+                                                ((3, 37, 45), 16, 1248), ((3, 37, 45), 16, 1249),
+                                                ((21, 200, 300), 64, 900), ((21, 200, 300), 64, 0)])
+def test_permuted_dense_output_by_cells_and_by_rows(grid, channels, rows):
+    """A permuted output is walked by its cells while they are at most rows x channels / 4, by the rows
+    beyond: both sides of the line, many more cells than rows, no rows; through a 1x1x1 rulebook, with
+    a capacity that says nothing of the rows."""
+    eng = _engine_mod()
+    rng = np.random.default_rng(rows)
+    ids, nodes = models._Ids(), []
+    y = models._conv(ids, rng, nodes, "0", 16, channels, (1, 1, 1), (1, 1, 1), (0, 0, 0), False, "down",
+                     "None", [0, 0], 20000)
+    d, t = ids.new(), ids.new()
+    nodes.append({"op": "dense", "name": "scatter0", "x": y, "out": d, "input_spatial_shape": list(grid),
+                  "format": "zyx", "output_shape": [1, channels, *grid]})
+    nodes.append({"op": "transpose", "name": "transpose0", "x": d, "out": t, "dims": [0, 1, 2, 4, 3]})
+    model = {"kind": "layer", "inputs": [("0", [1, 16])], "nodes": nodes, "in_channels": 16,
+             "outputs": [(t, [1, channels, grid[0], grid[2], grid[1]])], "roles": {"conv_input": [0]}}
+    cells = np.sort(rng.choice(int(np.prod(grid)), rows, replace=False))
+    coords = np.zeros((max(rows, 1), 4), np.int32)
+    coords[:rows, 1:] = np.stack(np.unravel_index(cells, grid), 1)
+    feats = rng.standard_normal((max(rows, 1), 16)).astype(np.float16)
+    e = eng.Engine.from_model(model, eng.PRECISION_FP16, eng.BUILD_KEEP_TENSORS)
+    for _ in range(2):
+        e.forward(_dev(feats), _dev(coords), grid, n=rows)
+        torch.cuda.synchronize()
+        assert e.status()[0] == 0
+        want = np.zeros((channels, int(np.prod(grid))), np.float16)
+        want[:, cells] = e.tensor(y)["features"][:rows].cpu().numpy().T
+        want = want.reshape(channels, *grid).swapaxes(-1, -2)
+        assert np.array_equal(e.output(0).cpu().numpy()[0].view(np.uint16), want.view(np.uint16))
+
+
 def test_batched_forward_equals_frame_by_frame():
     """Several frames in one engine call (told apart by the batch column of the indices) give,
     frame for frame, the bits of single-frame calls: dense output slices and every stage's rows.
