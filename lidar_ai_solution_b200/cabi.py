@@ -7,7 +7,6 @@ if the shared object is missing, loading raises.
 from __future__ import annotations
 
 import ctypes as C
-import functools
 import os
 
 _PKG = os.path.dirname(os.path.abspath(__file__))
@@ -144,14 +143,12 @@ def lib() -> C.CDLL:
     return _LIB
 
 
-@functools.lru_cache(maxsize=1024)
-def _i3(v):
-    return (C.c_int32 * 3)(*[int(x) for x in v])
+_Int3 = C.c_int32 * 3
 
 
 def i3(v):
-    """Three numbers as the int32[3] the library reads (shared between calls: not to be written)."""
-    return _i3(tuple(v))
+    """Three numbers as the int32[3] the library reads."""
+    return _Int3(*map(int, v))
 
 
 def check(code: int, what: str = "spconvb call"):

@@ -79,6 +79,17 @@ def test_argument_checks_come_before_any_device_work():
     assert lib.spconvb_convert(fake, cabi.F16, 5, cabi.F16, 4, 1.0, fake, 100, fake, None) == -1
 
 
+def test_triples_are_made_anew_from_any_numbers():
+    """Whatever int() takes is a triple's number, hashable or not; every call's array is its own."""
+    cabi, _ = _lib()
+    for v in ((41, 8, 9), [41.0, np.int64(8), np.uint8(9)], np.array([41, 8, 9]),
+              (np.array(41), np.array(8), np.array(9)), iter((41, 8, 9))):
+        assert list(cabi.i3(v)) == [41, 8, 9]
+    a = cabi.i3((1, 2, 3))
+    a[0] = 7
+    assert list(cabi.i3((1, 2, 3))) == [1, 2, 3]
+
+
 def test_workspace_of_a_strided_rulebook_keeps_its_size():
     """Two words for 32 cells, one for 1 024 of those, 16 to spare: what decides which grids the
     allocation-free entry point takes, up to 16 768 768 cells in a row and no more."""
