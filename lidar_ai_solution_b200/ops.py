@@ -15,8 +15,14 @@ from . import cabi
 from .cabi import ACT_NONE, ACT_RELU, F16, I8  # noqa: F401
 
 
+# torch's own way to the current stream's handle, a microsecond cheaper a call; not a public one
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def _stream():
-    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+    if _raw_stream is None:
+        return torch.cuda.current_stream().cuda_stream
+    return _raw_stream(torch.cuda.current_device())
 
 
 def _ptr(t):

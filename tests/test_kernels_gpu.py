@@ -33,6 +33,17 @@ def _status_ok(status):
     assert s[0] == 0, "device status %s" % s
 
 
+def test_calls_go_to_the_current_stream(monkeypatch):
+    """By torch's own shortcut to its handle, and without it."""
+    ops = _ops()
+    side = torch.cuda.Stream()
+    for shortcut in (ops._raw_stream, None):
+        monkeypatch.setattr(ops, "_raw_stream", shortcut)
+        assert ops._stream() == torch.cuda.current_stream().cuda_stream != side.cuda_stream
+        with torch.cuda.stream(side):
+            assert ops._stream() == side.cuda_stream
+
+
 # ------------------------------------------------------------------ rulebooks
 @pytest.mark.parametrize("n,grid,seed", [(20000, (41, 180, 180), 0), (20000, (41, 180, 180), 3),
                                          (120000, (41, 1440, 1440), 1), (1, (41, 180, 180), 0),
