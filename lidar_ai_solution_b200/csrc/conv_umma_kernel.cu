@@ -385,12 +385,14 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
         break;
       tc_fence_after();  // the epilogue's reads of this accumulator come before these MMAs
       const uint32_t d_tmem = tmem_base + buf * kTileRows;
-      // No fence before the MMAs of a stage: its rows arrive by cp.async completions on the stage's
-      // mbarrier, which is what the MMA's shared-memory reads are ordered behind.
+      // The rows of a stage are written by cp.async, through the generic proxy, and read by the MMAs
+      // through the async proxy: the stage's mbarrier orders the threads, the fence the proxies.  (It
+      // costs nothing that shows: 120 000 voxels 638.7 us without, 638.8 with it.)
       uint32_t accumulate = 0u;
 #pragma unroll 1
       for (int j = nchunk - 1; j > 0; --j) {
         if (leader) {
+          fence_proxy_async();
           umma_lohi<INT8>(d_tmem, wd, rd, desc_hi, idesc, accumulate);
           umma_lohi<INT8>(d_tmem, wd + 2u, rd + 2u, desc_hi, idesc, 1u);
           umma_lohi<INT8>(d_tmem, wd + 4u, rd + 4u, desc_hi, idesc, 1u);
@@ -406,6 +408,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
       }
       if (!alive) break;
       if (leader) {
+        fence_proxy_async();
         for (int ks = 0; ks < last_ksteps; ++ks) {
           umma_lohi<INT8>(d_tmem, wd + 2u * ks, rd + 2u * ks, desc_hi, idesc, accumulate);
           accumulate = 1u;
