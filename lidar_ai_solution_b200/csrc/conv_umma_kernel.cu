@@ -337,7 +337,9 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
     }
     cp_async_wait_all();  // nothing of this thread may still be writing when the CTA exits
     __syncwarp();
-    if (shared_tail && tile >= ntiles && tiles_done > 0u) {
+    // As one warp: where a launch gives up, some lanes may have left at a stage that came too late for
+    // them and others not, and the drain exchanges between all 32.
+    if (__all_sync(0xffffffffu, shared_tail && tile >= ntiles && tiles_done > 0u)) {
       drains = true;
       drain_tile = tile - gridDim.x;
       drain_tl = tiles_done - 1u;
