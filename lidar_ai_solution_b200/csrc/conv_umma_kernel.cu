@@ -376,15 +376,18 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
       wd += w_step;
       if (wd == w_end) wd = w_lo0;
     };
-    auto stage_full = [&]() -> bool {
-      return mbar_test_wait(bar, ph) || mbar_wait_spin(bar, ph, abort_flag, a.status, 3u);
+    // A lane that gives up walks on without waiting, and the issuing one without issuing: the lanes
+    // never part, so none asks about a stage a whole ring behind another (whose phase it would take
+    // for the one after), and none waits at a warp barrier for one that has left.
+    bool alive = true;
+    auto stage_full = [&]() {
+      alive = alive && (mbar_test_wait(bar, ph) || mbar_wait_spin(bar, ph, abort_flag, a.status, 3u));
     };
     // The loop is entered with the current chunk's stage known to be full.
-    bool alive = blockIdx.x < ntiles && stage_full();
-    for (uint32_t tile = blockIdx.x; tile < ntiles && alive; tile += gridDim.x, ++tl) {
+    if (blockIdx.x < ntiles) stage_full();
+    for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++tl) {
       const uint32_t buf = tl & 1u;
-      if (!mbar_wait_spin(bar_tempty + 8 * buf, ((tl >> 1) & 1u) ^ 1u, abort_flag, a.status, 2u))
-        break;
+      alive = alive && mbar_wait_spin(bar_tempty + 8 * buf, ((tl >> 1) & 1u) ^ 1u, abort_flag, a.status, 2u);
       tc_fence_after();  // the epilogue's reads of this accumulator come before these MMAs
       const uint32_t d_tmem = tmem_base + buf * kTileRows;
       // The rows of a stage are written by cp.async, through the generic proxy, and read by the MMAs
@@ -393,7 +396,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
       uint32_t accumulate = 0u;
 #pragma unroll 1
       for (int j = nchunk - 1; j > 0; --j) {
-        if (leader) {
+        if (leader && alive) {
           fence_proxy_async();
           umma_lohi<INT8>(d_tmem, wd, rd, desc_hi, idesc, accumulate);
           umma_lohi<INT8>(d_tmem, wd + 2u, rd + 2u, desc_hi, idesc, 1u);
@@ -401,15 +404,12 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
           umma_lohi<INT8>(d_tmem, wd + 6u, rd + 6u, desc_hi, idesc, 1u);
           tc_commit(bar + kToEmpty);
         }
+        __syncwarp();
         accumulate = 1u;
         next_stage();
-        if (!stage_full()) {
-          alive = false;
-          break;
-        }
+        stage_full();
       }
-      if (!alive) break;
-      if (leader) {
+      if (leader && alive) {
         fence_proxy_async();
         for (int ks = 0; ks < last_ksteps; ++ks) {
           umma_lohi<INT8>(d_tmem, wd + 2u * ks, rd + 2u * ks, desc_hi, idesc, accumulate);
@@ -420,7 +420,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
       }
       __syncwarp();
       next_stage();
-      if (tile + gridDim.x < ntiles) alive = stage_full();
+      if (tile + gridDim.x < ntiles) stage_full();
     }
     __syncwarp();
   }
