@@ -810,7 +810,7 @@ def layer_case(torch, c, n, fp16, reps, flush, seed=0):
 
     def conv():
         ops.conv_forward(x, m, n_ptr, wts, act=ops.ACT_RELU, out_kind=out_kind, inv_out_scale=8.0,
-                         status=st, out=out, n_in_ptr=n_ptr)
+                         status=st, out=out)
 
     conv()
     torch.cuda.synchronize()

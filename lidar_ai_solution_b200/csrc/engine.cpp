@@ -1103,8 +1103,6 @@ int Engine::forward(const void* features, const int32_t* indices, uint32_t cap_r
         const LayerWeights& w = weights[s.weights];
         spconvb_conv_params p = s.cp;
         p.res = s.in1 >= 0 ? rt[s.in1].data : nullptr;
-        p.n_in_ptr = cs_n(R.in_cs);
-        p.cap_in = cs_cap(R.in_cs);
         rc = spconvb_conv_forward(&p, rt[s.in0].data, R.map, coordsets[R.out_cs].cap,
                                   cs_n(R.out_cs), cs_launch(R.out_cs), w.plain, w.packed, w.scale,
                                   w.bias, rt[s.out].data, status, st);
