@@ -61,8 +61,8 @@ def test_rotated_iou_matches_the_restatement():
 
 @pytest.mark.parametrize("mean_logit,seed", [(-6.0, 17), (-3.0, 22)])
 def test_decode_and_nms_match_the_restatement(mean_logit, seed):
-    """-6: a few hundred candidates per task (the sort alone); -3: several thousand, more than
-    nms_pre_max_size, so the radix select chooses the best 1000 first."""
+    """-6: a few hundred candidates per task, all of them ranked; -3: several thousand, more than
+    nms_pre_max_size, so the histogram of the scores bounds the best 1000 first."""
     post = _post()
     heads = scenes.make_centerpoint_heads(seed, mean_logit=mean_logit)
     ref = _oracle_frame(heads, post.TASK_LABEL_OFFSET)
@@ -120,8 +120,8 @@ def test_empty_and_single_task_frames():
 @pytest.mark.parametrize("max_det", [64, 1000])
 def test_tied_scores_rank_by_cell_index(max_det):
     """Heat maps with only five distinct logits: thousands of cells tie exactly, all pass the
-    score filter, and the radix select has to cut inside a run of equal scores.  The ranking is
-    then decided by the cell index, on the device as in the restatement."""
+    score filter, no list holds a run of equal scores, and the radix select has to cut inside one.
+    The ranking is then decided by the cell index, on the device as in the restatement."""
     post = _post()
     rng = np.random.default_rng(2)
     H, W = 64, 80

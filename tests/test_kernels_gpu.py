@@ -426,8 +426,8 @@ def test_conv_int8_bit_exact(c, simt):
 @pytest.mark.parametrize("n", [120000, 200000])
 def test_conv_int8_bit_exact_at_benchmark_sizes(c, n):
     """The layer sweep of the benchmark configurations: SubM 3x3x3, Cin = Cout = c, on the
-    41x1440x1440 grid with 120 k and 200 k voxels (many tiles per CTA, balanced tile heights,
-    the L2 prefetch running ahead of the gather): identical to the oracle."""
+    41x1440x1440 grid with 120 k and 200 k voxels (many tiles per CTA, balanced tile heights):
+    identical to the oracle, with the input's row count given as a hint."""
     got, ref = _int8_layer(n, c, c, seed=c + n, simt=False, out_kind=orc.KIND_I8,
                            grid=(41, 1440, 1440), hint=True)
     assert got.dtype == np.int8 and np.array_equal(got, ref)
@@ -460,8 +460,8 @@ def test_conv_int8_ragged_row_counts(n):
 @pytest.mark.parametrize("n", [1, 3, 255, 256, 257, 511, 513])
 @pytest.mark.parametrize("out_kind", ["i8", "f16"])
 def test_conv_int8_ragged_row_counts_wide_outputs(n, out_kind):
-    """Tiles are 256 rows and the epilogue stores groups of 4 rows per lane quad: partial
-    tiles, partial groups, single-row inputs, with 2 weight replicas on the lanes."""
+    """The epilogue takes 16 rows at a time, an element a lane: partial tiles, partial groups,
+    single-row inputs, with 2 copies of the weights on the accumulator lanes."""
     kind = orc.KIND_I8 if out_kind == "i8" else orc.KIND_F16
     got, ref = _int8_layer(n, 32, 64, seed=100 + n, simt=False, out_kind=kind, grid=(7, 11, 13))
     assert np.array_equal(got.view(np.uint8), ref.view(np.uint8))
@@ -500,6 +500,29 @@ def test_conv_int8_tile_heights_and_shared_tail(n, cin, cout, kvol):
     torch.cuda.synchronize()
     _status_ok(st)
     assert torch.equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("n", [1, 33, 148 * 32, 148 * 96 + 1, 148 * 224 - 5, 148 * 256 + 1])
+@pytest.mark.parametrize("cin,cout,kvol", [(8, 16, 27), (16, 16, 27), (64, 64, 27), (128, 128, 27),
+                                           (128, 32, 3), (32, 128, 1)])
+def test_conv_fp16_tile_heights_and_shared_tail(n, cin, cout, kvol):
+    """The same row counts in fp16, up to the 256-byte rows and 54 chunks a tile of the widest layer,
+    against the CUDA-core kernel.  Operands are small whole numbers: every sum stays below 2^24, so fp32
+    holds it whatever the order, and the two kernels agree bit for bit."""
+    ops = _ops()
+    rng = np.random.default_rng(n + cin)
+    nin = max(n // 2, 1)
+    m = _dev(np.where(rng.random((kvol, n)) < 0.5, rng.integers(0, nin, (kvol, n)), -1).astype(np.int32))
+    x = _dev(rng.integers(-4, 5, (nin, cin)).astype(np.float16))
+    res = _dev(rng.integers(-40, 41, (n, cout)).astype(np.float16))
+    wts = ops.ConvWeights(rng.integers(-3, 4, (cout, kvol, cin)).astype(np.float16), ops.F16, None,
+                          rng.integers(-9, 10, cout).astype(np.float32))
+    n_ptr, st = ops.device_count(n), ops.new_status()
+    out = [ops.conv_forward(x, m, n_ptr, wts, out_kind=ops.F16, res=res, mid_kind=ops.F16,
+                            res_relu=True, force_simt=simt, status=st) for simt in (False, True)]
+    torch.cuda.synchronize()
+    _status_ok(st)
+    assert bool(out[0].any()) and torch.equal(out[0], out[1])
 
 
 @pytest.mark.parametrize("c", [16, 32, 64, 128])
@@ -822,9 +845,8 @@ def _shape_sweep_cases():
 
 @pytest.mark.parametrize("cin,cout,n,kind,i8_out,seed", _shape_sweep_cases())
 def test_conv_int8_shape_sweep_bit_exact(cin, cout, n, kind, i8_out, seed):
-    """Channel pairs select how many copies of the weights sit on the accumulator lanes and
-    whether they stay resident; row counts select the tile height (32..256) and leave
-    partial tiles; the three rulebook kinds give 27 or 3 taps.  Everything int8, so the
+    """Channel pairs select how many copies of the weights sit on the accumulator lanes; row counts
+    select the tile height (32..256), and with it the depth of the rings, and leave partial tiles; the three rulebook kinds give 27 or 3 taps.  Everything int8, so the
     tensor-core kernel must match the oracle bit for bit."""
     ops = _ops()
     grid = (41, 180, 180)
