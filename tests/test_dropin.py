@@ -48,7 +48,9 @@ def test_own_drivers_compile_and_link(tmp_path):
     assert os.path.exists(_compile_driver(tmp_path, v10=True))
 
 
-@pytest.mark.skipif(not os.path.isdir(REF), reason="reference checkout not mounted")
+@pytest.mark.skipif(not os.path.isfile(os.path.join(REF, "libraries", "3DSparseConvolution", "src",
+                                                    "main.cpp")),
+                    reason="reference checkout not mounted")
 def test_reference_sources_compile_and_link_unchanged(tmp_path):
     """The reference's own demo (`pro`: src/main.cpp + src/voxelization.cu) and its BEVFusion
     lidar wrapper (lidar-scn.cpp + lidar-voxelization.cu) are compiled where they lie, against
