@@ -235,9 +235,9 @@ def step_work(line, rows_of, pairs_of, dense_elems):
 # DRAM bytes (read + write) per algorithmic byte of a convolution launch, by the row width
 # of its input in bytes: from one ncu counter pass over every launch of a batch of 4 frames
 # of this workload (`--workload frame_once --batch 4`; dram__bytes_read.sum +
-# dram__bytes_write.sum of the launches of a width over their algorithmic bytes; 0.92 over
+# dram__bytes_write.sum of the launches of a width over their algorithmic bytes; 0.86 over
 # all 21).  A frame's traffic is these ratios weighted by each layer's bytes.
-CONV_DRAM_RATIO = {16: 0.91, 32: 0.93, 64: 0.96, 128: 0.79, 256: 0.79}
+CONV_DRAM_RATIO = {16: 0.87, 32: 0.89, 64: 0.89, 128: 0.70, 256: 0.70}
 
 
 # ------------------------------------------------------------ reference arm
