@@ -344,6 +344,7 @@ typedef struct spconvb_voxel_params {
   int32_t order;          /* 0: indices (0,z,y,x); 1: indices (0,x,y,z) */
 } spconvb_voxel_params;
 
+/* Device bytes of workspace for up to max_points points; it may start at any multiple of 4 bytes. */
 SPCONVB_API size_t spconvb_voxelize_workspace_bytes(const spconvb_voxel_params* p,
                                                     uint32_t max_points);
 
