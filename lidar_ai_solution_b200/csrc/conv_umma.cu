@@ -46,7 +46,7 @@ int conv_umma_pack(int compute, int cin, int cout, int kvol, const void* w, void
 int conv_umma_launch(const spconvb_conv_params& p, const void* in, const int32_t* map,
                      uint32_t cap, const uint32_t* n_out_ptr, uint32_t launch_rows,
                      const void* w_packed, const float* scale, const float* bias, void* out,
-                     uint32_t* status, cudaStream_t st) {
+                     uint32_t* status, bool rules_ready, cudaStream_t st) {
   if (!w_packed) return SPCONVB_E_ARG;
   if (p.kvol > kMaxTaps) return SPCONVB_E_UNSUPPORTED;
   if (p.compute == SPCONVB_I8 && !scale) return SPCONVB_E_ARG;
@@ -64,6 +64,7 @@ int conv_umma_launch(const spconvb_conv_params& p, const void* in, const int32_t
   a.out = (uint8_t*)out;
   a.status = status;
   a.kvol = p.kvol;
+  a.rules_ready = rules_ready ? 1 : 0;
   a.wait_test = p.wait_test;
   const int rb = row_bytes(p.compute, p.cin);
   a.ep = make_epilogue(p);

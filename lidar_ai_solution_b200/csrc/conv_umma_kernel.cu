@@ -141,7 +141,15 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
 
   const int warp = threadIdx.x >> 5;
   const uint32_t lane = threadIdx.x & 31;
-  pdl_trigger();
+  // The row count, the first neighbour indices and the weights are fetched under the kernel before,
+  // where that one has nothing to do with them; its results are waited for before the first gather
+  // and the first drain.  (One launch after the other, all waiting here / waiting there, us: int8
+  // 16 -> 16 of 14 000 rows 5.8 / 5.35, of 120 000 15.3 / 14.0; 128 -> 128 11.8 / 11.5, 41.5 / 40.7.)
+  if (!a.rules_ready) {
+    pdl_wait();
+    pdl_trigger();
+  }
+  const uint32_t n_out = min(load_after_wait(a.n_out_ptr), a.cap);
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kMaxStages; ++s) {
@@ -163,8 +171,6 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
-  pdl_wait();  // nothing above reads or writes what an earlier kernel may still be working on
-  const uint32_t n_out = min(load_after_wait(a.n_out_ptr), a.cap);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -333,6 +339,8 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
     advance2(ntile, nj);
     load_idx(ntile, nj, idx_b);
     advance2(ntile, nj);
+    pdl_wait();
+    pdl_trigger();
     while (step(idx_a) && step(idx_b)) {
     }
     cp_async_wait_all();  // nothing of this thread may still be writing when the CTA exits
@@ -431,6 +439,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
     // as one saturating round-to-nearest-even convert, and the layer-wide switches
     // hoisted out of the element loops.
     const Epilogue ep = a.ep;
+    pdl_wait();  // residual rows are read, and rows written that the kernel before may still read
     // Accumulator row m (TMEM lane m) holds channel m % COUT of weight copy m / COUT.  Copy c
     // owns cols_rep rows of the tile from c * cols_rep on, and the warps of a lane quadrant take
     // its groups of 16 rows in turn: two warps, in the CTA's last tile six.

@@ -1038,6 +1038,8 @@ int Engine::forward(const void* features, const int32_t* indices, uint32_t cap_r
     return cs_cap(c);
   };
 
+  // The rulebooks launched or waited for so far are older than the last launch on the stream.
+  bool rules_ready = false;
   bool clear_dense = true;  // false while a dense step's output was zeroed ahead of time
   auto run_step = [&](const Step& s) -> int {
     int rc = SPCONVB_OK;
@@ -1103,9 +1105,9 @@ int Engine::forward(const void* features, const int32_t* indices, uint32_t cap_r
         const LayerWeights& w = weights[s.weights];
         spconvb_conv_params p = s.cp;
         p.res = s.in1 >= 0 ? rt[s.in1].data : nullptr;
-        rc = spconvb_conv_forward(&p, rt[s.in0].data, R.map, coordsets[R.out_cs].cap,
-                                  cs_n(R.out_cs), cs_launch(R.out_cs), w.plain, w.packed, w.scale,
-                                  w.bias, rt[s.out].data, status, st);
+        rc = conv_forward_launch(&p, rt[s.in0].data, R.map, coordsets[R.out_cs].cap,
+                                 cs_n(R.out_cs), cs_launch(R.out_cs), w.plain, w.packed, w.scale,
+                                 w.bias, rt[s.out].data, status, rules_ready, st);
         last_launches += 1;
         break;
       }
@@ -1213,11 +1215,15 @@ int Engine::forward(const void* features, const int32_t* indices, uint32_t cap_r
           if (cudaStreamWaitEvent(caller_stream, level_ev_[upto], 0) != cudaSuccess)
             rc = SPCONVB_E_DEVICE;
           waited = upto;
+          rules_ready = false;
         }
       } else {
+        const size_t launched = next_wave;
         rc = launch_waves(level, st);
+        if (next_wave != launched) rules_ready = false;
       }
       if (rc == SPCONVB_OK) rc = run_step(s);
+      rules_ready = true;
     } else {
       // Per-step device time: rulebook steps change state and run once; the
       // others overwrite their output and are repeated, each time behind an L2

@@ -1,9 +1,13 @@
 // Programmatic dependent launch.  A kernel launched with launch_pdl() may be scheduled while the
 // kernel before it in the stream is still running; it must call pdl_wait() before it touches
-// global memory (the wait ends when every kernel before it has finished and its writes are
-// visible).  pdl_trigger() lets the kernel after it start its own prologue.  Launch latency and
-// prologue (2-4 us of a kernel's ~10 on small frames) then overlap with the tail of the kernel
-// before.
+// what that kernel may still be working on (the wait ends when every kernel before it has finished
+// and its writes are visible).  pdl_trigger() lets the kernel after it start its own prologue.
+// Launch latency and prologue (2-4 us of a kernel's ~10 on small frames) then overlap with the tail
+// of the kernel before.
+//
+// Every kernel here triggers behind its own wait, never before it.  So when a kernel starts, all
+// but the one launch directly before it are complete, and what those wrote may be read before
+// pdl_wait().
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
