@@ -69,7 +69,6 @@ namespace {
 constexpr int kTileRows = 256;  // most voxel rows per tile: the largest N of the MMA
 constexpr int kEpiWarps = 8;
 constexpr int kMmaWarp = 8;
-constexpr int kProdThreads = 512;   // two groups of 8 producer warps
 constexpr int kProdWarp0 = 9;       // 9, 10, ... 24: four of them on every TMEM lane quadrant
 constexpr int kWeightWarp = 25;
 constexpr int kCtaThreads = 32 * 26;
@@ -153,7 +152,6 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kMaxStages; ++s) {
-      mbar_init(bar_full + 8 * s, kProdThreads / 2 + 1);  // a group's threads + the weights
       mbar_init(bar_empty + 8 * s, 1);
     }
     for (int b = 0; b < 2; ++b) {
@@ -171,10 +169,6 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem_base = *tmem_holder;
 
   // Tile height: the rows are dealt out in rounds over the CTAs, so a fixed 256-row tile
   // can leave most CTAs idle in the last round (227 tiles on 148 CTAs run as long as 296).
@@ -195,6 +189,19 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
   const uint32_t nwst = min((uint32_t)kMaxStages, kRingBytes / (kWeightBytes + row_stage));
   const uint32_t nst = min((uint32_t)kMaxStages, (kRingBytes - nwst * kWeightBytes) / row_stage);
   const uint32_t sW = smem_u32(smem), sR = sW + nwst * kWeightBytes;
+  // Only the producers that own rows of the tile take part, two groups of t32 warps.  (Warps that
+  // only kept the barriers going cost low tiles a third of a chunk's time: fp16 128 -> 128 of 4 700
+  // rows, 32 a tile, 18.2 to 15.0 us, int8 10.8 to 9.1.)
+  if (warp == 0) {
+    if (lane < (uint32_t)kMaxStages)
+      mbar_init(bar_full + 8 * lane, 32u * t32 + 1u);  // a group's threads + the weights
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    fence_proxy_async();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_holder;
 
   const bool is_producer = warp > kMmaWarp && warp != kWeightWarp;
   // Who drains accumulators: the epilogue warps every tile of the CTA; the producers, which have
@@ -204,6 +211,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
   // the last tile, or about to be, only if a tile has at least as many chunks as the ring.
   const bool shared_tail = (uint32_t)nchunk >= nst;
   uint32_t drain_tile = blockIdx.x, drain_tl = 0;
+  const uint32_t help_sets = t32 >> 1;  // sets of four warps, one a lane quadrant, among the producers
   bool drains = warp < kEpiWarps;
   if (warp == kWeightWarp) {
     // -------------------------------------------------------------- weights
@@ -248,7 +256,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
     // piece of it).  Missing neighbours are zero-filled copies, so the 8 items are
     // branch-free and their address arithmetic and copies overlap.
     const uint32_t pw_all = (uint32_t)(warp - kProdWarp0);
-    const uint32_t grp = pw_all >> 3, pw = pw_all & 7u;
+    const uint32_t grp = pw_all >= t32 ? 1u : 0u, pw = grp ? pw_all - t32 : pw_all;
     const uint32_t seg = lane & 7u;        // 16-byte segment of the chunk this thread copies
     const uint32_t slot = lane >> 3;       // its 8 rows of the warp's 32
     // row R of the tile lives at (R / 8) * 1024 + (R % 8) * 128, its segments XOR-ed
@@ -257,7 +265,6 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
     // tap (within the chunk) and byte offset (within the neighbour row) of `seg`
     const uint32_t seg_tap = RB <= kChunk ? seg / SPO : 0u;
     const uint32_t seg_byte = RB <= kChunk ? (seg % SPO) * 16u : seg * 16u;
-    const bool has_rows = pw * 32u < tile_rows;  // else this warp only keeps the barriers going
     const uint32_t row_in_tile = pw * 32u + slot * 8u;
     // 16-byte index loads need the map rows 16-byte aligned and whole groups of 8 inside them
     const bool vec_ok = (a.cap & 7u) == 0u && ((uintptr_t)a.map & 15u) == 0u;
@@ -269,7 +276,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
     auto load_idx = [&](uint32_t tile, int j, int32_t (&v)[8]) {
       const int k = RB <= kChunk ? j * OPC + (int)seg_tap : j / CPT;
       const uint32_t row = tile * tile_rows + row_in_tile;
-      const bool live = has_rows && tile < ntiles && k < a.kvol && row < n_out;
+      const bool live = tile < ntiles && k < a.kvol && row < n_out;
       const int32_t* src = a.map + (size_t)k * a.cap + row;
       if (live && vec_ok && row + 8u <= n_out) {
         const int4 lo = __ldg((const int4*)src), hi = __ldg((const int4*)src + 1);
@@ -289,7 +296,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
         tile += gridDim.x;
       }
     };
-    uint32_t tile = blockIdx.x;
+    uint32_t tile = pw < t32 ? blockIdx.x : ntiles;  // a warp without rows has no chunks
     int j = grp == 1u ? 1 : 0;
     while (j >= nchunk) {
       j -= nchunk;
@@ -309,7 +316,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
       // segments of the last chunk that lie in K steps past the kernel's last tap are never
       // read by an MMA: nothing to copy, nothing to zero
       const bool dead_seg = j == nchunk - 1 && (int)(seg >> 1) >= last_ksteps;
-      if (has_rows && !dead_seg) {
+      if (!dead_seg) {
         const uint8_t* src = a.in + seg_byte + (RB > kChunk ? (uint32_t)(j % CPT) * kChunk : 0u);
         const uint32_t stage_addr = sR + s * row_stage + dst_base;
 #pragma unroll
@@ -347,7 +354,8 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
     __syncwarp();
     // As one warp: where a launch gives up, some lanes may have left at a stage that came too late for
     // them and others not, and the drain exchanges between all 32.
-    if (__all_sync(0xffffffffu, shared_tail && tile >= ntiles && tiles_done > 0u)) {
+    if (__all_sync(0xffffffffu, shared_tail && (pw_all >> 2) < help_sets && tile >= ntiles &&
+                                    tiles_done > 0u)) {
       drains = true;
       drain_tile = tile - gridDim.x;
       drain_tl = tiles_done - 1u;
@@ -474,7 +482,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
     uint32_t tl = drain_tl;
     for (uint32_t tile = drain_tile; tile < ntiles; tile += gridDim.x, ++tl) {
       const uint32_t buf = tl & 1u;
-      const uint32_t step = shared_tail && tile + gridDim.x >= ntiles ? 6u * 16u : 2u * 16u;
+      const uint32_t step = shared_tail && tile + gridDim.x >= ntiles ? (2u + help_sets) * 16u : 2u * 16u;
       const uint32_t trow0 = tile * tile_rows;
       uint32_t col = 16u * part;  // of the copy
       // the first residual rows are fetched before the accumulator is waited for; after that
