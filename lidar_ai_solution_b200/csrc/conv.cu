@@ -9,7 +9,8 @@ int conv_umma_pack(int compute, int cin, int cout, int kvol, const void* w, void
 int conv_umma_launch(const spconvb_conv_params& p, const void* in, const int32_t* map,
                      uint32_t cap, const uint32_t* n_out_ptr, uint32_t launch_rows,
                      const void* w_packed, const float* scale, const float* bias, void* out,
-                     uint32_t* status, bool rules_ready, cudaStream_t st);
+                     uint32_t* status, bool rules_ready, bool w_replicated,
+                     cudaStream_t st);
 int conv_simt_launch(const spconvb_conv_params& p, const void* in, const int32_t* map,
                      uint32_t cap, const uint32_t* n_out_ptr, uint32_t launch_rows,
                      const void* w_plain, const float* scale, const float* bias, void* out,
@@ -19,7 +20,7 @@ int conv_forward_launch(const spconvb_conv_params* p, const void* in, const int3
                         uint32_t cap, const uint32_t* n_out_ptr, uint32_t launch_rows,
                         const void* w_plain, const void* w_packed, const float* scale,
                         const float* bias, void* out, uint32_t* status, bool rules_ready,
-                        void* stream) {
+                        bool w_replicated, void* stream) {
   if (!p || !in || !map || !n_out_ptr || !out) return SPCONVB_E_ARG;
   if (p->compute != SPCONVB_I8 && p->compute != SPCONVB_F16) return SPCONVB_E_ARG;
   if (p->out_kind != SPCONVB_I8 && p->out_kind != SPCONVB_F16) return SPCONVB_E_ARG;
@@ -30,7 +31,7 @@ int conv_forward_launch(const spconvb_conv_params* p, const void* in, const int3
   if (!p->force_simt && w_packed && p->kvol <= 27 &&
       conv_umma_supported(p->compute, p->cin, p->cout))
     return conv_umma_launch(*p, in, map, cap, n_out_ptr, launch_rows, w_packed, scale, bias, out,
-                            status, rules_ready, st);
+                            status, rules_ready, w_replicated, st);
   return conv_simt_launch(*p, in, map, cap, n_out_ptr, launch_rows, w_plain, scale, bias, out,
                           st);
 }
@@ -60,7 +61,7 @@ int spconvb_conv_forward(const spconvb_conv_params* p, const void* in, const int
                          const float* bias, void* out, uint32_t* status, void* stream) {
   // the launch before this one may be the caller's map, or what it copies the weights with
   return conv_forward_launch(p, in, map, cap, n_out_ptr, launch_rows, w_plain, w_packed, scale,
-                             bias, out, status, false, stream);
+                             bias, out, status, false, false, stream);
 }
 
 const char* spconvb_version(void) { return "spconvb 0.1 (sm_100a)"; }

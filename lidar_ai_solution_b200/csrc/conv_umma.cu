@@ -1,5 +1,9 @@
 // Tensor-core convolution, host side: the supported shapes, the pre-swizzled weight
 // image the kernel streams, argument checks and the launch.
+#include <string.h>
+
+#include <vector>
+
 #include "umma_common.cuh"
 
 namespace spconvb {
@@ -43,10 +47,20 @@ int conv_umma_pack(int compute, int cin, int cout, int kvol, const void* w, void
   return SPCONVB_OK;
 }
 
+std::vector<uint8_t> conv_replicate_weights(const std::vector<uint8_t>& packed, int cout) {
+  const size_t piece = (size_t)cout * kChunk, nchunk = packed.size() / piece;
+  std::vector<uint8_t> out(nchunk * 128 * kChunk);
+  for (size_t j = 0; j < nchunk; ++j)
+    for (int c = 0; c < 128 / cout; ++c)
+      memcpy(out.data() + j * 128 * kChunk + c * piece, packed.data() + j * piece, piece);
+  return out;
+}
+
 int conv_umma_launch(const spconvb_conv_params& p, const void* in, const int32_t* map,
                      uint32_t cap, const uint32_t* n_out_ptr, uint32_t launch_rows,
                      const void* w_packed, const float* scale, const float* bias, void* out,
-                     uint32_t* status, bool rules_ready, cudaStream_t st) {
+                     uint32_t* status, bool rules_ready, bool w_replicated,
+                     cudaStream_t st) {
   if (!w_packed) return SPCONVB_E_ARG;
   if (p.kvol > kMaxTaps) return SPCONVB_E_UNSUPPORTED;
   if (p.compute == SPCONVB_I8 && !scale) return SPCONVB_E_ARG;
@@ -65,6 +79,7 @@ int conv_umma_launch(const spconvb_conv_params& p, const void* in, const int32_t
   a.status = status;
   a.kvol = p.kvol;
   a.rules_ready = rules_ready ? 1 : 0;
+  a.w_replicated = w_replicated ? 1 : 0;
   a.wait_test = p.wait_test;
   const int rb = row_bytes(p.compute, p.cin);
   a.ep = make_epilogue(p);

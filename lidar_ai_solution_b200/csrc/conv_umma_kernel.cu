@@ -186,7 +186,13 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
   // Two rings share the buffer: row stages as high as this launch's tile, and weight stages.
   // Low tiles get deeper rings: as many of both as fit, and what is left over goes to the rows.
   const uint32_t row_stage = tile_rows * kChunk;
-  const uint32_t nwst = min((uint32_t)kMaxStages, kRingBytes / (kWeightBytes + row_stage));
+  // Weights of which all chunks fit stay where they are after the first tile (a chunk in its own
+  // stage): int8 16 -> 16, four chunks, 120 000 rows 16.1 / 14.9 us, with the copies above.  There are
+  // never more weight stages than row stages: a chunk's weights are signed for on its row stage's
+  // barrier as soon as their own stage is free, so a longer ring would sign a phase twice.
+  const uint32_t fit = min((uint32_t)kMaxStages, kRingBytes / (kWeightBytes + row_stage));
+  const bool resident = (uint32_t)nchunk <= fit;
+  const uint32_t nwst = resident ? (uint32_t)nchunk : fit;
   const uint32_t nst = min((uint32_t)kMaxStages, (kRingBytes - nwst * kWeightBytes) / row_stage);
   const uint32_t sW = smem_u32(smem), sR = sW + nwst * kWeightBytes;
   // Only the producers that own rows of the tile take part, two groups of t32 warps.  (Warps that
@@ -222,7 +228,8 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
       uint32_t os = 0, oph = 0;  // row stage and phase of the chunk `nwst` before
       uint32_t it = 0;
       bool alive = true;
-      for (uint32_t tile = blockIdx.x; tile < ntiles && alive; tile += gridDim.x)
+      for (uint32_t tile = blockIdx.x; tile < ntiles && alive && !(resident && it > 0u);
+           tile += gridDim.x)
         for (int j = 0; j < nchunk; ++j, ++it) {
           if (it >= nwst) {
             // spinning: one lane, and every chunk waits for it (a launch of 4 736 rows 0.2 us less)
@@ -236,10 +243,19 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
             }
           }
           mbar_expect_tx(bar_full + 8 * s, kWeightBytes);
+          // A bulk copy takes about 70 cycles of issue whatever its size (eight of 2 KB a chunk
+          // instead of one of 16 KB: fp16 128 -> 128 of 4 700 rows 15.6 / 28.9 us), so the copies of
+          // narrow weights are made in global memory where the caller can hold them: fp16 16 -> 16 of
+          // 120 000 rows 20.4 / 19.2 us, 32 -> 32 29.7 / 26.7.
+          const uint32_t dst = sW + ws * kWeightBytes;
+          if (kRep > 1 && a.w_replicated) {
+            bulk_g2s(dst, a.wpk + (size_t)j * kWeightBytes, kWeightBytes, bar_full + 8 * s);
+          } else {
 #pragma unroll
-          for (uint32_t c = 0; c < kRep; ++c)
-            bulk_g2s(sW + ws * kWeightBytes + c * (COUT * kChunk),
-                     a.wpk + (size_t)j * (COUT * kChunk), COUT * kChunk, bar_full + 8 * s);
+            for (uint32_t c = 0; c < kRep; ++c)
+              bulk_g2s(dst + c * (COUT * kChunk), a.wpk + (size_t)j * (COUT * kChunk), COUT * kChunk,
+                       bar_full + 8 * s);
+          }
           if (++s == nst) s = 0;
           if (++ws == nwst) ws = 0;
         }
@@ -306,6 +322,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
     uint32_t ntile = tile;  // the chunk whose indices are loaded next
     int nj = j;
     uint32_t it = grp, s = grp % nst, ph = (grp / nst) & 1u;
+    const uint32_t first_thread = 32u * (kProdWarp0 + grp * t32);  // of this group
     // One chunk: its rows go from the indices in `idx` into the stage, and `idx` is then
     // refilled for the chunk after next.  Two register sets take turns and are never copied,
     // so the load has a whole chunk of the group's time to arrive.
@@ -328,6 +345,8 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
       }
       if (!(a.wait_test > 0 && it + 1u >= (uint32_t)a.wait_test))
         cp_async_arrive_noinc(bar_full + 8 * s);
+      // the weights' arrival, where they are there already
+      if (resident && tile != blockIdx.x && threadIdx.x == first_thread) mbar_arrive(bar_full + 8 * s);
       load_idx(ntile, nj, idx);
       advance2(ntile, nj);
       const uint32_t was = tile;

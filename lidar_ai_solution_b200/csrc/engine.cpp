@@ -445,6 +445,7 @@ int Engine::compile(const Builder& b, int precision, uint32_t build_flags, cudaS
           if (umma) {
             std::vector<uint8_t> packed(spconvb_conv_packed_bytes(compute, cpad, n.cout, kvol));
             rc = spconvb_conv_pack_weights(compute, cpad, n.cout, kvol, plain.data(), packed.data());
+            packed = conv_replicate_weights(packed, n.cout);
             if (rc == SPCONVB_OK) rc = upload(&lw.packed, packed.data(), packed.size());
           } else {
             rc = upload(&lw.plain, plain.data(), plain.size());
@@ -1107,7 +1108,7 @@ int Engine::forward(const void* features, const int32_t* indices, uint32_t cap_r
         p.res = s.in1 >= 0 ? rt[s.in1].data : nullptr;
         rc = conv_forward_launch(&p, rt[s.in0].data, R.map, coordsets[R.out_cs].cap,
                                  cs_n(R.out_cs), cs_launch(R.out_cs), w.plain, w.packed, w.scale,
-                                 w.bias, rt[s.out].data, status, rules_ready, st);
+                                 w.bias, rt[s.out].data, status, rules_ready, true, st);
         last_launches += 1;
         break;
       }

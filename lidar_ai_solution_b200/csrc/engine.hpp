@@ -18,13 +18,17 @@ namespace spconvb {
 void log_msg(int level, const char* fmt, ...);
 enum { LOG_VERB = 0, LOG_WARN = 1, LOG_ERROR = 2 };
 
-// spconvb_conv_forward; rules_ready: the map, the row count and the weights are older than the last
-// launch on the stream, so the kernel may read them while that launch is still running
+// spconvb_conv_forward.  rules_ready: the map, the row count and the weights are older than the last
+// launch on the stream, so the kernel may read them while that launch is still running.
+// w_replicated: `w_packed` is what conv_replicate_weights() makes of the packed image.
 int conv_forward_launch(const spconvb_conv_params* p, const void* in, const int32_t* map,
                         uint32_t cap, const uint32_t* n_out_ptr, uint32_t launch_rows,
                         const void* w_plain, const void* w_packed, const float* scale,
                         const float* bias, void* out, uint32_t* status, bool rules_ready,
-                        void* stream);
+                        bool w_replicated, void* stream);
+// The packed image with the rows of every chunk repeated to 128, as the kernel keeps them in shared
+// memory: one bulk copy a chunk.
+std::vector<uint8_t> conv_replicate_weights(const std::vector<uint8_t>& packed, int cout);
 int launch_set_count(uint32_t* dst, uint32_t value, cudaStream_t st);
 int launch_clamp_count(uint32_t* dst, const uint32_t* src, uint32_t cap, uint32_t* status,
                        cudaStream_t st);

@@ -25,6 +25,7 @@ struct UmmaArgs {
   uint8_t* out;
   uint32_t* status;
   int kvol;
+  int w_replicated;   // wpk holds 128 rows a chunk, not Cout (conv_replicate_weights)
   int rules_ready;    // the map and *n_out_ptr are older than the launch before this one (pdl.cuh)
   uint32_t grid_inv;  // about 2^32 / thread blocks of the launch
   int wait_test;   // > 0: producers withhold "stage full" from this chunk on (self-test)
