@@ -298,20 +298,15 @@ __device__ __forceinline__ void task_mark_rows(const RuleTask& t, uint32_t first
   }
 }
 
-// Up to 64 bits of a bitmap starting at cell `line + x0` of a line of `gx` cells that starts
-// at linear cell `line`: bit i of the result is cell x0 + i, zero outside the line.
+// 64 bits of a bitmap from cell `start` on, zero beyond its words (there is no cell 0xffffffff).
 __device__ __forceinline__ unsigned long long line_bits64(const uint32_t* __restrict__ bitmap,
-                                                          uint32_t words, uint32_t line, int x0,
-                                                          int count, int gx) {
-  const int lo = max(x0, 0), hi = min(x0 + count - 1, gx - 1);
-  if (lo > hi) return 0ull;
-  const uint32_t start = line + (uint32_t)lo, w = start >> 5, off = start & 31u;
-  unsigned long long v = (unsigned long long)__ldg(bitmap + w) >> off;
-  if (w + 1 < words) v |= (unsigned long long)__ldg(bitmap + w + 1) << (32u - off);
-  if (off && w + 2 < words) v |= (unsigned long long)__ldg(bitmap + w + 2) << (64u - off);
-  const int nb = hi - lo + 1;
-  if (nb < 64) v &= (1ull << nb) - 1ull;
-  return v << (lo - x0);
+                                                          uint32_t words, uint32_t start) {
+  const uint32_t w = start >> 5, off = start & 31u;
+  const uint32_t a = w < words ? __ldg(bitmap + w) : 0u;
+  const uint32_t b = w + 1 < words ? __ldg(bitmap + w + 1) : 0u;
+  const uint32_t c = w + 2 < words ? __ldg(bitmap + w + 2) : 0u;
+  const uint32_t low = __funnelshift_r(a, b, off), high = __funnelshift_r(b, c, off);
+  return (unsigned long long)high << 32 | low;
 }
 
 // The mark step when the input rows were made by a strided rulebook themselves: the output
@@ -341,18 +336,29 @@ __device__ __forceinline__ void task_mark_bitmap(const RuleTask& t, uint32_t fir
     const int o0 = (int)(plane - (uint32_t)b * (uint32_t)gout.g[0]);
     const int x0 = ox0 * kr.s[2] - kr.p[2];
     const int count = (ncell - 1) * kr.s[2] + kr.k[2];  // <= 64 (mark_from_bitmap)
+    const int lo = max(x0, 0), hi = min(x0 + count - 1, gin.g[2] - 1);
+    if (lo > hi) continue;
     unsigned long long win = 0ull;
     for (int k0 = 0; k0 < kr.k[0]; ++k0) {
       const int i0 = o0 * kr.s[0] - kr.p[0] + k0;
       if ((unsigned)i0 >= (unsigned)gin.g[0]) continue;
-#pragma unroll 3
-      for (int k1 = 0; k1 < kr.k[1]; ++k1) {
-        const int i1 = o1 * kr.s[1] - kr.p[1] + k1;
-        if ((unsigned)i1 >= (unsigned)gin.g[1]) continue;
-        win |= line_bits64(t.in_ws.bitmap, t.in_ws.words, voxel_key(b, i0, i1, 0, gin), x0,
-                           count, gin.g[2]);
+      for (int k1 = 0; k1 < kr.k[1]; k1 += 3) {
+        // Three lines at once, without branches: nine loads in flight.  (A line after the other, each
+        // behind its tests: 10 800 voxels 221.5 us the whole call, this way 216.8; BEVFusion's frame 261,
+        // 258.)
+        unsigned long long v[3];
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+          const int i1 = o1 * kr.s[1] - kr.p[1] + k1 + q;
+          const bool in = k1 + q < kr.k[1] && (unsigned)i1 < (unsigned)gin.g[1];
+          v[q] = line_bits64(t.in_ws.bitmap, t.in_ws.words,
+                             in ? voxel_key(b, i0, i1, lo, gin) : 0xffffffffu);
+        }
+        win |= v[0] | v[1] | v[2];
       }
     }
+    if (hi - lo < 63) win &= (1ull << (hi - lo + 1)) - 1ull;
+    win <<= lo - x0;
     if (!win) continue;
     uint32_t r = 0;
 #pragma unroll
