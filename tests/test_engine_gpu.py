@@ -336,6 +336,36 @@ def test_auxiliary_stream_changes_no_result():
         assert np.array_equal(fast.output(0).cpu().numpy().view(np.uint16), want.view(np.uint16))
 
 
+@pytest.mark.parametrize("flags", [0, "BUILD_SINGLE_STREAM"])
+@pytest.mark.parametrize("kind", ["centerpoint", "bevfusion"])
+def test_frames_queued_back_to_back(kind, flags):
+    """A convolution fetches its row count, first neighbour indices and weights while the launch before
+    it is running.  Frames of other sizes (one row, a lone tile, several) queued without a wait on one
+    engine give the bits that the same frames give one at a time."""
+    eng = _engine_mod()
+    flags = getattr(eng, flags) if flags else 0
+    frames = [[_dev(a) for a in _frame(n, seed=s)] for n, s in ((12000, 1), (1, 2), (33, 3), (20000, 4), (257, 5))]
+    model = _quantized(kind, *_frame(9000, seed=9)) if kind == "centerpoint" else _small_model(kind, 0)
+    precision = eng.PRECISION_INT8 if kind == "centerpoint" else eng.PRECISION_FP16
+    alone = eng.Engine.from_model(model, precision, flags)
+    want = []
+    for feats, coords in frames:
+        alone.forward(feats, coords, GRID)
+        torch.cuda.synchronize()
+        assert alone.status()[0] == 0
+        want.append(alone.output(0).clone())
+    queued = eng.Engine.from_model(model, precision, flags)
+    got = []
+    for _ in range(3):
+        for feats, coords in frames:
+            queued.forward(feats, coords, GRID)
+            got.append(queued.output(0).clone())
+    torch.cuda.synchronize()
+    assert queued.status()[0] == 0
+    for i, g in enumerate(got):
+        assert torch.equal(g.view(torch.int16), want[i % len(frames)].view(torch.int16)), i
+
+
 @pytest.mark.parametrize("single_stream", [False, True])
 def test_many_rulebooks_on_one_level(single_stream):
     """More independent rulebooks than one launch of rulebook tasks holds: ten strided convolutions
