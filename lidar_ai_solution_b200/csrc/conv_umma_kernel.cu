@@ -23,8 +23,8 @@
 //               64 -> 64 with a residual 51.8 us, this way 45.9.)
 //   warp  8     allocates TMEM; walks the chunks converged, one elected lane issues
 //               tcgen05.mma (kind::i8 with int32 accumulators or kind::f16 with fp32)
-//   warps 9-24  producers, two groups of 8 warps that take the chunks in turn (the
-//               work of a warp per chunk is a chain of dependent steps - wait for
+//   warps 9-24  producers, two groups of as many warps as the tile has 32 rows that take
+//               the chunks in turn (the work of a warp per chunk is a chain of dependent steps - wait for
 //               the stage, neighbour indices, addresses, copies, arrival - that
 //               takes longer than the tensor pipe needs for the chunk; two groups
 //               give each warp two chunk periods for it).  Within a group each warp
@@ -37,7 +37,7 @@
 //               them arrive on the stage's mbarrier when they land, so all free
 //               stages of the ring are in flight.
 //   warp  25    streams the pre-swizzled weight chunks with bulk async copies into a
-//               ring of their own
+//               ring of their own, or keeps all of them there
 //
 // What bounds it.  The round trip of a stage - freed, gathered (a cp.async takes about a
 // microsecond under load), multiplied, freed - over the number of stages in flight, not a
@@ -48,6 +48,10 @@
 // rows and 4 of weights; 160 rows: 6 and 6), and no work beside the MMAs in the issuing warp.
 // Measured with both, int8, us: 208 071 rows 64 -> 64 49.2 to 41.3, 128 -> 128 86.9 to 69.3
 // (730 cycles a chunk), fp16 181.6 to 158.1; 30 000 rows 128 -> 128 18.9 to 16.4.
+//
+// On low tiles the issuing warp is what a chunk waits for: 32-row tiles, 128 channels, 412 cycles a
+// chunk in it, of which 74 are its look at the stage's barrier; 628 and 121 on 224 rows, where the
+// MMAs fill the rest (clock counts of one CTA).
 //
 // K is walked in chunks of 128 bytes (one swizzle atom per row): a chunk is 8
 // taps of a 16-byte row, ..., 1 tap of a 128-byte row, or half a 256-byte row.
@@ -263,7 +267,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
     __syncwarp();
   } else if (is_producer) {
     // ------------------------------------------------------------ producers
-    // Two groups of 8 warps take the chunks in turn (group g the chunks g, g + 2, ...), so a
+    // Two groups of t32 warps take the chunks in turn (group g the chunks g, g + 2, ...), so a
     // warp has two chunk periods for the round trip of one chunk: wait for the stage, look
     // up the neighbours, issue the copies.  Within a group, warp w owns rows 32w..32w+31 of
     // the tile.  A chunk of the row tile is 256 rows x 8 segments of 16 bytes = 2048 copies,
