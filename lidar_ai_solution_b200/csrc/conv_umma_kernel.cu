@@ -385,7 +385,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
     }
   } else if (warp == kMmaWarp) {
     // ------------------------------------------------------------ MMA issue
-    // The whole warp walks the chunks and one elected lane issues: the loop's values stay
+    // The whole warp walks the chunks and one elected lane issues, by predicate: the loop's values stay
     // warp-uniform, so an MMA costs its own time (measured in isolation, M = 128, N = 256: 513
     // cycles per chunk against 583 when a single lane runs the loop, whose descriptors are moved
     // to uniform registers one MMA after the other).
@@ -421,6 +421,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
     bool alive = true;
     auto stage_full = [&]() {
       alive = alive && (mbar_test_wait(bar, ph) || mbar_wait_spin(bar, ph, abort_flag, a.status, 3u));
+      __syncwarp();  // (a wait that runs out may part them)
     };
     // The loop is entered with the current chunk's stage known to be full.
     if (blockIdx.x < ntiles) stage_full();
@@ -435,29 +436,25 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
       uint32_t accumulate = 0u;
 #pragma unroll 1
       for (int j = nchunk - 1; j > 0; --j) {
-        if (leader && alive) {
-          fence_proxy_async();
-          umma_lohi<INT8>(d_tmem, wd, rd, desc_hi, idesc, accumulate);
-          umma_lohi<INT8>(d_tmem, wd + 2u, rd + 2u, desc_hi, idesc, 1u);
-          umma_lohi<INT8>(d_tmem, wd + 4u, rd + 4u, desc_hi, idesc, 1u);
-          umma_lohi<INT8>(d_tmem, wd + 6u, rd + 6u, desc_hi, idesc, 1u);
-          tc_commit(bar + kToEmpty);
-        }
-        __syncwarp();
+        const uint32_t issue = leader && alive ? 1u : 0u;
+        fence_proxy_async();
+        umma_if<INT8>(issue, d_tmem, wd, rd, desc_hi, idesc, accumulate);
+        umma_if<INT8>(issue, d_tmem, wd + 2u, rd + 2u, desc_hi, idesc, 1u);
+        umma_if<INT8>(issue, d_tmem, wd + 4u, rd + 4u, desc_hi, idesc, 1u);
+        umma_if<INT8>(issue, d_tmem, wd + 6u, rd + 6u, desc_hi, idesc, 1u);
+        tc_commit_if(issue, bar + kToEmpty);
         accumulate = 1u;
         next_stage();
         stage_full();
       }
-      if (leader && alive) {
-        fence_proxy_async();
-        for (int ks = 0; ks < last_ksteps; ++ks) {
-          umma_lohi<INT8>(d_tmem, wd + 2u * ks, rd + 2u * ks, desc_hi, idesc, accumulate);
-          accumulate = 1u;
-        }
-        tc_commit(bar + kToEmpty);
-        tc_commit(bar_tfull + 8 * buf);
+      const uint32_t issue = leader && alive ? 1u : 0u;
+      fence_proxy_async();
+      for (int ks = 0; ks < last_ksteps; ++ks) {
+        umma_if<INT8>(issue, d_tmem, wd + 2u * ks, rd + 2u * ks, desc_hi, idesc, accumulate);
+        accumulate = 1u;
       }
-      __syncwarp();
+      tc_commit_if(issue, bar + kToEmpty);
+      tc_commit_if(issue, bar_tfull + 8 * buf);
       next_stage();
       if (tile + gridDim.x < ntiles) stage_full();
     }
