@@ -1014,8 +1014,9 @@ int Engine::forward(const void* features, const int32_t* indices, uint32_t cap_r
   // (the convert step that a wave does in its place takes no empty buffer either)
   if (pad_step_ >= 0 && n_dev && cap_rows == 0) return SPCONVB_E_ARG;
   last_launches = 0;
-  // Where the host knows the rows their table takes eight slots a row, not what the model's bound
-  // would: less to clear and closer together (10 800 voxels of 200 000: 1 MB for 8).
+  // Where the host knows the rows their table takes eight slots a row where the model's bound gives
+  // that many, not what the bound would: less to clear and closer together (10 800 voxels of 200 000:
+  // 1 MB for 8).  Eight hold for any rows: a probe may go on to every slot (common.cuh).
   uint32_t in_slots = in.slots;
   size_t clear_bytes = zero_bytes_;
   if (in.need_table && !n_dev && !prof) {

@@ -366,6 +366,45 @@ def test_frames_queued_back_to_back(kind, flags):
         assert torch.equal(g.view(torch.int16), want[i % len(frames)].view(torch.int16)), i
 
 
+def _forward_us(e, feats, coords, grid):
+    """Shortest of five forwards, device time."""
+    best = float("inf")
+    for _ in range(6):  # the first one warms up
+        t0, t1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        t0.record()
+        e.forward(feats, coords, grid)
+        t1.record()
+        torch.cuda.synchronize()
+        best = min(best, t0.elapsed_time(t1) * 1e3)
+    return best
+
+
+@pytest.mark.parametrize("n", [1024, 16000, 16384])
+def test_rows_of_one_plane_cost_what_spread_rows_do(n):
+    """With a row count the host knows the table has eight slots a row.  Rows that all have the same
+    position in their runs of eight along x (a plane) get the same map in about the same time as rows
+    all over the grid.  (When a collision kept the position, a row had an eighth of the table: full at
+    16 384 rows, so every lookup of an absent neighbour went through all of it.)"""
+    eng = _engine_mod()
+    grid = (64, 360, 360)
+    model = models.single_layer(5, 16, seed=5, output_bound=200000)
+    e = eng.Engine.from_model(model, eng.PRECISION_FP16, 0)
+    spread = scenes.make_coords(n, grid, 7)
+    cells = np.random.default_rng(7).choice(64 * 360, n, replace=False)
+    plane = np.zeros((n, 4), np.int32)
+    plane[:, 1], plane[:, 2], plane[:, 3] = cells // 360, cells % 360, 203
+    us = []
+    for coords in (spread, plane):
+        feats = _dev(scenes.make_point_features(coords, 7))
+        us.append(_forward_us(e, feats, _dev(coords), grid))
+        assert e.status()[0] == 0
+        m, n_out, _ = e.rules()[0]
+        assert n_out == n
+        assert np.array_equal(m[:, :n].cpu().numpy(), orc.subm_map(coords, grid)[0])
+    # a probe or two a lookup in both (1.2 and 1.4 on average); without it two orders of magnitude
+    assert us[1] < 3 * us[0], us
+
+
 @pytest.mark.parametrize("single_stream", [False, True])
 def test_many_rulebooks_on_one_level(single_stream):
     """More independent rulebooks than one launch of rulebook tasks holds: ten strided convolutions

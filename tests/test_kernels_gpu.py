@@ -84,6 +84,30 @@ def test_subm_map_capacity_larger_than_rows():
     assert np.array_equal(m.cpu().numpy(), ref)
 
 
+@pytest.mark.parametrize("x_step", [0, 8])
+@pytest.mark.parametrize("n,slots", [(4, 8), (8, 16), (128, 256), (4000, 8192), (14000, 32768)])
+def test_subm_map_of_rows_that_share_a_place_in_their_runs(n, slots, x_step):
+    """Cells in one x plane, or every eighth: all have the same position in their aligned runs of eight
+    along x.  They are found like any others, in the smallest table the rows may have."""
+    ops = _ops()
+    from lidar_ai_solution_b200 import cabi
+    grid = (41, 360, 360)
+    rng = np.random.default_rng(n)
+    cells = rng.choice(41 * 360 * (45 if x_step else 1), n, replace=False)
+    coords = np.zeros((n, 4), np.int32)
+    coords[:, 1], coords[:, 2] = cells % 41, cells // 41 % 360
+    coords[:, 3] = 5 + x_step * (cells // (41 * 360)) if x_step else 203
+    ref, _ = orc.subm_map(coords, grid)
+    dc, n_ptr, st = _dev(coords), ops.device_count(n), ops.new_status()
+    table = torch.empty(slots, dtype=torch.int64, device="cuda")
+    cabi.check(cabi.lib().spconvb_hash_build(dc.data_ptr(), n_ptr.data_ptr(), n, 0, cabi.i3(grid), 1,
+                                             table.data_ptr(), slots, 0, st.data_ptr(), ops._stream()))
+    m = ops.subm_map(dc, n_ptr, grid, table, status=st)
+    torch.cuda.synchronize()
+    _status_ok(st)
+    assert np.array_equal(m.cpu().numpy(), ref)
+
+
 def test_hash_reports_duplicates_and_range():
     ops = _ops()
     grid = (8, 8, 8)
