@@ -382,7 +382,7 @@ __global__ void __launch_bounds__(kRankThreads) cp_rank_kernel(const PostArgs a)
   __shared__ uint32_t s_need, s_list, s_own;
   pdl_wait();
 
-  const uint32_t n = min(load_after_wait(b.n_cand), (uint32_t)HW);
+  const uint32_t n = min(load_in_order(b.n_cand), (uint32_t)HW);
   const uint32_t K = min(n, (uint32_t)a.p.max_det);
   if (part == 0 && tid == 0) *b.n_det = K;
   if (tid == 0) { s_list = 0u; s_own = 0u; s_need = 0u; }
@@ -779,7 +779,7 @@ __global__ void __launch_bounds__(kMaskThreads) cp_mask_kernel(const PostArgs a)
   __shared__ uint32_t queued;
   __shared__ bool s_last;
   pdl_wait();
-  const int m = (int)load_after_wait(b.n_det);
+  const int m = (int)load_in_order(b.n_det);
   const float threshold = a.p.nms_iou_threshold;
   // tiles on or below the diagonal: 4 row groups of 16 in block row G, G + 1 tiles each
   const int groups = (m + kMaskRows - 1) / kMaskRows, whole = groups / 4;

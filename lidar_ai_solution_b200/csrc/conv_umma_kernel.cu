@@ -97,22 +97,24 @@ __device__ __forceinline__ constexpr uint32_t make_idesc() {
   return INT8 ? ((2u << 4) | (1u << 7) | (1u << 10)) : (1u << 4);
 }
 
-// Bytes or halves of 16 rows of one channel, `pitch` bytes apart; `n` rows exist.
+// Bytes or halves of 16 rows of one channel, `pitch` bytes apart; `n` rows exist.  The residual may be
+// the output of the launch directly before, and neither its address nor the row count says so: both may
+// be known before that launch is over.
 template <bool I8>
 __device__ __forceinline__ void load_rows16(const uint8_t* p, uint32_t pitch, uint32_t n,
                                             int32_t (&v)[16]) {
   if (n >= 16u) {
 #pragma unroll
     for (uint32_t i = 0; i < 16; ++i)
-      v[i] = I8 ? (int32_t)__ldg((const int8_t*)(p + i * pitch))
-                : (int32_t)__ldg((const uint16_t*)(p + i * pitch));
+      v[i] = I8 ? load_in_order((const int8_t*)(p + i * pitch))
+                : load_in_order((const uint16_t*)(p + i * pitch));
   } else {
 #pragma unroll
     for (uint32_t i = 0; i < 16; ++i) {
       v[i] = 0;
       if (i < n)
-        v[i] = I8 ? (int32_t)__ldg((const int8_t*)(p + i * pitch))
-                  : (int32_t)__ldg((const uint16_t*)(p + i * pitch));
+        v[i] = I8 ? load_in_order((const int8_t*)(p + i * pitch))
+                  : load_in_order((const uint16_t*)(p + i * pitch));
     }
   }
 }
@@ -152,7 +154,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
     pdl_wait();
     pdl_trigger();
   }
-  const uint32_t n_out = min(load_after_wait(a.n_out_ptr), a.cap);
+  const uint32_t n_out = min(load_in_order(a.n_out_ptr), a.cap);
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kMaxStages; ++s) {

@@ -195,7 +195,7 @@ __global__ void __launch_bounds__(256)
   pdl_wait();
   const int gp[3] = {g.g[p0], g.g[p1], g.g[p2]};
   const size_t vol = (size_t)gp[0] * gp[1] * gp[2];
-  const uint32_t rows = min(load_after_wait(n_ptr), cap);
+  const uint32_t rows = min(load_in_order(n_ptr), cap);
   const uint32_t cells = RANKED ? (uint32_t)vol * g.batch : 0u;
   const bool by_cell = RANKED && cells <= (unsigned long long)rows * channels / 4;
   const uint32_t n = by_cell ? cells : rows;

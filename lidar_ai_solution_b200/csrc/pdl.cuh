@@ -19,11 +19,24 @@ __device__ __forceinline__ void pdl_trigger() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
-// A word an earlier kernel wrote.  Volatile: stays behind pdl_wait(), whatever the compiler knows
-// about the pointer.  (Loads that depend on its value stay behind it with it.)
-__device__ __forceinline__ uint32_t load_after_wait(const uint32_t* p) {
+// What an earlier kernel wrote, read where the source reads it: volatile, and through the coherent path.
+// The compiler takes what __ldg() reads for constant while the kernel runs and may move such a load to
+// before pdl_wait(), unless it depends on a value that load_in_order() reads behind the wait.  So
+// whatever the launch directly before may have written is read with these; __ldg() is for what is older,
+// or hangs on a row count read behind the wait.
+__device__ __forceinline__ uint32_t load_in_order(const uint32_t* p) {
   uint32_t v;
   asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ int32_t load_in_order(const int8_t* p) {
+  int32_t v;
+  asm volatile("ld.global.s8 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ int32_t load_in_order(const uint16_t* p) {
+  int32_t v;
+  asm volatile("ld.global.u16 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
 

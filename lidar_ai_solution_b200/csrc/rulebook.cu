@@ -26,7 +26,7 @@ constexpr int kTaskWarps = kTaskThreads / 32;
 constexpr uint32_t kScanWords = kTaskThreads;  // bitmap words per scan block: one a thread
 
 __device__ __forceinline__ uint32_t task_rows(const RuleTask& t) {
-  return min(t.n_ptr ? load_after_wait(t.n_ptr) : t.n_host, t.cap);
+  return min(t.n_ptr ? load_in_order(t.n_ptr) : t.n_host, t.cap);
 }
 
 // v % s == 0 and v / s for v >= 0, without the integer division when the stride is a power
@@ -47,7 +47,7 @@ __host__ __device__ inline bool is_k333(const Kernel3& kr) {
 // ---------------------------------------------------------------- the caller's rows
 __device__ __forceinline__ void task_count(const RuleTask& t) {
   if (threadIdx.x != 0) return;
-  const uint32_t n = t.n_ptr ? load_after_wait(t.n_ptr) : t.n_host;
+  const uint32_t n = t.n_ptr ? load_in_order(t.n_ptr) : t.n_host;
   if (n > t.cap) set_status(t.status, SPCONVB_ST_OVERFLOW, n);
   *t.n_out = min(n, t.cap);
 }

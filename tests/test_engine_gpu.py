@@ -366,6 +366,53 @@ def test_frames_queued_back_to_back(kind, flags):
         assert torch.equal(g.view(torch.int16), want[i % len(frames)].view(torch.int16)), i
 
 
+@pytest.mark.parametrize("precision", ["int8", "fp16"])
+def test_residual_made_by_the_launch_directly_before(precision):
+    """conv3 adds the output of conv2, the launch before it, to its result: its row count and indices are
+    read while conv2 is running, the residual must not be.  Frames of other contents and sizes are queued
+    without a wait, so that a value read too early is another frame's."""
+    eng = _engine_mod()
+    rng = np.random.default_rng(3)
+    ids, nodes, counter, c = models._Ids(), [], [0, 0], 32
+
+    def conv(x, cin, act):
+        return models._conv(ids, rng, nodes, x, cin, c, (3, 3, 3), (1, 1, 1), (1, 1, 1), True, "subm0", act,
+                            counter, 40000)
+
+    x0 = conv("0", 16, "ReLU")
+    main, skip = conv(x0, c, "ReLU"), conv(x0, c, "None")
+    y = conv(main, c, "None")
+    nodes.append({"op": "add", "name": "add0", "a": y, "b": skip, "out": ids.new()})
+    nodes.append({"op": "relu", "name": "relu0", "x": nodes[-1]["out"], "out": ids.new()})
+    model = {"kind": "layer", "inputs": [("0", [1, 16])], "outputs": [(nodes[-1]["out"], [1, c])],
+             "nodes": nodes, "roles": {"conv_input": [0]}, "in_channels": 16}
+    frames = []
+    for i, n in enumerate((40000, 39000, 900, 20000, 33)):
+        coords = scenes.make_coords(n, GRID, 20 + i)
+        frames.append((rng.standard_normal((n, 16)).astype(np.float16), coords))
+    if precision == "int8":
+        model = models.quantize(model, eng.calibrate(model, _dev(frames[0][0]), _dev(frames[0][1]), GRID))
+    want = [graph_oracle.run(model, f, c, GRID, precision)[0][0] for f, c in frames]
+    e = eng.Engine.from_model(model, getattr(eng, "PRECISION_" + precision.upper()), 0)
+    convs = [ln for ln in e.describe().split("\n") if ln.startswith(("conv ", "add "))]
+    assert [ln.split()[1] for ln in convs] == ["conv0", "conv1", "conv2", "conv3+add0"]
+    dev = [(_dev(f), _dev(c)) for f, c in frames]
+    got = []
+    for _ in range(3):
+        for f, c in dev:
+            e.forward(f, c, GRID)
+            got.append(e.output(0)[:len(f)].clone())
+    torch.cuda.synchronize()
+    assert e.status()[0] == 0
+    for i, g in enumerate(got):
+        ref, g = want[i % len(frames)], g.cpu().numpy()
+        if precision == "int8":
+            assert np.array_equal(g.view(np.uint8), ref.view(np.uint8)), i
+        else:
+            ref = ref.astype(np.float32)
+            assert float(np.abs(g.astype(np.float32) - ref).max()) <= 1e-2 * float(np.abs(ref).max()), i
+
+
 def _forward_us(e, feats, coords, grid):
     """Shortest of five forwards, device time."""
     best = float("inf")

@@ -79,6 +79,22 @@ def test_argument_checks_come_before_any_device_work():
     assert lib.spconvb_convert(fake, cabi.F16, 5, cabi.F16, 4, 1.0, fake, 100, fake, None) == -1
 
 
+def _source(name):
+    with open(os.path.join(ROOT, "lidar_ai_solution_b200", "csrc", name)) as f:
+        return f.read()
+
+
+def test_residual_rows_are_not_read_as_constants():
+    """A convolution starts while the launch before it is running and may know its row count by then;
+    the residual may be that launch's output, so no load of it may be one that the compiler can move to
+    before the wait."""
+    src = _source("conv_umma_kernel.cu")
+    body = src[src.index("void load_rows16("):src.index("conv_umma_kernel(const UmmaArgs a)")]
+    assert "load_in_order(" in body and "__ldg" not in body
+    loads = re.findall(r"ld\.global\S*", _source("pdl.cuh"))
+    assert loads and not [ld for ld in loads if ".nc" in ld]
+
+
 def test_triples_are_made_anew_from_any_numbers():
     """Whatever int() takes is a triple's number, hashable or not; every call's array is its own."""
     cabi, _ = _lib()
