@@ -232,39 +232,44 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
     if (lane == 0) {
       uint32_t s = 0, ws = 0;    // row stage (whose barrier the copy signs), weight stage
       uint32_t os = 0, oph = 0;  // row stage and phase of the chunk `nwst` before
-      uint32_t it = 0;
-      bool alive = true;
-      for (uint32_t tile = blockIdx.x; tile < ntiles && alive && !(resident && it > 0u);
-           tile += gridDim.x)
-        for (int j = 0; j < nchunk; ++j, ++it) {
-          if (it >= nwst) {
-            // spinning: one lane, and every chunk waits for it (a launch of 4 736 rows 0.2 us less)
-            if (!mbar_wait_spin(bar_empty + 8 * os, oph, abort_flag, a.status, 6u)) {
-              alive = false;
-              break;
-            }
-            if (++os == nst) {
-              os = 0;
-              oph ^= 1u;
-            }
-          }
-          mbar_expect_tx(bar_full + 8 * s, kWeightBytes);
-          // A bulk copy takes about 70 cycles of issue whatever its size (eight of 2 KB a chunk
-          // instead of one of 16 KB: fp16 128 -> 128 of 4 700 rows 15.6 / 28.9 us), so the copies of
-          // narrow weights are made in global memory where the caller can hold them: fp16 16 -> 16 of
-          // 120 000 rows 20.4 / 19.2 us, 32 -> 32 29.7 / 26.7.
-          const uint32_t dst = sW + ws * kWeightBytes;
-          if (kRep > 1 && a.w_replicated) {
-            bulk_g2s(dst, a.wpk + (size_t)j * kWeightBytes, kWeightBytes, bar_full + 8 * s);
-          } else {
+      uint32_t tile = blockIdx.x;
+      int j = 0;
+      auto fetch = [&]() {
+        mbar_expect_tx(bar_full + 8 * s, kWeightBytes);
+        // A bulk copy takes about 70 cycles of issue whatever its size (eight of 2 KB a chunk
+        // instead of one of 16 KB: fp16 128 -> 128 of 4 700 rows 15.6 / 28.9 us), so the copies of
+        // narrow weights are made in global memory where the caller can hold them: fp16 16 -> 16 of
+        // 120 000 rows 20.4 / 19.2 us, 32 -> 32 29.7 / 26.7.
+        const uint32_t dst = sW + ws * kWeightBytes;
+        if (kRep > 1 && a.w_replicated) {
+          bulk_g2s(dst, a.wpk + (size_t)j * kWeightBytes, kWeightBytes, bar_full + 8 * s);
+        } else {
 #pragma unroll
-            for (uint32_t c = 0; c < kRep; ++c)
-              bulk_g2s(dst + c * (COUT * kChunk), a.wpk + (size_t)j * (COUT * kChunk), COUT * kChunk,
-                       bar_full + 8 * s);
-          }
-          if (++s == nst) s = 0;
-          if (++ws == nwst) ws = 0;
+          for (uint32_t c = 0; c < kRep; ++c)
+            bulk_g2s(dst + c * (COUT * kChunk), a.wpk + (size_t)j * (COUT * kChunk), COUT * kChunk,
+                     bar_full + 8 * s);
         }
+        if (++s == nst) s = 0;
+        if (++ws == nwst) ws = 0;
+        if (++j == nchunk) {
+          j = 0;
+          tile += gridDim.x;
+        }
+      };
+#pragma unroll 1
+      for (uint32_t n = 0; n < nwst && tile < ntiles; ++n) fetch();
+      // No stage is freed before the rows are gathered, and the limit of a wait is for this launch,
+      // not for what is left of the one before.
+      pdl_wait();
+      while (!resident && tile < ntiles) {
+        // spinning: one lane, and every chunk waits for it (a launch of 4 736 rows 0.2 us less)
+        if (!mbar_wait_spin(bar_empty + 8 * os, oph, abort_flag, a.status, 6u)) break;
+        if (++os == nst) {
+          os = 0;
+          oph ^= 1u;
+        }
+        fetch();
+      }
     }
     __syncwarp();
   } else if (is_producer) {
@@ -425,6 +430,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
       alive = alive && (mbar_test_wait(bar, ph) || mbar_wait_spin(bar, ph, abort_flag, a.status, 3u));
       __syncwarp();  // (a wait that runs out may part them)
     };
+    pdl_wait();  // no stage fills before; the limit of a wait is for this launch, as above
     // The loop is entered with the current chunk's stage known to be full.
     if (blockIdx.x < ntiles) stage_full();
     for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++tl) {

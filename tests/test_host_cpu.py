@@ -95,6 +95,19 @@ def test_residual_rows_are_not_read_as_constants():
     assert loads and not [ld for ld in loads if ".nc" in ld]
 
 
+def test_limits_of_waits_do_not_count_the_launch_before():
+    """Every role of the convolution waits for the launch before it ahead of its first bounded wait, else
+    a launch before that runs into its own limit takes this one with it."""
+    src = _source("conv_umma_kernel.cu")
+    body = src[src.index("conv_umma_kernel(const UmmaArgs a)"):src.index("-- teardown")]
+    roles = re.split(r"// -{20,} (weights|producers|MMA issue|epilogue)\n", body)
+    for name, text in zip(roles[1::2], roles[2::2]):
+        first = {"producers": "step(idx_a)", "MMA issue": "    if (blockIdx.x < ntiles) stage_full();"}.get(
+            name, "mbar_wait")
+        assert 0 < text.find("pdl_wait") < text.index(first), name
+    assert len(roles) == 9
+
+
 def test_triples_are_made_anew_from_any_numbers():
     """Whatever int() takes is a triple's number, hashable or not; every call's array is its own."""
     cabi, _ = _lib()
