@@ -82,7 +82,7 @@ constexpr uint32_t kTmemCols = 2 * kTileRows;
 // less a rulebook block fits and the two do overlap, but the convolutions then take 3 % longer,
 // which is what the overlap saves (batch of 8 frames 4.25 ms against 4.34).
 constexpr uint32_t kRingBytes = 5 * kTileRows * kChunk + 4 * 128 * kChunk;
-constexpr size_t kSmemBytes = kRingBytes + 1024 + 256;  // alignment slack, barriers
+constexpr size_t kSmemBytes = kRingBytes + 1024 + 768;  // alignment slack, barriers
 
 // ceil(2^32 / n): with it x / n = umulhi(x, .) for x < 2^29
 __constant__ const uint32_t kReciprocal[9] = {0u,          0u,          0x80000000u,
@@ -136,13 +136,17 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
   const uint32_t raw_addr = smem_u32(smem_raw);
   uint8_t* smem = smem_raw + ((1024u - (raw_addr & 1023u)) & 1023u);
   uint64_t* bars = (uint64_t*)(smem + kRingBytes);
-  uint32_t* tmem_holder = (uint32_t*)(bars + 2 * kMaxStages + 4);
+  uint32_t* tmem_holder = (uint32_t*)(bars + (kTileRows / 32 + 1) * kMaxStages + 4);
   volatile uint32_t* abort_flag = tmem_holder + 1;
 
-  const uint32_t bar_full = smem_u32(bars);
-  const uint32_t bar_empty = bar_full + 8 * kMaxStages;
+  // "Stage empty", "accumulator full" and "empty", then "stage full" once for every tile height: how
+  // many threads sign it depends on the height, and so on the row count.  All are made before that is
+  // known.  (Made behind it, with their fences, they stood in the way of the first gather; one launch
+  // after the other, waiting first, us: fp16 8 -> 16 of 28 000 rows 6.8 / 6.5, int8 16 -> 16 6.8 / 6.5.)
+  const uint32_t bar_empty = smem_u32(bars);
   const uint32_t bar_tfull = bar_empty + 8 * kMaxStages;
   const uint32_t bar_tempty = bar_tfull + 16;
+  const uint32_t bar_full0 = bar_tempty + 16;
 
   const int warp = threadIdx.x >> 5;
   const uint32_t lane = threadIdx.x & 31;
@@ -150,21 +154,18 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
   // where that one has nothing to do with them; its results are waited for before the first gather
   // and the first drain.  (One launch after the other, all waiting here / waiting there, us: int8
   // 16 -> 16 of 14 000 rows 5.8 / 5.35, of 120 000 15.3 / 14.0; 128 -> 128 11.8 / 11.5, 41.5 / 40.7.)
-  if (!a.rules_ready) {
-    pdl_wait();
-    pdl_trigger();
-  }
-  const uint32_t n_out = min(load_in_order(a.n_out_ptr), a.cap);
+  uint32_t n_out = 0;
+  if (a.rules_ready) n_out = load_in_order(a.n_out_ptr);
 
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < kMaxStages; ++s) {
-      mbar_init(bar_empty + 8 * s, 1);
+  if (threadIdx.x < kTileRows / 32 * kMaxStages) {
+    // a group of producers, as many warps as the tile has 32 rows, and the weights
+    mbar_init(bar_full0 + 8 * threadIdx.x, 32u * (threadIdx.x / kMaxStages + 1u) + 1u);
+    if (threadIdx.x < kMaxStages) mbar_init(bar_empty + 8 * threadIdx.x, 1);
+    if (threadIdx.x < 2) {
+      mbar_init(bar_tfull + 8 * threadIdx.x, 1);
+      mbar_init(bar_tempty + 8 * threadIdx.x, kEpiWarps);
     }
-    for (int b = 0; b < 2; ++b) {
-      mbar_init(bar_tfull + 8 * b, 1);
-      mbar_init(bar_tempty + 8 * b, kEpiWarps);
-    }
-    *abort_flag = 0u;
+    if (threadIdx.x == 0) *abort_flag = 0u;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     fence_proxy_async();
   }
@@ -175,6 +176,17 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
+
+  if (!a.rules_ready) {
+    pdl_wait();
+    pdl_trigger();
+    n_out = load_in_order(a.n_out_ptr);
+  }
+  n_out = min(n_out, a.cap);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_holder;
 
   // Tile height: the rows are dealt out in rounds over the CTAs, so a fixed 256-row tile
   // can leave most CTAs idle in the last round (227 tiles on 148 CTAs run as long as 296).
@@ -204,16 +216,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
   // Only the producers that own rows of the tile take part, two groups of t32 warps.  (Warps that
   // only kept the barriers going cost low tiles a third of a chunk's time: fp16 128 -> 128 of 4 700
   // rows, 32 a tile, 18.2 to 15.0 us, int8 10.8 to 9.1.)
-  if (warp == 0) {
-    if (lane < (uint32_t)kMaxStages)
-      mbar_init(bar_full + 8 * lane, 32u * t32 + 1u);  // a group's threads + the weights
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    fence_proxy_async();
-  }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem_base = *tmem_holder;
+  const uint32_t bar_full = bar_full0 + 8 * kMaxStages * (t32 - 1u);
 
   const bool is_producer = warp > kMmaWarp && warp != kWeightWarp;
   // Who drains accumulators: the epilogue warps every tile of the CTA; the producers, which have
@@ -221,7 +224,9 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
   // on a small frame the only tile (128 channels, 224 rows: 6 200 cycles with 8 warps, with a
   // residual 15 000, beside 17 000 of MMAs).  A producer that is done knows that the MMAs are in
   // the last tile, or about to be, only if a tile has at least as many chunks as the ring.
-  const bool shared_tail = (uint32_t)nchunk >= nst;
+  // With 16 channels a tile has 32 columns, a group of 16 for each of the epilogue's two sets of warps:
+  // nothing to help with (fp16 16 -> 16 of 28 000 rows 7.6 us with the producers there, 7.2 without).
+  const bool shared_tail = COUT > 16 && (uint32_t)nchunk >= nst;
   uint32_t drain_tile = blockIdx.x, drain_tl = 0;
   const uint32_t help_sets = t32 >> 1;  // sets of four warps, one a lane quadrant, among the producers
   bool drains = warp < kEpiWarps;
@@ -409,7 +414,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
     const uint32_t w_step = kWeightBytes >> 4, r_step = row_stage >> 4;
     const uint32_t w_lo0 = (uint32_t)wdesc0, r_lo0 = (uint32_t)rdesc0;
     const uint32_t w_end = w_lo0 + nwst * w_step, bar_end = bar_full + 8 * nst;
-    constexpr uint32_t kToEmpty = 8 * kMaxStages;  // from a stage's full barrier to its empty one
+    const uint32_t to_empty = bar_empty - bar_full;  // from a stage's full barrier to its empty one
     uint32_t bar = bar_full, rd = r_lo0, wd = w_lo0, ph = 0, tl = 0;
     auto next_stage = [&]() {
       bar += 8;
@@ -450,7 +455,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
         umma_if<INT8>(issue, d_tmem, wd + 2u, rd + 2u, desc_hi, idesc, 1u);
         umma_if<INT8>(issue, d_tmem, wd + 4u, rd + 4u, desc_hi, idesc, 1u);
         umma_if<INT8>(issue, d_tmem, wd + 6u, rd + 6u, desc_hi, idesc, 1u);
-        tc_commit_if(issue, bar + kToEmpty);
+        tc_commit_if(issue, bar + to_empty);
         accumulate = 1u;
         next_stage();
         stage_full();
@@ -461,7 +466,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
         umma_if<INT8>(issue, d_tmem, wd + 2u * ks, rd + 2u * ks, desc_hi, idesc, accumulate);
         accumulate = 1u;
       }
-      tc_commit_if(issue, bar + kToEmpty);
+      tc_commit_if(issue, bar + to_empty);
       tc_commit_if(issue, bar_tfull + 8 * buf);
       next_stage();
       if (tile + gridDim.x < ntiles) stage_full();

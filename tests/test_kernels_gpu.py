@@ -526,6 +526,25 @@ def test_conv_int8_tile_heights_and_shared_tail(n, cin, cout, kvol):
     assert torch.equal(out[0], out[1])
 
 
+@pytest.mark.parametrize("n", [148 * 32 * h - 5 for h in range(1, 9)] + [148 * 64 * h - 5 for h in range(5, 8)])
+@pytest.mark.parametrize("cin,cout", [(16, 16), (64, 32)])
+def test_conv_int8_every_tile_height(n, cin, cout):
+    """Every height a tile can have, as a CTA's only tile and (from 160 rows on) with a second one: each
+    height has barriers of its own.  One layer keeps its weights in shared memory, the other streams them."""
+    ops = _ops()
+    rng = np.random.default_rng(n + cin)
+    m = torch.randint(-n, n, (27, n), dtype=torch.int32, device="cuda").clamp_(min=-1)
+    x = _dev(rng.integers(-128, 128, (n, cin)).astype(np.int8))
+    wts = ops.ConvWeights(rng.integers(-127, 128, (cout, 27, cin)).astype(np.int8), ops.I8,
+                          np.full(cout, 2e-4, np.float32), rng.standard_normal(cout))
+    n_ptr, st = ops.device_count(n), ops.new_status()
+    out = [ops.conv_forward(x, m, n_ptr, wts, out_kind=ops.I8, inv_out_scale=9.0, force_simt=simt,
+                            status=st) for simt in (False, True)]
+    torch.cuda.synchronize()
+    _status_ok(st)
+    assert torch.equal(out[0], out[1])
+
+
 @pytest.mark.parametrize("n", [1, 33, 148 * 32, 148 * 96 + 1, 148 * 224 - 5, 148 * 256 + 1])
 @pytest.mark.parametrize("cin,cout,kvol", [(8, 16, 27), (16, 16, 27), (64, 64, 27), (128, 128, 27),
                                            (128, 32, 3), (32, 128, 1)])
