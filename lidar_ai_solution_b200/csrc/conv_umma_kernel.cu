@@ -178,8 +178,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
   }
 
   if (!a.rules_ready) {
-    pdl_wait();
-    pdl_trigger();
+    pdl_wait_and_trigger();
     n_out = load_in_order(a.n_out_ptr);
   }
   n_out = min(n_out, a.cap);
@@ -381,8 +380,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
     advance2(ntile, nj);
     load_idx(ntile, nj, idx_b);
     advance2(ntile, nj);
-    pdl_wait();
-    pdl_trigger();
+    pdl_wait_and_trigger();
     while (step(idx_a) && step(idx_b)) {
     }
     cp_async_wait_all();  // nothing of this thread may still be writing when the CTA exits

@@ -1,13 +1,14 @@
 // Programmatic dependent launch.  A kernel launched with launch_pdl() may be scheduled while the
 // kernel before it in the stream is still running; it must call pdl_wait() before it touches
 // what that kernel may still be working on (the wait ends when every kernel before it has finished
-// and its writes are visible).  pdl_trigger() lets the kernel after it start its own prologue.
+// and its writes are visible).  A trigger lets the kernel after it start its own prologue.
 // Launch latency and prologue (2-4 us of a kernel's ~10 on small frames) then overlap with the tail
 // of the kernel before.
 //
-// Every kernel here triggers behind its own wait, never before it.  So when a kernel starts, all
-// but the one launch directly before it are complete, and what those wrote may be read before
-// pdl_wait().
+// A kernel that triggers does it behind its own wait, in one call (pdl_wait_and_trigger()), and a
+// kernel launched this way leaves no CTA before its wait; the others' dependents start when they are
+// over.  So when a kernel starts, all but the one launch directly before it are complete, and what those
+// wrote may be read before pdl_wait(): the convolutions do.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -15,8 +16,10 @@
 namespace spconvb {
 
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_trigger() {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+// The kernel after this one may start once every CTA has been here.  (Nothing triggers without a wait:
+// that kernel would start beside two others, and read what the first is still writing.)
+__device__ __forceinline__ void pdl_wait_and_trigger() {
+  asm volatile("griddepcontrol.wait;\n\tgriddepcontrol.launch_dependents;" ::: "memory");
 }
 
 // What an earlier kernel wrote, read where the source reads it: volatile, and through the coherent path.

@@ -95,6 +95,28 @@ def test_residual_rows_are_not_read_as_constants():
     assert loads and not [ld for ld in loads if ".nc" in ld]
 
 
+def test_no_kernel_triggers_its_dependents_before_its_own_wait():
+    """The convolutions read row counts, indices and weights before they wait, because all but the one
+    launch directly before are complete when a kernel starts.  That holds as long as nothing triggers
+    without a wait ahead of it, and no CTA of a kernel launched to overlap leaves before its wait."""
+    csrc = os.path.join(ROOT, "lidar_ai_solution_b200", "csrc")
+    code = {f: re.sub(r"//[^\n]*", "", _source(f)) for f in sorted(os.listdir(csrc)) if f.endswith((".cu", ".cuh"))}
+    triggers = [(f, m.start()) for f, src in code.items() for m in
+                re.finditer(r"launch_dependents|cudaTriggerProgrammaticLaunchCompletion", src)]
+    assert [f for f, _ in triggers] == ["pdl.cuh"]
+    assert re.search(r'asm volatile\("griddepcontrol\.wait;[^"]*griddepcontrol\.launch_dependents;"', code["pdl.cuh"])
+    overlapping = {k for f, src in code.items() if f != "pdl.cuh" for k in re.findall(r"launch_pdl\((\w+)", src)}
+    assert "kernel" in overlapping  # a variable: an instance of the dense output's kernel
+    overlapping = overlapping - {"kernel"} | {"scatter_dense_kernel"}
+    assert {"conv_umma_kernel", "rule_wave_kernel"} <= overlapping
+    for k in sorted(overlapping):
+        src, = [src for src in code.values() if re.search(r"__global__[^;{}]*\b%s\(" % k, src)]
+        at = re.search(r"__global__[^;{}]*\b%s\(" % k, src).start()
+        body = src[src.index("{\n", at):src.index("\n}", at)]
+        wait = body.find("pdl_wait")
+        assert wait >= 0 and "return" not in body[:wait], k
+
+
 def test_limits_of_waits_do_not_count_the_launch_before():
     """Every role of the convolution waits for the launch before it ahead of its first bounded wait, else
     a launch before that runs into its own limit takes this one with it."""
