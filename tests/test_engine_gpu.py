@@ -336,34 +336,51 @@ def test_auxiliary_stream_changes_no_result():
         assert np.array_equal(fast.output(0).cpu().numpy().view(np.uint16), want.view(np.uint16))
 
 
-@pytest.mark.parametrize("flags", [0, "BUILD_SINGLE_STREAM"])
-@pytest.mark.parametrize("kind", ["centerpoint", "bevfusion"])
+@pytest.mark.parametrize("flags", ["", "BUILD_SINGLE_STREAM", "BUILD_NO_FUSION"])
+@pytest.mark.parametrize("kind", ["centerpoint", "bevfusion", "encoder_decoder"])
 def test_frames_queued_back_to_back(kind, flags):
-    """A convolution fetches its row count, first neighbour indices and weights while the launch before
-    it is running.  Frames of other sizes (one row, a lone tile, several) queued without a wait on one
-    engine give the bits that the same frames give one at a time."""
+    """In a forward a convolution fetches its row count, first neighbour indices and weights while the
+    launch before it is running, and where the host knows the row count the caller's table is as large as
+    that needs.  The profiling pass does neither: every launch starts when the one before is over, and the
+    table is the whole one.  Frames of other sizes (one row, a lone tile, several), their counts on the
+    host and on the device in turn, queued without a wait on one engine, give that pass's bits."""
     eng = _engine_mod()
     flags = getattr(eng, flags) if flags else 0
-    frames = [[_dev(a) for a in _frame(n, seed=s)] for n, s in ((12000, 1), (1, 2), (33, 3), (20000, 4), (257, 5))]
-    model = _quantized(kind, *_frame(9000, seed=9)) if kind == "centerpoint" else _small_model(kind, 0)
+    sizes = ((12000, 1), (1, 2), (33, 3), (20000, 4), (257, 5))
+    if kind == "encoder_decoder":  # an inverse rulebook, an add, two sparse outputs
+        grid = (21, 200, 200)
+        model = models.encoder_decoder(32, seed=5, in_channels=16, output_bound=60000)
+        frames = [(np.random.default_rng(s).standard_normal((n, 16)).astype(np.float16),
+                   scenes.make_coords(n, grid, s)) for n, s in sizes]
+    else:
+        grid = GRID
+        frames = [_frame(n, seed=s) for n, s in sizes]
+        model = _quantized(kind, *_frame(9000, seed=9)) if kind == "centerpoint" else _small_model(kind, 0)
     precision = eng.PRECISION_INT8 if kind == "centerpoint" else eng.PRECISION_FP16
-    alone = eng.Engine.from_model(model, precision, flags)
-    want = []
+    frames = [(_dev(f), _dev(c)) for f, c in frames]
+    one = eng.Engine.from_model(model, precision, flags)
+    want, rows = [], []
     for feats, coords in frames:
-        alone.forward(feats, coords, GRID)
+        one.profile(feats, coords, grid, reps=1)
         torch.cuda.synchronize()
-        assert alone.status()[0] == 0
-        want.append(alone.output(0).clone())
+        assert one.status()[0] == 0
+        rows.append([one.tensor(t)["n"] if kind == "encoder_decoder" else None for t, _ in model["outputs"]])
+        want.append([one.output(k)[:r].clone() for k, r in enumerate(rows[-1])])
     queued = eng.Engine.from_model(model, precision, flags)
+    counts = [torch.tensor([len(f)], dtype=torch.int32, device="cuda") for f, _ in frames]
     got = []
-    for _ in range(3):
-        for feats, coords in frames:
-            queued.forward(feats, coords, GRID)
-            got.append(queued.output(0).clone())
+    for turn in range(4):
+        for i, (feats, coords) in enumerate(frames):
+            if (turn + i) % 2:
+                queued.forward_dds(feats, coords, counts[i], grid)
+            else:
+                queued.forward(feats, coords, grid)
+            got.append([queued.output(k)[:r].clone() for k, r in enumerate(rows[i])])
     torch.cuda.synchronize()
     assert queued.status()[0] == 0
-    for i, g in enumerate(got):
-        assert torch.equal(g.view(torch.int16), want[i % len(frames)].view(torch.int16)), i
+    for i, outs in enumerate(got):
+        for k, (g, w) in enumerate(zip(outs, want[i % len(frames)])):
+            assert torch.equal(g.view(torch.int16), w.view(torch.int16)), (i, k)
 
 
 @pytest.mark.parametrize("precision", ["int8", "fp16"])
