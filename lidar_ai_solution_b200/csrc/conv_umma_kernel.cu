@@ -39,11 +39,11 @@
 //   warp  25    streams the pre-swizzled weight chunks with bulk async copies into a
 //               ring of their own, or keeps all of them there
 //
-// What bounds it.  The round trip of a stage - freed, gathered (a cp.async takes about a
-// microsecond under load), multiplied, freed - over the number of stages in flight, not a
-// pipe: in isolation the MMAs of a 256-row chunk take 513 cycles, its gather 460 (cp.async.cg;
-// 640 with .ca, which keeps a copy in L1 that nothing reads again) and its weights 310, and
-// they overlap freely, but with four stages of rows and weights together a chunk took 1000.
+// What bounds it.  On tall tiles the round trip of a stage - freed, gathered (a cp.async takes
+// about a microsecond under load), multiplied, freed - over the number of stages in flight, and
+// then shared memory: in isolation the MMAs of a 256-row chunk take 513 cycles, its gather 460
+// (cp.async.cg; 640 with .ca, which keeps a copy in L1 that nothing reads again) and its weights
+// 310, and they overlap, but with four stages of rows and weights together a chunk took 1000.
 // Hence two rings that are sized to the tile's height in the kernel (256 rows: 5 stages of
 // rows and 4 of weights; 160 rows: 6 and 6), and no work beside the MMAs in the issuing warp.
 // Measured with both, int8, us: 208 071 rows 64 -> 64 49.2 to 41.3, 128 -> 128 86.9 to 69.3
@@ -51,7 +51,8 @@
 //
 // On low tiles the issuing warp is what a chunk waits for: 32-row tiles, 128 channels, 412 cycles a
 // chunk in it, of which 74 are its look at the stage's barrier; 628 and 121 on 224 rows, where the
-// MMAs fill the rest (clock counts of one CTA).
+// MMAs fill the rest (clock counts of one CTA).  Close behind lies what a chunk brings into every SM,
+// 16 KB of weights and 4 KB of rows: 50 bytes a cycle, the same weights 148 times over from L2.
 //
 // K is walked in chunks of 128 bytes (one swizzle atom per row): a chunk is 8
 // taps of a 16-byte row, ..., 1 tap of a 128-byte row, or half a 256-byte row.
@@ -400,7 +401,7 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
     // cycles per chunk against 583 when a single lane runs the loop, whose descriptors are moved
     // to uniform registers one MMA after the other).
     //
-    // MMAs are queued: what a chunk costs here is the issue of its instructions, and with 24 other
+    // MMAs are queued: what a chunk costs here is the issue of its instructions, and with up to 24 other
     // warps around every one takes tens of cycles.  So the loop carries addresses and nothing
     // else, and a chunk is four MMAs, a commit and one test of the next stage's barrier.
     const bool leader = elect_one();
@@ -481,7 +482,8 @@ __global__ void __launch_bounds__(kCtaThreads, 1) conv_umma_kernel(const UmmaArg
     pdl_wait();  // residual rows are read, and rows written that the kernel before may still read
     // Accumulator row m (TMEM lane m) holds channel m % COUT of weight copy m / COUT.  Copy c
     // owns cols_rep rows of the tile from c * cols_rep on, and the warps of a lane quadrant take
-    // its groups of 16 rows in turn: two warps, in the CTA's last tile six.
+    // its groups of 16 rows in turn: two warps, and where the producers help with the last tile one more
+    // for every 64 rows of its height (2 to 6).
     const uint32_t q = (uint32_t)warp & 3u;        // TMEM lane quadrant of this warp
     const uint32_t part = is_producer ? 2u + (((uint32_t)warp - kProdWarp0) >> 2) : (uint32_t)warp >> 2;
     const uint32_t acc_row = 32u * q + lane, acc_row0 = 32u * q;
